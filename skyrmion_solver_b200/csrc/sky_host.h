@@ -20,6 +20,15 @@ int ew_blocks(int64_t n);
 int choose_xc(int X, int tiles_yz, int resident);
 int option(int key);
 
+// The buffers of a drop-in step (C N values each).
+struct StepBuffers {
+    double *V, *F, *eg;
+    double *k[4], *l[4];
+    double* temp;
+};
+int arrested_step(int theory, const Params& p, const StepBuffers& b, double* s_e, double* s_m, double prev_energy,
+                  double* new_energy, double* err, cudaStream_t st);
+int choose_chunk(int X, int tiles_yz, int resident);
 int gradient_fp64(int theory, const Params& p, const double* f, double* eg, double* l, cudaStream_t st);
 int density_fp64(int theory, const Params& p, int mode, const double* f, double* dens, double* scratch,
                  double* out_dev, cudaStream_t st);

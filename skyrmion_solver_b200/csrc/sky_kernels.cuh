@@ -37,6 +37,42 @@ struct DensTile {  // first derivatives only, FP64 arithmetic
     using type = TileShape<C, 32, (C > 5 ? 4 : 8), (C > 5 ? 1 : 2)>;
 };
 
+// RK4 arithmetic of the drop-in path, with every rounding spelled out: the separate kernels
+// and the fused stages give the same bits whatever the compiler contracts around them.
+// do_rk4_step_kernel (core/integrator.py:50-92): k = dt (v + f l), X = F + f k.
+__device__ __forceinline__ double rk4_slope(double dt, double v, double f, double l) {
+    return __dmul_rn(dt, __fma_rn(f, l, v));
+}
+__device__ __forceinline__ double rk4_field(double F, double f, double k) { return __fma_rn(f, k, F); }
+// _do_rk4_kernel (core/integrator.py:163-175): v + (a + 2 b + 2 c + d) / 6
+__device__ __forceinline__ double rk4_sum(double v, double a, double b, double c, double d) {
+    return __fma_rn(1.0 / 6.0, __dadd_rn(__fma_rn(2.0, c, __fma_rn(2.0, b, a)), d), v);
+}
+// The normalisation of the first nsky components and the projection of the velocity
+// orthogonal to them that end an RK4 step (compute_norm_skyrme_field /
+// project_orthogonal_skyrme_field, th/nuclear_skyrme/kernels.py:196-272).
+template <int C>
+__device__ __forceinline__ void rk4_constrain(double (&fv)[C], double (&vv)[C], int nsky, int constrain) {
+    if (!constrain) return;
+    double ss = 0.0;
+#pragma unroll
+    for (int a = 0; a < C; ++a)
+        if (a < nsky) ss = __fma_rn(fv[a], fv[a], ss);
+    ss = sqrt(ss);
+    if (ss != 0.0) {
+#pragma unroll
+        for (int a = 0; a < C; ++a)
+            if (a < nsky) fv[a] = __ddiv_rn(fv[a], ss);
+    }
+    double lm = 0.0;
+#pragma unroll
+    for (int a = 0; a < C; ++a)
+        if (a < nsky) lm = __fma_rn(vv[a], fv[a], lm);
+#pragma unroll
+    for (int a = 0; a < C; ++a)
+        if (a < nsky) vv[a] = __fma_rn(-lm, fv[a], vv[a]);
+}
+
 struct TileGrid {
     int nz, ny, nx;
     __host__ __device__ int count() const { return nz * ny * nx; }

@@ -36,17 +36,18 @@ namespace sky {
 // in z; a chunk crossing z = Z copies its in-lattice part and zero-fills the rest.
 constexpr size_t kMaxSmemPerBlock = 232448;  // 227 KB of dynamic shared memory per block
 
-template <int C_, int BY_, bool WIDE_ = false>
+// ZP: columns staged on each side of a wide row's 32 (4, or 2 for 8-byte values, whose
+// 16-byte chunks start at z0 - 2).
+template <int C_, int BY_, bool WIDE_ = false, int ZP = 4>
 struct MarchShape {
     static constexpr int C = C_, BY = BY_, BZ = 32;
     static constexpr bool WIDE = WIDE_;
-    static constexpr int HY = BY + 4, HZ = WIDE ? BZ + 8 : BZ + 4;
-    static constexpr int ZOFF = WIDE ? 4 : 2;
+    static constexpr int ZOFF = WIDE ? ZP : 2;
+    static constexpr int HY = BY + 4, HZ = BZ + 2 * ZOFF;
     static constexpr int PLANE = HY * HZ;  // one component of one plane, with halo
     static constexpr int SLOT = C * PLANE;  // all components of one plane
     static constexpr int RING = 5;
     static constexpr int NTHREADS = BZ * BY;
-    static constexpr int NPER = (SLOT + NTHREADS - 1) / NTHREADS;  // plane elements per thread
     // Sources staged through shared memory: all nsrc, or only the first two when
     // three would not fit in one block's 227 KB (FP64 rho); the third source is
     // then read from global memory while the plane is combined.
@@ -138,14 +139,14 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // global offset within the x-plane is c*N + gy*Z + gz (int32), or -1 when the
 // point lies outside the lattice in y or z (or idx is past the slot).  The
 // host guarantees C*N < 2^31 for marching launches.
-template <class M>
+template <class M, int NT = M::NTHREADS>
 struct PlaneOffsets {
-    int off[M::NPER];
-    __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0) {
-        const int tid = threadIdx.x + M::BZ * threadIdx.y;
+    static constexpr int NPER = (M::SLOT + NT - 1) / NT;
+    int off[NPER];
+    __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0, int tid) {
 #pragma unroll
-        for (int k = 0; k < M::NPER; ++k) {
-            const int idx = tid + k * M::NTHREADS;
+        for (int k = 0; k < NPER; ++k) {
+            const int idx = tid + k * NT;
             const int row = idx / M::HZ;
             const int zz = idx - row * M::HZ;
             const int c = row / M::HY;
@@ -160,20 +161,19 @@ struct PlaneOffsets {
 // Wide rows: per-thread 16-byte chunks of the haloed plane.  Chunk k of thread tid
 // is ci = tid + k*NTHREADS; its global element offset within the x-plane and the
 // number of its bytes inside the lattice (0 when outside or past the slot).
-template <class M, typename T>
+template <class M, typename T, int NT = M::NTHREADS>
 struct PlaneChunks {
     static constexpr int VW = 16 / int(sizeof(T));
     static constexpr int CPR = M::HZ / VW;
     static constexpr int NCHS = M::C * M::HY * CPR;
-    static constexpr int NCH = (NCHS + M::NTHREADS - 1) / M::NTHREADS;
+    static constexpr int NCH = (NCHS + NT - 1) / NT;
     int off[NCH];
     int nb[NCH];
-    __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0) {
+    __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0, int tid) {
         static_assert(M::WIDE && M::HZ % VW == 0, "16-byte chunks need the wide row layout");
-        const int tid = threadIdx.x + M::BZ * threadIdx.y;
 #pragma unroll
         for (int k = 0; k < NCH; ++k) {
-            const int ci = tid + k * M::NTHREADS;
+            const int ci = tid + k * NT;
             const int row = ci / CPR;
             const int cz = ci - row * CPR;
             const int c = row / M::HY;
@@ -186,37 +186,37 @@ struct PlaneChunks {
     }
 };
 
-// Source s of a plane lands at stage + s * DST (DST = M::SLOT: consecutive staging
+// `any`: a readable address for copies that only zero-fill.  Source s of a plane lands at stage + s * DST (DST = M::SLOT: consecutive staging
 // slots; a ring of R slots per source when the plane goes straight into the ring).
-template <class M, int NSRC, typename T, int DST = M::SLOT>
-__device__ __forceinline__ void plane_issue_wide(T* __restrict__ stage, const PlaneChunks<M, T>& pc,
-                                                 const T* const (&src)[3], int64_t plane_base, bool xok) {
-    using PC = PlaneChunks<M, T>;
-    const int tid = threadIdx.x + M::BZ * threadIdx.y;
+template <class M, int NSRC, typename T, int DST = M::SLOT, int NT = M::NTHREADS>
+__device__ __forceinline__ void plane_issue_wide(T* __restrict__ stage, const PlaneChunks<M, T, NT>& pc,
+                                                 const T* const (&src)[3], int64_t plane_base, bool xok, int tid,
+                                                 const T* any) {
+    using PC = PlaneChunks<M, T, NT>;
 #pragma unroll
     for (int k = 0; k < PC::NCH; ++k) {
-        const int ci = tid + k * M::NTHREADS;
-        if (PC::NCHS % M::NTHREADS == 0 || ci < PC::NCHS) {
+        const int ci = tid + k * NT;
+        if (PC::NCHS % NT == 0 || ci < PC::NCHS) {
 #pragma unroll
             for (int s = 0; s < NSRC; ++s) {
                 const T* g = src[s];
                 const int n = (xok && g != nullptr) ? pc.nb[k] : 0;
                 cp_async16(stage + s * DST + ci * PC::VW, n ? (const void*)(g + plane_base + pc.off[k])
-                                                                : (const void*)src[0], n);
+                                                                : (const void*)any, n);
             }
         }
     }
     cp_async_commit();
 }
 
-template <class M, int NSRC, typename T, typename S = T>
-__device__ __forceinline__ void plane_combine_wide(T* __restrict__ slot, const S* __restrict__ stage, T a, T b) {
-    using PC = PlaneChunks<M, S>;
-    const int tid = threadIdx.x + M::BZ * threadIdx.y;
+template <class M, int NSRC, typename T, typename S = T, int NT = M::NTHREADS>
+__device__ __forceinline__ void plane_combine_wide(T* __restrict__ slot, const S* __restrict__ stage, T a, T b,
+                                                   int tid) {
+    using PC = PlaneChunks<M, S, NT>;
 #pragma unroll
     for (int k = 0; k < PC::NCH; ++k) {
-        const int ci = tid + k * M::NTHREADS;
-        if (PC::NCHS % M::NTHREADS == 0 || ci < PC::NCHS) {
+        const int ci = tid + k * NT;
+        if (PC::NCHS % NT == 0 || ci < PC::NCHS) {
             T v[PC::VW];
 #pragma unroll
             for (int e = 0; e < PC::VW; ++e) v[e] = T(stage[ci * PC::VW + e]);
@@ -236,22 +236,22 @@ __device__ __forceinline__ void plane_combine_wide(T* __restrict__ slot, const S
 
 // Issue the cp.async copies of one x-plane (element offset plane_base) of the
 // NSRC source arrays into the staging slots; a null source reads as zero.
-template <class M, int NSRC, typename T, int DST = M::SLOT>
-__device__ __forceinline__ void plane_issue(T* __restrict__ stage, const PlaneOffsets<M>& po, const T* const (&src)[3],
-                                            int64_t plane_base, bool xok) {
+template <class M, int NSRC, typename T, int DST = M::SLOT, int NT = M::NTHREADS>
+__device__ __forceinline__ void plane_issue(T* __restrict__ stage, const PlaneOffsets<M, NT>& po,
+                                            const T* const (&src)[3], int64_t plane_base, bool xok, int tid,
+                                            const T* any) {
     // T here is the source (staging) type
-    const int tid = threadIdx.x + M::BZ * threadIdx.y;
 #pragma unroll
-    for (int k = 0; k < M::NPER; ++k) {
-        const int idx = tid + k * M::NTHREADS;
-        if (M::SLOT % M::NTHREADS == 0 || idx < M::SLOT) {
+    for (int k = 0; k < PlaneOffsets<M, NT>::NPER; ++k) {
+        const int idx = tid + k * NT;
+        if (M::SLOT % NT == 0 || idx < M::SLOT) {
             const bool ok = xok && po.off[k] >= 0;
 #pragma unroll
             for (int s = 0; s < NSRC; ++s) {
                 const T* g = src[s];
                 const bool v = ok && g != nullptr;
                 cp_async<sizeof(T)>(stage + s * DST + idx,
-                                    v ? (const void*)(g + plane_base + po.off[k]) : (const void*)src[0], v);
+                                    v ? (const void*)(g + plane_base + po.off[k]) : (const void*)any, v);
             }
         }
     }
@@ -260,13 +260,12 @@ __device__ __forceinline__ void plane_issue(T* __restrict__ stage, const PlaneOf
 
 // Combine the thread's own staged elements (source type S) into a ring slot of
 // type T: X = F + a V + b L.
-template <class M, int NSRC, typename T, typename S = T>
-__device__ __forceinline__ void plane_combine(T* __restrict__ slot, const S* __restrict__ stage, T a, T b) {
-    const int tid = threadIdx.x + M::BZ * threadIdx.y;
+template <class M, int NSRC, typename T, typename S = T, int NT = M::NTHREADS>
+__device__ __forceinline__ void plane_combine(T* __restrict__ slot, const S* __restrict__ stage, T a, T b, int tid) {
 #pragma unroll
-    for (int k = 0; k < M::NPER; ++k) {
-        const int idx = tid + k * M::NTHREADS;
-        if (M::SLOT % M::NTHREADS == 0 || idx < M::SLOT) {
+    for (int k = 0; k < PlaneOffsets<M, NT>::NPER; ++k) {
+        const int idx = tid + k * NT;
+        if (M::SLOT % NT == 0 || idx < M::SLOT) {
             T v = T(stage[idx]);
             if (NSRC > 1) v += a * T(stage[M::SLOT + idx]);
             if (NSRC > 2) v += b * T(stage[2 * M::SLOT + idx]);
@@ -288,19 +287,19 @@ __device__ __forceinline__ void plane_combine_g(T* __restrict__ slot, const S* _
     const int tid = threadIdx.x + M::BZ * threadIdx.y;
     const bool any = xok && src2 != nullptr;
 #pragma unroll
-    for (int k0 = 0; k0 < M::NPER; k0 += G) {
+    for (int k0 = 0; k0 < PlaneOffsets<M>::NPER; k0 += G) {
         T l[G];
 #pragma unroll
         for (int j = 0; j < G; ++j) {
             const int k = k0 + j;
             l[j] = T(0);
-            if (k < M::NPER && any && po.off[k] >= 0) l[j] = T(__ldg(src2 + plane_base + po.off[k]));
+            if (k < PlaneOffsets<M>::NPER && any && po.off[k] >= 0) l[j] = T(__ldg(src2 + plane_base + po.off[k]));
         }
 #pragma unroll
         for (int j = 0; j < G; ++j) {
             const int k = k0 + j;
             const int idx = tid + k * M::NTHREADS;
-            if (k < M::NPER && (M::SLOT % M::NTHREADS == 0 || idx < M::SLOT))
+            if (k < PlaneOffsets<M>::NPER && (M::SLOT % M::NTHREADS == 0 || idx < M::SLOT))
                 slot[idx] = T(stage[idx]) + a * T(stage[M::SLOT + idx]) + b * l[j];
         }
     }
@@ -312,7 +311,7 @@ __device__ __forceinline__ void plane_prefetch_l2(const PlaneOffsets<M>& po, con
                                                   bool xok) {
     if (!xok || src == nullptr) return;
 #pragma unroll
-    for (int k = 0; k < M::NPER; ++k)
+    for (int k = 0; k < PlaneOffsets<M>::NPER; ++k)
         if (po.off[k] >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + plane_base + po.off[k]));
 }
 
@@ -387,7 +386,7 @@ __device__ __forceinline__ bool march_tile(T* __restrict__ sm, const Params& p, 
     // element offsets (narrow rows) or 16-byte chunks (wide rows) of the haloed plane
     using PO = typename std::conditional<M::WIDE, PlaneChunks<M, S>, PlaneOffsets<M>>::type;
     PO po;
-    po.init(p, N, y0, z0);
+    po.init(p, N, y0, z0, tx + M::BZ * ty);
     constexpr int CQ = QUEUE ? C : 1;
     T uq[CQ][5], wq[CQ][5];  // uy / uz queues for planes x-2 .. x+2
 #pragma unroll
@@ -399,9 +398,9 @@ __device__ __forceinline__ bool march_tile(T* __restrict__ sm, const Params& p, 
     auto issue = [&](int64_t base, bool xok, int dslot) {
         S* dst = DIRECT ? reinterpret_cast<S*>(ring + dslot * M::SLOT) : stage;
         if constexpr (M::WIDE) {
-            plane_issue_wide<M, NST, S, DST>(dst, po, src, base, xok);
+            plane_issue_wide<M, NST, S, DST>(dst, po, src, base, xok, tx + M::BZ * ty, src[0]);
         } else {
-            plane_issue<M, NST, S, DST>(dst, po, src, base, xok);
+            plane_issue<M, NST, S, DST>(dst, po, src, base, xok, tx + M::BZ * ty, src[0]);
             if constexpr (NST < NSRC) plane_prefetch_l2<M, S>(po, src[2], base, xok);
         }
     };
@@ -507,9 +506,9 @@ __device__ __forceinline__ bool march_tile(T* __restrict__ sm, const Params& p, 
                     plane_combine_g<M, T, S>(ring + slot * M::SLOT, stage, a, b, po, src[2], (int64_t)q * YZ,
                                              q >= 0 && q < p.X);
             } else if constexpr (M::WIDE) {
-                plane_combine_wide<M, NSRC, T, S>(ring + slot * M::SLOT, stage, a, b);
+                plane_combine_wide<M, NSRC, T, S>(ring + slot * M::SLOT, stage, a, b, tx + M::BZ * ty);
             } else {
-                plane_combine<M, NSRC, T, S>(ring + slot * M::SLOT, stage, a, b);
+                plane_combine<M, NSRC, T, S>(ring + slot * M::SLOT, stage, a, b, tx + M::BZ * ty);
             }
             if (q < q1) issue((int64_t)(q + 1) * YZ, q + 1 >= 0 && q + 1 < p.X, 0);
             __syncthreads();  // (B) slot complete

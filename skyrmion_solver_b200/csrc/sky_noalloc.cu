@@ -115,38 +115,9 @@ extern "C" int sky_arrested_newton_step_noalloc(int theory, const int32_t* p_i, 
     double* base = nullptr;
     if ((rc = noalloc_scratch(&base))) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    double* ks[4] = {base, base + cn, base + 2 * cn, base + 3 * cn};
-    double* ls[4] = {base + 4 * cn, base + 5 * cn, base + 6 * cn, base + 7 * cn};
-    double* temp = base + 8 * cn;
+    const StepBuffers b{velocity, field, energy_gradient, {base, base + cn, base + 2 * cn, base + 3 * cn},
+                        {base + 4 * cn, base + 5 * cn, base + 6 * cn, base + 7 * cn}, base + 8 * cn};
     double* s_e = base + 9 * cn;
-    double* s_m = s_e + kScratchDoubles;
-    // core/integrator.py:382-398; every slope and the stage field are written before they are read
-    const double fac[4] = {0.0, 0.5, 0.5, 1.0};
-    for (int s = 0; s < 4; ++s) {
-        const double* lin = s == 0 ? velocity : ls[s - 1];
-        const double* kprev = s == 0 ? field : ks[s - 1];
-        if ((rc = rk4_stage(p, ks[s], velocity, lin, temp, field, kprev, fac[s], st))) return rc;
-        if ((rc = gradient_fp64(theory, p, temp, energy_gradient, ls[s], st))) return rc;
-    }
-    if ((rc = rk4_finalize(theory, p, velocity, field, ks[0], ks[1], ks[2], ks[3], ls[0], ls[1], ls[2], ls[3], st)))
-        return rc;
-    // energy (core/integrator.py:402) and err = signed max of the stage-4 gradient (:409); the
-    // reduction launchers clear their completion counters before each use
-    if ((rc = density_fp64(theory, p, 0, field, nullptr, s_e, nullptr, st))) return rc;
-    if ((rc = reduce(1, energy_gradient, cn, s_m, nullptr, st))) return rc;
-    double res[2];
-    if ((rc = check_cuda(cudaMemcpyAsync(&res[0], s_e + 2 * kMaxRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, st),
-                         "memcpy", __LINE__)))
-        return rc;
-    if ((rc = check_cuda(cudaMemcpyAsync(&res[1], s_m + 2 * kMaxRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, st),
-                         "memcpy", __LINE__)))
-        return rc;
-    if ((rc = check_cuda(cudaStreamSynchronize(st), "sync", __LINE__))) return rc;
-    *new_energy_host = res[0];
-    *err_host = res[1];
-    // arrest (core/integrator.py:403-407)
-    if (p.killkinen && res[0] > prev_energy) {
-        if ((rc = fill(velocity, cn, 0.0, st))) return rc;
-    }
-    return SKY_OK;
+    // every slope and the stage field are written before they are read
+    return arrested_step(theory, p, b, s_e, s_e + kScratchDoubles, prev_energy, new_energy_host, err_host, st);
 }

@@ -5,8 +5,8 @@
 #include <string.h>
 
 #include "sky_host.h"
+#include "sky_grad.cuh"
 #include "sky_kernels.cuh"
-#include "sky_march.cuh"
 
 namespace sky {
 
@@ -19,14 +19,12 @@ __global__ void k_rk4_stage(int64_t total, double dt, double factor, double* __r
                             const double* __restrict__ v, const double* __restrict__ lin, double* __restrict__ temp,
                             const double* __restrict__ f, const double* __restrict__ kprev) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        kout[i] = dt * (v[i] + factor * lin[i]);
-        temp[i] = f[i] + factor * kprev[i];
+        kout[i] = rk4_slope(dt, v[i], factor, lin[i]);
+        temp[i] = rk4_field(f[i], factor, kprev[i]);
     }
 }
 
-// _do_rk4_kernel (core/integrator.py:163-175) with compute_norm_skyrme_field /
-// project_orthogonal_skyrme_field (th/nuclear_skyrme/kernels.py:196-272) over
-// the first nsky components; constrain = 0 gives do_rk4_kernel_no_constraint.
+// _do_rk4_kernel (core/integrator.py:163-175); constrain = 0 gives do_rk4_kernel_no_constraint.
 template <int C>
 __global__ void k_rk4_finalize(int64_t N, int nsky, int constrain, double* __restrict__ v, double* __restrict__ f,
                                const double* __restrict__ k1, const double* __restrict__ k2,
@@ -38,28 +36,10 @@ __global__ void k_rk4_finalize(int64_t N, int nsky, int constrain, double* __res
 #pragma unroll
         for (int a = 0; a < C; ++a) {
             const int64_t i = a * N + s;
-            vv[a] = v[i] + (1.0 / 6.0) * (l1[i] + 2.0 * l2[i] + 2.0 * l3[i] + l4[i]);
-            fv[a] = f[i] + (1.0 / 6.0) * (k1[i] + 2.0 * k2[i] + 2.0 * k3[i] + k4[i]);
+            vv[a] = rk4_sum(v[i], l1[i], l2[i], l3[i], l4[i]);
+            fv[a] = rk4_sum(f[i], k1[i], k2[i], k3[i], k4[i]);
         }
-        if (constrain) {
-            double ss = 0.0;
-#pragma unroll
-            for (int a = 0; a < C; ++a)
-                if (a < nsky) ss += fv[a] * fv[a];
-            ss = sqrt(ss);
-            if (ss != 0.0) {
-#pragma unroll
-                for (int a = 0; a < C; ++a)
-                    if (a < nsky) fv[a] /= ss;
-            }
-            double lm = 0.0;
-#pragma unroll
-            for (int a = 0; a < C; ++a)
-                if (a < nsky) lm += vv[a] * fv[a];
-#pragma unroll
-            for (int a = 0; a < C; ++a)
-                if (a < nsky) vv[a] -= lm * fv[a];
-        }
+        rk4_constrain<C>(fv, vv, nsky, constrain);
 #pragma unroll
         for (int a = 0; a < C; ++a) {
             v[a * N + s] = vv[a];
@@ -75,8 +55,8 @@ __global__ void k_rk4_finalize_any(int64_t total, double* __restrict__ v, double
                                    const double* __restrict__ l1, const double* __restrict__ l2,
                                    const double* __restrict__ l3, const double* __restrict__ l4) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        v[i] += (1.0 / 6.0) * (l1[i] + 2.0 * l2[i] + 2.0 * l3[i] + l4[i]);
-        f[i] += (1.0 / 6.0) * (k1[i] + 2.0 * k2[i] + 2.0 * k3[i] + k4[i]);
+        v[i] = rk4_sum(v[i], l1[i], l2[i], l3[i], l4[i]);
+        f[i] = rk4_sum(f[i], k1[i], k2[i], k3[i], k4[i]);
     }
 }
 
@@ -317,6 +297,22 @@ int choose_xc(int X, int tiles_yz, int resident) {
     return best;
 }
 
+// x-chunk of a walk whose first planes are loaded at once (sky_grad.cuh): minimise (waves of
+// tiles) x (planes computed + about one and a half planes' time to fill the ring).
+int choose_chunk(int X, int tiles_yz, int resident) {
+    int best = X;
+    int64_t best_cost = -1;
+    for (int xc = 1; xc <= X; ++xc) {
+        const int64_t nt = (int64_t)tiles_yz * ((X + xc - 1) / xc);
+        const int64_t cost = ((nt + resident - 1) / resident) * (2 * xc + 3);
+        if (best_cost < 0 || cost < best_cost || (cost == best_cost && xc > best)) {
+            best_cost = cost;
+            best = xc;
+        }
+    }
+    return best;
+}
+
 // Library options (sky_set_option): key 0 = kernel family of the
 // reference-layout gradient and densities (1 = marching kernels, 0 = 3-D tile
 // kernels); key 1 = x-chunk of those marching launches (0 = automatic); key 2 =
@@ -357,6 +353,68 @@ int launch_gradient_march(const Params& p, const T* field, T* eg, T* l, cudaStre
     kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, mg, field, eg, l);
     return check_cuda(cudaGetLastError(), "launch march gradient", __LINE__);
 }
+
+// Geometry of a walk's launch: x-chunk (xc_opt, or 0: chosen), tiles and persistent blocks; one-time kernel attributes.
+template <class M, class K>
+int walk_geometry(K kern, size_t smem, const Params& p, int cap, int xc_opt, int* per_sm, MarchGrid* mg, int* blocks) {
+    if (*per_sm == 0) {
+        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                            "cudaFuncSetAttribute(walk)", __LINE__);
+        if (rc) return rc;
+        int n = 0;
+        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, M::NTHREADS, smem), "occupancy",
+                        __LINE__);
+        if (rc) return rc;
+        *per_sm = n < 1 ? 1 : n;
+    }
+    int resident = num_sms() * *per_sm;
+    if (cap > 0 && resident > cap) resident = cap;
+    const MarchGrid g0 = march_grid<M>(p, p.X);
+    *mg = march_grid<M>(p, xc_opt > 0 ? (xc_opt < p.X ? xc_opt : p.X) : choose_chunk(p.X, g0.nz * g0.ny, resident));
+    *blocks = mg->count() < resident ? mg->count() : resident;
+    return SKY_OK;
+}
+
+// 16-byte copies need a 16-byte aligned array and Z a multiple of two doubles.
+static bool wide64(const Params& p, const double* f) {
+    return p.Z % 2 == 0 && (reinterpret_cast<uintptr_t>(f) & 15) == 0;
+}
+template <template <typename> class Th, bool WIDE>
+using Shape64 = MarchShape<Th<double>::C, grad_rows64<Th>(), WIDE, 2>;
+
+template <template <typename> class Th, bool WIDE>
+int launch_gradient_walk(const Params& p, const double* field, double* eg, double* l, cudaStream_t st) {
+    using M = Shape64<Th, WIDE>;
+    auto kern = k_grad_plain<Th, M>;
+    const size_t smem = GradPipe<Th, M, double, double, 1, false>::bytes;
+    static int per_sm = 0;
+    MarchGrid mg;
+    int blocks;
+    int rc = walk_geometry<M>(kern, smem, p, 0, option(1), &per_sm, &mg, &blocks);
+    if (rc) return rc;
+    MarchCoef<double> k;
+    k.init(p);
+    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, field, eg, l);
+    return check_cuda(cudaGetLastError(), "launch gradient walk", __LINE__);
+}
+
+template <template <typename> class Th, bool WIDE, int STAGE>
+int launch_stage_walk(const Params& p, const double* in, const StageArrays& a, double* counter_e, double* scratch_m,
+                      double* err, cudaStream_t st) {
+    using M = Shape64<Th, WIDE>;
+    auto kern = k_plain_stage<Th, M, STAGE>;
+    const size_t smem = GradPipe<Th, M, double, double, 1, false>::bytes;
+    static int per_sm = 0;
+    MarchGrid mg;
+    int blocks;
+    int rc = walk_geometry<M>(kern, smem, p, kMaxRedBlocks, 0, &per_sm, &mg, &blocks);
+    if (rc) return rc;
+    MarchCoef<double> k;
+    k.init(p);
+    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, in, a, counter_e, scratch_m, err);
+    return check_cuda(cudaGetLastError(), "launch stage walk", __LINE__);
+}
+
 template <template <typename> class Th, typename T, typename S>
 int launch_gradient(const Params& p, const S* field, S* eg, S* l, cudaStream_t st) {
     using Shape = typename GradTile<Th<T>::C, T>::type;
@@ -418,71 +476,92 @@ int launch_density(const Params& p, const S* field, double* dens, double* scratc
 
 template <template <typename> class Th>
 int grad64(const Params& p, const double* f, double* eg, double* l, cudaStream_t st) {
-    if constexpr (Th<double>::C <= 5) {
-        if (option(0) == 1 && (int64_t)p.C * n_sites(p) < ((int64_t)1 << 31)) {
-            // 16-byte staging needs a 16-byte aligned field and Z a multiple of two doubles
-            if (p.Z % 2 == 0 && (reinterpret_cast<uintptr_t>(f) & 15) == 0)
-                return launch_gradient_march<Th, double, true>(p, f, eg, l, st);
-            return launch_gradient_march<Th, double, false>(p, f, eg, l, st);
-        }
-    } else {
-        if (option(0) == 1 && (int64_t)p.C * n_sites(p) < ((int64_t)1 << 31))
+    if (option(0) == 1 && (int64_t)p.C * n_sites(p) < ((int64_t)1 << 31)) {
+        if constexpr (Th<double>::C <= 5)
+            return wide64(p, f) ? launch_gradient_walk<Th, true>(p, f, eg, l, st)
+                                : launch_gradient_walk<Th, false>(p, f, eg, l, st);
+        else
             return launch_gradient_march<Th, double, false, 4>(p, f, eg, l, st);
     }
     return launch_gradient<Th, double, double>(p, f, eg, l, st);
 }
-// Marching FP64 density with its fused compensated sum (energy: all components,
-// in 4-row tiles for rho; baryon: phi_0..3 of any theory).
-template <template <typename> class Th, int MODE, bool WIDE, int BY = 8>
-int launch_density_march(const Params& p, const double* field, double* dens, double* scratch, double* out_dev,
-                         cudaStream_t st) {
-    using M = MarchShape<(MODE == 0 ? Th<double>::C : 4), BY, WIDE>;
-    auto kern = k_march_density<Th, M, MODE>;
-    const size_t smem = M::template smem_bytes<double>(1);
+// FP64 density walk with its fused compensated sum (energy: all components, in 6-row tiles for
+// rho, whose 13-component ring of more rows would not fit; baryon: phi_0..3 of any theory).
+// clear: set the reduction's completion counter to 0 first.
+template <template <typename> class Th, int MODE, bool WIDE>
+int launch_density_walk(const Params& p, const double* field, double* dens, double* scratch, double* out_dev,
+                        bool clear, cudaStream_t st) {
+    constexpr int C = MODE == 0 ? Th<double>::C : 4;
+    using M = MarchShape<C, (C > 5 ? 6 : 16), WIDE, 2>;
+    auto kern = k_dens_plain<Th, M, MODE>;
+    const size_t smem = PlanePipe<M, double, double, 1, false, M::NTHREADS>::bytes;
     static int per_sm = 0;
-    if (per_sm == 0) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(march density)", __LINE__);
-        if (rc) return rc;
-        int n = 0;
-        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, M::NTHREADS, smem), "occupancy",
-                        __LINE__);
-        if (rc) return rc;
-        per_sm = n < 1 ? 1 : n;
-    }
-    int resident = num_sms() * per_sm;
-    if (resident > kMaxRedBlocks) resident = kMaxRedBlocks;
-    const MarchGrid g0 = march_grid<M>(p, p.X);
-    const MarchGrid mg = march_grid<M>(p, choose_xc(p.X, g0.nz * g0.ny, resident));
-    const int blocks = mg.count() < resident ? mg.count() : resident;
-    if (scratch) {
-        int rc = check_cuda(cudaMemsetAsync(scratch + 2 * kMaxRedBlocks + 1, 0, sizeof(double), st), "memset",
-                            __LINE__);
+    MarchGrid mg;
+    int blocks;
+    int rc = walk_geometry<M>(kern, smem, p, kMaxRedBlocks, 0, &per_sm, &mg, &blocks);
+    if (rc) return rc;
+    if (scratch && clear) {
+        rc = check_cuda(cudaMemsetAsync(scratch + 2 * kMaxRedBlocks + 1, 0, sizeof(double), st), "memset", __LINE__);
         if (rc) return rc;
     }
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, mg, field, dens, scratch, out_dev);
-    return check_cuda(cudaGetLastError(), "launch march density", __LINE__);
-}
-
-template <template <typename> class Th, int MODE>
-int density_march(const Params& p, const double* f, double* dens, double* scratch, double* out_dev, cudaStream_t st) {
-    if (p.Z % 2 == 0 && (reinterpret_cast<uintptr_t>(f) & 15) == 0)
-        return launch_density_march<Th, MODE, true>(p, f, dens, scratch, out_dev, st);
-    return launch_density_march<Th, MODE, false>(p, f, dens, scratch, out_dev, st);
+    MarchCoef<double> k;
+    k.init(p);
+    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, field, dens, scratch, out_dev);
+    return check_cuda(cudaGetLastError(), "launch density walk", __LINE__);
 }
 
 template <template <typename> class Th>
-int dens64(const Params& p, int mode, const double* f, double* dens, double* scratch, double* out_dev,
+int dens64(const Params& p, int mode, const double* f, double* dens, double* scratch, double* out_dev, bool clear,
            cudaStream_t st) {
-    const bool march = option(0) == 1 && (int64_t)p.C * n_sites(p) < ((int64_t)1 << 31);
-    if (march && mode == 1) return density_march<Th, 1>(p, f, dens, scratch, out_dev, st);
-    if constexpr (Th<double>::C <= 5) {
-        if (march) return density_march<Th, 0>(p, f, dens, scratch, out_dev, st);
-    } else {
-        if (march) return launch_density_march<Th, 0, false, 4>(p, f, dens, scratch, out_dev, st);
+    if (option(0) == 1 && (int64_t)p.C * n_sites(p) < ((int64_t)1 << 31)) {
+        if (mode == 1)
+            return wide64(p, f) ? launch_density_walk<Th, 1, true>(p, f, dens, scratch, out_dev, clear, st)
+                                : launch_density_walk<Th, 1, false>(p, f, dens, scratch, out_dev, clear, st);
+        return wide64(p, f) ? launch_density_walk<Th, 0, true>(p, f, dens, scratch, out_dev, clear, st)
+                            : launch_density_walk<Th, 0, false>(p, f, dens, scratch, out_dev, clear, st);
     }
     return mode == 0 ? launch_density<Th, 0, double>(p, f, dens, scratch, out_dev, st)
                      : launch_density<Th, 1, double>(p, f, dens, scratch, out_dev, st);
+}
+
+// The four stages of a drop-in step as walks (C <= 5): k, l, Temp, EG, V and F as the separate
+// kernels leave them (k_plain_stage), the signed maximum of EG at *err.  `done` tells whether
+// they ran: not for rho, the tile-kernel option, lattices past the walks' 32-bit plane offsets,
+// or buffers that overlap, which keep the separate kernels.
+template <template <typename> class Th>
+int stages64(const Params& p, const StepBuffers& b, double* counter_e, double* scratch_m, double* err, bool* done,
+             cudaStream_t st) {
+    *done = false;
+    if constexpr (Th<double>::C <= 5) {
+        const int64_t n = (int64_t)p.C * n_sites(p);
+        if (option(0) != 1 || n >= ((int64_t)1 << 31)) return SKY_OK;
+        const double* all[] = {b.V, b.F, b.eg, b.k[0], b.k[1], b.k[2], b.k[3], b.l[0], b.l[1], b.l[2], b.l[3], b.temp};
+        constexpr int na = int(sizeof(all) / sizeof(all[0]));
+        for (int i = 0; i < na; ++i)
+            for (int j = i + 1; j < na; ++j)
+                if (all[i] < all[j] + n && all[j] < all[i] + n) return SKY_OK;
+        const bool w = wide64(p, b.F) && wide64(p, b.temp) && wide64(p, b.eg);
+        const StageArrays s1{b.V, b.F, b.l[0], b.l[1], b.l[2], b.k[0], b.l[0], b.temp};
+        const StageArrays s2{b.V, b.F, b.l[0], b.l[1], b.l[2], b.k[1], b.l[1], b.eg};
+        const StageArrays s3{b.V, b.F, b.l[0], b.l[1], b.l[2], b.k[2], b.l[2], b.temp};
+        const StageArrays s4{b.V, b.F, b.l[0], b.l[1], b.l[2], b.k[3], b.l[3], b.eg};
+        int rc;
+        if (w) {
+            if ((rc = launch_stage_walk<Th, true, 1>(p, b.F, s1, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, true, 2>(p, b.temp, s2, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, true, 3>(p, b.eg, s3, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, true, 4>(p, b.temp, s4, counter_e, scratch_m, err, st)))
+                return rc;
+        } else {
+            if ((rc = launch_stage_walk<Th, false, 1>(p, b.F, s1, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, false, 2>(p, b.temp, s2, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, false, 3>(p, b.eg, s3, counter_e, scratch_m, err, st)) ||
+                (rc = launch_stage_walk<Th, false, 4>(p, b.temp, s4, counter_e, scratch_m, err, st)))
+                return rc;
+        }
+        *done = true;
+    }
+    return SKY_OK;
 }
 
 // Baryon moments (k_march_moments): at most kScratchDoubles / 18 blocks, so the
@@ -571,7 +650,15 @@ int gradient_fp64(int theory, const Params& p, const double* f, double* eg, doub
 
 int density_fp64(int theory, const Params& p, int mode, const double* f, double* dens, double* scratch,
                  double* out_dev, cudaStream_t st) {
-    SKY_DISPATCH(theory, dens64, p, mode, f, dens, scratch, out_dev, st)
+    SKY_DISPATCH(theory, dens64, p, mode, f, dens, scratch, out_dev, true, st)
+}
+static int density_uncleared(int theory, const Params& p, int mode, const double* f, double* dens, double* scratch,
+                             double* out_dev, cudaStream_t st) {
+    SKY_DISPATCH(theory, dens64, p, mode, f, dens, scratch, out_dev, false, st)
+}
+static int stages_fp64(int theory, const Params& p, const StepBuffers& b, double* counter_e, double* scratch_m,
+                       double* err, bool* done, cudaStream_t st) {
+    SKY_DISPATCH(theory, stages64, p, b, counter_e, scratch_m, err, done, st)
 }
 
 int rk4_stage(const Params& p, double* kout, const double* v, const double* lin, double* temp, const double* f,
@@ -627,6 +714,43 @@ int reduce(int kind, const double* v, int64_t n, double* scratch, double* out_de
     else
         k_min<<<(int)b, 256, 0, st>>>(v, n, scratch, out_dev);
     return check_cuda(cudaGetLastError(), "launch reduce", __LINE__);
+}
+
+// One drop-in step on the caller's buffers (core/integrator.py:382-409); s_e and s_m: two
+// reduction scratch areas.  Reads the new energy and err and, on an arrest, zeroes the velocity.
+int arrested_step(int theory, const Params& p, const StepBuffers& b, double* s_e, double* s_m, double prev_energy,
+                  double* new_energy, double* err, cudaStream_t st) {
+    int rc;
+    double res[3];
+    // the step's two results side by side: the energy at s_e[2 kMaxRedBlocks], err two places on
+    double* out = s_e + 2 * kMaxRedBlocks;
+    bool done;
+    if ((rc = stages_fp64(theory, p, b, out + 1, s_m, out + 2, &done, st))) return rc;
+    if (done) {
+        if ((rc = density_uncleared(theory, p, 0, b.F, nullptr, s_e, nullptr, st))) return rc;
+    } else {
+        const double fac[4] = {0.0, 0.5, 0.5, 1.0};
+        for (int s = 0; s < 4; ++s) {
+            const double* lin = s == 0 ? b.V : b.l[s - 1];
+            const double* kprev = s == 0 ? b.F : b.k[s - 1];
+            if ((rc = rk4_stage(p, b.k[s], b.V, lin, b.temp, b.F, kprev, fac[s], st))) return rc;
+            if ((rc = gradient_fp64(theory, p, b.temp, b.eg, b.l[s], st))) return rc;
+        }
+        if ((rc = rk4_finalize(theory, p, b.V, b.F, b.k[0], b.k[1], b.k[2], b.k[3], b.l[0], b.l[1], b.l[2], b.l[3],
+                               st)))
+            return rc;
+        // new energy (core/integrator.py:402) and err = signed max of the stage-4 EG (:409)
+        if ((rc = density_fp64(theory, p, 0, b.F, nullptr, s_e, nullptr, st))) return rc;
+        if ((rc = reduce(1, b.eg, (int64_t)p.C * n_sites(p), s_m, out + 2, st))) return rc;
+    }
+    if ((rc = check_cuda(cudaMemcpyAsync(res, out, sizeof(res), cudaMemcpyDeviceToHost, st), "memcpy", __LINE__)))
+        return rc;
+    if ((rc = check_cuda(cudaStreamSynchronize(st), "sync", __LINE__))) return rc;
+    *new_energy = res[0];
+    *err = res[2];
+    // arrest (core/integrator.py:403-407)
+    if (p.killkinen && res[0] > prev_energy) return fill(b.V, (int64_t)p.C * n_sites(p), 0.0, st);
+    return SKY_OK;
 }
 
 int read_result(double* scratch, double* out_host, cudaStream_t st) {
@@ -862,37 +986,8 @@ int sky_arrested_newton_step(int theory, const int32_t* p_i, int32_t n_pi, const
     if (!new_energy_host || !err_host) return invalid("null host output");
     if (!scratch || n_scratch < 2 * kScratchDoubles) return SKY_ERR_NOMEM;
     cudaStream_t st = SKY_STREAM(stream);
-    // core/integrator.py:382-398
-    double* ks[4] = {k1, k2, k3, k4};
-    double* ls[4] = {l1, l2, l3, l4};
-    const double fac[4] = {0.0, 0.5, 0.5, 1.0};
-    for (int s = 0; s < 4; ++s) {
-        const double* lin = s == 0 ? velocity : ls[s - 1];
-        const double* kprev = s == 0 ? field : ks[s - 1];
-        if ((rc = rk4_stage(p, ks[s], velocity, lin, temp, field, kprev, fac[s], st))) return rc;
-        if ((rc = gradient_fp64(theory, p, temp, energy_gradient, ls[s], st))) return rc;
-    }
-    if ((rc = rk4_finalize(theory, p, velocity, field, k1, k2, k3, k4, l1, l2, l3, l4, st))) return rc;
-    // new energy (core/integrator.py:402) and err = signed max of the stage-4 EG (:409)
-    double* s_e = scratch;
-    double* s_m = scratch + kScratchDoubles;
-    if ((rc = density_fp64(theory, p, 0, field, nullptr, s_e, nullptr, st))) return rc;
-    if ((rc = reduce(1, energy_gradient, (int64_t)p.C * n_sites(p), s_m, nullptr, st))) return rc;
-    double res[2];
-    if ((rc = check_cuda(cudaMemcpyAsync(&res[0], s_e + 2 * kMaxRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, st),
-                         "memcpy", __LINE__)))
-        return rc;
-    if ((rc = check_cuda(cudaMemcpyAsync(&res[1], s_m + 2 * kMaxRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, st),
-                         "memcpy", __LINE__)))
-        return rc;
-    if ((rc = check_cuda(cudaStreamSynchronize(st), "sync", __LINE__))) return rc;
-    *new_energy_host = res[0];
-    *err_host = res[1];
-    // arrest (core/integrator.py:403-407)
-    if (p.killkinen && res[0] > prev_energy) {
-        if ((rc = fill(velocity, (int64_t)p.C * n_sites(p), 0.0, st))) return rc;
-    }
-    return SKY_OK;
+    const StepBuffers b{velocity, field, energy_gradient, {k1, k2, k3, k4}, {l1, l2, l3, l4}, temp};
+    return arrested_step(theory, p, b, scratch, scratch + kScratchDoubles, prev_energy, new_energy_host, err_host, st);
 }
 
 }  // extern "C"

@@ -89,6 +89,51 @@ __device__ __forceinline__ void skyrme_quartic(T* g, const T (&D)[3][C], const T
     for (int a = 0; a < 4; ++a) g[a] -= coef * acc[a];
 }
 
+// skyrme_quartic with the second derivatives taken one component at a time, pure ones with
+// the opposite sign: begin() needs the first derivatives only; add(a) consumes component a's
+// S = (-S_xx, -S_yy, -S_zz, S_xy, S_xz, S_yz) and returns its complete part of the sum that
+// skyrme_quartic subtracts, negated; rest(a), after all components, returns the other part.
+template <typename T, int C>
+struct QuarticStream {
+    T w[3], d[3];    // n_j + n_k, and 2 F_i . F_j of the pairs xy, xz, yz
+    T ci[3], cj[3];  // F_j.S_ij - S_jj.F_i and F_i.S_ij - S_ii.F_j of the pairs
+    __device__ __forceinline__ void begin(const T (&D)[3][C]) {
+        T n[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            n[i] = D[i][0] * D[i][0] + D[i][1] * D[i][1] + D[i][2] * D[i][2] + D[i][3] * D[i][3];
+        w[0] = n[1] + n[2];
+        w[1] = n[0] + n[2];
+        w[2] = n[0] + n[1];
+        const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int i = pi[q], j = pj[q];
+            const T f = D[i][0] * D[j][0] + D[i][1] * D[j][1] + D[i][2] * D[j][2] + D[i][3] * D[j][3];
+            d[q] = f + f;
+            ci[q] = cj[q] = T(0);
+        }
+    }
+    __device__ __forceinline__ T add(int a, const T (&S)[6], const T (&D)[3][C]) {
+        const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+        T acc = w[0] * S[0] + w[1] * S[1] + w[2] * S[2];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int i = pi[q], j = pj[q];
+            acc += d[q] * S[3 + q];
+            ci[q] += D[j][a] * S[3 + q];
+            ci[q] += S[j] * D[i][a];
+            cj[q] += D[i][a] * S[3 + q];
+            cj[q] += S[i] * D[j][a];
+        }
+        return acc;
+    }
+    // the part of components' sums, which skyrme_quartic subtracts times its coefficient
+    __device__ __forceinline__ T rest(int a, const T (&D)[3][C]) const {
+        return (ci[0] + ci[1]) * D[0][a] + (cj[0] + ci[2]) * D[1][a] + (cj[1] + cj[2]) * D[2][a];
+    }
+};
+
 // sum_{ijk} eps_ijk d_i(aux) det[e_mu, phi, d_j phi, d_k phi] for mu = 0..3, and
 // (into *negdet) -det[phi, d_x phi, d_y phi, d_z phi], which shares the (y, z)
 // cross product.  Used by the omega (th/omega_skyrme/kernels.py:633-690) and
@@ -131,6 +176,24 @@ struct Nuclear {
         g[0] -= mpi2;
         project<T, C>(g, phi, p.nsky);
     }
+    // gradient() with the second derivatives taken one component at a time (QuarticStream's S)
+    struct Stream {
+        QuarticStream<T, C> q;
+        T coef;
+        __device__ __forceinline__ void begin(const T*, const T (&D)[3][C], const Params& p) {
+            coef = T(p.c1 * p.c1);
+            q.begin(D);
+        }
+        __device__ __forceinline__ void add(int a, const T (&S)[6], const T*, const T (&D)[3][C], T* g) {
+            g[a] = coef * q.add(a, S, D) + (S[0] + S[1] + S[2]);
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) g[a] -= coef * q.rest(a, D);
+            g[0] -= T(p.c0 * p.c0);
+            project<T, C>(g, phi, p.nsky);
+        }
+    };
     // th/nuclear_skyrme/kernels.py:277-347
     __device__ static T energy(const T* phi, const T (&D)[3][C], const Params& p) {
         T n[3];
@@ -174,6 +237,25 @@ struct Omega {
         const T b0 = nd / T(2.0 * M_PI * M_PI);
         g[4] = phi[4] - (S[0][4] + S[1][4] + S[2][4]) + cw * b0;
     }
+    // gradient() with the second derivatives taken one component at a time (QuarticStream's S)
+    struct Stream {
+        __device__ __forceinline__ void begin(const T*, const T (&)[3][C], const Params&) {}
+        __device__ __forceinline__ void add(int a, const T (&S)[6], const T*, const T (&)[3][C], T* g) {
+            g[a] = S[0] + S[1] + S[2];
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+            const T cw = T(p.c1);
+            const T daux[3] = {D[0][4], D[1][4], D[2][4]};
+            T cs[4], nd;
+            cs_coupling<T, C>(cs, phi, D, daux, &nd);
+            const T k = T(p.c1 / (4.0 * M_PI * M_PI));
+#pragma unroll
+            for (int mu = 0; mu < 4; ++mu) g[mu] = k * cs[mu] + T(0.25) * g[mu];
+            g[0] -= T(0.25 * p.c0 * p.c0);
+            project<T, C>(g, phi, p.nsky);
+            g[4] += cw * (nd * T(1.0 / (2.0 * M_PI * M_PI))) + phi[4];
+        }
+    };
     // th/omega_skyrme/kernels.py:231-302 (no -c_omega*omega*B0 term, :301)
     __device__ static T energy(const T* phi, const T (&D)[3][C], const Params& p) {
         T n = T(0);
@@ -219,6 +301,28 @@ struct Coulomb {
         const T b0 = nd / T(2.0 * M_PI * M_PI);
         g[4] = -(kap * (S[0][4] + S[1][4] + S[2][4]) + kap * b0);
     }
+    // gradient() with the second derivatives taken one component at a time (QuarticStream's S)
+    struct Stream {
+        QuarticStream<T, C> q;
+        __device__ __forceinline__ void begin(const T*, const T (&D)[3][C], const Params&) { q.begin(D); }
+        __device__ __forceinline__ void add(int a, const T (&S)[6], const T*, const T (&D)[3][C], T* g) {
+            g[a] = S[0] + S[1] + S[2];
+            if (a < 4) g[a] += q.add(a, S, D);
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) g[a] -= q.rest(a, D);
+            g[0] -= T(p.c0 * p.c0);
+            const T daux[3] = {D[0][4], D[1][4], D[2][4]};
+            T cs[4], nd;
+            cs_coupling<T, C>(cs, phi, D, daux, &nd);
+            const T k = T(p.c1 / (4.0 * M_PI * M_PI));
+#pragma unroll
+            for (int mu = 0; mu < 4; ++mu) g[mu] -= k * cs[mu];
+            project<T, C>(g, phi, p.nsky);
+            g[4] = T(p.c1) * (g[4] - nd * T(1.0 / (2.0 * M_PI * M_PI)));
+        }
+    };
     // th/coulomb_skyrme/kernels.py:231-306 (no A0*B0 term, :305)
     __device__ static T energy(const T* phi, const T (&D)[3][C], const Params& p) {
         T n[3];
@@ -438,6 +542,18 @@ struct Berger {
         g[0] -= mpi2;
         project<T, C>(g, phi, p.nsky);
     }
+    // gradient() with the second derivatives taken one component at a time (QuarticStream's S)
+    struct Stream {
+        T S6[6][C];
+        __device__ __forceinline__ void begin(const T*, const T (&)[3][C], const Params&) {}
+        __device__ __forceinline__ void add(int a, const T (&S)[6], const T*, const T (&)[3][C], T*) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) S6[i][a] = i < 3 ? -S[i] : S[i];
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+            gradient(phi, D, S6, p, g);
+        }
+    };
     // th/berger_skyrme/kernels.py:251-337
     __device__ static T energy(const T* phi, const T (&D)[3][C], const Params& p) {
         T n[3];
@@ -484,6 +600,26 @@ struct LightlyBound {
         g[0] -= T(4) * al * om * om * om;
         project<T, C>(g, phi, p.nsky);
     }
+    // gradient() with the second derivatives taken one component at a time (QuarticStream's S)
+    struct Stream {
+        QuarticStream<T, C> q;
+        T w;
+        __device__ __forceinline__ void begin(const T*, const T (&D)[3][C], const Params& p) {
+            w = T(2.0 * (1.0 - p.c1));
+            q.begin(D);
+        }
+        __device__ __forceinline__ void add(int a, const T (&S)[6], const T*, const T (&D)[3][C], T* g) {
+            g[a] = w * (S[0] + S[1] + S[2]) + q.add(a, S, D);
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+            const T om = T(1) - phi[0];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) g[a] -= q.rest(a, D);
+            g[0] -= T(2.0 * (1.0 - p.c1) * p.c0 * p.c0);
+            g[0] -= T(4.0 * p.c1) * om * om * om;
+            project<T, C>(g, phi, p.nsky);
+        }
+    };
     // th/lightly_bound_skyrme/kernels.py:275-346
     __device__ static T energy(const T* phi, const T (&D)[3][C], const Params& p) {
         T n[3];
