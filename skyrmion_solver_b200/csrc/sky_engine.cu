@@ -10,328 +10,74 @@
 #include <vector>
 
 #include "sky_engine.cuh"
+#include "sky_engine_host.h"
 #include "sky_host.h"
 
 namespace sky {
 
 constexpr int kStatsCap = 8192;
 constexpr int kGraphSteps = 8;  // steps captured per graph replay
-
-struct HostInst {
-    int id = -1;
-    int theory = 0;
-    int prec = 0;  // storage: 0 = FP32 storage/arithmetic, 1 = FP64
-    int comp = 0;    // FP32 storage with a compensated (hi + lo) field
-    int defect = 0;  // ... and a defect-corrected gradient (precision 3)
-    int defect_period = kDefectRefresh;  // steps between refreshes of the correction
-    Params p{};
-    int64_t N = 0;
-    int C = 0;
-    void* F[2] = {nullptr, nullptr};
-    void* Flo[2] = {nullptr, nullptr};
-    void* Dlt = nullptr;
-    void* V[2] = {nullptr, nullptr};
-    void* L[3] = {nullptr, nullptr, nullptr};
-    KSum* epart = nullptr;
-    KSum* bpart = nullptr;
-    double* gpart = nullptr;
-    StepStats* stats = nullptr;
-    int ntiles = 0, tnz = 0, tny = 0, tnx = 0;
-    int xc = 0;          // x-chunk of the marching kernels
-    int xc_request = 0;  // x-chunk asked for by the caller (0: automatic)
-    bool tma = false;    // the stage kernels stage this instance with TMA box copies
-    bool pair = false;   // ... with z-pair tiles (FP32 theories without mixed derivatives, option 3)
-    int group_slot = -1;
-    int64_t steps = 0;  // host mirror of the device step counter
-    bool active = true;
-    size_t bytes = 0;
-};
-
-struct Group {
-    int theory = 0, prec = 0;
-    std::vector<int> members;  // instance ids in slot order
-    void* d_desc = nullptr;    // InstDesc<S>[cap]
-    int* d_tile_inst = nullptr;
-    int* d_done = nullptr;     // blocks of the current tail stage launch finished (0 between launches)
-    int desc_cap = 0, tile_cap = 0;
-    int ntiles = 0;
-    bool any_comp = false;  // holds a compensated-field instance (stage 1 stages the low parts too)
-    bool all_wide = true;   // every member can use the wide-row (16-byte staged) kernels
-    bool any_defect = false;  // holds a defect-corrected instance (launch the defect refresh)
-    bool all_tma = false;     // every member has TMA plane maps (launch the TMA stage kernels)
-    bool all_pair = false;    // ... and runs as z-pair tiles (option 3 at admission)
-};
+// Steps launched kernel by kernel after a change of the instance set before they are captured:
+// capturing and instantiating eight steps takes about as long as launching 64 (a millisecond),
+// and a server that admits or retires a request every chunk of 64 steps would do it every chunk.
+constexpr int kDirectSteps = 64;
 
 struct Engine {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;  // stage 4 of a captured step, beside the work on the new field
+    cudaEvent_t forked = nullptr, joined = nullptr;
     std::map<int, HostInst> insts;
     int next_id = 0;
     Group groups[6][2];
     cudaGraphExec_t graph = nullptr;   // kGraphSteps steps
     cudaGraphExec_t graph1 = nullptr;  // one step (the remainder of a step call)
-    bool graph_valid = false;
+    bool graph_valid = false, graph1_valid = false;
     int graph_pdl = -1;                // option 4 when the graphs were captured
+    int direct_steps = 0;              // steps launched kernel by kernel since the instance set changed
     int64_t bytes = 0;
     int* d_status = nullptr;  // device error word the stage kernels set (bit 0: a TMA wait gave up)
 };
 
-// ---------------------------------------------------------------------------
-// shapes and launches per (theory, precision)
-// ---------------------------------------------------------------------------
-// Every theory runs the marching kernels (sky_march.cuh) in both precisions.
-// Tiles are 8 rows x 32 columns, except for FP64 rho (13 components): its
-// 4-row tiles keep the five-plane ring at 150 KB, narrow rows only, with two
-// of stage 3/4's three sources staged (one block per SM).
-constexpr int kMarchBY = 8;
-template <template <typename> class Th, typename T>
-constexpr int march_by() {
-    return (Th<float>::C > 5 && sizeof(T) == 8) ? 4 : kMarchBY;
+const TheoryOps& theory_ops(int theory) {
+    switch (theory) {
+        case SKY_THEORY_NUCLEAR: return kNuclearOps;
+        case SKY_THEORY_OMEGA: return kOmegaOps;
+        case SKY_THEORY_COULOMB: return kCoulombOps;
+        case SKY_THEORY_RHO: return kRhoOps;
+        case SKY_THEORY_BERGER: return kBergerOps;
+        default: return kLightlyBoundOps;
+    }
 }
-template <template <typename> class Th, typename T>
-constexpr bool march_wide_allowed() {
-    return !(Th<float>::C > 5 && sizeof(T) == 8);
+static int launch_stage_group(int stage, const Group& g, const StageArgs& a, cudaStream_t st) {
+    return theory_ops(g.theory).stage(g.prec, stage, g, a, st);
 }
-// Wide-row (16-byte staged) or narrow-row march shape.
-template <template <typename> class Th, typename T, bool WIDE>
-using MShape = MarchShape<Th<T>::C, march_by<Th, T>(), WIDE && march_wide_allowed<Th, T>()>;
-
-template <int STAGE>
-constexpr int stage_nsrc() {
-    return STAGE == 1 ? 1 : (STAGE == 2 ? 2 : 3);
+static int launch_energy(const Group& g, const StageArgs& a, cudaStream_t st) {
+    return energy_walk(g.theory, g.prec) ? theory_ops(g.theory).energy(g, a, st) : SKY_OK;
 }
-
-// Resident blocks per SM the marching stages are compiled for (__launch_bounds__):
-// two for FP32 (registers capped at 128, no spills for C = 5), one for FP64
-// (whose shared memory allows no more).
-template <template <typename> class Th, typename T>
-constexpr int march_minb() {
-    return (sizeof(T) == 4 && Th<float>::C <= 5) ? 2 : 1;
+// Defect refresh of the group's defect-corrected FP32 instances (those whose refresh is due;
+// the others' tiles are skipped).
+static int launch_defect(const Group& g, cudaStream_t st) {
+    return g.prec || !g.any_defect ? SKY_OK : theory_ops(g.theory).defect(g, st);
 }
+static int setup_group(const Group& g) { return theory_ops(g.theory).setup(g.prec); }
 
 // Whether every instance of a group can use the wide-row kernels: Z a multiple of
 // 16 / sizeof(T) (the buffers are cudaMalloc'd, hence 256-byte aligned).
 static bool wide_ok(int prec, int Z) { return Z % (prec ? 2 : 4) == 0; }
 
-// One-time kernel attribute setup (kept out of stream capture); returns the
-// number of resident blocks per SM.
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool LO = false, bool TMA = false>
-static size_t stage_smem() {
-    using M = MShape<Th, T, WIDE>;
-    return stage_smem_bytes<M, T, STAGE, march_minb<Th, T>(), LO, TMA>();
-}
-
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool LO = false, bool TMA = false,
-          bool PAIR = false>
-static int stage_setup_w(int* per_sm_out) {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int rc, n = 0;
-        using M = MShape<Th, T, WIDE>;
-        auto kern = k_march_stage<Th, M, T, STAGE, march_minb<Th, T>(), LO, TMA, PAIR>;
-        const size_t smem = stage_smem<Th, T, STAGE, WIDE, LO, TMA>();
-        rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                        "cudaFuncSetAttribute(march stage)", __LINE__);
-        if (rc) return rc;
-        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, stage_threads<M, PAIR>(), smem),
-                        "occupancy query", __LINE__);
-        if (rc) return rc;
-        per_sm = n < 1 ? 1 : n;
-    }
-    *per_sm_out = per_sm;
-    return SKY_OK;
-}
-
-template <template <typename> class Th, typename T, int STAGE>
-static int stage_setup(int* per_sm_out) {
-    return stage_setup_w<Th, T, STAGE, true>(per_sm_out);
-}
-
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool LO = false, bool TMA = false,
-          bool PAIR = false>
-static int launch_stage_w(const Group& g, int t_begin, int t_end, cudaStream_t st, int tail) {
-    int per_sm = 1;
-    int rc = stage_setup_w<Th, T, STAGE, WIDE, LO, TMA, PAIR>(&per_sm);
-    if (rc) return rc;
-    int n = t_end - t_begin;
-    if (n <= 0) return SKY_OK;
-    const int blocks = n < num_sms() * per_sm ? n : num_sms() * per_sm;
-    InstDesc<T>* d = reinterpret_cast<InstDesc<T>*>(g.d_desc);
-    using M = MShape<Th, T, WIDE>;
-    const size_t smem = stage_smem<Th, T, STAGE, WIDE, LO, TMA>();
-    const dim3 block(PAIR ? PairShape<M>::TZ : M::BZ, M::BY);
-    auto kern = k_march_stage<Th, M, T, STAGE, march_minb<Th, T>(), LO, TMA, PAIR>;
-    int* done = tail ? g.d_done : nullptr;
-    if (option(4) == 1) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = block;
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return check_cuda(cudaLaunchKernelEx(&cfg, kern, static_cast<const InstDesc<T>*>(d), d,
-                                             static_cast<const int*>(g.d_tile_inst), t_begin, t_end, done),
-                          "launch engine stage", __LINE__);
-    }
-    kern<<<blocks, block, smem, st>>>(d, d, g.d_tile_inst, t_begin, t_end, done);
-    return check_cuda(cudaGetLastError(), "launch engine stage", __LINE__);
-}
-
-// Whether the FP32 stages of Th run as z-pair tiles (option 3, TMA groups, theories
-// without mixed second derivatives).
-template <template <typename> class Th, typename T>
-constexpr bool pair_allowed() {
-    return sizeof(T) == 4 && !Th<float>::kMixed && Th<float>::C <= 5;
-}
-
-// Whether the stage kernels of (Th, T) can stage with TMA: wide rows must be allowed.
-template <template <typename> class Th, typename T>
-constexpr bool tma_allowed() {
-    return march_wide_allowed<Th, T>();
-}
-
-template <template <typename> class Th, typename T, int STAGE>
-static int launch_stage(const Group& g, int t_begin, int t_end, cudaStream_t st, int tail) {
-    if constexpr (tma_allowed<Th, T>()) {
-        if (g.all_tma) {
-            if constexpr (pair_allowed<Th, T>()) {
-                if (g.all_pair) {
-                    if constexpr (STAGE == 1) {
-                        if (g.any_comp) return launch_stage_w<Th, T, 1, true, true, true, true>(g, t_begin, t_end, st, tail);
-                    }
-                    return launch_stage_w<Th, T, STAGE, true, false, true, true>(g, t_begin, t_end, st, tail);
-                }
-            }
-            if constexpr (STAGE == 1 && sizeof(T) == 4 && Th<float>::C <= 5) {
-                if (g.any_comp) return launch_stage_w<Th, T, 1, true, true, true>(g, t_begin, t_end, st, tail);
-            }
-            return launch_stage_w<Th, T, STAGE, true, false, true>(g, t_begin, t_end, st, tail);
-        }
-    }
-    // stage 1 of a group with compensated-field instances stages the low parts too,
-    // in wide rows when two blocks per SM still fit (the two six-slot rings take
-    // 112.5 KB per block for C = 5), else in narrow rows; rho's 13 components leave
-    // no room for the second ring at all: its FP64 densities use the high parts
-    if constexpr (STAGE == 1 && sizeof(T) == 4 && Th<float>::C <= 5) {
-        if (g.any_comp) {
-            if (g.all_wide) {
-                int n = 0;
-                const int rc = stage_setup_w<Th, T, 1, true, true>(&n);
-                if (rc) return rc;
-                if (n >= 2) return launch_stage_w<Th, T, 1, true, true>(g, t_begin, t_end, st, tail);
-            }
-            return launch_stage_w<Th, T, 1, false, true>(g, t_begin, t_end, st, tail);
-        }
-    }
-    if (g.all_wide) return launch_stage_w<Th, T, STAGE, true>(g, t_begin, t_end, st, tail);
-    return launch_stage_w<Th, T, STAGE, false>(g, t_begin, t_end, st, tail);
-}
-
-template <template <typename> class Th, typename T>
-static int launch_stage_any(int stage, const Group& g, int tb, int te, cudaStream_t st, int tail) {
-    switch (stage) {
-        case 1: return launch_stage<Th, T, 1>(g, tb, te, st, tail);
-        case 2: return launch_stage<Th, T, 2>(g, tb, te, st, tail);
-        case 3: return launch_stage<Th, T, 3>(g, tb, te, st, tail);
-        default: return launch_stage<Th, T, 4>(g, tb, te, st, tail);
-    }
-}
-
-template <template <typename> class Th>
-static int stage_dispatch_prec(int prec, int stage, const Group& g, int tb, int te, cudaStream_t st, int tail) {
-    return prec ? launch_stage_any<Th, double>(stage, g, tb, te, st, tail)
-                : launch_stage_any<Th, float>(stage, g, tb, te, st, tail);
-}
-
-template <template <typename> class Th, typename T>
-static int setup_all() {
-    int n, rc;
-    if ((rc = stage_setup<Th, T, 1>(&n)) || (rc = stage_setup<Th, T, 2>(&n)) || (rc = stage_setup<Th, T, 3>(&n)) ||
-        (rc = stage_setup<Th, T, 4>(&n)))
-        return rc;
-    if constexpr (sizeof(T) == 4 && Th<float>::C <= 5) {  // stage 1 with the low parts
-        if ((rc = stage_setup_w<Th, T, 1, true, true>(&n)) || (rc = stage_setup_w<Th, T, 1, false, true>(&n)))
-            return rc;
-    }
-    if constexpr (tma_allowed<Th, T>()) {
-        if ((rc = stage_setup_w<Th, T, 1, true, false, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 2, true, false, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 3, true, false, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 4, true, false, true>(&n)))
-            return rc;
-        if constexpr (sizeof(T) == 4 && Th<float>::C <= 5) {
-            if ((rc = stage_setup_w<Th, T, 1, true, true, true>(&n))) return rc;
-        }
-    }
-    if constexpr (tma_allowed<Th, T>() && pair_allowed<Th, T>()) {
-        if ((rc = stage_setup_w<Th, T, 1, true, false, true, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 2, true, false, true, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 3, true, false, true, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 4, true, false, true, true>(&n)) ||
-            (rc = stage_setup_w<Th, T, 1, true, true, true, true>(&n)))
-            return rc;
-    }
-    return SKY_OK;
-}
-
-template <template <typename> class Th>
-static int setup_prec(int prec) {
-    return prec ? setup_all<Th, double>() : setup_all<Th, float>();
-}
-
-static int setup_group(const Group& g) {
-    switch (g.theory) {
-        case SKY_THEORY_NUCLEAR: return setup_prec<Nuclear>(g.prec);
-        case SKY_THEORY_OMEGA: return setup_prec<Omega>(g.prec);
-        case SKY_THEORY_COULOMB: return setup_prec<Coulomb>(g.prec);
-        case SKY_THEORY_RHO: return setup_prec<Rho>(g.prec);
-        case SKY_THEORY_BERGER: return setup_prec<Berger>(g.prec);
-        case SKY_THEORY_LIGHTLY_BOUND: return setup_prec<LightlyBound>(g.prec);
-    }
-    return invalid("unknown theory id");
-}
-
-// tail = 1: stage 4 also advances each instance and stage 1 also runs its control
-// (the step's launch sequence); 0: the stage alone (admission, precision change).
-static int launch_stage_group(int stage, const Group& g, int tb, int te, cudaStream_t st, int tail = 0) {
-    switch (g.theory) {
-        case SKY_THEORY_NUCLEAR: return stage_dispatch_prec<Nuclear>(g.prec, stage, g, tb, te, st, tail);
-        case SKY_THEORY_OMEGA: return stage_dispatch_prec<Omega>(g.prec, stage, g, tb, te, st, tail);
-        case SKY_THEORY_COULOMB: return stage_dispatch_prec<Coulomb>(g.prec, stage, g, tb, te, st, tail);
-        case SKY_THEORY_RHO: return stage_dispatch_prec<Rho>(g.prec, stage, g, tb, te, st, tail);
-        case SKY_THEORY_BERGER: return stage_dispatch_prec<Berger>(g.prec, stage, g, tb, te, st, tail);
-        case SKY_THEORY_LIGHTLY_BOUND: return stage_dispatch_prec<LightlyBound>(g.prec, stage, g, tb, te, st, tail);
-    }
-    return invalid("unknown theory id");
-}
-
-// Tile geometry of a (theory, precision): (bz, by, tx) = (32, BY, 0) for the
-// marching kernels, whose x-chunk is chosen per instance; per_sm = resident
-// stage-4 blocks per SM.
-template <template <typename> class Th>
-static int shape_of(int prec, int& bz, int& by, int& tx, int& per_sm) {
-    per_sm = 1;
-    if (prec) {
-        bz = 32, by = march_by<Th, double>(), tx = 0;
-        return stage_setup<Th, double, 4>(&per_sm);
-    }
-    bz = 32, by = march_by<Th, float>(), tx = 0;
-    return stage_setup<Th, float, 4>(&per_sm);
-}
-
-static int tile_shape(int theory, int prec, int& bz, int& by, int& tx, int& per_sm) {
-    switch (theory) {
-        case SKY_THEORY_NUCLEAR: return shape_of<Nuclear>(prec, bz, by, tx, per_sm);
-        case SKY_THEORY_OMEGA: return shape_of<Omega>(prec, bz, by, tx, per_sm);
-        case SKY_THEORY_COULOMB: return shape_of<Coulomb>(prec, bz, by, tx, per_sm);
-        case SKY_THEORY_RHO: return shape_of<Rho>(prec, bz, by, tx, per_sm);
-        case SKY_THEORY_BERGER: return shape_of<Berger>(prec, bz, by, tx, per_sm);
-        default: return shape_of<LightlyBound>(prec, bz, by, tx, per_sm);
-    }
+// Stage tiles of an instance for x-chunk request `xc` (0: chosen).
+static void tile_geometry(const HostInst& h, int request, int* xc, int* nz, int* ny, int* nx) {
+    const TileShapeInfo sh = theory_ops(h.theory).shape(h.prec);
+    *nz = (h.p.Z + 31) / 32;
+    *ny = (h.p.Y + sh.rows - 1) / sh.rows;
+    const int resident = num_sms() * sh.blocks;
+    if (request > 0)
+        *xc = request < h.p.X ? request : h.p.X;
+    else
+        *xc = theory_components(h.theory) <= 5 ? choose_chunk(h.p.X, *nz * *ny, resident)
+                                               : choose_xc(h.p.X, *nz * *ny, resident);
+    *nx = (h.p.X + *xc - 1) / *xc;
 }
 
 static int launch_control(const Group& g, int ib, int ie, int mode, cudaStream_t st) {
@@ -343,50 +89,6 @@ static int launch_control(const Group& g, int ib, int ie, int mode, cudaStream_t
     return check_cuda(cudaGetLastError(), "launch engine control", __LINE__);
 }
 
-
-// Defect refresh of the group's defect-corrected FP32 instances (those whose
-// refresh flag the stage-4 advance just set; the others' tiles are skipped).
-template <template <typename> class Th, bool WIDE>
-static int launch_defect_t(const Group& g, cudaStream_t st) {
-    using M = MarchShape<Th<double>::C, march_by<Th, double>(), WIDE && march_wide_allowed<Th, double>()>;
-    auto kern = k_march_defect<Th, M, march_by<Th, float>()>;
-    const size_t smem = M::template smem_bytes<double, float>(2);
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(defect)", __LINE__);
-        if (rc) return rc;
-        int n = 0;
-        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, M::NTHREADS, smem), "occupancy",
-                        __LINE__);
-        if (rc) return rc;
-        per_sm = n < 1 ? 1 : n;
-    }
-    const int n = g.ntiles;
-    if (n <= 0) return SKY_OK;
-    const int blocks = n < num_sms() * per_sm ? n : num_sms() * per_sm;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(reinterpret_cast<InstDesc<float>*>(g.d_desc), g.d_tile_inst, 0,
-                                                   n);
-    return check_cuda(cudaGetLastError(), "launch defect refresh", __LINE__);
-}
-
-template <template <typename> class Th>
-static int launch_defect_w(const Group& g, cudaStream_t st) {
-    return g.all_wide ? launch_defect_t<Th, true>(g, st) : launch_defect_t<Th, false>(g, st);
-}
-
-static int launch_defect(const Group& g, cudaStream_t st) {
-    if (g.prec || !g.any_defect) return SKY_OK;
-    switch (g.theory) {
-        case SKY_THEORY_NUCLEAR: return launch_defect_w<Nuclear>(g, st);
-        case SKY_THEORY_OMEGA: return launch_defect_w<Omega>(g, st);
-        case SKY_THEORY_COULOMB: return launch_defect_w<Coulomb>(g, st);
-        case SKY_THEORY_BERGER: return launch_defect_w<Berger>(g, st);
-        case SKY_THEORY_LIGHTLY_BOUND: return launch_defect_w<LightlyBound>(g, st);
-        case SKY_THEORY_RHO: return launch_defect_w<Rho>(g, st);
-        default: return SKY_OK;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // conversion kernels (FP64 reference layout <-> engine storage)
@@ -428,29 +130,32 @@ __global__ void k_f32c_to_f64(int64_t n, const float* __restrict__ hi, const flo
 // ---------------------------------------------------------------------------
 // descriptors
 // ---------------------------------------------------------------------------
-// TMA plane maps of an instance's staged arrays (box: 40 z-values x (BY + 4) rows x 1
-// plane x C components, the marching kernels' wide-row plane).
+// TMA plane maps of an instance's staged arrays: box hz z-values x (rows + 4) y x 1 plane x C
+// components, the haloed plane of a stage tile; and of an energy tile.
 template <typename S>
-static int encode_maps(const HostInst& h, InstDesc<S>& d, int by) {
-    const void* arrs[kNumCentreMaps] = {h.F[0], h.F[1], h.Flo[0], h.Flo[1], h.V[0], h.V[1],
-                                        h.L[0], h.L[1], h.L[2], h.Dlt};
-    for (int k = 0; k < kNumCentreMaps; ++k) {
+static int encode_maps(const HostInst& h, InstDesc<S>& d) {
+    const TileShapeInfo sh = theory_ops(h.theory).shape(h.prec);
+    const void* arrs[kNumMaps] = {h.F[0], h.F[1], h.Flo[0], h.Flo[1], h.V[0], h.V[1],
+                                  h.L[0], h.L[1], h.L[2], h.Dlt};
+    for (int k = 0; k < kNumMaps; ++k) {
         if (!arrs[k]) continue;
-        int rc = SKY_OK;
-        if (k < kNumMaps)
-            rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, 40, by + 4);
-        // centre box: the tile's 32 z-values x BY rows, no halo
-        if (!rc) rc = encode_plane_map(&d.tmc[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, 32, by);
+        int rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, sh.hz, sh.rows + 4);
+        if (!rc && k < kNumEnergyMaps && energy_walk(h.theory, h.prec))
+            rc = encode_plane_map(&d.tme[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, 40, kEnergyRows + 4);
         if (rc) return rc;
     }
     return SKY_OK;
 }
 
 template <typename S>
-static InstDesc<S> make_desc(const HostInst& h, int tile_begin) {
+static InstDesc<S> make_desc(const HostInst& h, int tile_begin, int e_tile_begin) {
     InstDesc<S> d;
     memset(&d, 0, sizeof(d));
     d.p = h.p;
+    d.coef.init(h.p);
+    MarchCoef<double> cd;
+    cd.init(h.p);
+    for (int i = 0; i < 3; ++i) d.r1d[i] = cd.r1[i];
     for (int i = 0; i < 2; ++i) {
         d.F[i] = reinterpret_cast<S*>(h.F[i]);
         d.Flo[i] = reinterpret_cast<S*>(h.Flo[i]);
@@ -469,6 +174,12 @@ static InstDesc<S> make_desc(const HostInst& h, int tile_begin) {
     d.tiles_ny = h.tny;
     d.tiles_nx = h.tnx;
     d.xc = h.xc;
+    d.e_tile_begin = e_tile_begin;
+    d.e_ntiles = h.entiles;
+    d.e_nz = h.etnz;
+    d.e_ny = h.etny;
+    d.e_nx = h.etnx;
+    d.e_xc = h.exc;
     d.active = h.active ? 1 : 0;
     d.refresh_period = h.defect_period;
     return d;
@@ -489,27 +200,22 @@ static int rebuild_group_t(Engine& e, Group& g) {
         if ((rc = check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__))) return rc;
     }
     std::vector<InstDesc<S>> descs;
-    std::vector<int> tile_inst;
+    std::vector<int> tile_inst, e_tile_inst;
     int tb = 0;
-    g.any_comp = false;
     g.all_wide = true;
     g.any_defect = false;
     g.all_tma = !g.members.empty();
-    g.all_pair = !g.members.empty();
     for (size_t k = 0; k < g.members.size(); ++k) {
         HostInst& h = e.insts[g.members[k]];
-        InstDesc<S> d = make_desc<S>(h, tb);
+        InstDesc<S> d = make_desc<S>(h, tb, (int)e_tile_inst.size());
         d.status = e.d_status;
         if (h.tma) {
-            int bz, by, tx, per_sm;
-            int rc = tile_shape(h.theory, h.prec, bz, by, tx, per_sm);
-            if (!rc) rc = encode_maps<S>(h, d, by);
+            const int rc = encode_maps<S>(h, d);
             if (rc) return rc;
             d.tma = 1;
         } else {
             g.all_tma = false;
         }
-        if (!h.pair) g.all_pair = false;
         if (h.group_slot >= 0 && h.group_slot < (int)dev_old.size()) {
             const InstDesc<S>& o = dev_old[h.group_slot];
             d.e_prev = o.e_prev;
@@ -519,14 +225,16 @@ static int rebuild_group_t(Engine& e, Group& g) {
             d.refresh = (o.refresh && d.Dlt != nullptr) ? 1 : 0;  // a pending defect refresh survives
         }
         h.group_slot = (int)k;
-        if (h.comp) g.any_comp = true;
         if (h.defect) g.any_defect = true;
         if (!wide_ok(h.prec, h.p.Z)) g.all_wide = false;
         descs.push_back(d);
         for (int t = 0; t < h.ntiles; ++t) tile_inst.push_back((int)k);
+        if (energy_walk(h.theory, h.prec)) e_tile_inst.insert(e_tile_inst.end(), h.entiles, (int)k);
         tb += h.ntiles;
     }
     g.ntiles = tb;
+    g.entiles = (int)e_tile_inst.size();
+    tile_inst.insert(tile_inst.end(), e_tile_inst.begin(), e_tile_inst.end());
     if ((int)descs.size() > g.desc_cap) {
         if (g.d_desc) cudaFree(g.d_desc);
         g.desc_cap = (int)descs.size() * 2 + 4;
@@ -555,7 +263,8 @@ static int rebuild_group_t(Engine& e, Group& g) {
                         "write tile list", __LINE__);
         if (rc) return rc;
     }
-    e.graph_valid = false;
+    e.graph_valid = e.graph1_valid = false;
+    e.direct_steps = 0;
     return check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__);
 }
 
@@ -585,7 +294,7 @@ static bool tma_possible(const HostInst& h) {
     return wide_ok(h.prec, h.p.Z) && !(h.prec && theory_components(h.theory) > 5);
 }
 static bool tma_ok_for(const HostInst& h) { return option(2) == 1 && tma_possible(h); }
-// Whether an instance can run as z-pair tiles (TMA staging, FP32, omega).
+// Whether the z-pair flag applies to an instance (TMA staging, FP32, omega).
 static bool pair_possible(const HostInst& h) { return h.prec == 0 && h.theory == SKY_THEORY_OMEGA; }
 
 static int alloc_inst(Engine& e, HostInst& h) {
@@ -593,17 +302,17 @@ static int alloc_inst(Engine& e, HostInst& h) {
     h.tma = tma_ok_for(h);
     h.pair = h.tma && option(3) == 1 && pair_possible(h);
     const size_t fb = es * (size_t)h.C * (size_t)h.N;
-    int bz, by, tx, per_sm;
-    int rc0 = tile_shape(h.theory, h.prec, bz, by, tx, per_sm);
-    if (rc0) return rc0;
-    h.tnz = (h.p.Z + bz - 1) / bz;
-    h.tny = (h.p.Y + by - 1) / by;
-    (void)tx;
     if ((int64_t)h.C * h.N >= ((int64_t)1 << 31)) return invalid("lattice too large for the marching kernels");
-    h.xc = h.xc_request > 0 ? (h.xc_request < h.p.X ? h.xc_request : h.p.X)
-                            : choose_xc(h.p.X, h.tnz * h.tny, num_sms() * per_sm);
-    h.tnx = (h.p.X + h.xc - 1) / h.xc;
+    tile_geometry(h, h.xc_request, &h.xc, &h.tnz, &h.tny, &h.tnx);
     h.ntiles = h.tnz * h.tny * h.tnx;
+    h.entiles = h.ntiles;
+    if (energy_walk(h.theory, h.prec)) {
+        h.etnz = h.tnz;
+        h.etny = (h.p.Y + kEnergyRows - 1) / kEnergyRows;
+        h.exc = choose_chunk(h.p.X, h.etnz * h.etny, num_sms());
+        h.etnx = (h.p.X + h.exc - 1) / h.exc;
+        h.entiles = h.etnz * h.etny * h.etnx;
+    }
     void** bufs[] = {&h.F[0], &h.F[1], &h.V[0], &h.V[1], &h.L[0], &h.L[1], &h.L[2]};
     for (void** b : bufs) {
         if (cudaMalloc(b, fb) != cudaSuccess) {
@@ -612,7 +321,7 @@ static int alloc_inst(Engine& e, HostInst& h) {
             return SKY_ERR_NOMEM;
         }
     }
-    if (cudaMalloc(&h.epart, sizeof(KSum) * h.ntiles) != cudaSuccess ||
+    if (cudaMalloc(&h.epart, sizeof(KSum) * h.entiles) != cudaSuccess ||
         cudaMalloc(&h.bpart, sizeof(KSum) * h.ntiles) != cudaSuccess ||
         cudaMalloc(&h.gpart, sizeof(double) * 4 * h.ntiles) != cudaSuccess ||
         cudaMalloc(&h.stats, sizeof(StepStats) * kStatsCap) != cudaSuccess) {
@@ -640,8 +349,8 @@ static int alloc_inst(Engine& e, HostInst& h) {
     }
     cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * h.ntiles, e.stream);
     cudaMemsetAsync(h.stats, 0, sizeof(StepStats) * kStatsCap, e.stream);
-    h.bytes = (h.comp ? 9 : 7) * fb + (h.defect ? fb : 0) + (sizeof(KSum) * 2 + sizeof(double) * 4) * h.ntiles +
-              sizeof(StepStats) * kStatsCap;
+    h.bytes = (h.comp ? 9 : 7) * fb + (h.defect ? fb : 0) + (sizeof(KSum) + sizeof(double) * 4) * h.ntiles +
+              sizeof(KSum) * h.entiles + sizeof(StepStats) * kStatsCap;
     return SKY_OK;
 }
 
@@ -681,50 +390,70 @@ static int upload(Engine& e, HostInst& h, const double* field, const double* vel
 // Stage 1 + control for one instance (admission or precision change).
 static int init_instance(Engine& e, HostInst& h, int mode) {
     Group& g = e.groups[h.theory][h.prec];
-    int tb = 0;
+    int tb = 0, eb = 0;
     for (int id : g.members) {
         if (id == h.id) break;
         tb += e.insts[id].ntiles;
+        eb += e.insts[id].entiles;
     }
-    int rc = launch_stage_group(1, g, tb, tb + h.ntiles, e.stream);
+    int rc = launch_energy(g, StageArgs{eb, eb + h.entiles, 0}, e.stream);
+    if (!rc) rc = launch_stage_group(1, g, StageArgs{tb, tb + h.ntiles, 0}, e.stream);
     if (rc) return rc;
     rc = launch_control(g, h.group_slot, h.group_slot + 1, mode, e.stream);
     if (rc) return rc;
     return check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__);
 }
 
-// Launch kinds of one step, in order: stage 2, 3, 4 (+ update), advance, the
-// defect refresh (groups with defect-corrected instances only), stage 1 (on the
-// updated field), control.  Groups are independent, so each kind is issued for
-// every non-empty group before the next kind.
-enum { kKindS2 = 0, kKindS3, kKindS4, kKindAdvance, kKindDefect, kKindS1, kKindControl, kNumKinds };
+// Launch kinds of one step: stage 2, stage 3 (+ the field's update), then stage 4 (+ the
+// velocity's) and, independent of it, the defect refresh (groups with defect-corrected instances
+// only), the energy of FP32 walks and stage 1, all on the new field.  Groups are independent, so
+// each kind is issued for every non-empty group before the next kind.
+enum { kKindS2 = 0, kKindS3, kKindS4, kKindDefect, kKindEnergy, kKindS1, kNumKinds };
 
-static int launch_kind(Engine& e, int kind) {
+static int launch_kind(Engine& e, int kind, cudaStream_t st) {
     for (int t = 0; t < 6; ++t)
         for (int pr = 0; pr < 2; ++pr) {
             Group& g = e.groups[t][pr];
             if (g.members.empty()) continue;
+            const StageArgs a{0, g.ntiles, 1};
             int rc = SKY_OK;
             switch (kind) {
-                case kKindS2: rc = launch_stage_group(2, g, 0, g.ntiles, e.stream); break;
-                case kKindS3: rc = launch_stage_group(3, g, 0, g.ntiles, e.stream); break;
-                case kKindS4: rc = launch_stage_group(4, g, 0, g.ntiles, e.stream, 1); break;
-                case kKindAdvance: break;  // folded into stage 4
-                case kKindDefect: rc = launch_defect(g, e.stream); break;
-                case kKindS1: rc = launch_stage_group(1, g, 0, g.ntiles, e.stream, 1); break;
-                default: break;  // the control is folded into stage 1
+                case kKindS2: rc = launch_stage_group(2, g, a, st); break;
+                case kKindS3: rc = launch_stage_group(3, g, a, st); break;
+                case kKindS4: rc = launch_stage_group(4, g, a, st); break;
+                case kKindDefect: rc = launch_defect(g, st); break;
+                case kKindEnergy: rc = launch_energy(g, StageArgs{0, g.entiles, 1}, st); break;
+                default: rc = launch_stage_group(1, g, a, st); break;
             }
             if (rc) return rc;
         }
     return SKY_OK;
 }
 
+// Record one step.  Stage 4 runs on a second stream beside the work on the new field, except
+// under programmatic dependent launch, which orders the kernels of one stream.
 static int record_step(Engine& e) {
-    for (int k = 0; k < kNumKinds; ++k) {
-        int rc = launch_kind(e, k);
-        if (rc) return rc;
+    int rc;
+    if ((rc = launch_kind(e, kKindS2, e.stream)) || (rc = launch_kind(e, kKindS3, e.stream))) return rc;
+    const bool fork = option(4) == 0;
+    cudaStream_t side = fork ? e.side : e.stream;
+    if (fork) {
+        if ((rc = check_cuda(cudaEventRecord(e.forked, e.stream), "fork", __LINE__)) ||
+            (rc = check_cuda(cudaStreamWaitEvent(side, e.forked, 0), "fork", __LINE__)))
+            return rc;
     }
-    return SKY_OK;
+    bool any_defect = false;
+    for (int t = 0; t < 6; ++t) any_defect = any_defect || e.groups[t][0].any_defect;
+    auto join = [&]() -> int {
+        if (!fork) return SKY_OK;
+        const int r = check_cuda(cudaEventRecord(e.joined, side), "join", __LINE__);
+        return r ? r : check_cuda(cudaStreamWaitEvent(e.stream, e.joined, 0), "join", __LINE__);
+    };
+    // the refresh replaces the correction that stage 4 reads: it and its stage 1 come after stage 4
+    if ((rc = launch_kind(e, kKindS4, side)) || (rc = launch_kind(e, kKindEnergy, e.stream))) return rc;
+    if (any_defect && ((rc = join()) || (rc = launch_kind(e, kKindDefect, e.stream)))) return rc;
+    if ((rc = launch_kind(e, kKindS1, e.stream))) return rc;
+    return any_defect ? SKY_OK : join();
 }
 
 static int count_launches(Engine& e) {
@@ -732,7 +461,8 @@ static int count_launches(Engine& e) {
     for (int t = 0; t < 6; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty())
-                n += 4 + ((pr == 0 && e.groups[t][pr].any_defect) ? 1 : 0);  // stages 2, 3, 4, [defect,] 1
+                // stages 2, 3, 4, [defect,] [energy,] 1
+                n += 4 + ((pr == 0 && e.groups[t][pr].any_defect) ? 1 : 0) + (energy_walk(t, pr) ? 1 : 0);
     return n;
 }
 
@@ -758,17 +488,17 @@ static int capture_steps(Engine& e, int nsteps, cudaGraphExec_t* exec) {
     return rc;
 }
 
-// The step graphs: kGraphSteps steps, and one step for the remainder of a call.
-// Each step depends only on device-side state, so replaying them is the same as
-// launching the kernels one by one.
-static int build_graph(Engine& e) {
+// The step graphs: kGraphSteps steps, and one step for the remainder of a call, each captured
+// when a call first wants it.  Each step depends only on device-side state, so replaying them is
+// the same as launching the kernels one by one.
+static int step_graph(Engine& e, int nsteps, cudaGraphExec_t* exec, bool* valid) {
+    if (*valid) return SKY_OK;
     int rc = SKY_OK;
     for (int t = 0; t < 6; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty() && (rc = setup_group(e.groups[t][pr]))) return rc;
-    if ((rc = capture_steps(e, kGraphSteps, &e.graph)) || (rc = capture_steps(e, 1, &e.graph1))) return rc;
-    e.graph_valid = true;
-    e.graph_pdl = option(4);
+    if ((rc = capture_steps(e, nsteps, exec))) return rc;
+    *valid = true;
     return SKY_OK;
 }
 
@@ -804,61 +534,6 @@ static int remove_from_group(Engine& e, HostInst& h) {
 
 using namespace sky;
 
-// ---------------------------------------------------------------------------
-// energy audit of the RK4 dynamics (k_engine_audit)
-// ---------------------------------------------------------------------------
-constexpr int kAuditBY = 4;  // 4-row tiles: a 13-component FP64 ring still fits
-
-template <template <typename> class Th, typename S>
-static int audit_t(Engine& e, const HostInst& h, double* out2) {
-    using M = MarchShape<Th<double>::C, kAuditBY, false>;
-    constexpr int NSRC = std::is_same<S, double>::value ? 1 : 2;
-    auto kern = k_engine_audit<Th, M, S>;
-    const size_t smem = M::template smem_bytes<double, S>(NSRC);
-    static bool configured = false;
-    if (!configured) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(audit)", __LINE__);
-        if (rc) return rc;
-        configured = true;
-    }
-    const MarchGrid mg = march_grid<M>(h.p, h.p.X < 16 ? h.p.X : 16);
-    const int blocks = mg.count() < num_sms() ? mg.count() : num_sms();
-    double* parts = nullptr;
-    int rc = check_cuda(cudaMalloc(&parts, sizeof(double) * 4 * blocks), "cudaMalloc(audit)", __LINE__);
-    if (rc) return rc;
-    const Group& g = e.groups[h.theory][h.prec];
-    const InstDesc<S>* d = reinterpret_cast<const InstDesc<S>*>(g.d_desc) + h.group_slot;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, e.stream>>>(d, mg, parts);
-    rc = check_cuda(cudaGetLastError(), "launch audit", __LINE__);
-    std::vector<double> hp(4 * (size_t)blocks);
-    if (!rc)
-        rc = check_cuda(cudaMemcpyAsync(hp.data(), parts, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, e.stream),
-                        "read audit", __LINE__);
-    if (!rc) rc = check_cuda(cudaStreamSynchronize(e.stream), "sync audit", __LINE__);
-    cudaFree(parts);
-    if (rc) return rc;
-    // fixed-order compensated sum of the block partials
-    for (int q = 0; q < 2; ++q) {
-        double sum = 0.0, comp = 0.0;
-        for (int b = 0; b < blocks; ++b) {
-            for (int k = 0; k < 2; ++k) {
-                const double v = hp[4 * b + 2 * q + k];
-                const double t = sum + v;
-                comp += (std::fabs(sum) >= std::fabs(v)) ? ((sum - t) + v) : ((v - t) + sum);
-                sum = t;
-            }
-        }
-        out2[q] = sum + comp;
-    }
-    return SKY_OK;
-}
-
-template <template <typename> class Th>
-static int audit_prec(Engine& e, const HostInst& h, double* out2) {
-    return h.prec ? audit_t<Th, double>(e, h, out2) : audit_t<Th, float>(e, h, out2);
-}
-
 // ===========================================================================
 // C ABI
 // ===========================================================================
@@ -870,10 +545,16 @@ int sky_engine_create(int device, void** out) {
     e->device = device;
     int rc = check_cuda(cudaSetDevice(device), "cudaSetDevice", __LINE__);
     if (!rc) rc = check_cuda(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream", __LINE__);
+    if (!rc) rc = check_cuda(cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking), "stream", __LINE__);
+    if (!rc) rc = check_cuda(cudaEventCreateWithFlags(&e->forked, cudaEventDisableTiming), "event", __LINE__);
+    if (!rc) rc = check_cuda(cudaEventCreateWithFlags(&e->joined, cudaEventDisableTiming), "event", __LINE__);
     if (!rc) rc = check_cuda(cudaMalloc(&e->d_status, sizeof(int)), "cudaMalloc(status)", __LINE__);
     if (!rc) rc = check_cuda(cudaMemset(e->d_status, 0, sizeof(int)), "memset(status)", __LINE__);
     if (rc) {
         if (e->d_status) cudaFree(e->d_status);
+        if (e->joined) cudaEventDestroy(e->joined);
+        if (e->forked) cudaEventDestroy(e->forked);
+        if (e->side) cudaStreamDestroy(e->side);
         if (e->stream) cudaStreamDestroy(e->stream);
         delete e;
         return rc;
@@ -902,6 +583,9 @@ int sky_engine_destroy(void* handle) {
             if (e->groups[t][p].d_done) cudaFree(e->groups[t][p].d_done);
         }
     if (e->d_status) cudaFree(e->d_status);
+    cudaEventDestroy(e->joined);
+    cudaEventDestroy(e->forked);
+    cudaStreamDestroy(e->side);
     cudaStreamDestroy(e->stream);
     delete e;
     return SKY_OK;
@@ -1065,15 +749,14 @@ int sky_engine_retile(void* handle, int id, int xc) {
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
     HostInst& h = *hp;
-    int bz, by, tx, per_sm;
-    int rc = tile_shape(h.theory, h.prec, bz, by, tx, per_sm);
-    if (rc) return rc;
-    const int tny = (h.p.Y + by - 1) / by, tnz = (h.p.Z + bz - 1) / bz;
-    const int nxc = xc > 0 ? (xc < h.p.X ? xc : h.p.X) : choose_xc(h.p.X, tnz * tny, num_sms() * per_sm);
-    const int ntiles = tnz * tny * ((h.p.X + nxc - 1) / nxc);
+    int rc, nxc, tnz, tny, tnx;
+    tile_geometry(h, xc, &nxc, &tnz, &tny, &tnx);
+    const int ntiles = tnz * tny * tnx;
+    const bool own_energy = energy_walk(h.theory, h.prec);  // its energy tiles stay as they are
+    const int entiles = own_energy ? h.entiles : ntiles;
     KSum *ep = nullptr, *bp = nullptr;
     double* gp = nullptr;
-    if (cudaMalloc(&ep, sizeof(KSum) * ntiles) != cudaSuccess || cudaMalloc(&bp, sizeof(KSum) * ntiles) != cudaSuccess ||
+    if (cudaMalloc(&ep, sizeof(KSum) * entiles) != cudaSuccess || cudaMalloc(&bp, sizeof(KSum) * ntiles) != cudaSuccess ||
         cudaMalloc(&gp, sizeof(double) * 4 * ntiles) != cudaSuccess) {
         cudaGetLastError();
         if (ep) cudaFree(ep);
@@ -1091,13 +774,15 @@ int sky_engine_retile(void* handle, int id, int xc) {
     h.bpart = bp;
     h.gpart = gp;
     cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * ntiles, e->stream);
-    const int64_t dbytes = (int64_t)(sizeof(KSum) * 2 + sizeof(double) * 4) * ((int64_t)ntiles - h.ntiles);
+    const int64_t dbytes = (int64_t)(sizeof(KSum) + sizeof(double) * 4) * ((int64_t)ntiles - h.ntiles) +
+                           (int64_t)sizeof(KSum) * ((int64_t)entiles - h.entiles);
     h.bytes += dbytes;
     e->bytes += dbytes;
     h.xc_request = xc;
     h.xc = nxc;
-    h.tnx = (h.p.X + nxc - 1) / nxc;
-    h.ntiles = ntiles;  // the staging (TMA, z-pairs) carries over
+    h.tnx = tnx;
+    h.ntiles = ntiles;  // the staging carries over
+    h.entiles = entiles;
     Group& g = e->groups[h.theory][h.prec];
     if ((rc = rebuild_group(*e, g))) return rc;
     return init_instance(*e, h, 2);
@@ -1138,15 +823,7 @@ int sky_engine_audit(void* handle, int id, double* out2) {
     HostInst* hp = find(e, id);
     if (!hp) return invalid("unknown instance id");
     cudaSetDevice(e->device);
-    switch (hp->theory) {
-        case SKY_THEORY_NUCLEAR: return audit_prec<Nuclear>(*e, *hp, out2);
-        case SKY_THEORY_OMEGA: return audit_prec<Omega>(*e, *hp, out2);
-        case SKY_THEORY_COULOMB: return audit_prec<Coulomb>(*e, *hp, out2);
-        case SKY_THEORY_RHO: return audit_prec<Rho>(*e, *hp, out2);
-        case SKY_THEORY_BERGER: return audit_prec<Berger>(*e, *hp, out2);
-        case SKY_THEORY_LIGHTLY_BOUND: return audit_prec<LightlyBound>(*e, *hp, out2);
-    }
-    return invalid("unknown theory id");
+    return theory_ops(hp->theory).audit(e->groups[hp->theory][hp->prec], *hp, e->stream, out2);
 }
 
 int sky_engine_set_defect_period(void* handle, int id, int period) {
@@ -1199,14 +876,24 @@ int sky_engine_step(void* handle, int nsteps) {
     cudaSetDevice(e->device);
     int rc;
     int done = 0;
-    if (e->graph_valid && e->graph_pdl != option(4)) e->graph_valid = false;
-    if (nsteps > 0 && !e->graph_valid && (rc = build_graph(*e))) return rc;
+    if (e->graph_pdl != option(4)) {
+        e->graph_valid = e->graph1_valid = false;
+        e->graph_pdl = option(4);
+    }
+    if (!e->graph_valid && !e->graph1_valid && e->direct_steps + nsteps <= kDirectSteps) {
+        for (; done < nsteps; ++done)
+            if ((rc = record_step(*e))) return rc;
+        e->direct_steps += nsteps;
+    }
     while (nsteps - done >= kGraphSteps) {
+        if ((rc = step_graph(*e, kGraphSteps, &e->graph, &e->graph_valid))) return rc;
         if ((rc = check_cuda(cudaGraphLaunch(e->graph, e->stream), "graph launch", __LINE__))) return rc;
         done += kGraphSteps;
     }
-    for (; done < nsteps; ++done)
+    for (; done < nsteps; ++done) {
+        if ((rc = step_graph(*e, 1, &e->graph1, &e->graph1_valid))) return rc;
         if ((rc = check_cuda(cudaGraphLaunch(e->graph1, e->stream), "graph launch", __LINE__))) return rc;
+    }
     for (auto& kv : e->insts)
         if (kv.second.active) kv.second.steps += nsteps;
     return SKY_OK;
@@ -1367,7 +1054,7 @@ int sky_engine_time_stages(void* handle, int nsteps, double* ms_out) {
     for (int s = 0; s < nsteps && rc == SKY_OK; ++s) {
         for (int k = 0; k < kNumKinds && rc == SKY_OK; ++k) {
             cudaEventRecord(ev[k], e->stream);
-            rc = launch_kind(*e, k);
+            rc = launch_kind(*e, k, e->stream);
         }
         if (rc) break;
         cudaEventRecord(ev[kNumKinds], e->stream);
@@ -1383,7 +1070,8 @@ int sky_engine_time_stages(void* handle, int nsteps, double* ms_out) {
     for (auto& kv : e->insts)
         if (kv.second.active) kv.second.steps += nsteps;
     // report in the order stage 1, 2, 3, 4, control, advance
-    ms_out[0] = (acc[kKindS1] + acc[kKindDefect]) / nsteps;  // stage 1 with the defect refresh
+    // stage 1 with the defect refresh and the FP32 energy walk
+    ms_out[0] = (acc[kKindS1] + acc[kKindDefect] + acc[kKindEnergy]) / nsteps;
     ms_out[1] = acc[kKindS2] / nsteps;
     ms_out[2] = acc[kKindS3] / nsteps;
     ms_out[3] = acc[kKindS4] / nsteps;

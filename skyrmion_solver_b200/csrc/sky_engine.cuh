@@ -6,25 +6,27 @@
 // stage inputs of the reference schedule are
 //   X1 = F,  X2 = F + (dt/2) V,  X3 = F + (dt/2)(V + l1/2),  X4 = F + dt (V + l2/2)
 // and the update is
-//   V' = V + (l1 + 2 l2 + 2 l3 + l4)/6,   F' = F + dt (V + (l1 + l2 + l3)/6)
+//   F' = F + dt (V + (l1 + l2 + l3)/6),   V' = V + (l1 + 2 l2 + 2 l3 + l4)/6
 // followed by the theory's normalisation of phi and projection of V'
 // (core/integrator.py:163-175).  Stage s builds X_s for its haloed tile on the
-// fly from F, V and the previous slope and writes only l_s; stage 4 applies the
-// update into the other half of a ping-pong pair.
+// fly from F, V and the previous slope.
 //
-// One step is: stage 2, stage 3, stage 4 (+ update; its tail advances each instance),
-// [the defect refresh,] stage 1 (its tail runs each instance's control).
-// Stage 1 runs on the freshly updated field, so besides l1 (needed by the next
-// step) it evaluates that field's energy and baryon density in FP64; the
-// control launch reduces them (compensated, fixed order), records the step's
-// (energy, err) exactly as do_arrested_newton_flow returns them, and takes the
-// arrest decision for the next step: the velocity is treated as zero when
-// killkinen is set and the energy rose (core/integrator.py:403-407).
+// F' needs no l4.  So stage 3 already writes the new field, into the other half of a
+// ping-pong pair, and P = V + (l1 + 2 l2 + 2 l3)/6 instead of l3; stage 4 adds l4 / 6,
+// projects and leaves V'.  The work on the new field -- its energy and the next step's l1
+// (stage 1) -- then depends on stage 3 only and runs beside stage 4:
+//   stage 2 -> stage 3 -> { stage 4 | [defect refresh,] [FP32 energy,] stage 1 } -> control.
+// The last block of the two branches to finish runs every instance's control: it reduces the
+// energy, baryon number and stage-4 gradient (compensated, fixed order), records the step's
+// (energy, err) exactly as do_arrested_newton_flow returns them, takes the arrest decision for
+// the next step (the velocity is treated as zero when killkinen is set and the energy rose,
+// core/integrator.py:403-407) and flips the halves.  l1 alternates between two buffers, since
+// stage 4 of an arrested step reads the old one (l2 = l1) while stage 1 writes the new one.
 #pragma once
 
+#include "sky_grad.cuh"
 #include "sky_kernels.cuh"
 #include "sky_march.cuh"
-#include "sky_march_pair.cuh"
 
 namespace sky {
 
@@ -42,26 +44,30 @@ struct StepStats {
     int reserved;
 };
 
-// Roles of an instance's TMA plane maps (InstDesc::tm).
-// Plane maps (tm) cover a tile's haloed plane, centre maps (tmc) its BY x 32 sites
-// (the stage-4 update's operands, which need no halo); the centre maps add the
-// defect correction at kMapDlt.
-enum { kMapF = 0, kMapFlo = 2, kMapV = 4, kMapL = 6, kNumMaps = 9, kMapDlt = 9, kNumCentreMaps = 10 };
+// Roles of an instance's TMA plane maps (InstDesc::tm): the haloed plane of a stage tile; the
+// field's also of an energy tile (InstDesc::tme, kMapF and kMapFlo).
+enum { kMapF = 0, kMapFlo = 2, kMapV = 4, kMapL = 6, kMapDlt = 9, kNumMaps = 10, kNumEnergyMaps = 4 };
+
+// Default number of steps between refreshes of the defect correction of an FP32
+// instance (sky_engine_set_defect_period changes it per instance).
+constexpr int kDefectRefresh = 16;
 
 // Device-resident state of one instance.
 template <typename S>
 struct InstDesc {
-    TmaMap tm[kNumMaps];  // plane maps of F[0..1], Flo[0..1], V[0..1], L[0..2] (when tma is set)
-    TmaMap tmc[kNumCentreMaps];  // centre maps of the same arrays and of Dlt (when tma is set)
+    TmaMap tm[kNumMaps];  // plane maps of F[0..1], Flo[0..1], V[0..1], L[0..2], Dlt (when tma is set)
+    TmaMap tme[kNumEnergyMaps];  // energy-tile maps of F and Flo (FP32 instances of at most five components)
     int tma;              // the stage kernels stage this instance's planes with TMA
     int* status;          // the engine's error word (bit 0: a wait for a TMA copy gave up)
     Params p;
+    MarchCoef<S> coef;   // stencil scales of the lattice
+    double r1d[3];       // ... of the FP64 energy's first derivatives
     S* F[2];           // ping-pong field
     S* Flo[2];         // ping-pong low parts of a compensated FP32 field (null otherwise)
     S* Dlt;            // defect correction g64 - g32 of a defect-corrected FP32 instance (null otherwise)
-    S* V[2];           // ping-pong velocity
-    S* L[3];           // stage slopes l1, l2, l3
-    KSum* epart;       // per-tile energy partials (stage 1)
+    S* V[2];           // ping-pong velocity (the next half holds P between stages 3 and 4)
+    S* L[3];           // slopes: l1 of this step and of the next in L[0] and L[2] (see cur_l1), l2 in L[1]
+    KSum* epart;       // energy partials, per energy tile (k_energy) or per stage tile (stage 1)
     KSum* bpart;       // per-tile baryon partials (stage 1)
     double* gpart;     // per-tile [signed max, abs max of stage-4 g, kinetic KSum (s, c)] (4 doubles / tile)
     StepStats* stats;  // ring of per-step records
@@ -70,73 +76,56 @@ struct InstDesc {
     int ntiles;
     int tiles_nz, tiles_ny, tiles_nx;
     int xc;            // x-chunk of the marching kernels
+    int e_tile_begin, e_ntiles, e_nz, e_ny, e_nx, e_xc;  // energy tiles (e_ntiles = ntiles where stage 1 sums it)
     // control state (device-updated)
     double e_prev;     // energy entering the previous step
     int step;          // steps taken
     int arrested;      // arrest flag for the current step
     int active;        // 0 = skip (retired / paused)
     int cur;           // which half of the F / V ping-pong pairs is current
-    int refresh;       // this step's stage 1 refreshes the defect correction
+    int refresh;       // the current l1 comes from a defect refresh
     int refresh_period;  // steps between refreshes of the defect correction
 };
 
-// RK4 update of one site (core/integrator.py:163-175): V' = V + (l1 + 2 l2 + 2 l3 + l4)/6,
-// F' = F + (k1 + 2 k2 + 2 k3 + k4)/6 = F + dt (V + (l1 + l2 + l3)/6), then the theory's
-// normalisation of the first nsky components and projection of V' orthogonal to them.
+// The field's update at one site: F' = F + dt (V + (l1 + l2 + l3)/6), then the theory's
+// normalisation of the first nsky components; and P = V + (l1 + 2 l2 + 2 l3)/6.
 // With a compensated field (comp) F is the unevaluated sum hi + lo of two FP32
-// values: the update, the normalisation and the projection run in FP64 and the result is
+// values: the update and the normalisation run in FP64 and the result is
 // split back into hi + lo, so increments far below one FP32 ulp of F still accumulate.
-template <typename T, typename S, int C>
-__device__ __forceinline__ void finalize_vals(int64_t s, int64_t N, const T (&f0)[C], const T (&flo)[C], bool comp,
-                                              const T (&v0)[C], const T (&l1)[C], const T (&l2)[C],
-                                              const T (&l3)[C], const T (&g)[C], T dtt, int nsky, int unit_length,
-                                              S* __restrict__ Fo, S* __restrict__ Flo_out, S* __restrict__ Vo,
-                                              T& v2) {
-    T vv[C], inc[C];
+template <typename T, int C>
+__device__ __forceinline__ void update_field(const T (&f0)[C], const T (&flo)[C], bool comp, const T (&v0)[C],
+                                             const T (&l1)[C], const T (&l2)[C], const T (&l3)[C], T dtt, int nsky,
+                                             int unit_length, T (&fo)[C], T (&lo)[C], T (&pv)[C]) {
+    T inc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        const T l4 = -dtt * g[c];
-        vv[c] = v0[c] + (l1[c] + T(2) * l2[c] + T(2) * l3[c] + l4) * T(1.0 / 6.0);
-        inc[c] = dtt * (v0[c] + (l1[c] + l2[c] + l3[c]) * T(1.0 / 6.0));
+        const T b = l2[c] + l3[c], a = l1[c] + b;
+        pv[c] = v0[c] + (a + b) * T(1.0 / 6.0);
+        inc[c] = dtt * (v0[c] + a * T(1.0 / 6.0));
+        lo[c] = T(0);
     }
     if (!comp) {
-        T fv[C];
 #pragma unroll
-        for (int c = 0; c < C; ++c) fv[c] = f0[c] + inc[c];
+        for (int c = 0; c < C; ++c) fo[c] = f0[c] + inc[c];
         if (unit_length) {
             // one reciprocal square root instead of a square root and nsky divisions
             // (within one unit in the last place of the quotients)
             T ss = T(0);
 #pragma unroll
             for (int c = 0; c < C; ++c)
-                if (c < nsky) ss += fv[c] * fv[c];
+                if (c < nsky) ss += fo[c] * fo[c];
             if (ss != T(0)) {
                 const T r = ss == T(1) ? T(1) : rsqrt(ss);  // unit fields (the vacuum shell) stay exact
 #pragma unroll
                 for (int c = 0; c < C; ++c)
-                    if (c < nsky) fv[c] *= r;
+                    if (c < nsky) fo[c] *= r;
             }
-            T lm = T(0);
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                if (c < nsky) lm += vv[c] * fv[c];
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                if (c < nsky) vv[c] -= lm * fv[c];
-        }
-        v2 = T(0);
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            __stcg(Fo + c * N + s, S(fv[c]));
-            __stcg(Vo + c * N + s, S(vv[c]));
-            v2 += vv[c] * vv[c];
         }
     } else {
         // hi + lo + inc in FP64, with the two small terms summed in FP32 first: lo and the
         // increment are both far below hi, so their FP32 sum loses no more than the FP32
         // increment and the FP32 low part already do (about 2^-49 of the field).  One
-        // reciprocal square root normalises.  The velocity is FP32 storage and is
-        // projected in FP32 on the rounded field.
+        // reciprocal square root normalises.
         double fd[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) fd[c] = double(f0[c]) + double(flo[c] + inc[c]);
@@ -152,55 +141,47 @@ __device__ __forceinline__ void finalize_vals(int64_t s, int64_t N, const T (&f0
                     if (c < nsky) fd[c] *= r;
             }
         }
-        T hi[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            hi[c] = T(fd[c]);
-            __stcg(Fo + c * N + s, S(hi[c]));
-            __stcg(Flo_out + c * N + s, S(fd[c] - double(hi[c])));
-        }
-        if (unit_length) {
-            T lm = T(0);
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                if (c < nsky) lm += vv[c] * hi[c];
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                if (c < nsky) vv[c] -= lm * hi[c];
-        }
-        v2 = T(0);
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            __stcg(Vo + c * N + s, S(vv[c]));
-            v2 += vv[c] * vv[c];
+            fo[c] = T(fd[c]);
+            lo[c] = T(fd[c] - double(fo[c]));
         }
     }
 }
 
-// finalize_vals with the inputs read from global memory (the stage-4 epilogue).
-template <typename T, typename S, int C>
-__device__ __forceinline__ void finalize_site(int64_t s, int64_t N, const S* __restrict__ F,
-                                              const S* __restrict__ Flo_in, const S* __restrict__ V,
-                                              const S* __restrict__ L1, const S* __restrict__ L2,
-                                              const S* __restrict__ L3, const T (&g)[C], T dtt, int nsky,
-                                              int unit_length, S* __restrict__ Fo, S* __restrict__ Flo_out,
-                                              S* __restrict__ Vo, T& v2) {
-    // the arrays are read-only during stage 4 (it writes the other halves of the
-    // ping-pong pairs): non-coherent global loads (the pointers come from the
-    // descriptor in global memory, so the compiler cannot infer the space itself)
-    T f0[C], flo[C], v0[C], a1[C], a2[C], a3[C];
+// The velocity's update: V' = P + l4 / 6, projected orthogonal to the first nsky components of
+// the new field (a compensated field's high parts); returns |V'|^2.
+template <typename T, int C>
+__device__ __forceinline__ T update_velocity(const T (&pv)[C], const T (&g)[C], const T (&fo)[C], T dtt, int nsky,
+                                             int unit_length, T (&vv)[C]) {
+    const T w = -dtt * T(1.0 / 6.0);
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-        const int64_t j = c * N + s;
-        f0[c] = T(__ldg(F + j));
-        flo[c] = Flo_in ? T(__ldg(Flo_in + j)) : T(0);
-        v0[c] = V ? T(__ldg(V + j)) : T(0);
-        a1[c] = T(__ldg(L1 + j));
-        a2[c] = T(__ldg(L2 + j));
-        a3[c] = T(__ldg(L3 + j));
+    for (int c = 0; c < C; ++c) vv[c] = pv[c] + w * g[c];
+    if (unit_length) {
+        T lm = T(0);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (c < nsky) lm += vv[c] * fo[c];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (c < nsky) vv[c] -= lm * fo[c];
     }
-    finalize_vals<T, S, C>(s, N, f0, flo, Flo_in != nullptr, v0, a1, a2, a3, g, dtt, nsky, unit_length, Fo, Flo_out,
-                           Vo, v2);
+    T v2 = T(0);
+#pragma unroll
+    for (int c = 0; c < C; ++c) v2 += vv[c] * vv[c];
+    return v2;
+}
+
+// Whether the work on the new field of the step in flight refreshes the defect correction.
+template <typename S>
+__device__ __forceinline__ bool refresh_due(const InstDesc<S>& in) {
+    const int period = in.refresh_period > 0 ? in.refresh_period : kDefectRefresh;
+    return in.Dlt != nullptr && (in.step + 1) % period == 0;
+}
+// The buffer of the current step's l1 (half 0) or of the next one's (half 1).
+template <typename S>
+__device__ __forceinline__ int l1_slot(const InstDesc<S>& in, int half) {
+    return (in.cur ^ half) ? 2 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -208,10 +189,10 @@ __device__ __forceinline__ void finalize_site(int64_t s, int64_t N, const S* __r
 // of the field entering this step) and the previous step's stage-4 gradient
 // partials, records StepStats and sets the arrest flag.
 // ---------------------------------------------------------------------------
-// mode 0: end of a step (arrest decision); 1: admission (step 0, no arrest);
-// 2: resume after a precision change (keeps the pending arrest decision).
+// mode 0: end of a step (advances the instance, arrest decision); 1: admission (step 0, no
+// arrest); 2: resume after a precision change (keeps the pending arrest decision).
 // The work is one warp's (the control kernel, or a warp of the last block to finish a
-// stage-1 launch, one warp per instance): lane-strided compensated sums of
+// step's stage-4 and stage-1 launches, one warp per instance): lane-strided compensated sums of
 // the per-tile partials and a fixed shuffle tree, so the order depends on the tile count
 // only.  The partials are read through L2: in the stage kernel they were written by
 // other blocks of the same launch.
@@ -220,8 +201,8 @@ __device__ __forceinline__ void engine_control_warp(InstDesc<S>& in, int mode) {
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
     KSum e{0.0, 0.0}, b{0.0, 0.0}, kin{0.0, 0.0};
     double gm = -1.0e300, ga = 0.0;
+    for (int t = lane; t < in.e_ntiles; t += 32) ksum_merge(e, KSum{__ldcg(&in.epart[t].s), __ldcg(&in.epart[t].c)});
     for (int t = lane; t < in.ntiles; t += 32) {
-        ksum_merge(e, KSum{__ldcg(&in.epart[t].s), __ldcg(&in.epart[t].c)});
         ksum_merge(b, KSum{__ldcg(&in.bpart[t].s), __ldcg(&in.bpart[t].c)});
         gm = fmax(gm, __ldcg(&in.gpart[4 * t]));
         ga = fmax(ga, __ldcg(&in.gpart[4 * t + 1]));
@@ -242,6 +223,11 @@ __device__ __forceinline__ void engine_control_warp(InstDesc<S>& in, int mode) {
     if (lane == 0) {
         const double en = e.s + e.c;
         if (mode == 1) in.step = 0;
+        if (mode == 0) {
+            in.refresh = refresh_due(in) ? 1 : 0;
+            in.step += 1;
+            in.cur ^= 1;
+        }
         const int n = in.step;
         // arrest (core/integrator.py:403-407): the energy after step n exceeds the one after step n-1
         int arrest = in.arrested;
@@ -263,14 +249,8 @@ __device__ __forceinline__ void engine_control_warp(InstDesc<S>& in, int mode) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// Control: one block per instance.  Reduces the stage-1 partials (energy and
-// baryon number of the field entering this step) and the previous step's
-// stage-4 gradient partials, records StepStats and sets the arrest flag.
-// ---------------------------------------------------------------------------
-// mode 0: end of a step (arrest decision); 1: admission (step 0, no arrest);
-// 2: resume after a precision change (keeps the pending arrest decision).
-// (The steps themselves fold mode 0 into stage 1: k_march_stage with tail.)
+// Control of the instances [i_begin, i_end), one block each (admission, precision change; the
+// steps themselves fold mode 0 into their last launches).
 template <typename S>
 __global__ void __launch_bounds__(32) k_engine_control(InstDesc<S>* __restrict__ insts, int i_begin, int i_end,
                                                        int mode) {
@@ -281,379 +261,584 @@ __global__ void __launch_bounds__(32) k_engine_control(InstDesc<S>* __restrict__
     engine_control_warp(in, mode);
 }
 
-// Default number of steps between refreshes of the defect correction of an FP32
-// instance (sky_engine_set_defect_period changes it per instance).
-constexpr int kDefectRefresh = 16;
 
-// Flip the ping-pong halves and advance the step counter (the tail of stage 4); flag
-// the defect refresh of the step that now begins.
-template <typename S>
-__device__ __forceinline__ void engine_advance_one(InstDesc<S>& in) {
-    in.step += 1;
-    in.cur ^= 1;
-    const int period = in.refresh_period > 0 ? in.refresh_period : kDefectRefresh;
-    in.refresh = (in.Dlt != nullptr && in.step % period == 0) ? 1 : 0;
+
+// ---------------------------------------------------------------------------
+// Stage kernels.  The stage input is built while the x-planes are staged; the epilogue
+// writes l_s, or applies the RK4 update at stage 4.  Theories of at most five components run
+// the gradient walk (sky_grad.cuh, k_grad_stage), rho the marching tile (sky_march.cuh,
+// k_march_stage).
+// ---------------------------------------------------------------------------
+// What a tile's stage reads and writes (both kernels).  `half`: stage 1 works on the new field
+// of the step in flight (1) or, at admission and after a precision change, on the current one (0).
+template <typename T>
+struct StageIo {
+    const T* src[3];   // sources of the stage input
+    T a, b;            // their weights
+    const T *F, *Flo, *V, *l1, *l2;  // stage 3: the update's operands (V null: zero; Flo null: not compensated)
+    // stages 1, 2: l_s.  Stage 3: F', its low parts and P.  Stage 4: F' (read) and P -> V'.
+    T *out, *out_lo, *pv;
+    T dtt;
+    bool l2_is_l1;
+};
+
+// An arrested step treats the velocity as zero, so its stage-2 input F + (dt/2) V is
+// the field itself: l2 = l1, and stage 2 has nothing to compute.  Stages 3 and 4 then
+// read l1 where they read l2.  Not after a defect refresh: that stage 1 formed l1 from
+// the FP64 gradient, and stage 2's FP32 gradient plus the new correction may differ
+// from it in the last bit.
+template <typename T>
+__device__ __forceinline__ bool l2_is_l1(const InstDesc<T>& in) {
+    return in.arrested && !in.refresh;
 }
 
+template <typename T, int STAGE>
+__device__ __forceinline__ StageIo<T> stage_io(const InstDesc<T>& in, const Params& p, int half) {
+    const int cur = STAGE == 1 ? in.cur ^ half : in.cur;
+    StageIo<T> io;
+    io.l2_is_l1 = l2_is_l1(in);
+    io.F = in.F[cur];
+    io.Flo = in.Flo[cur];
+    io.V = in.arrested ? nullptr : in.V[cur];
+    io.l1 = in.L[l1_slot(in, 0)];
+    io.l2 = io.l2_is_l1 ? io.l1 : in.L[1];  // the step's l2
+    io.dtt = T(p.dt);
+    const T hdt = T(0.5 * p.dt);
+    io.src[0] = io.F;
+    io.src[1] = io.V;
+    io.src[2] = STAGE == 3 ? io.l1 : io.l2;
+    io.a = STAGE == 4 ? io.dtt : hdt;
+    io.b = STAGE == 3 ? T(0.25) * io.dtt : T(0.5) * io.dtt;
+    io.out = STAGE == 1 ? in.L[l1_slot(in, half)] : STAGE == 2 ? in.L[1] : in.F[cur ^ 1];
+    io.out_lo = in.Flo[cur ^ 1];
+    io.pv = in.V[cur ^ 1];
+    return io;
+}
 
+// The maps of a tile's sources (null: the source reads as zero).
+template <typename T, int STAGE>
+__device__ __forceinline__ void stage_maps(const InstDesc<T>& in, const StageIo<T>& io, int half, TmaTile& tt) {
+    const int cur = STAGE == 1 ? in.cur ^ half : in.cur;
+    tt.map[0] = &in.tm[kMapF + cur];
+    tt.map[1] = io.V != nullptr ? &in.tm[kMapV + cur] : nullptr;
+    tt.map[2] = STAGE > 2 ? &in.tm[kMapL + (STAGE == 3 || io.l2_is_l1 ? l1_slot(in, 0) : 1)] : nullptr;
+    tt.status = in.status;
+}
 
-// ---------------------------------------------------------------------------
-// Marching stage kernel (C <= 5 theories): the stage input is built while the
-// x-planes are staged (sky_march.cuh); the epilogue writes l_s, or applies the
-// RK4 update at stage 4.
-// ---------------------------------------------------------------------------
-// The stage-4 update's operands for one plane of a tile, staged by TMA centre-box
-// copies into shared memory (k_march_stage with TMA; sky_march.cuh, the plane_begin
-// hook): F, F_lo, V, l1, l2, l3 and the defect correction, each C x BY x 32 values in
-// [c][y][z] order; a null map means the operand is absent (reads as zero).
+// The stage-4 statistics of a thread's sites.
 template <typename T>
-struct CentreStage {
-    T* buf;                     // kCentreArrays boxes
-    uint64_t* bar;              // the mbarrier the copies complete on
-    const TmaMap* map[7];       // F, F_lo, V, l1, l2, l3, Dlt
-    int* status;                // the engine's error word (bit 1: a centre-box wait gave up)
-    int z0, y0, box;            // tile origin; values per box
-    uint32_t phase;             // parity of the copies' next phase
-    uint32_t pending;           // parity of the phase this plane's copies complete
-};
-constexpr int kCentreArrays = 7;
-
-// CC: components of the theory.
-// CENTRE: stage 4 reads the update's operands from shared memory (CentreStage).
-// NL: sites per thread (2 for the z-pair tiles: lane l is the thread's site l).
-template <typename T, int STAGE, int CC, bool CENTRE = false, int NL = 1>
-struct EngineEpi {
-    // the correction of the thread's next site is held in registers (prefetched a plane
-    // ahead) for CC <= 5; with more components it is read at the site
-    static constexpr bool kPrefetch = CC <= 5;
-    // inputs of the stage-4 update, read from global memory at the site (prefetching them
-    // into shared memory with cp.async measured slower: more instructions and shared memory)
-    const T* fin_src[6];  // F, F_lo (null unless compensated), V (null when arrested), l1, l2, l3
-    T* out0;              // l_STAGE (stages 1-3) or F' (stage 4)
-    T* out1;              // V' (stage 4)
-    T* Flo_out;           // compensated field: low parts out (stage 4)
-    T dtt;
-    int nsky;
-    int unit_length;
+struct StageStats {
     T gmx, gab;   // signed and absolute maxima of the thread's stage-4 gradients (exact in T)
-    T hvol;       // h^3 / 2
     // (1/2) h^3 sum |V'|^2 over the thread's sites: compensated FP64 for an FP64 instance; an
     // FP32 instance's per-site |V'|^2 is an FP32 value and its thread partial (at most one
     // x-chunk of sites) is summed in FP32, then merged per block in FP64
     KSum kin;
     T kin_t;
-    T* dlt;       // defect correction (null unless defect-corrected)
-    int refresh;  // stage 1 of a refresh step: dlt holds g64 of the field; replace it by g64 - g32
-    CentreStage<T>* cs = nullptr;  // CENTRE: the plane's staged operands
-    int zbase = 0;                 // z of the thread's first site within the tile
-    T d[NL][kPrefetch ? CC : 1];   // the site's correction
-    T dn[NL][kPrefetch ? CC : 1];  // the correction of the thread's site on the next plane, in flight
-    int64_t dn_tag[NL];            // 1 + the site dn belongs to (0: none; value-initialised)
-    // CENTRE: thread 0 copies the update's operands of plane x (every thread calls this
-    // right after the plane barrier, before the stencil arithmetic).
-    __device__ __forceinline__ void plane_begin(int x) {
-        if constexpr (CENTRE) {
-            cs->pending = cs->phase;
-            cs->phase ^= 1u;
-            if (threadIdx.x == 0 && threadIdx.y == 0) {
-                uint32_t n = 0;
-#pragma unroll
-                for (int k = 0; k < kCentreArrays; ++k) n += cs->map[k] != nullptr ? 1u : 0u;
-                mbar_arrive_expect_tx(cs->bar, n * uint32_t(cs->box * sizeof(T)));
-#pragma unroll
-                for (int k = 0; k < kCentreArrays; ++k)
-                    if (cs->map[k]) tma_load_plane(cs->buf + k * cs->box, cs->map[k], cs->z0, cs->y0, x, 0, cs->bar);
-            }
-        }
+    T hvol;       // h^3 / 2
+    __device__ __forceinline__ explicit StageStats(double vol)
+        : gmx(T(-INFINITY)), gab(T(0)), kin{0.0, 0.0}, kin_t(T(0)), hvol(T(0.5 * vol)) {}
+    __device__ __forceinline__ void gradient(T g) {
+        if (g > gmx) gmx = g;  // (a NaN changes neither, as with fmax)
+        if (fabs(g) > gab) gab = fabs(g);
     }
-    // A thread walks its (y, z) column along x.  The correction of the next plane's
-    // site is loaded while this site is computed, so that its global-memory latency
-    // overlaps a whole plane of stencil and point arithmetic.
-    __device__ __forceinline__ void begin_site(int64_t s, int64_t N, int64_t next, int l = 0) {
-        if constexpr (CENTRE) return;  // the correction comes with the staged operands
-        if constexpr (kPrefetch) {
-            if (dlt) {
-                if (dn_tag[l] == s + 1) {
-#pragma unroll
-                    for (int c = 0; c < CC; ++c) d[l][c] = dn[l][c];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < CC; ++c) d[l][c] = __ldcg(dlt + c * N + s);
-                }
-                if (next >= 0) {
-#pragma unroll
-                    for (int c = 0; c < CC; ++c) dn[l][c] = __ldcg(dlt + c * N + next);
-                }
-                dn_tag[l] = next + 1;
-            }
-        }
-    }
-    template <int C>
-    __device__ __forceinline__ void operator()(int64_t s, int64_t N, const T (&)[C], const T (&g32)[C], int l = 0) {
-        static_assert(C == CC, "component count");
-        T g[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) g[c] = g32[c];
-        if constexpr (CENTRE) {
-            static_assert(STAGE == 4, "staged operands are the stage-4 update's");
-            if (!mbar_wait_bounded(cs->bar, cs->pending)) atomicOr(cs->status, 2);
-            // the site within the staged boxes: [c][y - y0][z - z0]
-            const int o = threadIdx.y * 32 + zbase + l;
-            const int bx = cs->box / C;
-            T f0[C], flo[C], v0[C], a1[C], a2[C], a3[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int j = c * bx + o;
-                f0[c] = cs->buf[j];
-                flo[c] = cs->map[1] ? cs->buf[cs->box + j] : T(0);
-                v0[c] = cs->map[2] ? cs->buf[2 * cs->box + j] : T(0);
-                a1[c] = cs->buf[3 * cs->box + j];
-                a2[c] = cs->buf[4 * cs->box + j];
-                a3[c] = cs->buf[5 * cs->box + j];
-                if (cs->map[6]) g[c] += cs->buf[6 * cs->box + j];
-            }
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                gmx = fmax(gmx, g[c]);
-                gab = fmax(gab, fabs(g[c]));
-            }
-            T v2;
-            finalize_vals<T, T, C>(s, N, f0, flo, cs->map[1] != nullptr, v0, a1, a2, a3, g, dtt, nsky, unit_length,
-                                   out0, Flo_out, out1, v2);
-            if constexpr (sizeof(T) == 8)
-                ksum_add(kin, hvol * v2);
-            else
-                kin_t += hvol * v2;
-            return;
-        }
-        if (dlt) {
-            T dd[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                if constexpr (kPrefetch)
-                    dd[c] = d[l][c];
-                else
-                    dd[c] = __ldcg(dlt + c * N + s);
-            }
-            if (STAGE == 1 && refresh) {   // dd = g64(F): the correction becomes g64 - g32(F)
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    __stcg(dlt + c * N + s, dd[c] - g32[c]);
-                    g[c] = dd[c];
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < C; ++c) g[c] = g32[c] + dd[c];
-            }
-        }
-        if (STAGE < 4) {
-#pragma unroll
-            for (int c = 0; c < C; ++c) __stcg(out0 + c * N + s, -dtt * g[c]);
-            return;
-        }
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            gmx = fmax(gmx, g[c]);
-            gab = fmax(gab, fabs(g[c]));
-        }
-        T v2;
-        finalize_site<T, T, C>(s, N, fin_src[0], fin_src[1], fin_src[2], fin_src[3], fin_src[4], fin_src[5], g, dtt,
-                               nsky, unit_length, out0, Flo_out, out1, v2);
+    __device__ __forceinline__ void velocity(T v2) {
         if constexpr (sizeof(T) == 8)
             ksum_add(kin, hvol * v2);
         else
             kin_t += hvol * v2;
     }
-    // the thread's kinetic partial as a compensated FP64 sum
-    __device__ __forceinline__ KSum kinetic() const {
-        if constexpr (sizeof(T) == 8)
-            return kin;
+    __device__ __forceinline__ KSum kinetic() const { return sizeof(T) == 8 ? kin : KSum{double(kin_t), 0.0}; }
+};
+
+// Loads that stay where they are written (a plain load may be moved down to its use, where
+// nothing is left to hide its latency).
+__device__ __forceinline__ double ld_early(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_early(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_early2(const float* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
+// Epilogue of the gradient walk's stages: a thread's pair of FP32 sites, or its FP64 site, at
+// once.  WIDE: Z is a multiple of four (FP32), so the pair is one aligned 8-byte access.
+// EARLY: stage 3's operands are loaded before the point arithmetic (where 168 registers hold
+// both: without mixed derivatives); stage 4's two always are.
+template <typename T, int STAGE, int C, bool WIDE, bool TMA, bool EARLY>
+struct GradEpi {
+    using L = Lanes<T>;
+    using V = typename L::V;
+    static constexpr int NL = L::NL;
+    StageIo<T> io;
+    StageStats<T> st;
+    int nsky, unit_length;
+    T* dlt;       // defect correction (null unless defect-corrected)
+    int refresh;  // stage 1 after the defect refresh: dlt holds g64 of the field; replace it by g64 - g32
+    const T* ahead[4];  // operands that the stage reads at the site only (null: none), and their maps
+    const TmaMap* ahead_map[4];
+    V d[NL > 1 ? C : 1];  // the correction of the site's pair
+    V op[STAGE == 3 ? 5 : STAGE == 4 ? 2 : 1][STAGE > 2 ? C : 1];  // the update's operands at the site
+
+    static __device__ __forceinline__ V get(const T* p, bool own1) {
+        if constexpr (NL == 1)
+            return ld_early(p);
+        else if constexpr (WIDE)
+            return P2(ld_early2(p));
         else
-            return KSum{double(kin_t), 0.0};
+            return P2(ld_early(p), own1 ? ld_early(p + 1) : 0.0f);
+    }
+    static __device__ __forceinline__ void store(T* p, V v, bool own1) {
+        if constexpr (NL == 1) {
+            __stcg(p, v);
+        } else if constexpr (WIDE) {
+            __stcg(reinterpret_cast<float2*>(p), v.v);
+        } else {
+            __stcg(p, v.v.x);
+            if (own1) __stcg(p + 1, v.v.y);
+        }
+    }
+    // The next plane of the operands into L2, so that the loads at the site do not wait for DRAM:
+    // box prefetches by one thread, or 128-byte lines by each row.
+    int z0, y0;
+    __device__ __forceinline__ void prefetch(int64_t s0, int64_t N, int lane, int n, int x) {
+        if constexpr (TMA) {
+            if (threadIdx.x == 0 && threadIdx.y == 0) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (ahead_map[k]) tma_prefetch_plane(ahead_map[k], z0, y0, x, 0);
+            }
+        } else {
+            constexpr int Q = sizeof(T) == 8 ? 3 : 2, PER = 128 / int(sizeof(T));  // lines a row can span
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (ahead[k] == nullptr) continue;
+                for (int i = lane; i < Q * C; i += M_TZ) {
+                    const int c = i / Q, q = i - Q * c;
+                    prefetch_l2(ahead[k] + c * N + s0 + min(PER * q, n - 1));
+                }
+            }
+        }
+    }
+    static constexpr int M_TZ = 32 / NL;
+    __device__ __forceinline__ void begin_site(int64_t s, int64_t N, bool own1) {
+        if constexpr (NL > 1) {
+            if (dlt) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) d[c] = get(dlt + at(c, N, s), own1);
+            }
+        }
+    }
+    // element index of component c at site s (C N < 2^31)
+    static __device__ __forceinline__ uint32_t at(int c, int64_t N, int64_t s) {
+        return uint32_t(c) * uint32_t(N) + uint32_t(s);
+    }
+    __device__ __forceinline__ void load(int64_t s, int64_t N, bool own1) {
+        if constexpr (EARLY || STAGE == 4) operands(s, N, own1);
+    }
+    __device__ __forceinline__ void operands(int64_t s, int64_t N, bool own1) {
+        if constexpr (STAGE == 3) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const uint32_t j = at(c, N, s);
+                op[0][c] = get(io.F + j, own1);
+                op[1][c] = io.Flo ? get(io.Flo + j, own1) : V(0.0f);
+                op[2][c] = io.V ? get(io.V + j, own1) : V(0.0f);
+                op[3][c] = get(io.l1 + j, own1);
+                op[4][c] = io.l2_is_l1 ? op[3][c] : get(io.l2 + j, own1);
+            }
+        }
+        if constexpr (STAGE == 4) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                op[0][c] = get(io.out + at(c, N, s), own1);
+                op[1][c] = get(io.pv + at(c, N, s), own1);
+            }
+        }
+    }
+    __device__ __forceinline__ void operator()(int64_t s, int64_t N, bool own1, const V (&)[C], const V (&g32)[C]) {
+        V g[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) g[c] = g32[c];
+        if constexpr (NL > 1) {
+            if (dlt) {
+                if (STAGE == 1 && refresh) {  // d = g64(F): the correction becomes g64 - g32(F)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        store(dlt + at(c, N, s), d[c] - g32[c], own1);
+                        g[c] = d[c];
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) g[c] = g32[c] + d[c];
+                }
+            }
+        }
+        if constexpr (STAGE < 3) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) store(io.out + at(c, N, s), V(-io.dtt) * g[c], own1);
+        } else if constexpr (STAGE == 3) {
+            if constexpr (!EARLY) operands(s, N, own1);
+            V fo[C], lo[C], pv[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) g[c] = V(-io.dtt) * g[c];  // l3
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                T F[C], Fl[C], v[C], b1[C], b2[C], b3[C], of[C], ol[C], pn[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    F[c] = L::get(op[0][c], l), Fl[c] = L::get(op[1][c], l), v[c] = L::get(op[2][c], l);
+                    b1[c] = L::get(op[3][c], l), b2[c] = L::get(op[4][c], l), b3[c] = L::get(g[c], l);
+                }
+                update_field<T, C>(F, Fl, io.Flo != nullptr, v, b1, b2, b3, io.dtt, nsky, unit_length, of, ol, pn);
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    L::set(fo[c], l, of[c]);
+                    L::set(lo[c], l, ol[c]);
+                    L::set(pv[c], l, pn[c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const uint32_t j = at(c, N, s);
+                store(io.out + j, fo[c], own1);
+                if (io.Flo) store(io.out_lo + j, lo[c], own1);
+                store(io.pv + j, pv[c], own1);
+            }
+        } else {
+            V (&fo)[C] = op[0], (&pv)[C] = op[1];
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                if (l == 1 && !own1) break;
+                T F[C], v[C], gg[C], ov[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    F[c] = L::get(fo[c], l), v[c] = L::get(pv[c], l), gg[c] = L::get(g[c], l);
+                    st.gradient(gg[c]);
+                }
+                st.velocity(update_velocity<T, C>(v, gg, F, io.dtt, nsky, unit_length, ov));
+#pragma unroll
+                for (int c = 0; c < C; ++c) L::set(pv[c], l, ov[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) store(io.pv + at(c, N, s), pv[c], own1);
+        }
     }
 };
 
-// Shared memory of a stage launch: the plane pipeline (sky_march.cuh), plus for a TMA
-// stage 4 the staged update operands when they fit (two FP32 blocks per SM keep
-// 2 x (dynamic + 1.3 KB) within the SM's 228 KB).
-template <class M, typename T>
-constexpr size_t centre_bytes() {
-    return size_t(kCentreArrays) * M::C * M::BY * M::BZ * sizeof(T);
-}
-template <class M, typename T, int STAGE, int MINB, bool TMA>
-constexpr bool stage_centre() {
-    return STAGE == 4 && TMA &&
-           M::template smem_bytes_tma<T>(3) + centre_bytes<M, T>() + 128 <= (MINB >= 2 ? 115000 : kMaxSmemPerBlock);
-}
-template <class M, typename T, int STAGE, int MINB, bool LO, bool TMA>
-constexpr size_t stage_smem_bytes() {
-    constexpr int nsrc = LO ? 2 : (STAGE == 1 ? 1 : (STAGE == 2 ? 2 : 3));
-    return TMA ? M::template smem_bytes_tma<T>(nsrc, LO) + 128 +
-                     (stage_centre<M, T, STAGE, MINB, TMA>() ? centre_bytes<M, T>() : 0)
-               : M::template smem_bytes<T>(nsrc, LO);
-}
-
-// TMA: planes staged by tensor-memory-accelerator box copies (every instance of
-// the launch has its maps encoded; wide rows), and for stage 4 the update's
-// operands too when they fit (stage_centre).  PAIR: z-pair tiles (FP32, TMA,
-// theories without mixed derivatives; sky_march_pair.cuh), 16 x BY threads.
-template <class M, bool PAIR>
-constexpr int stage_threads() {
-    return PAIR ? PairShape<M>::NT : M::NTHREADS;
-}
-
-template <template <typename> class Th, class M, typename T, int STAGE, int MINB, bool LO = false, bool TMA = false,
-          bool PAIR = false>
-__global__ void __launch_bounds__(stage_threads<M, PAIR>(), MINB)
-    k_march_stage(const InstDesc<T>* __restrict__ insts, InstDesc<T>* ctl, const int* __restrict__ tile_inst,
-                  int t_begin, int t_end, int* done) {
-    static_assert(!PAIR || (TMA && sizeof(T) == 4), "z-pair tiles: FP32 with TMA staging");
-    constexpr int NSRC = STAGE == 1 ? (LO ? 2 : 1) : (STAGE == 2 ? 2 : 3);
-    constexpr bool CENTRE = stage_centre<M, T, STAGE, MINB, TMA>();
-    extern __shared__ __align__(128) unsigned char smraw[];
-    // TMA box copies land on 128-byte boundaries: the launch adds 128 bytes of slack
-    // and the ring starts at the first 128-byte boundary of the dynamic segment
-    T* sm = reinterpret_cast<T*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
-    __shared__ KSum shk[M::NTHREADS / 32];  // one entry per warp (kept small: two blocks
-    __shared__ double shm[M::NTHREADS / 32];  // per SM need all but 1 KB of shared memory)
-    __shared__ uint64_t tma_bar[3];
-    TmaTile tt{tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
-    CentreStage<T> cst;
-    if constexpr (TMA) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            mbar_init(&tma_bar[0], 1);
-            mbar_init(&tma_bar[1], 1);
-            if (CENTRE) mbar_init(&tma_bar[2], 1);
-        }
-        __syncthreads();
-    }
-    // the previous launch of the step (its tail writes the control state) must be complete
-    grid_dep_wait();
-    if constexpr (CENTRE) {
-        cst.buf = sm + M::template smem_bytes_tma<T>(3) / sizeof(T);
-        cst.bar = &tma_bar[2];
-        cst.box = M::C * M::BY * M::BZ;
-        cst.phase = 0u;
-        cst.pending = 0u;
-    }
-    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
-        const int ii = __ldg(tile_inst + t);
-        const InstDesc<T>& in = insts[ii];
-        if (!in.active) continue;  // uniform across the block
-        // An arrested step treats the velocity as zero, so its stage-2 input F + (dt/2) V is
-        // the field itself: l2 = l1, and stage 2 has nothing to compute.  Stages 3 and 4 then
-        // read l1 where they read l2.  Not after a defect refresh: that stage 1 formed l1 from
-        // the FP64 gradient, and stage 2's FP32 gradient plus the new correction may differ
-        // from it in the last bit.
-        const bool l2_is_l1 = in.arrested && !in.refresh;
-        if (STAGE == 2 && l2_is_l1) continue;
-        const Params p = in.p;
-        const int parity = in.cur;
-        const int lt = t - in.tile_begin;
-        const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
-        int xa, xe, y0, z0;
-        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
-        const T* F = in.F[parity];
-        const T* V = in.arrested ? nullptr : in.V[parity];
-        const T dtt = T(p.dt), hdt = T(0.5 * p.dt);
-        T* const L2 = l2_is_l1 ? in.L[0] : in.L[1];  // the step's l2
-        const T* const src[3] = {F, LO ? in.Flo[parity] : V, STAGE == 3 ? in.L[0] : L2};
-        const T a = STAGE == 4 ? dtt : hdt;
-        const T b = STAGE == 3 ? T(0.25) * dtt : T(0.5) * dtt;
-        using Epi = EngineEpi<T, STAGE, M::C, CENTRE, PAIR ? 2 : 1>;
-        Epi epi{{F, in.Flo[parity], V, in.L[0], L2, in.L[2]},
-                                STAGE < 4 ? in.L[STAGE - 1] : in.F[parity ^ 1],
-                                STAGE < 4 ? nullptr : in.V[parity ^ 1],
-                                in.Flo[parity ^ 1],
-                                dtt, p.nsky, p.unit_length, T(-INFINITY), T(0), T(0.5 * p.vol), KSum{0.0, 0.0},
-                                T(0), in.Dlt, in.refresh};
-        KSum es{0.0, 0.0}, bs{0.0, 0.0};
-        if constexpr (TMA) {
-            tt.map[0] = &in.tm[kMapF + parity];
-            tt.map[1] = LO ? &in.tm[kMapFlo + parity] : (V != nullptr ? &in.tm[kMapV + parity] : nullptr);
-            tt.map[2] = NSRC > 2 ? &in.tm[kMapL + (STAGE == 3 || l2_is_l1 ? 0 : 1)] : nullptr;
-            tt.status = in.status;
-        }
-        if constexpr (CENTRE) {
-            cst.map[0] = &in.tmc[kMapF + parity];
-            cst.map[1] = in.Flo[parity] != nullptr ? &in.tmc[kMapFlo + parity] : nullptr;
-            cst.map[2] = V != nullptr ? &in.tmc[kMapV + parity] : nullptr;
-            cst.map[3] = &in.tmc[kMapL];
-            cst.map[4] = &in.tmc[kMapL + (l2_is_l1 ? 0 : 1)];
-            cst.map[5] = &in.tmc[kMapL + 2];
-            cst.map[6] = in.Dlt != nullptr ? &in.tmc[kMapDlt] : nullptr;
-            cst.status = in.status;
-            cst.z0 = z0;
-            cst.y0 = y0;
-            epi.cs = &cst;
-        }
-        epi.zbase = PAIR ? 2 * int(threadIdx.x) : int(threadIdx.x);
-        bool ok;
-        if constexpr (PAIR)
-            ok = march_tile_pair<Th, M, NSRC, STAGE == 1, Epi, LO>(sm, p, a, b, xa, xe, y0, z0, epi, es, bs, &tt);
-        else
-            ok = march_tile<Th, M, T, NSRC, STAGE == 1, Epi, LO, T, true, TMA>(sm, p, src, a, b, xa, xe, y0, z0, epi,
-                                                                             es, bs, TMA ? &tt : nullptr);
-        // !ok: a copy did not arrive; the block's error bit is set and its partials stay stale
-        if (ok && STAGE == 1) {
+// A finished tile's partials: stage 1 the baryon number and (FP64) the energy, stage 4 the
+// gradient maxima and the kinetic sum.
+template <typename T, int STAGE>
+__device__ __forceinline__ void tile_partials(const InstDesc<T>& in, int lt, const KSum& es, const KSum& bs,
+                                              const StageStats<T>& st, bool energy, KSum* shk, double* shm) {
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if constexpr (STAGE == 1) {
+        const KSum bb = block_ksum(bs, shk);
+        if (first) in.bpart[lt] = bb;
+        if (energy) {
             const KSum be = block_ksum(es, shk);
-            const KSum bb = block_ksum(bs, shk);
-            if (threadIdx.x == 0 && threadIdx.y == 0) {
-                in.epart[lt] = be;
-                in.bpart[lt] = bb;
-            }
+            if (first) in.epart[lt] = be;
         }
-        if (ok && STAGE == 4) {
-            // a thread without sites keeps -inf, which block_max maps below every gradient
-            const double ga = block_max(fmax(double(epi.gmx), -1.0e300), shm);
-            const double gb = block_max(double(epi.gab), shm);
-            const KSum kk = block_ksum(epi.kinetic(), shk);
-            if (threadIdx.x == 0 && threadIdx.y == 0) {
-                in.gpart[4 * lt] = ga;
-                in.gpart[4 * lt + 1] = gb;
-                in.gpart[4 * lt + 2] = kk.s;
-                in.gpart[4 * lt + 3] = kk.c;
-            }
-        }
-        if (!ok) break;
     }
-    grid_dep_launch();  // the next launch may be scheduled while the last blocks finish
-    // tail (done != null, stages 1 and 4): the last block of the launch to finish runs the
-    // advance (stage 4) or the control (stage 1: reductions, statistics, arrest decision) of
-    // every active instance of the launch, one warp per instance, so a step needs no separate
-    // launches for them.  Each block publishes its partials (fence) before it is counted; the
-    // counter returns to 0 for the next launch.  The tail sits after the tile loop so that its
-    // registers do not add to the stencil loop's.
+    if constexpr (STAGE == 4) {
+        // a thread without sites keeps -inf, which block_max maps below every gradient
+        const double ga = block_max(fmax(double(st.gmx), -1.0e300), shm);
+        const double gb = block_max(double(st.gab), shm);
+        const KSum kk = block_ksum(st.kinetic(), shk);
+        if (first) {
+            in.gpart[4 * lt] = ga;
+            in.gpart[4 * lt + 1] = gb;
+            in.gpart[4 * lt + 2] = kk.s;
+            in.gpart[4 * lt + 3] = kk.c;
+        }
+    }
+}
+
+// Tail of a step's stage-4 and stage-1 launches (total > 0: their blocks together): the last
+// block of the two to finish runs the control of every active instance of the group, one warp
+// per instance, so a step needs no separate launch for it.  Each block publishes its partials
+// (fence) before it is counted; the counter returns to 0 for the next step.  The tail sits after
+// the tile loop so that its registers do not add to the stencil loop's.
+template <typename T, int STAGE>
+__device__ __forceinline__ void stage_tail(InstDesc<T>* ctl, const int* tile_inst, int t_begin, int t_end, int* done,
+                                           int total) {
     if constexpr (STAGE == 1 || STAGE == 4) {
-        if (done != nullptr) {
+        if (total > 0) {
             __shared__ int last_block;
             const int ltid = threadIdx.x + blockDim.x * threadIdx.y;
+            __syncthreads();
             if (ltid == 0) {
                 __threadfence();
-                last_block = atomicAdd(done, 1) == int(gridDim.x) - 1 ? 1 : 0;
+                last_block = atomicAdd(done, 1) == total - 1 ? 1 : 0;
             }
             __syncthreads();
             if (last_block) {
                 __threadfence();
                 const int nw = int(blockDim.x * blockDim.y) >> 5;
                 const int i1 = __ldg(tile_inst + t_end - 1) + 1;
-                for (int i = __ldg(tile_inst + t_begin) + (ltid >> 5); i < i1; i += nw) {
-                    if (!ctl[i].active) continue;
-                    if constexpr (STAGE == 4) {
-                        if ((ltid & 31) == 0) engine_advance_one(ctl[i]);
-                    } else {
-                        engine_control_warp(ctl[i], 0);
-                    }
-                }
+                for (int i = __ldg(tile_inst + t_begin) + (ltid >> 5); i < i1; i += nw)
+                    if (ctl[i].active) engine_control_warp(ctl[i], 0);
                 if (ltid == 0) *done = 0;
             }
         }
     }
 }
 
+template <int STAGE>
+constexpr int stage_nsrc() {
+    return STAGE == 1 ? 1 : (STAGE == 2 ? 2 : 3);
+}
+
+// Shared memory of a walk's stage launch (TMA boxes land on 128-byte boundaries).
+template <template <typename> class Th, class M, typename T, int STAGE, bool TMA>
+constexpr size_t grad_stage_bytes() {
+    return GradPipe<Th, M, T, T, stage_nsrc<STAGE>(), TMA>::bytes + (TMA ? 128 : 0);
+}
+
+template <template <typename> class Th, class M, typename T, int STAGE, int MINB, bool TMA>
+__global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
+    k_grad_stage(const InstDesc<T>* __restrict__ insts, InstDesc<T>* ctl, const int* __restrict__ tile_inst,
+                 int t_begin, int t_end, int half, int* done, int total) {
+    constexpr int NSRC = stage_nsrc<STAGE>();
+    constexpr int NW = GradBlock<M, T>::NT / 32;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    T* sm = reinterpret_cast<T*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    __shared__ KSum shk[NW];
+    __shared__ double shm[NW];
+    __shared__ uint64_t tma_bar;
+    __shared__ MarchCoef<T> coef;
+    TmaTile tt{&tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if constexpr (TMA) {
+        if (first) mbar_init(&tma_bar, 1);
+        __syncthreads();
+    }
+    // the previous launch of the step (its tail writes the control state) must be complete
+    grid_dep_wait();
+    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
+        const InstDesc<T>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;  // uniform across the block
+        if (STAGE == 2 && l2_is_l1(in)) continue;
+        const Params p = in.p;
+        const int lt = t - in.tile_begin;
+        const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
+        int xa, xe, y0, z0;
+        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
+        using Epi = GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>;
+        Epi epi{stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
+                STAGE == 1 && half && refresh_due(in), {nullptr, nullptr, nullptr, nullptr},
+                {nullptr, nullptr, nullptr, nullptr}};
+        epi.z0 = z0;
+        epi.y0 = y0;
+        // what the staged sources have not brought into L2 already
+        auto ahead = [&](int k, const T* a, int map) {
+            epi.ahead[k] = a;
+            epi.ahead_map[k] = a != nullptr ? &in.tm[map] : nullptr;
+        };
+        if constexpr (STAGE == 3) {
+            ahead(0, epi.io.Flo, kMapFlo + in.cur);
+            ahead(1, epi.io.l2_is_l1 ? nullptr : epi.io.l2, kMapL + 1);
+        }
+        if constexpr (STAGE == 4) {
+            ahead(0, epi.io.out, kMapF + (in.cur ^ 1));
+            ahead(1, epi.io.pv, kMapV + (in.cur ^ 1));
+        }
+        ahead(3, in.Dlt, kMapDlt);
+        if constexpr (TMA) stage_maps<T, STAGE>(in, epi.io, half, tt);
+        __syncthreads();  // the previous tile's readers of coef are done
+        if (first) coef = in.coef;
+        __syncthreads();
+        KSum es{0.0, 0.0}, bs{0.0, 0.0};
+        const bool ok = grad_tile<Th, M, T, NSRC, STAGE == 1, Epi, T, TMA>(sm, p, coef, epi.io.src, epi.io.a, epi.io.b,
+                                                                           xa, xe, y0, z0, epi, es, bs, &tt);
+        if (!ok) break;  // a copy did not arrive; the error bit is set and the tile's partials stay stale
+        tile_partials<T, STAGE>(in, lt, es, bs, epi.st, sizeof(T) == 8, shk, shm);
+    }
+    grid_dep_launch();  // the next launch may be scheduled while the last blocks finish
+    stage_tail<T, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
+}
+
 // ---------------------------------------------------------------------------
-// Defect refresh: for every defect-corrected FP32 instance whose refresh flag is
-// set, the FP64 gradient of its compensated field hi + lo (staged from the FP32
+// Energy of FP32 instances: the FP64 density of the field (high plus low parts of a
+// compensated one), evaluated in its own walk.  Each value is converted once as it enters an
+// FP64 ring.  (Inside stage 1 the 60 tap differences of a five-component site each needed an
+// exact FP32 difference and two conversions: half of that stage's instructions.)
+// ---------------------------------------------------------------------------
+constexpr int kEnergyRows = 16;
+
+template <template <typename> class Th>
+struct EnergyOp {
+    const Params& p;
+    KSum sum;
+    __device__ __forceinline__ void operator()(int64_t, const double (&phi)[Th<double>::C],
+                                               const double (&D)[3][Th<double>::C]) {
+        ksum_add(sum, Th<double>::energy(phi, D, p));
+    }
+};
+
+template <template <typename> class Th, class M, bool TMA>
+__global__ void __launch_bounds__(M::NTHREADS)
+    k_energy(const InstDesc<float>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end,
+             int half) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    double* sm = reinterpret_cast<double*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    __shared__ KSum shk[M::NTHREADS / 32];
+    __shared__ uint64_t tma_bar;
+    TmaTile tt{&tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
+    if constexpr (TMA) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(&tma_bar, 1);
+        __syncthreads();
+    }
+    grid_dep_wait();
+    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
+        const InstDesc<float>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;
+        const Params p = in.p;
+        const int lt = t - in.e_tile_begin, cur = in.cur ^ half;
+        const MarchGrid mg{in.e_nz, in.e_ny, in.e_nx, in.e_xc};
+        int xa, xe, y0, z0;
+        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
+        const float* const src[3] = {in.F[cur], in.Flo[cur], nullptr};
+        const double r1[3] = {in.r1d[0], in.r1d[1], in.r1d[2]};
+        if constexpr (TMA) {
+            tt.map[0] = &in.tme[kMapF + cur];
+            tt.map[1] = in.Flo[cur] != nullptr ? &in.tme[kMapFlo + cur] : nullptr;
+            tt.status = in.status;
+        }
+        EnergyOp<Th> op{p, KSum{0.0, 0.0}};
+        if (!dens_tile<M, float, 2, TMA>(sm, p, r1, src, xa, xe, y0, z0, op, &tt)) break;
+        const KSum e = block_ksum(op.sum, shk);
+        if (threadIdx.x == 0 && threadIdx.y == 0) in.epart[lt] = e;
+    }
+    grid_dep_launch();
+}
+
+// ---------------------------------------------------------------------------
+// Rho's stages (13 components): the marching tile, one site per thread.
+// ---------------------------------------------------------------------------
+template <typename T, int STAGE, int CC>
+struct EngineEpi {
+    StageIo<T> io;
+    StageStats<T> st;
+    int nsky, unit_length;
+    T* dlt;
+    int refresh;
+    template <int C>
+    __device__ __forceinline__ void operator()(int64_t s, int64_t N, const T (&)[C], const T (&g32)[C]) {
+        static_assert(C == CC, "component count");
+        T g[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) g[c] = g32[c];
+        if (dlt) {
+            if (STAGE == 1 && refresh) {  // dlt = g64(F): the correction becomes g64 - g32(F)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    g[c] = __ldcg(dlt + c * N + s);
+                    __stcg(dlt + c * N + s, g[c] - g32[c]);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < C; ++c) g[c] = g32[c] + __ldcg(dlt + c * N + s);
+            }
+        }
+        if constexpr (STAGE < 3) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) __stcg(io.out + c * N + s, -io.dtt * g[c]);
+        } else if constexpr (STAGE == 3) {
+            T f0[C], fl[C], v0[C], a1[C], a2[C], fo[C], lo[C], pv[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int64_t j = c * N + s;
+                f0[c] = __ldcg(io.F + j);
+                fl[c] = io.Flo ? __ldcg(io.Flo + j) : T(0);
+                v0[c] = io.V ? __ldcg(io.V + j) : T(0);
+                a1[c] = __ldcg(io.l1 + j);
+                a2[c] = io.l2_is_l1 ? a1[c] : __ldcg(io.l2 + j);
+                g[c] = -io.dtt * g[c];  // l3
+            }
+            update_field<T, C>(f0, fl, io.Flo != nullptr, v0, a1, a2, g, io.dtt, nsky, unit_length, fo, lo, pv);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int64_t j = c * N + s;
+                __stcg(io.out + j, fo[c]);
+                if (io.Flo) __stcg(io.out_lo + j, lo[c]);
+                __stcg(io.pv + j, pv[c]);
+            }
+        } else {
+            T fo[C], pv[C], vv[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                st.gradient(g[c]);
+                fo[c] = __ldcg(io.out + c * N + s);
+                pv[c] = __ldcg(io.pv + c * N + s);
+            }
+            st.velocity(update_velocity<T, C>(pv, g, fo, io.dtt, nsky, unit_length, vv));
+#pragma unroll
+            for (int c = 0; c < C; ++c) __stcg(io.pv + c * N + s, vv[c]);
+        }
+    }
+};
+
+template <class M, typename T, int STAGE, bool TMA>
+constexpr size_t march_stage_bytes() {
+    constexpr int nsrc = stage_nsrc<STAGE>();
+    return TMA ? M::template smem_bytes_tma<T>(nsrc) + 128 : M::template smem_bytes<T>(nsrc);
+}
+
+template <template <typename> class Th, class M, typename T, int STAGE, bool TMA>
+__global__ void __launch_bounds__(M::NTHREADS)
+    k_march_stage(const InstDesc<T>* __restrict__ insts, InstDesc<T>* ctl, const int* __restrict__ tile_inst,
+                  int t_begin, int t_end, int half, int* done, int total) {
+    constexpr int NSRC = stage_nsrc<STAGE>();
+    extern __shared__ __align__(128) unsigned char smraw[];
+    // TMA box copies land on 128-byte boundaries: the launch adds 128 bytes of slack
+    // and the ring starts at the first 128-byte boundary of the dynamic segment
+    T* sm = reinterpret_cast<T*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    __shared__ KSum shk[M::NTHREADS / 32];
+    __shared__ double shm[M::NTHREADS / 32];
+    __shared__ uint64_t tma_bar[2];
+    TmaTile tt{tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
+    if constexpr (TMA) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) {
+            mbar_init(&tma_bar[0], 1);
+            mbar_init(&tma_bar[1], 1);
+        }
+        __syncthreads();
+    }
+    grid_dep_wait();
+    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
+        const InstDesc<T>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;  // uniform across the block
+        if (STAGE == 2 && l2_is_l1(in)) continue;
+        const Params p = in.p;
+        const int lt = t - in.tile_begin;
+        const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
+        int xa, xe, y0, z0;
+        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
+        using Epi = EngineEpi<T, STAGE, M::C>;
+        Epi epi{stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
+                STAGE == 1 && half && refresh_due(in)};
+        if constexpr (TMA) stage_maps<T, STAGE>(in, epi.io, half, tt);
+        KSum es{0.0, 0.0}, bs{0.0, 0.0};
+        const bool ok = march_tile<Th, M, T, NSRC, STAGE == 1, Epi, false, T, true, TMA>(
+            sm, p, epi.io.src, epi.io.a, epi.io.b, xa, xe, y0, z0, epi, es, bs, TMA ? &tt : nullptr);
+        if (!ok) break;  // a copy did not arrive; the error bit is set and the tile's partials stay stale
+        tile_partials<T, STAGE>(in, lt, es, bs, epi.st, true, shk, shm);
+    }
+    grid_dep_launch();  // the next launch may be scheduled while the last blocks finish
+    stage_tail<T, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
+}
+
+// ---------------------------------------------------------------------------
+// Defect refresh: for every defect-corrected FP32 instance whose refresh is due, the FP64
+// gradient of the step's new compensated field hi + lo (staged from the FP32
 // arrays into an FP64 ring) is written to Dlt; the following stage 1 turns it
 // into the correction g64 - g32.
 // ---------------------------------------------------------------------------
@@ -663,6 +848,11 @@ struct DefectEpi {
     __device__ __forceinline__ void operator()(int64_t s, int64_t N, const double (&)[C], const double (&g)[C]) {
 #pragma unroll
         for (int c = 0; c < C; ++c) dlt[c * N + s] = float(g[c]);
+    }
+    template <int C>
+    __device__ __forceinline__ void operator()(int64_t s, int64_t N, bool, const double (&phi)[C],
+                                               const double (&g)[C]) {
+        (*this)(s, N, phi, g);
     }
 };
 
@@ -678,18 +868,25 @@ __global__ void __launch_bounds__(M::NTHREADS, 1)
     for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
         const int ii = __ldg(tile_inst + t);
         const InstDesc<float>& in = insts[ii];
-        if (!in.active || !in.refresh || in.Dlt == nullptr) continue;  // uniform across the block
+        if (!in.active || !refresh_due(in)) continue;  // uniform across the block
         const Params p = in.p;
         const int lt = t - in.tile_begin;
         const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
         int xa, xe, y0, z0;
         march_origin(mg, lt, TBY, xa, xe, y0, z0, p.X);
-        const float* const src[3] = {in.F[in.cur], in.Flo[in.cur], nullptr};
+        const float* const src[3] = {in.F[in.cur ^ 1], in.Flo[in.cur ^ 1], nullptr};  // the new field
         DefectEpi epi{in.Dlt};
         KSum es{0.0, 0.0}, bs{0.0, 0.0};
-        for (int sy = 0; sy < TBY && y0 + sy < p.Y; sy += M::BY)
-            march_tile<Th, M, double, 2, false, DefectEpi, false, float>(sm, p, src, 1.0, 0.0, xa, xe, y0 + sy, z0,
-                                                                         epi, es, bs);
+        [[maybe_unused]] MarchCoef<double> k;
+        if constexpr (M::C <= 5) k.init(p);
+        for (int sy = 0; sy < TBY && y0 + sy < p.Y; sy += M::BY) {
+            if constexpr (M::C <= 5)
+                grad_tile<Th, M, double, 2, 0, DefectEpi, float>(sm, p, k, src, 1.0, 0.0, xa, xe, y0 + sy, z0, epi, es,
+                                                                 bs);
+            else
+                march_tile<Th, M, double, 2, false, DefectEpi, false, float>(sm, p, src, 1.0, 0.0, xa, xe, y0 + sy,
+                                                                             z0, epi, es, bs);
+        }
     }
 }
 
@@ -701,12 +898,14 @@ __global__ void __launch_bounds__(M::NTHREADS, 1)
 // block writes its two compensated partial sums to parts[4 * block].
 // ---------------------------------------------------------------------------
 template <template <typename> class Th, typename S>
-struct AuditEpi {
+struct AuditOp {
+    const Params& p;
     const S* V;  // null: the velocity is zero (arrested)
     int64_t N;
-    double hvol;  // h^3 / 2
-    KSum kin;
-    __device__ __forceinline__ void density(int64_t s, double) {
+    KSum pot, kin;
+    __device__ __forceinline__ void operator()(int64_t s, const double (&phi)[Th<double>::C],
+                                               const double (&D)[3][Th<double>::C]) {
+        ksum_add(pot, Dynamics<Th>::potential(phi, D, p));
         if (!V) return;
         double k = 0.0;
 #pragma unroll
@@ -714,7 +913,7 @@ struct AuditEpi {
             const double v = double(V[c * N + s]);
             k += Dynamics<Th>::kinetic_sign(c) * v * v;
         }
-        ksum_add(kin, hvol * k);
+        ksum_add(kin, 0.5 * p.vol * k);
     }
 };
 
@@ -728,16 +927,15 @@ __global__ void __launch_bounds__(M::NTHREADS, 1)
     const Params p = d->p;
     const int cur = d->cur;
     const S* const src[3] = {d->F[cur], NSRC == 2 ? d->Flo[cur] : nullptr, nullptr};
-    AuditEpi<Th, S> epi{d->arrested ? nullptr : d->V[cur], n_sites(p), 0.5 * p.vol, KSum{0.0, 0.0}};
-    KSum es{0.0, 0.0}, unused{0.0, 0.0};
+    const double r1[3] = {d->r1d[0], d->r1d[1], d->r1d[2]};
+    AuditOp<Th, S> op{p, d->arrested ? nullptr : d->V[cur], n_sites(p), KSum{0.0, 0.0}, KSum{0.0, 0.0}};
     for (int t = blockIdx.x; t < mg.count(); t += gridDim.x) {
         int xa, xe, y0, z0;
         march_origin(mg, t, M::BY, xa, xe, y0, z0, p.X);
-        march_tile<Th, M, double, NSRC, 4, AuditEpi<Th, S>, false, S, false>(sm, p, src, 1.0, 0.0, xa, xe, y0, z0,
-                                                                             epi, es, unused);
+        dens_tile<M, S, NSRC, false>(sm, p, r1, src, xa, xe, y0, z0, op);
     }
-    const KSum pe = block_ksum(es, shk);
-    const KSum pk = block_ksum(epi.kin, shk);
+    const KSum pe = block_ksum(op.pot, shk);
+    const KSum pk = block_ksum(op.kin, shk);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         parts[4 * blockIdx.x] = pe.s;
         parts[4 * blockIdx.x + 1] = pe.c;

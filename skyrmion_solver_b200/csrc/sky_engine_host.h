@@ -1,0 +1,82 @@
+// Host structures of the resident engine, and what each theory's translation unit provides.
+#pragma once
+
+#include <vector>
+
+#include "sky_common.cuh"
+#include "sky_host.h"
+
+namespace sky {
+
+struct StepStats;
+
+struct HostInst {
+    int id = -1;
+    int theory = 0;
+    int prec = 0;  // storage: 0 = FP32 storage/arithmetic, 1 = FP64
+    int comp = 0;    // FP32 storage with a compensated (hi + lo) field
+    int defect = 0;  // ... and a defect-corrected gradient (precision 3)
+    int defect_period = kDefectRefresh;  // steps between refreshes of the correction
+    Params p{};
+    int64_t N = 0;
+    int C = 0;
+    void* F[2] = {nullptr, nullptr};
+    void* Flo[2] = {nullptr, nullptr};
+    void* Dlt = nullptr;
+    void* V[2] = {nullptr, nullptr};
+    void* L[3] = {nullptr, nullptr, nullptr};
+    KSum* epart = nullptr;
+    KSum* bpart = nullptr;
+    double* gpart = nullptr;
+    StepStats* stats = nullptr;
+    int ntiles = 0, tnz = 0, tny = 0, tnx = 0;
+    int entiles = 0, etnz = 0, etny = 0, etnx = 0, exc = 0;  // energy tiles (entiles = ntiles: stage 1 sums it)
+    int xc = 0;          // x-chunk of the marching kernels
+    int xc_request = 0;  // x-chunk asked for by the caller (0: automatic)
+    bool tma = false;    // the stage kernels stage this instance with TMA box copies
+    bool pair = false;   // the caller's z-pair flag (option 3): every FP32 walk computes z-pairs
+    int group_slot = -1;
+    int64_t steps = 0;  // host mirror of the device step counter
+    bool active = true;
+    size_t bytes = 0;
+};
+
+struct Group {
+    int theory = 0, prec = 0;
+    std::vector<int> members;  // instance ids in slot order
+    void* d_desc = nullptr;    // InstDesc<S>[cap]
+    int* d_tile_inst = nullptr;   // stage tiles, then energy tiles (FP32 walks)
+    int* d_done = nullptr;     // blocks of the current step's stage-1 and stage-4 launches finished (0 between steps)
+    int desc_cap = 0, tile_cap = 0;
+    int ntiles = 0, entiles = 0;
+    bool all_wide = true;   // every member can use the wide-row (16-byte staged) kernels
+    bool any_defect = false;  // holds a defect-corrected instance (launch the defect refresh)
+    bool all_tma = false;     // every member has TMA plane maps (launch the TMA stage kernels)
+};
+
+// Shapes and launches of one theory (sky_engine_launch.cuh, instantiated per theory in
+// sky_engine_<theory>.cu).
+struct TileShapeInfo {
+    int rows, blocks, hz;  // rows of a stage tile; resident blocks per SM its x-chunk is chosen for; staged columns
+};
+// Tiles [t_begin, t_end) of a stage or energy launch.  in_step: part of a step (the work on the
+// new field; stages 1 and 4 share the control tail); 0: on the current field alone (admission,
+// precision change).
+struct StageArgs {
+    int t_begin, t_end, in_step;
+};
+struct TheoryOps {
+    TileShapeInfo (*shape)(int prec);
+    int (*setup)(int prec);
+    int (*stage)(int prec, int stage, const Group& g, const StageArgs& a, cudaStream_t st);
+    int (*energy)(const Group& g, const StageArgs& a, cudaStream_t st);  // FP32 groups
+    int (*defect)(const Group& g, cudaStream_t st);
+    int (*audit)(const Group& g, const HostInst& h, cudaStream_t st, double* out2);
+};
+const TheoryOps& theory_ops(int theory);
+extern const TheoryOps kNuclearOps, kOmegaOps, kCoulombOps, kRhoOps, kBergerOps, kLightlyBoundOps;
+
+// FP32 instances of theories with at most five components have their own energy walk.
+inline bool energy_walk(int theory, int prec) { return prec == 0 && theory_components(theory) <= 5; }
+
+}  // namespace sky

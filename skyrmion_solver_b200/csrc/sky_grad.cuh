@@ -52,13 +52,28 @@ struct MarchCoef {
     }
 };
 
-// Optional hook of a gradient walk's epilogue: prefetch(s, N, lane, n) is called by every
-// thread of a row with the row's first site on the next plane and its number of sites.
+// Optional hook of a gradient walk's epilogue: prefetch(s, N, lane, n, x) is called by every
+// thread of a row with the row's first site on the next plane, its number of sites and that plane.
 template <class E, class = void>
 struct HasPrefetch : std::false_type {};
 template <class E>
-struct HasPrefetch<E, std::void_t<decltype(std::declval<E&>().prefetch(int64_t(0), int64_t(0), 0, 0))>>
+struct HasPrefetch<E, std::void_t<decltype(std::declval<E&>().prefetch(int64_t(0), int64_t(0), 0, 0, 0))>>
     : std::true_type {};
+// load(s, N, own1): at the site, between the plane's pure derivatives and its point arithmetic
+// (before the barrier in between, where there is one): operands loaded here arrive while the
+// point arithmetic runs.
+template <class E, class = void>
+struct HasLoad : std::false_type {};
+template <class E>
+struct HasLoad<E, std::void_t<decltype(std::declval<E&>().load(int64_t(0), int64_t(0), true))>> : std::true_type {};
+
+// begin_site(s, N, own1): at the site, before its plane is computed.
+template <class E, class = void>
+struct HasGradBegin : std::false_type {};
+template <class E>
+struct HasGradBegin<E, std::void_t<decltype(std::declval<E&>().begin_site(int64_t(0), int64_t(0), true))>>
+    : std::true_type {};
+
 __device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
 // Lanes of a thread: one FP64 site, or a packed pair of FP32 sites (z, z + 1).
@@ -74,6 +89,7 @@ struct Lanes {
     }
     static __device__ __forceinline__ V mask(V v, bool m0, bool) { return m0 ? v : V(0); }
     static __device__ __forceinline__ T get(V v, int) { return v; }
+    static __device__ __forceinline__ void set(V& v, int, T a) { v = a; }
 };
 template <>
 struct Lanes<float> {
@@ -90,6 +106,7 @@ struct Lanes<float> {
     }
     static __device__ __forceinline__ V mask(V v, bool m0, bool m1) { return p2_mask(v, m0, m1); }
     static __device__ __forceinline__ float get(V v, int l) { return l ? v.v.y : v.v.x; }
+    static __device__ __forceinline__ void set(V& v, int l, float a) { (l ? v.v.y : v.v.x) = a; }
 };
 
 // The stencils' integer tap sums (MarchCoef).
@@ -124,26 +141,27 @@ __device__ __forceinline__ void axpy16(double2& v, double a, const double2& u) {
 // ---------------------------------------------------------------------------
 // The plane pipeline of a walk: a ring of six haloed planes and its copies.
 //
-// S = T: the first source is copied straight into the ring.  Further sources pass through
-// staging slots and are added in (X = F + a V + b L): with TMA through one slot, one after the
-// other, which costs a second wait per plane and leaves room for two 16-row FP32 blocks per
-// SM; with cp.async through a slot each, added by the thread that copied the element.
+// S = T: the first source is copied straight into the ring.  Further sources pass through a
+// staging slot each and are added in (X = F + a V + b L).  The ring has six slots, so that a
+// plane travels while the whole previous one is computed.  The late ring (LATE, three sources by
+// TMA) has five, and a plane travels during the point arithmetic only: for tiles of which 7 slots
+// leave two blocks on an SM and 8 do not.
 // S != T (float arrays, FP64 ring): every source is staged and converted; X = F + a V.
 // Planes outside the lattice and points outside it in y and z read as zero.
 // ---------------------------------------------------------------------------
-template <class M, typename T, typename S, int NSRC, bool TMA, int NT>
+template <class M, typename T, typename S, int NSRC, bool TMA, int NT, bool LATE_ = false>
 struct PlanePipe {
     static constexpr bool SAME = std::is_same<S, T>::value;
     static constexpr bool DIRECT = SAME && NSRC == 1;
-    // the second extra source is copied after the first one has been added
-    static constexpr bool TWO = TMA && SAME && NSRC == 3;
-    static constexpr int R = 6;
+    static constexpr bool LATE = LATE_;
+    static constexpr int R = LATE ? 5 : 6;
     static constexpr int SLOT = M::SLOT;
-    static constexpr int NSTG = SAME ? (TMA ? (NSRC > 1 ? 1 : 0) : NSRC - 1) : NSRC;
+    static constexpr int NSTG = SAME ? NSRC - 1 : NSRC;
     static constexpr size_t ring_bytes = size_t(R) * SLOT * sizeof(T);
     static constexpr size_t stage_bytes = size_t(NSTG) * SLOT * sizeof(S);
     static constexpr size_t bytes = ring_bytes + stage_bytes;
     static_assert(!TMA || M::WIDE, "TMA staging: wide rows");
+    static_assert(!LATE || (TMA && SAME && NSRC == 3), "the late ring is the staged TMA pipeline's");
     static_assert(SAME || NSRC <= 2, "converted sources: a field and its low parts");
 
     T* ring;
@@ -153,20 +171,20 @@ struct PlanePipe {
     TmaTile* tma;
     int tid, y0, z0, X;
     int64_t YZ;
-    int ns;       // extra sources present
-    int e[2];     // which they are
+    int ns;       // extra sources present (TMA: V may be absent, then L takes the first staging slot)
+    int e0;       // the first of them
     using PO = typename std::conditional<M::WIDE, PlaneChunks<M, S, NT>, PlaneOffsets<M, NT>>::type;
     PO po;
 
     __device__ __forceinline__ PlanePipe(T* sm, const Params& p, const S* const (&src_)[3], T a, T b, int tid_, int y0_,
                                          int z0_, TmaTile* tma_)
         : ring(sm), stage(reinterpret_cast<S*>(reinterpret_cast<char*>(sm) + ring_bytes)), src(src_), w{T(1), a, b},
-          tma(tma_), tid(tid_), y0(y0_), z0(z0_), X(p.X), YZ((int64_t)p.Y * p.Z), ns(0), e{1, 2} {
+          tma(tma_), tid(tid_), y0(y0_), z0(z0_), X(p.X), YZ((int64_t)p.Y * p.Z), ns(0), e0(1) {
         if constexpr (!TMA) po.init(p, n_sites(p), y0, z0, tid);
 #pragma unroll
         for (int s = 1; s < NSRC; ++s)
             if (TMA ? tma->map[s] != nullptr : src[s] != nullptr) {
-                if (ns == 0 && s == 2) e[0] = 2;
+                if (ns == 0) e0 = s;
                 ++ns;
             }
     }
@@ -175,15 +193,26 @@ struct PlanePipe {
     }
     static constexpr uint32_t kBox = uint32_t(SLOT * sizeof(S));
 
-    // Start the copies of plane q into `slot` (TWO: without the second extra source).
+    // Plane q of every source into L2.
+    __device__ __forceinline__ void ahead(int q) {
+        if constexpr (TMA) {
+            if (q >= X) return;
+            tma_prefetch_plane(tma->map[0], z0 - M::ZOFF, y0 - 2, q, 0);
+            if (NSRC > 1 && ns > 0) tma_prefetch_plane(tma->map[e0], z0 - M::ZOFF, y0 - 2, q, 0);
+            if (NSRC > 2 && ns > 1) tma_prefetch_plane(tma->map[2], z0 - M::ZOFF, y0 - 2, q, 0);
+        }
+    }
+    // Start the copies of plane q into `slot`.
     __device__ __forceinline__ void issue(int q, int slot) {
         if constexpr (TMA) {
             if (tid == 0) {
                 fence_proxy_async_smem();
-                const bool one = NSRC > 1 && ns > 0;
-                mbar_arrive_expect_tx(tma->bar, (one ? 2u : 1u) * kBox);
+                mbar_arrive_expect_tx(tma->bar, uint32_t(1 + (NSRC > 1 ? ns : 0)) * kBox);
                 box(SAME ? (void*)(ring + slot * SLOT) : (void*)stage, 0, q);
-                if (one) box(SAME ? stage : stage + SLOT, e[0], q);
+                S* d = SAME ? stage : stage + SLOT;
+                if (NSRC > 1 && ns > 0) box(d, e0, q);
+                if (NSRC > 2 && ns > 1) box(d + SLOT, 2, q);
+                ahead(q + 2);
             }
         } else {
             const bool xok = q >= 0 && q < X;
@@ -224,18 +253,35 @@ struct PlanePipe {
             }
         }
     }
-    // ring[slot] = buf0 + w1 buf1, converted (S != T)
+    // ring[slot] = buf0 + w1 buf1, converted (S != T): pairs of consecutive values per lane, or,
+    // with cp.async, the chunks the thread copied itself
     __device__ __forceinline__ void convert(int slot) {
         if constexpr (!SAME) {
-            T* d = ring + slot * SLOT;
-            constexpr int VW = M::WIDE ? 16 / int(sizeof(S)) : 1;  // the chunks this thread copied itself
-#pragma unroll 2
-            for (int i = tid; i < SLOT / VW; i += NT) {
+            static_assert(sizeof(S) == 4 && sizeof(T) == 8 && SLOT % 4 == 0, "FP32 sources of an FP64 ring");
+            double* d = reinterpret_cast<double*>(ring + slot * SLOT);
+            const float* u = reinterpret_cast<const float*>(stage);
+            const bool two = NSRC > 1 && ns > 0;
+            const double wt = w[1];
+            if constexpr (TMA) {
+                for (int i = tid; i < SLOT / 2; i += NT) {
+                    const float2 a = reinterpret_cast<const float2*>(u)[i];
+                    double2 v = make_double2(a.x, a.y);
+                    if (two) {
+                        const float2 b = reinterpret_cast<const float2*>(u + SLOT)[i];
+                        v.x += wt * double(b.x);
+                        v.y += wt * double(b.y);
+                    }
+                    reinterpret_cast<double2*>(d)[i] = v;
+                }
+            } else {
+                constexpr int VW = M::WIDE ? 4 : 1;
+                for (int i = tid; i < SLOT / VW; i += NT) {
 #pragma unroll
-                for (int j = 0; j < VW; ++j) {
-                    T v = T(stage[i * VW + j]);
-                    if (NSRC > 1 && ns > 0) v += w[1] * T(stage[SLOT + i * VW + j]);
-                    d[i * VW + j] = v;
+                    for (int j = 0; j < VW; ++j) {
+                        double v = double(u[i * VW + j]);
+                        if (two) v += wt * double(u[SLOT + i * VW + j]);
+                        d[i * VW + j] = v;
+                    }
                 }
             }
         }
@@ -257,30 +303,11 @@ struct PlanePipe {
             convert(slot);
         } else if constexpr (NSRC > 1) {
             if constexpr (TMA) {
-                if (ns > 0) add(slot, stage, e[0] == 1 ? w[1] : w[2]);
+                if (ns > 0) add(slot, stage, e0 == 1 ? w[1] : w[2]);
+                if (NSRC > 2 && ns > 1) add(slot, stage + SLOT, w[2]);
             } else {
                 if (src[1] != nullptr) add(slot, stage, w[1]);
                 if (NSRC > 2 && src[2] != nullptr) add(slot, stage + SLOT, w[2]);
-            }
-        }
-        return ok;
-    }
-    // TWO: the second extra source of plane q, once every thread has added the first.
-    __device__ __forceinline__ void issue2(int q) {
-        if constexpr (TWO) {
-            if (tid == 0 && ns > 1) {
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(tma->bar, kBox);
-                box(stage, 2, q);
-            }
-        }
-    }
-    __device__ __forceinline__ bool land2(int slot) {
-        bool ok = true;
-        if constexpr (TWO) {
-            if (ns > 1) {
-                ok = wait();
-                add(slot, stage, w[2]);
             }
         }
         return ok;
@@ -305,17 +332,21 @@ struct PlanePipe {
         }
     }
     // Planes q0 .. q0 + 4 into slots 0 .. 4, complete and visible to the block.  `spare` is
-    // shared memory of at least `nspare` slots that the walk does not use yet: with slot 5 and
-    // the staging slot it lets several staged planes travel at once.
+    // shared memory of at least `nspare` slots that the walk does not use yet, so that several
+    // staged planes travel at once.
     __device__ __forceinline__ bool prologue(int q0, S* spare, int nspare) {
         meet(true);  // the previous tile's readers are done
         bool ok = true;
         if constexpr (TMA && SAME) {
-            const int nb = DIRECT ? 0 : 2 + nspare;
+            // staged planes travel through the staging slots, a sixth ring slot and the spare ones
+            constexpr int own = NSTG + (R - 5);
+            const int nb = DIRECT ? 0 : own + nspare;
             const int items = NSRC > 1 ? 5 * ns : 0;
             auto buf = [&](int k) -> S* {
-                return k == 0 ? stage : k == 1 ? reinterpret_cast<S*>(ring + 5 * SLOT) : spare + (k - 2) * SLOT;
+                return k < NSTG ? stage + k * SLOT
+                                : k < own ? reinterpret_cast<S*>(ring + 5 * SLOT) : spare + (k - own) * SLOT;
             };
+            auto which = [&](int i) { return ns == 1 ? e0 : 1 + i % 2; };
             for (int it = 0; it == 0 || it < items;) {
                 const int n = min(nb, items - it);
                 if (tid == 0) {
@@ -323,10 +354,10 @@ struct PlanePipe {
                     mbar_arrive_expect_tx(tma->bar, uint32_t((it == 0 ? 5 : 0) + n) * kBox);
                     if (it == 0)
                         for (int j = 0; j < 5; ++j) box(ring + j * SLOT, 0, q0 + j);
-                    for (int k = 0; k < n; ++k) box(buf(k), e[(it + k) % ns], q0 + (it + k) / ns);
+                    for (int k = 0; k < n; ++k) box(buf(k), which(it + k), q0 + (it + k) / ns);
                 }
                 ok = wait();
-                for (int k = 0; k < n; ++k) add((it + k) / ns, buf(k), e[(it + k) % ns] == 1 ? w[1] : w[2]);
+                for (int k = 0; k < n; ++k) add((it + k) / ns, buf(k), which(it + k) == 1 ? w[1] : w[2]);
                 it += n > 0 ? n : 1;
                 if (meet(ok)) {
                     give_up();
@@ -357,16 +388,20 @@ struct PlanePipe {
 // (8-row tiles with the register queues of the earlier form: 154, 119, 200 and 173 us).
 template <template <typename> class Th>
 constexpr int grad_rows64() {
-    return Th<double>::kId == SKY_THEORY_COULOMB || Th<double>::kId == SKY_THEORY_BERGER ? 12 : 16;
+    return 12;
 }
 
 // Shared memory of a gradient walk.
 template <template <typename> class Th, class M, typename T, typename S, int NSRC, bool TMA>
 struct GradPipe {
-    using Pipe = PlanePipe<M, T, S, NSRC, TMA, GradBlock<M, T>::NT>;
     static constexpr bool GH = Th<T>::kMixed;
     static constexpr int CM = 4;  // components with mixed derivatives: the pion field
     static constexpr size_t gh_bytes = GH ? size_t(CM) * (M::PLANE + M::HY * M::BZ) * sizeof(T) : 0;
+    // the late ring where the full one would leave one FP32 block on an SM (228 KB, less 1 KB and
+    // the static variables of each block)
+    static constexpr bool LATE = TMA && NSRC == 3 && sizeof(T) == 4 && sizeof(S) == 4 &&
+                                 size_t(8) * M::SLOT * sizeof(T) + gh_bytes > 114000;
+    using Pipe = PlanePipe<M, T, S, NSRC, TMA, GradBlock<M, T>::NT, LATE>;
     static constexpr size_t bytes = Pipe::bytes + gh_bytes;
     // staging slots that G and H can stand in for during the prologue
     static constexpr int nspare = int(gh_bytes / (size_t(M::SLOT) * sizeof(S)));
@@ -390,8 +425,8 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
     constexpr int NL = L::NL;
     constexpr int C = M::C, R = Pipe::R, SLOT = M::SLOT, PLANE = M::PLANE, HZ = M::HZ;
     constexpr bool GH = P::GH;
-    // two barriers per plane: between writing and reading G and H, and for a second staged source
-    constexpr bool PHASED = GH || Pipe::TWO;
+    // two barriers per plane: between writing and reading G and H, and for the late ring
+    constexpr bool LATE = Pipe::LATE, PHASED = GH || LATE;
     static_assert(Th<T>::C == C && C <= 5, "component count");
     T* ring = sm;
     T* Gs = reinterpret_cast<T*>(reinterpret_cast<char*>(sm) + Pipe::bytes);
@@ -413,38 +448,34 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
 
     Pipe pipe(sm, p, src, a, b, tx + GradBlock<M, T>::TZ * ty, y0, z0, tma);
     if (!pipe.prologue(q0, reinterpret_cast<S*>(Gs), P::nspare)) return false;
-    if (q0 + 5 <= q1) pipe.issue(q0 + 5, 5);
+    if (!LATE && q0 + 5 <= q1) pipe.issue(q0 + 5, 5);
 
-    // ring offsets of planes x-2 .. x+3
+    // ring offsets of planes x-2 .. x+2 (and, with six slots, x+3)
     int o0 = 0, o1 = SLOT, o2 = 2 * SLOT, o3 = 3 * SLOT, o4 = 4 * SLOT, o5 = 5 * SLOT;
-    int nslot = 0;  // slot of plane x + 4 (that of plane x - 2)
+    int nslot = 0;  // slot of plane x - 2
     int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
     // the second derivatives are taken with the opposite sign, as the streamed point arithmetic
     // wants them (no negations to issue)
     const V r1x = V(k.r1[0]), r1y = V(k.r1[1]), r1z = V(k.r1[2]);
     const V r2x = V(-k.r2[0]), r2y = V(-k.r2[1]), r2z = V(-k.r2[2]);
     for (int x = xa; x < xe; ++x, s += YZ) {
-        const bool more = x + 3 <= q1;
-        const int islot = nslot == 0 ? R - 1 : nslot - 1;  // slot of plane x + 3
+        const int pslot = nslot == 0 ? R - 1 : nslot - 1;  // slot of plane x + 3, or of x + 2 in the late ring
         if constexpr (PHASED) {
-            // plane x - 1 is finished: G and H (and the staged update operands) may be overwritten
-            if constexpr (Pipe::TWO) {
-                const bool ok = more ? pipe.land(islot) : true;
+            // plane x - 1 is finished: G and H may be overwritten; in the late ring plane x + 2 is in
+            if (x > xa) {
+                const bool ok = LATE ? pipe.land(pslot) : true;
                 if (pipe.meet(ok)) {
                     pipe.give_up();
                     return false;
                 }
-                if (more) pipe.issue2(x + 3);
-            } else if (x > xa) {
-                pipe.meet(true);
             }
         }
-        if constexpr (HasBeginSite<Epi>::value) {
-            if (own) epi.begin_site(s, N, x + 1 < xe ? s + YZ : int64_t(-1), own1);
+        if constexpr (HasGradBegin<Epi>::value) {
+            if (own) epi.begin_site(s, N, own1);
         }
         if constexpr (HasPrefetch<Epi>::value) {
             // the row's operands of plane x + 1, while this plane is computed
-            if (y < p.Y && x + 1 < xe) epi.prefetch(s - NL * tx + YZ, N, tx, min(M::BZ, p.Z - z0));
+            if (y < p.Y && x + 1 < xe) epi.prefetch(s - NL * tx + YZ, N, tx, min(M::BZ, p.Z - z0), x + 1);
         }
         const bool px = x >= hl && x < p.X - hl;
         // ---- pure derivatives; G and H ----
@@ -513,6 +544,9 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
                 if constexpr (sizeof(T) == 8) ksum_add(esum, Th<double>::energy(phi, D, p));
             }
         }
+        if constexpr (HasLoad<Epi>::value) {
+            if (own) epi.load(s, N, own1);
+        }
         auto point = [&]() {
             const bool mx = px && x > hl;
             V g[C];
@@ -544,19 +578,19 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
         if constexpr (!PHASED) {
             if (own) point();
         }
-        // ---- plane x + 3 is in; plane x + 4 follows into the slot of plane x - 2 ----
-        bool ok = true;
-        if (more) ok = Pipe::TWO ? pipe.land2(islot) : pipe.land(islot);
+        // ---- plane x + 3 is in; the slot of plane x - 2 takes the next plane ----
+        const bool ok = !LATE && x + 3 <= q1 ? pipe.land(pslot) : true;
         if (pipe.meet(ok)) {
             pipe.give_up();
             return false;
         }
-        if (x + 4 <= q1) pipe.issue(x + 4, nslot);
+        constexpr int next = LATE ? 3 : 4;
+        if (x + next <= q1) pipe.issue(x + next, nslot);
         if constexpr (PHASED) {
             if (own) point();
         }
         const int t0 = o0;
-        o0 = o1, o1 = o2, o2 = o3, o3 = o4, o4 = o5, o5 = t0;
+        o0 = o1, o1 = o2, o2 = o3, o3 = o4, o4 = LATE ? t0 : o5, o5 = t0;
         nslot = nslot + 1 == R ? 0 : nslot + 1;
     }
     return true;
@@ -583,9 +617,17 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
     Pipe pipe(sm, p, src, 1.0, 1.0, tx + M::BZ * ty, y0, z0, tma);
     if (!pipe.prologue(q0, nullptr, 0)) return false;
     if (q0 + 5 <= q1) pipe.issue(q0 + 5, 5);
-    int o0 = 0, o1 = SLOT, o2 = 2 * SLOT, o3 = 3 * SLOT, o4 = 4 * SLOT, o5 = 5 * SLOT;
+    int o2 = 2 * SLOT, o4 = 4 * SLOT;  // ring offsets of planes x and x + 2
     int nslot = 0;
     int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
+    // the thread's own column: planes x-2 .. x+1 of the next site (its x-taps and its value; the
+    // walk is bound by shared-memory reads)
+    double qm2[C], qm1[C], q0v[C], qp1[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const int co = lofs + c * PLANE;
+        qm2[c] = sm[co], qm1[c] = sm[SLOT + co], q0v[c] = sm[2 * SLOT + co], qp1[c] = sm[3 * SLOT + co];
+    }
     for (int x = xa; x < xe; ++x, s += YZ) {
         if (own) {
             const bool px = x >= hl && x < p.X - hl;
@@ -594,10 +636,12 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
             for (int c = 0; c < C; ++c) {
                 const int co = lofs + c * PLANE;
                 const double* f = sm + o2 + co;
-                phi[c] = f[0];
-                D[0][c] = px ? r1[0] * tap_first(sm[o0 + co], sm[o1 + co], sm[o3 + co], sm[o4 + co]) : 0.0;
+                const double p2 = sm[o4 + co];
+                phi[c] = q0v[c];
+                D[0][c] = px ? r1[0] * tap_first(qm2[c], qm1[c], qp1[c], p2) : 0.0;
                 D[1][c] = py ? r1[1] * tap_first(f[-2 * HZ], f[-HZ], f[HZ], f[2 * HZ]) : 0.0;
                 D[2][c] = pz ? r1[2] * tap_first(f[-2], f[-1], f[1], f[2]) : 0.0;
+                qm2[c] = qm1[c], qm1[c] = q0v[c], q0v[c] = qp1[c], qp1[c] = p2;
             }
             op(s, phi, D);
         }
@@ -607,8 +651,8 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
             return false;
         }
         if (x + 4 <= q1) pipe.issue(x + 4, nslot);
-        const int t0 = o0;
-        o0 = o1, o1 = o2, o2 = o3, o3 = o4, o4 = o5, o5 = t0;
+        o2 = o2 + SLOT == R * SLOT ? 0 : o2 + SLOT;
+        o4 = o4 + SLOT == R * SLOT ? 0 : o4 + SLOT;
         nslot = nslot + 1 == R ? 0 : nslot + 1;
     }
     return true;
@@ -676,7 +720,7 @@ struct PlainStageEpi {
     // plane ahead: the loads at the site then wait for L2 and not for DRAM (omega 128^3,
     // stage 4: 280 -> 206 us, stage 2: 135 -> 129; loading the operands into registers before
     // the point arithmetic gained nothing, 12 rows of them 229 us)
-    __device__ __forceinline__ void prefetch(int64_t s0, int64_t N, int lane, int n) {
+    __device__ __forceinline__ void prefetch(int64_t s0, int64_t N, int lane, int n, int) {
         for (int i = lane; i < 3 * NA * C; i += 32) {
             const int k = i / (3 * C), r = i - k * 3 * C, c = r / 3, q = r - 3 * c;
             prefetch_l2(operand(k) + c * N + s0 + min(16 * q, n - 1));

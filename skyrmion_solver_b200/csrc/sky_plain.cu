@@ -298,13 +298,13 @@ int choose_xc(int X, int tiles_yz, int resident) {
 }
 
 // x-chunk of a walk whose first planes are loaded at once (sky_grad.cuh): minimise (waves of
-// tiles) x (planes computed + about one and a half planes' time to fill the ring).
+// tiles) x (planes computed + about three planes' time to fill the ring).
 int choose_chunk(int X, int tiles_yz, int resident) {
     int best = X;
     int64_t best_cost = -1;
     for (int xc = 1; xc <= X; ++xc) {
         const int64_t nt = (int64_t)tiles_yz * ((X + xc - 1) / xc);
-        const int64_t cost = ((nt + resident - 1) / resident) * (2 * xc + 3);
+        const int64_t cost = ((nt + resident - 1) / resident) * (xc + 3);
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && xc > best)) {
             best_cost = cost;
             best = xc;

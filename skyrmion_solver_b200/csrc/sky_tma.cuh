@@ -104,6 +104,13 @@ __device__ __forceinline__ void tma_load_plane(void* dst, const TmaMap* map, int
         : "memory");
 }
 
+// The same box into L2 only, for a later tma_load_plane.
+__device__ __forceinline__ void tma_prefetch_plane(const TmaMap* map, int z, int y, int x, int c) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(&map->m), "r"(z), "r"(y),
+                 "r"(x), "r"(c)
+                 : "memory");
+}
+
 // Host: encode the plane-box map of a C-component lattice array of element size
 // `esize` (4 or 8) with dimensions (X, Y, Z): box (hz, hy, 1, C).  Returns 0 on
 // success, else a sky_status (invalid argument when an alignment rule fails).
