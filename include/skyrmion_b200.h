@@ -146,6 +146,11 @@ int sky_baryon_moments(int theory, const int32_t* p_i, int32_t n_pi, const doubl
 int sky_nuclear_diagnostics(const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf,
                             const double* field, const double* com_host, double* scratch, int64_t n_scratch,
                             double* out28_host, void* stream);
+/* The same for one group of the 28 sums (which = 1: U, 2: V, 4: W, 8: Q, 16: D, or 31: all); the
+ * other entries of out28_host are left as they are.  U does not depend on com_host. */
+int sky_nuclear_diagnostics_part(const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf, int which,
+                                 const double* field, const double* com_host, double* scratch, int64_t n_scratch,
+                                 double* out28_host, void* stream);
 
 /* Initial field on the device (replaces the reference's initial-configuration
  * kernels, th/nuclear_skyrme/initial_config.py:583-627, 664-698, 941-953,

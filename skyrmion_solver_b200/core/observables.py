@@ -124,16 +124,24 @@ def _sym(v6):
     return np.array([[a, b, c], [b, d, e], [c, e, f]], dtype=np.float64)
 
 
-def _nuclear_diag(theory_id, Field, gridsum_partial, p_i, p_f, moments=None):
-    """(centre of mass, the 28 fused sums of sky_nuclear_diagnostics).  `moments`: the nine
-    baryon moments of the same field when the caller already has them (sky_baryon_moments)."""
+# groups of the 28 sums of sky_nuclear_diagnostics (the `which` of sky_nuclear_diagnostics_part)
+GROUP_U, GROUP_V, GROUP_W, GROUP_Q, GROUP_D, GROUP_ALL = 1, 2, 4, 8, 16, 31
+
+
+def _nuclear_diag(theory_id, Field, gridsum_partial, p_i, p_f, moments=None, which=GROUP_ALL):
+    """(centre of mass, the fused sums of sky_nuclear_diagnostics that `which` selects, the others
+    zero).  `moments`: the nine baryon moments of the same field when the caller already has them
+    (sky_baryon_moments).  U alone does not need the centre of mass: it is then None."""
     import numpy as np
-    m = _moments(theory_id, Field, gridsum_partial, p_i, p_f) if moments is None else moments
-    com = np.zeros(3) if abs(m[0]) < 1.0e-30 else m[1:4] / m[0]
+    com = None
+    if which != GROUP_U:
+        m = _moments(theory_id, Field, gridsum_partial, p_i, p_f) if moments is None else moments
+        com = np.zeros(3) if abs(m[0]) < 1.0e-30 else m[1:4] / m[0]
     hi, hf = host_params(p_i, p_f)
     scratch = pick_scratch(gridsum_partial)
     out = np.zeros(28)
-    _lib.call("sky_nuclear_diagnostics", i32p(hi), len(hi), f64p(hf), len(hf), dptr(Field), f64p(np.ascontiguousarray(com)),
+    at = np.ascontiguousarray(com if com is not None else np.zeros(3))
+    _lib.call("sky_nuclear_diagnostics_part", i32p(hi), len(hi), f64p(hf), len(hf), int(which), dptr(Field), f64p(at),
               dptr(scratch), _numel(scratch), f64p(out), stream_ptr())
     return com, out
 
@@ -156,7 +164,8 @@ class UTensorObservable:
         self.theory_id = theory_id
 
     def __call__(self, Field, d1fd1x, obs9, tensor_scratch, entmp, gridsum_partial, p_i_d, p_f_d, p_i_h=None):
-        _, out = _nuclear_diag(self.theory_id, Field, gridsum_partial, p_i_h if p_i_h is not None else p_i_d, p_f_d)
+        _, out = _nuclear_diag(self.theory_id, Field, gridsum_partial, p_i_h if p_i_h is not None else p_i_d, p_f_d,
+                               which=GROUP_U)
         return _sym(out[0:6])
 
 
@@ -170,13 +179,15 @@ class _ComTensorObservable:
     def __call__(self, Field, grid, d1fd1x, obs9, tensor_scratch, entmp, gridsum_partial, obs4, com_d, p_i_d, p_f_d,
                  p_i_h=None):
         com, out = _nuclear_diag(self.theory_id, Field, gridsum_partial, p_i_h if p_i_h is not None else p_i_d,
-                                 p_f_d)
+                                 p_f_d, which=self.group)
         _store_com(com_d, com)
         return self.pick(out)
 
 
 class VTensorObservable(_ComTensorObservable):
     """compute_V_tensor: the spin inertia tensor (observables.py:308-349)."""
+
+    group = GROUP_V
 
     @staticmethod
     def pick(out):
@@ -186,6 +197,8 @@ class VTensorObservable(_ComTensorObservable):
 class WTensorObservable(_ComTensorObservable):
     """compute_W_tensor: the mixed inertia tensor (observables.py:352-393)."""
 
+    group = GROUP_W
+
     @staticmethod
     def pick(out):
         return out[12:21].reshape(3, 3).copy()
@@ -193,6 +206,8 @@ class WTensorObservable(_ComTensorObservable):
 
 class QuadrupoleTensorObservable(_ComTensorObservable):
     """compute_quadrupole_tensor: the baryon quadrupole tensor (observables.py:396-437)."""
+
+    group = GROUP_Q
 
     @staticmethod
     def pick(out):
@@ -211,7 +226,7 @@ class DTermObservable:
                  p_i_h=None, p_f_h=None):
         p_i = p_i_h if p_i_h is not None else p_i_d
         p_f = p_f_h if p_f_h is not None else p_f_d
-        com, out = _nuclear_diag(self.theory_id, Field, gridsum_partial, p_i, p_f)
+        com, out = _nuclear_diag(self.theory_id, Field, gridsum_partial, p_i, p_f, which=GROUP_D)
         _store_com(com_d, com)
         E = _total("sky_total_energy", self.theory_id, Field, en, entmp, gridsum_partial, p_i, p_f)
         return -(2.0 / 5.0) * E * float(out[27])

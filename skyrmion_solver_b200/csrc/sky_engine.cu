@@ -309,7 +309,7 @@ static int alloc_inst(Engine& e, HostInst& h) {
     if (energy_walk(h.theory, h.prec)) {
         h.etnz = h.tnz;
         h.etny = (h.p.Y + kEnergyRows - 1) / kEnergyRows;
-        h.exc = choose_chunk(h.p.X, h.etnz * h.etny, num_sms());
+        h.exc = choose_chunk(h.p.X, h.etnz * h.etny, 2 * num_sms());
         h.etnx = (h.p.X + h.exc - 1) / h.exc;
         h.entiles = h.etnz * h.etny * h.etnx;
     }

@@ -671,20 +671,20 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
 // FP64 ring.  (Inside stage 1 the 60 tap differences of a five-component site each needed an
 // exact FP32 difference and two conversions: half of that stage's instructions.)
 // ---------------------------------------------------------------------------
-constexpr int kEnergyRows = 16;
+constexpr int kEnergyRows = kDensRows;
 
 template <template <typename> class Th>
 struct EnergyOp {
     const Params& p;
     KSum sum;
-    __device__ __forceinline__ void operator()(int64_t, const double (&phi)[Th<double>::C],
+    __device__ __forceinline__ void operator()(int64_t, int, const double (&phi)[Th<double>::C],
                                                const double (&D)[3][Th<double>::C]) {
         ksum_add(sum, Th<double>::energy(phi, D, p));
     }
 };
 
 template <template <typename> class Th, class M, bool TMA>
-__global__ void __launch_bounds__(M::NTHREADS)
+__global__ void __launch_bounds__(M::NTHREADS, 2)
     k_energy(const InstDesc<float>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end,
              int half) {
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -903,7 +903,7 @@ struct AuditOp {
     const S* V;  // null: the velocity is zero (arrested)
     int64_t N;
     KSum pot, kin;
-    __device__ __forceinline__ void operator()(int64_t s, const double (&phi)[Th<double>::C],
+    __device__ __forceinline__ void operator()(int64_t s, int, const double (&phi)[Th<double>::C],
                                                const double (&D)[3][Th<double>::C]) {
         ksum_add(pot, Dynamics<Th>::potential(phi, D, p));
         if (!V) return;

@@ -29,7 +29,7 @@ constexpr bool is_walk() {
 template <template <typename> class Th, typename T>
 constexpr int stage_rows() {
     if (!is_walk<Th>()) return sizeof(T) == 8 ? 4 : 8;
-    if (sizeof(T) == 8) return grad_rows64<Th>();
+    if (sizeof(T) == 8) return grad_rows64<Th>(true);
     constexpr int id = Th<float>::kId;
     return (id == SKY_THEORY_NUCLEAR || id == SKY_THEORY_LIGHTLY_BOUND) ? 16 : 12;
 }
@@ -148,7 +148,7 @@ template <template <typename> class Th, bool WIDE, bool TMA>
 static int energy_setup(int* per_sm_out) {
     static int per_sm = 0;
     using M = MarchShape<Th<double>::C, kEnergyRows, WIDE, 4>;
-    using Pipe = PlanePipe<M, double, float, 2, TMA, M::NTHREADS>;
+    using Pipe = DensPipe<M, float, 2, TMA>;
     if (per_sm == 0) {
         const int rc = kernel_setup(k_energy<Th, M, TMA>, Pipe::bytes + (TMA ? 128 : 0), M::NTHREADS, &per_sm);
         if (rc) return rc;
@@ -159,7 +159,7 @@ static int energy_setup(int* per_sm_out) {
 template <template <typename> class Th, bool WIDE, bool TMA>
 static int launch_energy_w(const Group& g, const StageArgs& a, cudaStream_t st) {
     using M = MarchShape<Th<double>::C, kEnergyRows, WIDE, 4>;
-    using Pipe = PlanePipe<M, double, float, 2, TMA, M::NTHREADS>;
+    using Pipe = DensPipe<M, float, 2, TMA>;
     int per_sm = 1;
     int rc = energy_setup<Th, WIDE, TMA>(&per_sm);
     if (rc) return rc;
@@ -267,7 +267,7 @@ static int launch_defect_w(const Group& g, cudaStream_t st) {
 // Energy audit of the RK4 dynamics (k_engine_audit).
 template <template <typename> class Th>
 constexpr int audit_rows() {
-    return Th<double>::C > 5 ? 4 : 16;  // a 13-component FP64 ring still fits
+    return Th<double>::C > 5 ? 4 : kDensRows;  // a 13-component FP64 ring with staged FP32 sources fits
 }
 
 template <template <typename> class Th, typename S>
@@ -275,7 +275,7 @@ static int audit_t(const Group& g, const HostInst& h, cudaStream_t st, double* o
     using M = MarchShape<Th<double>::C, audit_rows<Th>(), false>;
     constexpr int NSRC = std::is_same<S, double>::value ? 1 : 2;
     auto kern = k_engine_audit<Th, M, S>;
-    const size_t smem = PlanePipe<M, double, S, NSRC, false, M::NTHREADS>::bytes;
+    const size_t smem = DensPipe<M, S, NSRC, false>::bytes;
     static bool configured = false;
     if (!configured) {
         int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),

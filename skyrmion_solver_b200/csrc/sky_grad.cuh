@@ -145,23 +145,28 @@ __device__ __forceinline__ void axpy16(double2& v, double a, const double2& u) {
 // staging slot each and are added in (X = F + a V + b L).  The ring has six slots, so that a
 // plane travels while the whole previous one is computed.  The late ring (LATE, three sources by
 // TMA) has five, and a plane travels during the point arithmetic only: for tiles of which 7 slots
-// leave two blocks on an SM and 8 do not.
+// leave two blocks on an SM and 8 do not.  The density walks, whose threads keep their own
+// column in registers, have four.
 // S != T (float arrays, FP64 ring): every source is staged and converted; X = F + a V.
 // Planes outside the lattice and points outside it in y and z read as zero.
 // ---------------------------------------------------------------------------
-template <class M, typename T, typename S, int NSRC, bool TMA, int NT, bool LATE_ = false>
+template <class M, typename T, typename S, int NSRC, bool TMA, int NT, int R_ = 6>
 struct PlanePipe {
     static constexpr bool SAME = std::is_same<S, T>::value;
     static constexpr bool DIRECT = SAME && NSRC == 1;
-    static constexpr bool LATE = LATE_;
-    static constexpr int R = LATE ? 5 : 6;
+    static constexpr int R = R_;
+    static constexpr bool LATE = R == 5;
+    static constexpr int FIRST = R < 5 ? R : 5;  // planes the prologue fills
     static constexpr int SLOT = M::SLOT;
     static constexpr int NSTG = SAME ? NSRC - 1 : NSRC;
     static constexpr size_t ring_bytes = size_t(R) * SLOT * sizeof(T);
     static constexpr size_t stage_bytes = size_t(NSTG) * SLOT * sizeof(S);
     static constexpr size_t bytes = ring_bytes + stage_bytes;
     static_assert(!TMA || M::WIDE, "TMA staging: wide rows");
+    static_assert(!TMA || (SLOT * sizeof(S) % 128 == 0 && SLOT * sizeof(T) % 128 == 0),
+                  "TMA boxes land on 128-byte boundaries");
     static_assert(!LATE || (TMA && SAME && NSRC == 3), "the late ring is the staged TMA pipeline's");
+    static_assert(R >= 5 || DIRECT || !SAME, "the density walks' ring");
     static_assert(SAME || NSRC <= 2, "converted sources: a field and its low parts");
 
     T* ring;
@@ -331,7 +336,7 @@ struct PlanePipe {
             }
         }
     }
-    // Planes q0 .. q0 + 4 into slots 0 .. 4, complete and visible to the block.  `spare` is
+    // Planes q0 .. q0 + FIRST - 1 into slots 0, 1, .., complete and visible to the block.  `spare` is
     // shared memory of at least `nspare` slots that the walk does not use yet, so that several
     // staged planes travel at once.
     __device__ __forceinline__ bool prologue(int q0, S* spare, int nspare) {
@@ -339,9 +344,9 @@ struct PlanePipe {
         bool ok = true;
         if constexpr (TMA && SAME) {
             // staged planes travel through the staging slots, a sixth ring slot and the spare ones
-            constexpr int own = NSTG + (R - 5);
+            constexpr int own = NSTG + (R > 5 ? 1 : 0);
             const int nb = DIRECT ? 0 : own + nspare;
-            const int items = NSRC > 1 ? 5 * ns : 0;
+            const int items = NSRC > 1 ? FIRST * ns : 0;
             auto buf = [&](int k) -> S* {
                 return k < NSTG ? stage + k * SLOT
                                 : k < own ? reinterpret_cast<S*>(ring + 5 * SLOT) : spare + (k - own) * SLOT;
@@ -351,9 +356,9 @@ struct PlanePipe {
                 const int n = min(nb, items - it);
                 if (tid == 0) {
                     fence_proxy_async_smem();
-                    mbar_arrive_expect_tx(tma->bar, uint32_t((it == 0 ? 5 : 0) + n) * kBox);
+                    mbar_arrive_expect_tx(tma->bar, uint32_t((it == 0 ? FIRST : 0) + n) * kBox);
                     if (it == 0)
-                        for (int j = 0; j < 5; ++j) box(ring + j * SLOT, 0, q0 + j);
+                        for (int j = 0; j < FIRST; ++j) box(ring + j * SLOT, 0, q0 + j);
                     for (int k = 0; k < n; ++k) box(buf(k), which(it + k), q0 + (it + k) / ns);
                 }
                 ok = wait();
@@ -365,11 +370,11 @@ struct PlanePipe {
                 }
             }
         } else if constexpr (DIRECT) {
-            for (int j = 0; j < 5; ++j) issue(q0 + j, j);
+            for (int j = 0; j < FIRST; ++j) issue(q0 + j, j);
             wait();
             meet(true);
         } else {
-            for (int j = 0; j < 5; ++j) {
+            for (int j = 0; j < FIRST; ++j) {
                 issue(q0 + j, j);
                 ok = land(j);
                 if (meet(ok)) {
@@ -382,13 +387,15 @@ struct PlanePipe {
     }
 };
 
-// Rows of an FP64 walk's tiles (32 threads each): 16 where the kernel fits 128 registers, else
-// 12 (168 registers).  Gradient of 128^3 sites: nuclear 110 us with 16 rows, 134 with 12;
-// omega 89 and 89; Coulomb 147 with 12 and 230 with 16, where it spills; Berger 140 with 12
-// (8-row tiles with the register queues of the earlier form: 154, 119, 200 and 173 us).
+// Rows of an FP64 gradient walk's tiles (32 threads each).  The drop-in kernels, whose scales and
+// couplings are kernel parameters, take 16 where they fit 128 registers (gradient of 128^3
+// sites: nuclear 110 us with 16 rows, 134 with 12; omega 89 and 89), else 12 at 168 registers
+// (Coulomb 147 with 12 and 230 with 16, where it spills; Berger 140).  8-row tiles with the
+// register queues of the earlier form: 154, 119, 200 and 173 us.  Every engine stage spills with
+// 16 (omega stage 1: 143 us against 114, stage 3: 222 against 173): 12.
 template <template <typename> class Th>
-constexpr int grad_rows64() {
-    return 12;
+constexpr int grad_rows64(bool engine) {
+    return engine || Th<double>::kId == SKY_THEORY_COULOMB || Th<double>::kId == SKY_THEORY_BERGER ? 12 : 16;
 }
 
 // Shared memory of a gradient walk.
@@ -401,7 +408,7 @@ struct GradPipe {
     // the static variables of each block)
     static constexpr bool LATE = TMA && NSRC == 3 && sizeof(T) == 4 && sizeof(S) == 4 &&
                                  size_t(8) * M::SLOT * sizeof(T) + gh_bytes > 114000;
-    using Pipe = PlanePipe<M, T, S, NSRC, TMA, GradBlock<M, T>::NT, LATE>;
+    using Pipe = PlanePipe<M, T, S, NSRC, TMA, GradBlock<M, T>::NT, LATE ? 5 : 6>;
     static constexpr size_t bytes = Pipe::bytes + gh_bytes;
     // staging slots that G and H can stand in for during the prologue
     static constexpr int nspare = int(gh_bytes / (size_t(M::SLOT) * sizeof(S)));
@@ -597,63 +604,71 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
 }
 
 // Density walk: the FP64 value and first derivatives of the first M::C components at every
-// site of a tile, handed to op(s, phi, D).  Sources: an FP64 array, or an FP32 one with
+// site of a tile, handed to op(s, x, phi, D).  Sources: an FP64 array, or an FP32 one with
 // optional low parts (S = float, NSRC = 2, weight 1), converted once as they enter the FP64
-// ring.  One barrier per plane.
+// ring.  The walk is bound by shared-memory reads and their latency: a thread keeps its own
+// column (x-2 .. x+1) in registers, which leaves nine reads per component and a ring of four
+// planes (x, whose y and z taps are read, x+1, x+2 and the one on its way), so that several
+// blocks share an SM.
+template <class M, typename S, int NSRC, bool TMA>
+using DensPipe = PlanePipe<M, double, S, NSRC, TMA, M::NTHREADS, 4>;
+
 template <class M, typename S, int NSRC, bool TMA, class Op>
 __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params& p, const double (&r1)[3],
                                           const S* const (&src)[3], int xa, int xe, int y0, int z0, Op& op,
                                           TmaTile* tma = nullptr) {
-    using Pipe = PlanePipe<M, double, S, NSRC, TMA, M::NTHREADS>;
-    constexpr int C = M::C, R = Pipe::R, SLOT = M::SLOT, PLANE = M::PLANE, HZ = M::HZ;
+    using Pipe = DensPipe<M, S, NSRC, TMA>;
+    constexpr int C = M::C, SLOT = M::SLOT, PLANE = M::PLANE, HZ = M::HZ;
     const int64_t YZ = (int64_t)p.Y * p.Z;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = y0 + ty, z = z0 + tx;
     const bool own = (y < p.Y) && (z < p.Z);
     const int hl = p.halo;
     const bool py = y >= hl && y < p.Y - hl, pz = z >= hl && z < p.Z - hl;
-    const int q0 = xa - 2, q1 = xe + 1;
+    const int q1 = xe + 1;
     const int lofs = (ty + 2) * HZ + (tx + M::ZOFF);
     Pipe pipe(sm, p, src, 1.0, 1.0, tx + M::BZ * ty, y0, z0, tma);
-    if (!pipe.prologue(q0, nullptr, 0)) return false;
-    if (q0 + 5 <= q1) pipe.issue(q0 + 5, 5);
-    int o2 = 2 * SLOT, o4 = 4 * SLOT;  // ring offsets of planes x and x + 2
-    int nslot = 0;
-    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
-    // the thread's own column: planes x-2 .. x+1 of the next site (its x-taps and its value; the
-    // walk is bound by shared-memory reads)
-    double qm2[C], qm1[C], q0v[C], qp1[C];
+    if (!pipe.prologue(xa - 2, nullptr, 0)) return false;
+    double qm2[C], qm1[C], qc[C], qp1[C];  // planes x-2 .. x+1 of the thread's column
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         const int co = lofs + c * PLANE;
-        qm2[c] = sm[co], qm1[c] = sm[SLOT + co], q0v[c] = sm[2 * SLOT + co], qp1[c] = sm[3 * SLOT + co];
+        qm2[c] = sm[co], qm1[c] = sm[SLOT + co], qc[c] = sm[2 * SLOT + co], qp1[c] = sm[3 * SLOT + co];
     }
+    pipe.meet(true);  // planes xa - 2 and xa - 1 have been read
+    pipe.issue(xa + 2, 0);
+    if (pipe.meet(pipe.land(0))) {
+        pipe.give_up();
+        return false;
+    }
+    if (xa + 3 <= q1) pipe.issue(xa + 3, 1);
+    int k = 2;  // slot of plane x
+    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
     for (int x = xa; x < xe; ++x, s += YZ) {
+        const double* P0 = sm + k * SLOT + lofs;
+        const double* P2 = sm + ((k + 2) & 3) * SLOT + lofs;
         if (own) {
             const bool px = x >= hl && x < p.X - hl;
             double phi[C], D[3][C];
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                const int co = lofs + c * PLANE;
-                const double* f = sm + o2 + co;
-                const double p2 = sm[o4 + co];
-                phi[c] = q0v[c];
+                const double* f = P0 + c * PLANE;
+                const double p2 = P2[c * PLANE];
+                phi[c] = qc[c];
                 D[0][c] = px ? r1[0] * tap_first(qm2[c], qm1[c], qp1[c], p2) : 0.0;
                 D[1][c] = py ? r1[1] * tap_first(f[-2 * HZ], f[-HZ], f[HZ], f[2 * HZ]) : 0.0;
                 D[2][c] = pz ? r1[2] * tap_first(f[-2], f[-1], f[1], f[2]) : 0.0;
-                qm2[c] = qm1[c], qm1[c] = q0v[c], q0v[c] = qp1[c], qp1[c] = p2;
+                qm2[c] = qm1[c], qm1[c] = qc[c], qc[c] = qp1[c], qp1[c] = p2;
             }
-            op(s, phi, D);
+            op(s, x, phi, D);
         }
-        const bool ok = x + 3 <= q1 ? pipe.land(nslot == 0 ? R - 1 : nslot - 1) : true;
+        const bool ok = x + 3 <= q1 ? pipe.land((k + 3) & 3) : true;
         if (pipe.meet(ok)) {
             pipe.give_up();
             return false;
         }
-        if (x + 4 <= q1) pipe.issue(x + 4, nslot);
-        o2 = o2 + SLOT == R * SLOT ? 0 : o2 + SLOT;
-        o4 = o4 + SLOT == R * SLOT ? 0 : o4 + SLOT;
-        nslot = nslot + 1 == R ? 0 : nslot + 1;
+        if (x + 4 <= q1) pipe.issue(x + 4, k);
+        k = (k + 1) & 3;
     }
     return true;
 }
@@ -803,7 +818,7 @@ struct DensOp {
     double* dens;
     KSum sum;
     template <int C>
-    __device__ __forceinline__ void operator()(int64_t s, const double (&phi)[C], const double (&D)[3][C]) {
+    __device__ __forceinline__ void operator()(int64_t s, int, const double (&phi)[C], const double (&D)[3][C]) {
         constexpr int CT = Th<double>::C;
         double ph[CT], d[3][CT];
 #pragma unroll
@@ -818,8 +833,13 @@ struct DensOp {
     }
 };
 
+// Rows of a density walk's tiles.  Two 8-row blocks per SM: 46 us for the nuclear energy of 128^3
+// sites and 55 for omega's (16 rows, one block: 50 and 56; a ring of six planes read at every
+// tap: 56 and 62).  Rho's 13 components: 8 rows, one block, 36 us at 64^3 (4 rows: 58).
+constexpr int kDensRows = 8;
+
 template <template <typename> class Th, class M, int MODE>
-__global__ void __launch_bounds__(M::NTHREADS)
+__global__ void __launch_bounds__(M::NTHREADS, M::C > 5 ? 1 : 2)
     k_dens_plain(Params p, const __grid_constant__ MarchCoef<double> k, MarchGrid mg, const double* __restrict__ field,
                  double* __restrict__ dens, double* __restrict__ scratch, double* __restrict__ out_dev) {
     extern __shared__ __align__(16) unsigned char smraw[];

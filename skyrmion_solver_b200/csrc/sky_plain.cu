@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include "sky_host.h"
+#include "sky_diag.cuh"
 #include "sky_grad.cuh"
 #include "sky_kernels.cuh"
 
@@ -380,7 +381,7 @@ static bool wide64(const Params& p, const double* f) {
     return p.Z % 2 == 0 && (reinterpret_cast<uintptr_t>(f) & 15) == 0;
 }
 template <template <typename> class Th, bool WIDE>
-using Shape64 = MarchShape<Th<double>::C, grad_rows64<Th>(), WIDE, 2>;
+using Shape64 = MarchShape<Th<double>::C, grad_rows64<Th>(false), WIDE, 2>;
 
 template <template <typename> class Th, bool WIDE>
 int launch_gradient_walk(const Params& p, const double* field, double* eg, double* l, cudaStream_t st) {
@@ -485,16 +486,16 @@ int grad64(const Params& p, const double* f, double* eg, double* l, cudaStream_t
     }
     return launch_gradient<Th, double, double>(p, f, eg, l, st);
 }
-// FP64 density walk with its fused compensated sum (energy: all components, in 6-row tiles for
-// rho, whose 13-component ring of more rows would not fit; baryon: phi_0..3 of any theory).
+// FP64 density walk with its fused compensated sum (energy: all components; baryon: phi_0..3 of
+// any theory).
 // clear: set the reduction's completion counter to 0 first.
 template <template <typename> class Th, int MODE, bool WIDE>
 int launch_density_walk(const Params& p, const double* field, double* dens, double* scratch, double* out_dev,
                         bool clear, cudaStream_t st) {
     constexpr int C = MODE == 0 ? Th<double>::C : 4;
-    using M = MarchShape<C, (C > 5 ? 6 : 16), WIDE, 2>;
+    using M = MarchShape<C, kDensRows, WIDE, 2>;
     auto kern = k_dens_plain<Th, M, MODE>;
-    const size_t smem = PlanePipe<M, double, double, 1, false, M::NTHREADS>::bytes;
+    const size_t smem = DensPipe<M, double, 1, false>::bytes;
     static int per_sm = 0;
     MarchGrid mg;
     int blocks;
@@ -564,84 +565,72 @@ int stages64(const Params& p, const StepBuffers& b, double* counter_e, double* s
     return SKY_OK;
 }
 
-// Baryon moments (k_march_moments): at most kScratchDoubles / 18 blocks, so the
-// per-block partials fit the standard reduction scratch.
-template <template <typename> class Th>
-int moments64(const Params& p, const double* f, double* scratch, double* out9, cudaStream_t st) {
-    using M = MarchShape<4, 8, false>;
-    auto kern = k_march_moments<Th, M>;
-    const size_t smem = M::template smem_bytes<double>(1);
-    static bool configured = false;
-    if (!configured) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(moments)", __LINE__);
-        if (rc) return rc;
-        configured = true;
-    }
-    const int cap = kScratchDoubles / (2 * kMoments);
-    const MarchGrid g0 = march_grid<M>(p, p.X);
-    const MarchGrid mg = march_grid<M>(p, choose_xc(p.X, g0.nz * g0.ny, num_sms()));
-    const int blocks = mg.count() < cap ? mg.count() : cap;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, mg, f, scratch);
-    int rc = check_cuda(cudaGetLastError(), "launch moments", __LINE__);
+// Launch a diagnostic walk (k_moments, k_diag) and read its n sums.  The grid is whole clusters;
+// one partial per cluster keeps the standard reduction scratch sufficient.
+template <class M, class K, class... A>
+int diag_walk(K kern, const Params& p, const double* f, double* scratch, int n, double* out, int* per_sm,
+              cudaStream_t st, A... args) {
+    const size_t smem = DensPipe<M, double, 1, false>::bytes;
+    MarchGrid mg;
+    int blocks;
+    const int cap = kScratchDoubles / (2 * n) * kDiagCluster;
+    int rc = walk_geometry<M>(kern, smem, p, cap, 0, per_sm, &mg, &blocks);
     if (rc) return rc;
-    double parts[2 * kMoments * (kScratchDoubles / (2 * kMoments))];
-    rc = check_cuda(cudaMemcpyAsync(parts, scratch, sizeof(double) * 2 * kMoments * blocks, cudaMemcpyDeviceToHost, st),
-                    "read moments", __LINE__);
+    blocks = (blocks + kDiagCluster - 1) / kDiagCluster * kDiagCluster;
+    rc = check_cuda(cudaMemsetAsync(scratch + 2 * kMaxRedBlocks + 1, 0, sizeof(double), st), "memset", __LINE__);
+    if (rc) return rc;
+    MarchCoef<double> k;
+    k.init(p);
+    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, f, scratch, args...);
+    rc = check_cuda(cudaGetLastError(), "launch diagnostic walk", __LINE__);
+    if (!rc) rc = check_cuda(cudaMemcpyAsync(out, scratch, sizeof(double) * n, cudaMemcpyDeviceToHost, st),
+                             "read diagnostics", __LINE__);
     if (!rc) rc = check_cuda(cudaStreamSynchronize(st), "sync", __LINE__);
-    if (rc) return rc;
-    for (int q = 0; q < kMoments; ++q) {   // fixed-order compensated sum over the blocks
-        double sum = 0.0, comp = 0.0;
-        for (int b = 0; b < blocks; ++b) {
-            for (int k = 0; k < 2; ++k) {
-                const double v = parts[2 * kMoments * b + 2 * q + k];
-                const double t = sum + v;
-                comp += (fabs(sum) >= fabs(v)) ? ((sum - t) + v) : ((v - t) + sum);
-                sum = t;
-            }
-        }
-        out9[q] = sum + comp;
-    }
-    return SKY_OK;
+    return rc;
 }
 
-// Nuclear diagnostics (k_march_diag): at most kScratchDoubles / 56 blocks.
-int diag64(const Params& p, const double* f, const double* com, double* scratch, double* out28, cudaStream_t st) {
-    using M = MarchShape<4, 8, false>;
-    auto kern = k_march_diag<M>;
-    const size_t smem = M::template smem_bytes<double>(1);
-    static bool configured = false;
-    if (!configured) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(diagnostics)", __LINE__);
-        if (rc) return rc;
-        configured = true;
-    }
-    const int cap = kScratchDoubles / (2 * kDiag);
-    const MarchGrid g0 = march_grid<M>(p, p.X);
-    const MarchGrid mg = march_grid<M>(p, choose_xc(p.X, g0.nz * g0.ny, num_sms()));
-    const int blocks = mg.count() < cap ? mg.count() : cap;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, mg, f, com[0], com[1], com[2], scratch);
-    int rc = check_cuda(cudaGetLastError(), "launch diagnostics", __LINE__);
+template <template <typename> class Th, bool WIDE>
+int moments_walk(const Params& p, const double* f, double* scratch, double* out9, cudaStream_t st) {
+    using M = MarchShape<4, kDensRows, WIDE, 2>;
+    static int per_sm = 0;
+    return diag_walk<M>(k_moments<Th, M>, p, f, scratch, kMoments, out9, &per_sm, st);
+}
+template <template <typename> class Th>
+int moments64(const Params& p, const double* f, double* scratch, double* out9, cudaStream_t st) {
+    return wide64(p, f) ? moments_walk<Th, true>(p, f, scratch, out9, st)
+                        : moments_walk<Th, false>(p, f, scratch, out9, st);
+}
+
+template <bool WIDE, int WHICH>
+int diag_parts(const Params& p, const double* f, const double* com, double* scratch, double* out28, cudaStream_t st) {
+    using M = MarchShape<4, kDensRows, WIDE, 2>;
+    static int per_sm = 0;
+    double sums[kDiag];
+    const int rc = diag_walk<M>(k_diag<M, WHICH>, p, f, scratch, diag_count(WHICH), sums, &per_sm, st, com[0], com[1],
+                                com[2]);
     if (rc) return rc;
-    double parts[2 * kDiag * (kScratchDoubles / (2 * kDiag))];
-    rc = check_cuda(cudaMemcpyAsync(parts, scratch, sizeof(double) * 2 * kDiag * blocks, cudaMemcpyDeviceToHost, st),
-                    "read diagnostics", __LINE__);
-    if (!rc) rc = check_cuda(cudaStreamSynchronize(st), "sync", __LINE__);
-    if (rc) return rc;
-    for (int q = 0; q < kDiag; ++q) {   // fixed-order compensated sum over the blocks
-        double sum = 0.0, comp = 0.0;
-        for (int b = 0; b < blocks; ++b) {
-            for (int k = 0; k < 2; ++k) {
-                const double v = parts[2 * kDiag * b + 2 * q + k];
-                const double t = sum + v;
-                comp += (fabs(sum) >= fabs(v)) ? ((sum - t) + v) : ((v - t) + sum);
-                sum = t;
-            }
-        }
-        out28[q] = sum + comp;
-    }
+    for (int g = 0, n = 0; g < 5; ++g)
+        if (WHICH >> g & 1)
+            for (int q = 0; q < kDiagSize[g]; ++q) out28[kDiagStart[g] + q] = sums[n++];
     return SKY_OK;
+}
+template <int WHICH>
+int diag_wide(const Params& p, const double* f, const double* com, double* scratch, double* out28, cudaStream_t st) {
+    return wide64(p, f) ? diag_parts<true, WHICH>(p, f, com, scratch, out28, st)
+                        : diag_parts<false, WHICH>(p, f, com, scratch, out28, st);
+}
+// The groups of `which` (bit 0: U, 1: V, 2: W, 3: Q, 4: D) of the 28 sums; the others stay.
+int diag64(const Params& p, int which, const double* f, const double* com, double* scratch, double* out28,
+           cudaStream_t st) {
+    switch (which) {
+        case 1: return diag_wide<1>(p, f, com, scratch, out28, st);
+        case 2: return diag_wide<2>(p, f, com, scratch, out28, st);
+        case 4: return diag_wide<4>(p, f, com, scratch, out28, st);
+        case 8: return diag_wide<8>(p, f, com, scratch, out28, st);
+        case 16: return diag_wide<16>(p, f, com, scratch, out28, st);
+        case 31: return diag_wide<31>(p, f, com, scratch, out28, st);
+        default: return invalid("which must be one of 1, 2, 4, 8, 16 and 31");
+    }
 }
 
 int gradient_fp64(int theory, const Params& p, const double* f, double* eg, double* l, cudaStream_t st) {
@@ -970,7 +959,19 @@ int sky_nuclear_diagnostics(const int32_t* p_i, int32_t n_pi, const double* p_f,
     if (!field || !com_host || !out28_host) return invalid("null buffer");
     if (!scratch || n_scratch < kScratchDoubles) return SKY_ERR_NOMEM;
     if ((int64_t)4 * n_sites(p) >= ((int64_t)1 << 31)) return invalid("lattice too large for the diagnostics kernel");
-    return diag64(p, field, com_host, scratch, out28_host, SKY_STREAM(stream));
+    return diag64(p, 31, field, com_host, scratch, out28_host, SKY_STREAM(stream));
+}
+
+int sky_nuclear_diagnostics_part(const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf, int which,
+                                 const double* field, const double* com_host, double* scratch, int64_t n_scratch,
+                                 double* out28_host, void* stream) {
+    Params p;
+    int rc = pack_params(SKY_THEORY_NUCLEAR, p_i, n_pi, p_f, n_pf, &p);
+    if (rc) return rc;
+    if (!field || !com_host || !out28_host) return invalid("null buffer");
+    if (!scratch || n_scratch < kScratchDoubles) return SKY_ERR_NOMEM;
+    if ((int64_t)4 * n_sites(p) >= ((int64_t)1 << 31)) return invalid("lattice too large for the diagnostics kernel");
+    return diag64(p, which, field, com_host, scratch, out28_host, SKY_STREAM(stream));
 }
 
 int sky_arrested_newton_step(int theory, const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf,

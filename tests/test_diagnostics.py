@@ -80,3 +80,28 @@ def test_engine_diagnostics_of_a_resident_instance():
         assert _close(g["center_of_mass"], O.center_of_mass(th, Fj, p_i, p_f))
         assert _close(g["U"], O.u_tensor(th, Fj, p_i, p_f))
         assert _close(g["D_term"], O.d_term(th, Fj, p_i, p_f))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(3, 8, 32), (6, 7, 31), (5, 9, 33), (37, 17, 66)])
+def test_diagnostic_walks_at_tile_edges(dims):
+    """Moments and each group of the inertia and shape sums on lattices at the edges of the 8-row,
+    32-column tiles (fewer tiles than a cluster has blocks, odd Z), and every group alone against
+    all 28 sums together.  The sums' terms are at most a few hundred; 1e-10 is the parity bound."""
+    from skyrmion_solver_b200.core import observables as ob
+    from tests._gpu import dev
+    from tests.test_march import inputs, params_for
+    th, p_i, p_f = params_for("nuclear", dims)
+    F, _ = inputs(4, dims, seed=11)
+    thd = O.THEORIES["nuclear"]
+    field = dev(F)
+    com, full = ob._nuclear_diag(0, field, None, p_i, p_f)
+    assert _close(com, O.center_of_mass(thd, F, p_i, p_f))
+    assert _close(ob._sym(full[0:6]), O.u_tensor(thd, F, p_i, p_f))
+    assert _close(ob._sym(full[6:12]), O.v_tensor(thd, F, p_i, p_f))
+    assert _close(full[12:21].reshape(3, 3), O.w_tensor(thd, F, p_i, p_f))
+    assert _close(ob._sym(full[21:27]), O.quadrupole_tensor(thd, F, p_i, p_f))
+    for which, sl in ((1, slice(0, 6)), (2, slice(6, 12)), (4, slice(12, 21)), (8, slice(21, 27)), (16, slice(27, 28))):
+        _, part = ob._nuclear_diag(0, field, None, p_i, p_f, which=which)
+        assert _close(part[sl], full[sl], 1e-12)
+        assert not np.any(np.delete(part, np.arange(28)[sl]))
