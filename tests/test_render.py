@@ -409,3 +409,37 @@ def test_renderer_draws_a_resident_engine_instance():
         assert r.extrema == (vmin, vmax)
         assert np.array_equal(r.volume.cpu().numpy(), want)
         assert _image_close(img.cpu().numpy(), R.render(want, inv_view_rows(), box=r.box_scale, width=40, height=30))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 3, 5), (17, 23, 31), (40, 9, 24)])
+@pytest.mark.parametrize("color_mode", [0, 1])
+def test_rays_across_empty_cells(dims, color_mode):
+    """Rays that cross cells whose corners show nothing: a bump in an empty volume (empty cells
+    before and behind it), random sparse texels (empty cells next to full ones), from outside and
+    inside the box, at the module's image tolerance against the oracle, which samples every step."""
+    import torch
+    X, Y, Z = dims
+    rng = np.random.default_rng(X * 100 + Y)
+    z, y, x = np.meshgrid(*[(np.arange(n) + 0.5) * 2.0 / n - 1.0 for n in (Z, Y, X)], indexing="ij")
+    bump = np.exp(-12.0 * ((x - 0.2) ** 2 + (y + 0.1) ** 2 + z ** 2))
+    sparse = np.where(rng.random(bump.shape) < 0.02, 0.5, 0.01)
+    n = rng.normal(size=(3,) + bump.shape)
+    n /= np.sqrt((n ** 2).sum(axis=0))
+
+    class _Sim:
+        p_i_h = np.array(dims, np.int32)
+        p_f_h = np.array(dims, np.float64)
+    for dens in (bump, sparse):
+        vol = np.concatenate([dens[None], n]).transpose(1, 2, 3, 0).astype(np.float32)
+        for rot, tr in [((20, -35, 0), (0.1, -0.1, -3.5)), ((10, 200, 0), (0, 0, -0.5))]:
+            r = HeadlessRenderer(40, 30)
+            r.bind_sim(_Sim())
+            r.set_display_mode(1 + color_mode)
+            r.set_camera_pose(view_rotation=rot, view_translation=tr)
+            r.set_render_params(opacity_scale=0.05, levelset=0.2, transfer_scale=4.0)
+            r.volume.copy_(torch.from_numpy(vol))
+            got = r.draw().cpu().numpy()
+            want = R.render(vol, inv_view_rows(rot, tr), box=r.box_scale, width=40, height=30,
+                            opacity_scale=0.05, color_mode=color_mode)
+            assert _image_close(got, want)
