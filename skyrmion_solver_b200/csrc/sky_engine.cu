@@ -29,7 +29,7 @@ struct Engine {
     cudaEvent_t forked = nullptr, joined = nullptr;
     std::map<int, HostInst> insts;
     int next_id = 0;
-    Group groups[6][2];
+    Group groups[kNumKernelSets][2];
     cudaGraphExec_t graph = nullptr;   // kGraphSteps steps
     cudaGraphExec_t graph1 = nullptr;  // one step (the remainder of a step call)
     bool graph_valid = false, graph1_valid = false;
@@ -39,28 +39,29 @@ struct Engine {
     int* d_status = nullptr;  // device error word the stage kernels set (bit 0: a TMA wait gave up)
 };
 
-const TheoryOps& theory_ops(int theory) {
-    switch (theory) {
+const TheoryOps& kernel_ops(int set) {
+    switch (set) {
         case SKY_THEORY_NUCLEAR: return kNuclearOps;
         case SKY_THEORY_OMEGA: return kOmegaOps;
         case SKY_THEORY_COULOMB: return kCoulombOps;
         case SKY_THEORY_RHO: return kRhoOps;
         case SKY_THEORY_BERGER: return kBergerOps;
+        case kFusedRho: return kFusedRhoOps;
         default: return kLightlyBoundOps;
     }
 }
 static int launch_stage_group(int stage, const Group& g, const StageArgs& a, cudaStream_t st) {
-    return theory_ops(g.theory).stage(g.prec, stage, g, a, st);
+    return kernel_ops(g.set).stage(g.prec, stage, g, a, st);
 }
 static int launch_energy(const Group& g, const StageArgs& a, cudaStream_t st) {
-    return energy_walk(g.theory, g.prec) ? theory_ops(g.theory).energy(g, a, st) : SKY_OK;
+    return energy_walk(g.set, g.prec) ? kernel_ops(g.set).energy(g, a, st) : SKY_OK;
 }
 // Defect refresh of the group's defect-corrected FP32 instances (those whose refresh is due;
 // the others' tiles are skipped).
 static int launch_defect(const Group& g, cudaStream_t st) {
-    return g.prec || !g.any_defect ? SKY_OK : theory_ops(g.theory).defect(g, st);
+    return g.prec || !g.any_defect ? SKY_OK : kernel_ops(g.set).defect(g, st);
 }
-static int setup_group(const Group& g) { return theory_ops(g.theory).setup(g.prec); }
+static int setup_group(const Group& g) { return kernel_ops(g.set).setup(g); }
 
 // Whether every instance of a group can use the wide-row kernels: Z a multiple of
 // 16 / sizeof(T) (the buffers are cudaMalloc'd, hence 256-byte aligned).
@@ -68,24 +69,23 @@ static bool wide_ok(int prec, int Z) { return Z % (prec ? 2 : 4) == 0; }
 
 // Stage tiles of an instance for x-chunk request `xc` (0: chosen).
 static void tile_geometry(const HostInst& h, int request, int* xc, int* nz, int* ny, int* nx) {
-    const TileShapeInfo sh = theory_ops(h.theory).shape(h.prec);
+    const TileShapeInfo sh = kernel_ops(h.set).shape(h.prec);
     *nz = (h.p.Z + 31) / 32;
     *ny = (h.p.Y + sh.rows - 1) / sh.rows;
     const int resident = num_sms() * sh.blocks;
     if (request > 0)
         *xc = request < h.p.X ? request : h.p.X;
     else
-        *xc = theory_components(h.theory) <= 5 ? choose_chunk(h.p.X, *nz * *ny, resident)
-                                               : choose_xc(h.p.X, *nz * *ny, resident);
+        *xc = choose_chunk(h.p.X, *nz * *ny, resident);
     *nx = (h.p.X + *xc - 1) / *xc;
 }
 
 static int launch_control(const Group& g, int ib, int ie, int mode, cudaStream_t st) {
     if (ie <= ib) return SKY_OK;
     if (g.prec)
-        k_engine_control<double><<<ie - ib, 32, 0, st>>>(reinterpret_cast<InstDesc<double>*>(g.d_desc), ib, ie, mode);
+        k_engine_control<double><<<ie - ib, 32 * kControlWarps, 0, st>>>(reinterpret_cast<InstDesc<double>*>(g.d_desc), ib, ie, mode);
     else
-        k_engine_control<float><<<ie - ib, 32, 0, st>>>(reinterpret_cast<InstDesc<float>*>(g.d_desc), ib, ie, mode);
+        k_engine_control<float><<<ie - ib, 32 * kControlWarps, 0, st>>>(reinterpret_cast<InstDesc<float>*>(g.d_desc), ib, ie, mode);
     return check_cuda(cudaGetLastError(), "launch engine control", __LINE__);
 }
 
@@ -134,21 +134,30 @@ __global__ void k_f32c_to_f64(int64_t n, const float* __restrict__ hi, const flo
 // components, the haloed plane of a stage tile; and of an energy tile.
 template <typename S>
 static int encode_maps(const HostInst& h, InstDesc<S>& d) {
-    const TileShapeInfo sh = theory_ops(h.theory).shape(h.prec);
+    const TileShapeInfo sh = kernel_ops(h.set).shape(h.prec);
     const void* arrs[kNumMaps] = {h.F[0], h.F[1], h.Flo[0], h.Flo[1], h.V[0], h.V[1],
                                   h.L[0], h.L[1], h.L[2], h.Dlt};
     for (int k = 0; k < kNumMaps; ++k) {
         if (!arrs[k]) continue;
-        int rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, sh.hz, sh.rows + 4);
-        if (!rc && k < kNumEnergyMaps && energy_walk(h.theory, h.prec))
-            rc = encode_plane_map(&d.tme[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.C, 40, kEnergyRows + 4);
+        int rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, sh.components, sh.hz,
+                                  sh.rows + 4);
+        if (!rc && h.set == SKY_THEORY_RHO)
+            // the rho components: those of one isospin component are 3 N apart, and its planes X long
+            rc = encode_plane_map(&d.tmr[k], reinterpret_cast<const S*>(arrs[k]) + 4 * h.N, (int)sizeof(S), 3 * h.p.X,
+                                  h.p.Y, h.p.Z, 3, sh.hz, sh.rho_rows + 4);
+        if (!rc && k < kNumEnergyMaps && split_energy(h.set, h.prec))
+            rc = encode_plane_map(&d.tmc[k], reinterpret_cast<const S*>(arrs[k]) + 4 * h.N, (int)sizeof(S), 3 * h.p.X,
+                                  h.p.Y, h.p.Z, 3, 40, kDensRows + 4);
+        if (!rc && k < kNumEnergyMaps && energy_walk(h.set, h.prec))
+            rc = encode_plane_map(&d.tme[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, sh.components, 40,
+                                  kDensRows + 4);
         if (rc) return rc;
     }
     return SKY_OK;
 }
 
 template <typename S>
-static InstDesc<S> make_desc(const HostInst& h, int tile_begin, int e_tile_begin) {
+static InstDesc<S> make_desc(const HostInst& h, int tile_begin, int e_tile_begin, int r_tile_begin) {
     InstDesc<S> d;
     memset(&d, 0, sizeof(d));
     d.p = h.p;
@@ -164,16 +173,21 @@ static InstDesc<S> make_desc(const HostInst& h, int tile_begin, int e_tile_begin
     }
     for (int i = 0; i < 3; ++i) d.L[i] = reinterpret_cast<S*>(h.L[i]);
     d.epart = h.epart;
+    d.curl = h.curl;
+    d.e_parts = energy_partials(h.set, h.prec, h.entiles);
     d.bpart = h.bpart;
     d.gpart = h.gpart;
     d.stats = h.stats;
     d.stats_cap = kStatsCap;
     d.tile_begin = tile_begin;
     d.ntiles = h.ntiles;
+    d.gtiles = grad_partials(h.set, h.ntiles, h.rgrid.count());
     d.tiles_nz = h.tnz;
     d.tiles_ny = h.tny;
     d.tiles_nx = h.tnx;
     d.xc = h.xc;
+    d.r_tile_begin = r_tile_begin;
+    d.r_grid = h.rgrid;
     d.e_tile_begin = e_tile_begin;
     d.e_ntiles = h.entiles;
     d.e_nz = h.etnz;
@@ -200,14 +214,14 @@ static int rebuild_group_t(Engine& e, Group& g) {
         if ((rc = check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__))) return rc;
     }
     std::vector<InstDesc<S>> descs;
-    std::vector<int> tile_inst, e_tile_inst;
+    std::vector<int> tile_inst, e_tile_inst, r_tile_inst;
     int tb = 0;
     g.all_wide = true;
     g.any_defect = false;
     g.all_tma = !g.members.empty();
     for (size_t k = 0; k < g.members.size(); ++k) {
         HostInst& h = e.insts[g.members[k]];
-        InstDesc<S> d = make_desc<S>(h, tb, (int)e_tile_inst.size());
+        InstDesc<S> d = make_desc<S>(h, tb, (int)e_tile_inst.size(), (int)r_tile_inst.size());
         d.status = e.d_status;
         if (h.tma) {
             const int rc = encode_maps<S>(h, d);
@@ -229,12 +243,15 @@ static int rebuild_group_t(Engine& e, Group& g) {
         if (!wide_ok(h.prec, h.p.Z)) g.all_wide = false;
         descs.push_back(d);
         for (int t = 0; t < h.ntiles; ++t) tile_inst.push_back((int)k);
-        if (energy_walk(h.theory, h.prec)) e_tile_inst.insert(e_tile_inst.end(), h.entiles, (int)k);
+        if (energy_walk(h.set, h.prec)) e_tile_inst.insert(e_tile_inst.end(), h.entiles, (int)k);
+        r_tile_inst.insert(r_tile_inst.end(), h.rgrid.count(), (int)k);
         tb += h.ntiles;
     }
     g.ntiles = tb;
     g.entiles = (int)e_tile_inst.size();
+    g.rtiles = (int)r_tile_inst.size();
     tile_inst.insert(tile_inst.end(), e_tile_inst.begin(), e_tile_inst.end());
+    tile_inst.insert(tile_inst.end(), r_tile_inst.begin(), r_tile_inst.end());
     if ((int)descs.size() > g.desc_cap) {
         if (g.d_desc) cudaFree(g.d_desc);
         g.desc_cap = (int)descs.size() * 2 + 4;
@@ -274,7 +291,7 @@ static int rebuild_group(Engine& e, Group& g) {
 
 static void free_inst(HostInst& h) {
     void* ptrs[] = {h.F[0], h.F[1], h.Flo[0], h.Flo[1], h.Dlt, h.V[0], h.V[1], h.L[0], h.L[1], h.L[2],
-                    h.epart, h.bpart, h.gpart, h.stats};
+                    h.curl, h.epart, h.bpart, h.gpart, h.stats};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     memset(h.F, 0, sizeof(h.F));
@@ -282,6 +299,7 @@ static void free_inst(HostInst& h) {
     h.Dlt = nullptr;
     memset(h.V, 0, sizeof(h.V));
     memset(h.L, 0, sizeof(h.L));
+    h.curl = nullptr;
     h.epart = h.bpart = nullptr;
     h.gpart = nullptr;
     h.stats = nullptr;
@@ -289,7 +307,7 @@ static void free_inst(HostInst& h) {
 
 // Whether an instance's planes can be staged by TMA box copies: the option is on,
 // the row pitch Z * sizeof(T) is a multiple of 16 bytes, and its (theory,
-// precision) uses wide rows (every one but FP64 rho).
+// precision) has TMA kernels (every one but FP64 rho).
 static bool tma_possible(const HostInst& h) {
     return wide_ok(h.prec, h.p.Z) && !(h.prec && theory_components(h.theory) > 5);
 }
@@ -299,6 +317,7 @@ static bool pair_possible(const HostInst& h) { return h.prec == 0 && h.theory ==
 
 static int alloc_inst(Engine& e, HostInst& h) {
     const size_t es = h.prec ? sizeof(double) : sizeof(float);
+    h.set = kernel_set(h.theory, h.prec, h.N);
     h.tma = tma_ok_for(h);
     h.pair = h.tma && option(3) == 1 && pair_possible(h);
     const size_t fb = es * (size_t)h.C * (size_t)h.N;
@@ -306,10 +325,18 @@ static int alloc_inst(Engine& e, HostInst& h) {
     tile_geometry(h, h.xc_request, &h.xc, &h.tnz, &h.tny, &h.tnx);
     h.ntiles = h.tnz * h.tny * h.tnx;
     h.entiles = h.ntiles;
-    if (energy_walk(h.theory, h.prec)) {
+    if (h.set == SKY_THEORY_RHO) {
+        const TileShapeInfo sh = kernel_ops(h.set).shape(h.prec);
+        h.rgrid.nz = h.tnz;
+        h.rgrid.ny = (h.p.Y + sh.rho_rows - 1) / sh.rho_rows;
+        h.rgrid.xc = choose_chunk(h.p.X, 3 * h.rgrid.nz * h.rgrid.ny, sh.rho_blocks * num_sms());
+        h.rgrid.nx = (h.p.X + h.rgrid.xc - 1) / h.rgrid.xc;
+    }
+    if (energy_walk(h.set, h.prec)) {
         h.etnz = h.tnz;
-        h.etny = (h.p.Y + kEnergyRows - 1) / kEnergyRows;
-        h.exc = choose_chunk(h.p.X, h.etnz * h.etny, 2 * num_sms());
+        h.etny = (h.p.Y + kDensRows - 1) / kDensRows;
+        h.exc = choose_chunk(h.p.X, h.etnz * h.etny,
+                             (h.C > 5 ? 1 : 2) * num_sms());
         h.etnx = (h.p.X + h.exc - 1) / h.exc;
         h.entiles = h.etnz * h.etny * h.etnx;
     }
@@ -321,9 +348,10 @@ static int alloc_inst(Engine& e, HostInst& h) {
             return SKY_ERR_NOMEM;
         }
     }
-    if (cudaMalloc(&h.epart, sizeof(KSum) * h.entiles) != cudaSuccess ||
+    if (cudaMalloc(&h.epart, sizeof(KSum) * energy_partials(h.set, h.prec, h.entiles)) != cudaSuccess ||
+        (split_energy(h.set, h.prec) && cudaMalloc(&h.curl, sizeof(double) * 9 * (size_t)h.N) != cudaSuccess) ||
         cudaMalloc(&h.bpart, sizeof(KSum) * h.ntiles) != cudaSuccess ||
-        cudaMalloc(&h.gpart, sizeof(double) * 4 * h.ntiles) != cudaSuccess ||
+        cudaMalloc(&h.gpart, sizeof(double) * 4 * grad_partials(h.set, h.ntiles, h.rgrid.count())) != cudaSuccess ||
         cudaMalloc(&h.stats, sizeof(StepStats) * kStatsCap) != cudaSuccess) {
         cudaGetLastError();
         free_inst(h);
@@ -347,10 +375,11 @@ static int alloc_inst(Engine& e, HostInst& h) {
         }
         cudaMemsetAsync(h.Dlt, 0, fb, e.stream);
     }
-    cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * h.ntiles, e.stream);
+    cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * grad_partials(h.set, h.ntiles, h.rgrid.count()), e.stream);
     cudaMemsetAsync(h.stats, 0, sizeof(StepStats) * kStatsCap, e.stream);
-    h.bytes = (h.comp ? 9 : 7) * fb + (h.defect ? fb : 0) + (sizeof(KSum) + sizeof(double) * 4) * h.ntiles +
-              sizeof(KSum) * h.entiles + sizeof(StepStats) * kStatsCap;
+    h.bytes = (h.comp ? 9 : 7) * fb + (h.defect ? fb : 0) + sizeof(KSum) * (h.ntiles + energy_partials(h.set, h.prec, h.entiles)) +
+              (h.curl ? sizeof(double) * 9 * (size_t)h.N : 0) +
+              sizeof(double) * 4 * grad_partials(h.set, h.ntiles, h.rgrid.count()) + sizeof(StepStats) * kStatsCap;
     return SKY_OK;
 }
 
@@ -389,15 +418,16 @@ static int upload(Engine& e, HostInst& h, const double* field, const double* vel
 
 // Stage 1 + control for one instance (admission or precision change).
 static int init_instance(Engine& e, HostInst& h, int mode) {
-    Group& g = e.groups[h.theory][h.prec];
-    int tb = 0, eb = 0;
+    Group& g = e.groups[h.set][h.prec];
+    int tb = 0, eb = 0, rb = 0;
     for (int id : g.members) {
         if (id == h.id) break;
         tb += e.insts[id].ntiles;
         eb += e.insts[id].entiles;
+        rb += e.insts[id].rgrid.count();
     }
-    int rc = launch_energy(g, StageArgs{eb, eb + h.entiles, 0}, e.stream);
-    if (!rc) rc = launch_stage_group(1, g, StageArgs{tb, tb + h.ntiles, 0}, e.stream);
+    int rc = launch_energy(g, StageArgs{eb, eb + h.entiles, 0, 0, 0, 0}, e.stream);
+    if (!rc) rc = launch_stage_group(1, g, StageArgs{tb, tb + h.ntiles, 0, rb, rb + h.rgrid.count(), 0}, e.stream);
     if (rc) return rc;
     rc = launch_control(g, h.group_slot, h.group_slot + 1, mode, e.stream);
     if (rc) return rc;
@@ -411,18 +441,19 @@ static int init_instance(Engine& e, HostInst& h, int mode) {
 enum { kKindS2 = 0, kKindS3, kKindS4, kKindDefect, kKindEnergy, kKindS1, kNumKinds };
 
 static int launch_kind(Engine& e, int kind, cudaStream_t st) {
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr) {
             Group& g = e.groups[t][pr];
             if (g.members.empty()) continue;
-            const StageArgs a{0, g.ntiles, 1};
+            const int chained = kind == kKindS3 || kind == kKindEnergy || kind == kKindS1;
+            const StageArgs a{0, g.ntiles, 1, 0, g.rtiles, chained};
             int rc = SKY_OK;
             switch (kind) {
                 case kKindS2: rc = launch_stage_group(2, g, a, st); break;
                 case kKindS3: rc = launch_stage_group(3, g, a, st); break;
                 case kKindS4: rc = launch_stage_group(4, g, a, st); break;
                 case kKindDefect: rc = launch_defect(g, st); break;
-                case kKindEnergy: rc = launch_energy(g, StageArgs{0, g.entiles, 1}, st); break;
+                case kKindEnergy: rc = launch_energy(g, StageArgs{0, g.entiles, 1, 0, 0, chained}, st); break;
                 default: rc = launch_stage_group(1, g, a, st); break;
             }
             if (rc) return rc;
@@ -443,7 +474,7 @@ static int record_step(Engine& e) {
             return rc;
     }
     bool any_defect = false;
-    for (int t = 0; t < 6; ++t) any_defect = any_defect || e.groups[t][0].any_defect;
+    for (int t = 0; t < kNumKernelSets; ++t) any_defect = any_defect || e.groups[t][0].any_defect;
     auto join = [&]() -> int {
         if (!fork) return SKY_OK;
         const int r = check_cuda(cudaEventRecord(e.joined, side), "join", __LINE__);
@@ -458,11 +489,12 @@ static int record_step(Engine& e) {
 
 static int count_launches(Engine& e) {
     int n = 0;
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty())
-                // stages 2, 3, 4, [defect,] [energy,] 1
-                n += 4 + ((pr == 0 && e.groups[t][pr].any_defect) ? 1 : 0) + (energy_walk(t, pr) ? 1 : 0);
+                // stages 2, 3, 4, 1 (rho: three kernels each), [defect,] [energy] (FP32 rho: two each)
+                n += 4 * (t == SKY_THEORY_RHO ? 3 : 1) + (energy_walk(t, pr) ? (split_energy(t, pr) ? 2 : 1) : 0) +
+                     ((pr == 0 && e.groups[t][pr].any_defect) ? (t == SKY_THEORY_RHO || t == kFusedRho ? 2 : 1) : 0);
     return n;
 }
 
@@ -494,7 +526,7 @@ static int capture_steps(Engine& e, int nsteps, cudaGraphExec_t* exec) {
 static int step_graph(Engine& e, int nsteps, cudaGraphExec_t* exec, bool* valid) {
     if (*valid) return SKY_OK;
     int rc = SKY_OK;
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty() && (rc = setup_group(e.groups[t][pr]))) return rc;
     if ((rc = capture_steps(e, nsteps, exec))) return rc;
@@ -518,7 +550,7 @@ static HostInst* find(Engine* e, int id) {
 }
 
 static int remove_from_group(Engine& e, HostInst& h) {
-    Group& g = e.groups[h.theory][h.prec];
+    Group& g = e.groups[h.set][h.prec];
     // the remaining members still carry their old slots, from which the
     // rebuild gathers their device control state
     std::vector<int> keep;
@@ -559,9 +591,9 @@ int sky_engine_create(int device, void** out) {
         delete e;
         return rc;
     }
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int p = 0; p < 2; ++p) {
-            e->groups[t][p].theory = t;
+            e->groups[t][p].set = t;
             e->groups[t][p].prec = p;
         }
     *out = e;
@@ -576,7 +608,7 @@ int sky_engine_destroy(void* handle) {
     if (e->graph) cudaGraphExecDestroy(e->graph);
     if (e->graph1) cudaGraphExecDestroy(e->graph1);
     for (auto& kv : e->insts) free_inst(kv.second);
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int p = 0; p < 2; ++p) {
             if (e->groups[t][p].d_desc) cudaFree(e->groups[t][p].d_desc);
             if (e->groups[t][p].d_tile_inst) cudaFree(e->groups[t][p].d_tile_inst);
@@ -615,7 +647,7 @@ int sky_engine_add(void* handle, int theory, const int32_t* p_i, int32_t n_pi, c
         return rc;
     }
     e->insts[h.id] = h;
-    Group& g = e->groups[theory][h.prec];
+    Group& g = e->groups[h.set][h.prec];
     g.members.push_back(h.id);
     if ((rc = rebuild_group(*e, g)) || (rc = init_instance(*e, e->insts[h.id], 1))) {
         g.members.pop_back();
@@ -658,7 +690,7 @@ int sky_engine_set_precision(void* handle, int id, int precision) {
     int cur = 0, arrested = 0, step = 0;
     double e_prev = 0.0;
     {
-        Group& g = e->groups[h.theory][h.prec];
+        Group& g = e->groups[h.set][h.prec];
         if (h.prec) {
             InstDesc<double> d;
             cudaMemcpy(&d, reinterpret_cast<InstDesc<double>*>(g.d_desc) + h.group_slot, sizeof(d),
@@ -679,6 +711,7 @@ int sky_engine_set_precision(void* handle, int id, int precision) {
     nh.group_slot = -1;
     for (int i = 0; i < 2; ++i) nh.F[i] = nh.Flo[i] = nh.V[i] = nullptr;
     for (int i = 0; i < 3; ++i) nh.L[i] = nullptr;
+    nh.curl = nullptr;
     nh.epart = nh.bpart = nullptr;
     nh.gpart = nullptr;
     nh.stats = nullptr;
@@ -722,7 +755,7 @@ int sky_engine_set_precision(void* handle, int id, int precision) {
     free_inst(h);
     e->bytes += (int64_t)nh.bytes - (int64_t)h.bytes;
     h = nh;
-    Group& g2 = e->groups[h.theory][h.prec];
+    Group& g2 = e->groups[h.set][h.prec];
     g2.members.push_back(h.id);
     if ((rc = rebuild_group(*e, g2))) return rc;
     // restore the control state, then recompute l1 / energy of the converted field
@@ -752,12 +785,13 @@ int sky_engine_retile(void* handle, int id, int xc) {
     int rc, nxc, tnz, tny, tnx;
     tile_geometry(h, xc, &nxc, &tnz, &tny, &tnx);
     const int ntiles = tnz * tny * tnx;
-    const bool own_energy = energy_walk(h.theory, h.prec);  // its energy tiles stay as they are
+    const bool own_energy = energy_walk(h.set, h.prec);  // its energy tiles stay as they are
     const int entiles = own_energy ? h.entiles : ntiles;
+    const int gtiles = grad_partials(h.set, ntiles, h.rgrid.count());
     KSum *ep = nullptr, *bp = nullptr;
     double* gp = nullptr;
-    if (cudaMalloc(&ep, sizeof(KSum) * entiles) != cudaSuccess || cudaMalloc(&bp, sizeof(KSum) * ntiles) != cudaSuccess ||
-        cudaMalloc(&gp, sizeof(double) * 4 * ntiles) != cudaSuccess) {
+    if (cudaMalloc(&ep, sizeof(KSum) * energy_partials(h.set, h.prec, entiles)) != cudaSuccess || cudaMalloc(&bp, sizeof(KSum) * ntiles) != cudaSuccess ||
+        cudaMalloc(&gp, sizeof(double) * 4 * gtiles) != cudaSuccess) {
         cudaGetLastError();
         if (ep) cudaFree(ep);
         if (bp) cudaFree(bp);
@@ -773,9 +807,9 @@ int sky_engine_retile(void* handle, int id, int xc) {
     h.epart = ep;
     h.bpart = bp;
     h.gpart = gp;
-    cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * ntiles, e->stream);
-    const int64_t dbytes = (int64_t)(sizeof(KSum) + sizeof(double) * 4) * ((int64_t)ntiles - h.ntiles) +
-                           (int64_t)sizeof(KSum) * ((int64_t)entiles - h.entiles);
+    cudaMemsetAsync(h.gpart, 0, sizeof(double) * 4 * gtiles, e->stream);
+    const int64_t dbytes = (int64_t)sizeof(KSum) * ((int64_t)ntiles - h.ntiles + entiles - h.entiles) +
+                           (int64_t)sizeof(double) * 4 * (gtiles - grad_partials(h.set, h.ntiles, h.rgrid.count()));
     h.bytes += dbytes;
     e->bytes += dbytes;
     h.xc_request = xc;
@@ -783,7 +817,7 @@ int sky_engine_retile(void* handle, int id, int xc) {
     h.tnx = tnx;
     h.ntiles = ntiles;  // the staging carries over
     h.entiles = entiles;
-    Group& g = e->groups[h.theory][h.prec];
+    Group& g = e->groups[h.set][h.prec];
     if ((rc = rebuild_group(*e, g))) return rc;
     return init_instance(*e, h, 2);
 }
@@ -803,7 +837,7 @@ int sky_engine_set_staging(void* handle, int id, int tma, int pair) {
     cudaStreamSynchronize(e->stream);
     h.tma = tma;
     h.pair = pair;
-    return rebuild_group(*e, e->groups[h.theory][h.prec]);  // keeps the control state
+    return rebuild_group(*e, e->groups[h.set][h.prec]);  // keeps the control state
 }
 
 int sky_engine_get_staging(void* handle, int id, int* tma, int* pair) {
@@ -823,7 +857,7 @@ int sky_engine_audit(void* handle, int id, double* out2) {
     HostInst* hp = find(e, id);
     if (!hp) return invalid("unknown instance id");
     cudaSetDevice(e->device);
-    return theory_ops(hp->theory).audit(e->groups[hp->theory][hp->prec], *hp, e->stream, out2);
+    return kernel_ops(hp->set).audit(e->groups[hp->set][hp->prec], *hp, e->stream, out2);
 }
 
 int sky_engine_set_defect_period(void* handle, int id, int period) {
@@ -835,7 +869,7 @@ int sky_engine_set_defect_period(void* handle, int id, int period) {
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
     hp->defect_period = period;
-    Group& g = e->groups[hp->theory][hp->prec];
+    Group& g = e->groups[hp->set][hp->prec];
     const size_t sz = hp->prec ? sizeof(InstDesc<double>) : sizeof(InstDesc<float>);
     const size_t off = hp->prec ? offsetof(InstDesc<double>, refresh_period) : offsetof(InstDesc<float>, refresh_period);
     char* base = reinterpret_cast<char*>(g.d_desc) + sz * hp->group_slot;
@@ -858,7 +892,7 @@ int sky_engine_set_active(void* handle, int id, int active) {
     HostInst* h = find(e, id);
     if (!h) return invalid("unknown instance id");
     h->active = active != 0;
-    Group& g = e->groups[h->theory][h->prec];
+    Group& g = e->groups[h->set][h->prec];
     const int a = h->active ? 1 : 0;
     size_t off = h->prec ? offsetof(InstDesc<double>, active) : offsetof(InstDesc<float>, active);
     size_t sz = h->prec ? sizeof(InstDesc<double>) : sizeof(InstDesc<float>);
@@ -1001,7 +1035,7 @@ int sky_engine_read(void* handle, int id, double* field, double* velocity, int o
     HostInst* h = find(e, id);
     if (!h) return invalid("unknown instance id");
     cudaSetDevice(e->device);
-    Group& g = e->groups[h->theory][h->prec];
+    Group& g = e->groups[h->set][h->prec];
     int cur = 0, arrested = 0;
     int rc;
     size_t sz = h->prec ? sizeof(InstDesc<double>) : sizeof(InstDesc<float>);
@@ -1044,7 +1078,7 @@ int sky_engine_time_stages(void* handle, int nsteps, double* ms_out) {
     if (nsteps < 1) return invalid("nsteps must be >= 1");
     cudaSetDevice(e->device);
     int rc = SKY_OK;
-    for (int t = 0; t < 6; ++t)
+    for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e->groups[t][pr].members.empty() && (rc = setup_group(e->groups[t][pr]))) return rc;
     cudaEvent_t ev[kNumKinds + 1];

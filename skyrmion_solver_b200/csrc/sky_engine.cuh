@@ -24,9 +24,12 @@
 // stage 4 of an arrested step reads the old one (l2 = l1) while stage 1 writes the new one.
 #pragma once
 
+#include <string.h>
+
 #include "sky_grad.cuh"
 #include "sky_kernels.cuh"
-#include "sky_march.cuh"
+#include "sky_rho.cuh"
+#include "sky_rho_march.cuh"
 
 namespace sky {
 
@@ -52,11 +55,26 @@ enum { kMapF = 0, kMapFlo = 2, kMapV = 4, kMapL = 6, kMapDlt = 9, kNumMaps = 10,
 // instance (sky_engine_set_defect_period changes it per instance).
 constexpr int kDefectRefresh = 16;
 
+// Sets of engine kernels: one per theory, and one for FP32 rho lattices of at most kFusedRhoSites
+// sites (k_rho_fused).
+constexpr int kFusedRho = 6, kNumKernelSets = 7;
+constexpr int64_t kFusedRhoSites = 56 * 56 * 56;
+inline int kernel_set(int theory, int prec, int64_t sites) {
+    return theory == SKY_THEORY_RHO && prec == 0 && sites <= kFusedRhoSites ? kFusedRho : theory;
+}
+// Whether a kernel set has its own energy walk; else stage 1 sums the energy.
+template <typename T>
+constexpr bool energy_walk(int set) {
+    return set != kFusedRho && (sizeof(T) == 4 || set == SKY_THEORY_RHO);
+}
+
 // Device-resident state of one instance.
 template <typename S>
 struct InstDesc {
     TmaMap tm[kNumMaps];  // plane maps of F[0..1], Flo[0..1], V[0..1], L[0..2], Dlt (when tma is set)
     TmaMap tme[kNumEnergyMaps];  // energy-tile maps of F and Flo (FP32 instances of at most five components)
+    TmaMap tmc[kNumEnergyMaps];  // FP32 rho: energy-tile maps of the rho components (as tmr)
+    TmaMap tmr[kNumMaps];  // rho: maps of the rho components, 3 planes-long x axes of one isospin component each
     int tma;              // the stage kernels stage this instance's planes with TMA
     int* status;          // the engine's error word (bit 0: a wait for a TMA copy gave up)
     Params p;
@@ -66,16 +84,21 @@ struct InstDesc {
     S* Flo[2];         // ping-pong low parts of a compensated FP32 field (null otherwise)
     S* Dlt;            // defect correction g64 - g32 of a defect-corrected FP32 instance (null otherwise)
     S* V[2];           // ping-pong velocity (the next half holds P between stages 3 and 4)
+    double* curl;      // FP32 rho: R^a_xy, R^a_xz, R^a_yz (at 3 a) of the field whose energy is being summed
     S* L[3];           // slopes: l1 of this step and of the next in L[0] and L[2] (see cur_l1), l2 in L[1]
-    KSum* epart;       // energy partials, per energy tile (k_energy) or per stage tile (stage 1)
+    KSum* epart;       // energy partials, per energy tile (k_energy; FP32 rho: four each) or per stage tile (stage 1)
     KSum* bpart;       // per-tile baryon partials (stage 1)
     double* gpart;     // per-tile [signed max, abs max of stage-4 g, kinetic KSum (s, c)] (4 doubles / tile)
     StepStats* stats;  // ring of per-step records
     int stats_cap;
     int tile_begin;    // first global tile index of this instance
     int ntiles;
+    int e_parts;       // entries of epart: e_ntiles, four times that for FP32 rho
+    int gtiles;        // entries of gpart: ntiles, and for rho those of the rho components' epilogue
     int tiles_nz, tiles_ny, tiles_nx;
     int xc;            // x-chunk of the marching kernels
+    int r_tile_begin;  // rho: tiles of the walk over the rho components (three items each)
+    MarchGrid r_grid;
     int e_tile_begin, e_ntiles, e_nz, e_ny, e_nx, e_xc;  // energy tiles (e_ntiles = ntiles where stage 1 sums it)
     // control state (device-updated)
     double e_prev;     // energy entering the previous step
@@ -191,85 +214,120 @@ __device__ __forceinline__ int l1_slot(const InstDesc<S>& in, int half) {
 // ---------------------------------------------------------------------------
 // mode 0: end of a step (advances the instance, arrest decision); 1: admission (step 0, no
 // arrest); 2: resume after a precision change (keeps the pending arrest decision).
-// The work is one warp's (the control kernel, or a warp of the last block to finish a
-// step's stage-4 and stage-1 launches, one warp per instance): lane-strided compensated sums of
-// the per-tile partials and a fixed shuffle tree, so the order depends on the tile count
-// only.  The partials are read through L2: in the stage kernel they were written by
-// other blocks of the same launch.
+// The work is four warps' (the control kernel, or warps of the last block to finish a step's
+// stage-4 and stage-1 launches): lane-strided compensated sums of the per-tile partials, a fixed
+// shuffle tree per warp and the warps in order, so the order depends on the tile count only.  The
+// partials are read through L2: in the stage kernel they were written by other blocks of the same
+// launch.  A step ends with this, so it is laid out for latency: several turns of loads in flight
+// (with one warp and one load after the other, 20 us for 1300 partials).
+constexpr int kControlWarps = 4;
+struct ControlSums {
+    KSum e, b, kin;
+    double gm, ga;
+    __device__ __forceinline__ void merge(const ControlSums& o) {
+        ksum_merge(e, o.e);
+        ksum_merge(b, o.b);
+        ksum_merge(kin, o.kin);
+        gm = fmax(gm, o.gm);
+        ga = fmax(ga, o.ga);
+    }
+};
+// warp: the calling warp's number among the instance's four; sh: three entries of shared memory;
+// bar: a barrier of the four warps.
 template <typename S>
-__device__ __forceinline__ void engine_control_warp(InstDesc<S>& in, int mode) {
+__device__ __forceinline__ void engine_control(InstDesc<S>& in, int mode, int warp, ControlSums* sh, int bar) {
     const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
-    KSum e{0.0, 0.0}, b{0.0, 0.0}, kin{0.0, 0.0};
-    double gm = -1.0e300, ga = 0.0;
-    for (int t = lane; t < in.e_ntiles; t += 32) ksum_merge(e, KSum{__ldcg(&in.epart[t].s), __ldcg(&in.epart[t].c)});
-    for (int t = lane; t < in.ntiles; t += 32) {
-        ksum_merge(b, KSum{__ldcg(&in.bpart[t].s), __ldcg(&in.bpart[t].c)});
-        gm = fmax(gm, __ldcg(&in.gpart[4 * t]));
-        ga = fmax(ga, __ldcg(&in.gpart[4 * t + 1]));
-        ksum_merge(kin, KSum{__ldcg(&in.gpart[4 * t + 2]), __ldcg(&in.gpart[4 * t + 3])});
+    ControlSums r{{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, -1.0e300, 0.0};
+    constexpr int U = 2, T = 32 * kControlWarps;
+    const int ne = in.e_parts, nb = in.ntiles, ng = in.gtiles, n = max(max(ne, nb), ng);
+    const KSum *ep = in.epart, *bp = in.bpart;
+    const double* gp = in.gpart;
+    for (int t0 = 32 * warp + lane; t0 < n; t0 += T * U) {
+        double le[U][2], lb[U][2], lg[U][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {  // loads past an array's end read its last entry
+            const int t = t0 + T * u;
+            const int te = min(t, ne - 1), tb = min(t, nb - 1), tg = min(t, ng - 1);
+            le[u][0] = __ldcg(&ep[te].s), le[u][1] = __ldcg(&ep[te].c);
+            lb[u][0] = __ldcg(&bp[tb].s), lb[u][1] = __ldcg(&bp[tb].c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) lg[u][k] = __ldcg(&gp[4 * tg + k]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t0 + T * u;
+            if (t < ne) ksum_merge(r.e, KSum{le[u][0], le[u][1]});
+            if (t < nb) ksum_merge(r.b, KSum{lb[u][0], lb[u][1]});
+            if (t < ng) {
+                r.gm = fmax(r.gm, lg[u][0]);
+                r.ga = fmax(r.ga, lg[u][1]);
+                ksum_merge(r.kin, KSum{lg[u][2], lg[u][3]});
+            }
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-        const KSum oe = ksum_shfl_down(e, off), ob = ksum_shfl_down(b, off), ok = ksum_shfl_down(kin, off);
-        const double om = __shfl_down_sync(0xffffffffu, gm, off), oa = __shfl_down_sync(0xffffffffu, ga, off);
-        if (lane + off < 32) {
-            ksum_merge(e, oe);
-            ksum_merge(b, ob);
-            ksum_merge(kin, ok);
-            gm = fmax(gm, om);
-            ga = fmax(ga, oa);
-        }
+        ControlSums o;
+        o.e = ksum_shfl_down(r.e, off), o.b = ksum_shfl_down(r.b, off), o.kin = ksum_shfl_down(r.kin, off);
+        o.gm = __shfl_down_sync(0xffffffffu, r.gm, off), o.ga = __shfl_down_sync(0xffffffffu, r.ga, off);
+        if (lane + off < 32) r.merge(o);
     }
-    if (lane == 0) {
-        const double en = e.s + e.c;
+    if (warp > 0 && lane == 0) sh[warp - 1] = r;
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory");
+    if (warp == 0 && lane == 0) {
+        for (int w = 1; w < kControlWarps; ++w) r.merge(sh[w - 1]);
+        const double en = r.e.s + r.e.c;
         if (mode == 1) in.step = 0;
         if (mode == 0) {
             in.refresh = refresh_due(in) ? 1 : 0;
             in.step += 1;
             in.cur ^= 1;
         }
-        const int n = in.step;
+        const int step = in.step;
         // arrest (core/integrator.py:403-407): the energy after step n exceeds the one after step n-1
         int arrest = in.arrested;
-        if (mode == 0) arrest = (n > 0 && in.p.killkinen && en > in.e_prev) ? 1 : 0;
+        if (mode == 0) arrest = (step > 0 && in.p.killkinen && en > in.e_prev) ? 1 : 0;
         if (mode == 1) arrest = 0;
-        StepStats& st = in.stats[n % in.stats_cap];
+        StepStats& st = in.stats[step % in.stats_cap];
         st.energy = en;
-        st.baryon = b.s + b.c;
+        st.baryon = r.b.s + r.b.c;
         if (mode != 2) {  // a resume keeps the step's gradient statistics
-            st.err = (n > 0) ? gm : 0.0;
-            st.kinetic = (n > 0) ? kin.s + kin.c : 0.0;
-            st.gabs = (n > 0) ? ga : 0.0;
+            st.err = (step > 0) ? r.gm : 0.0;
+            st.kinetic = (step > 0) ? r.kin.s + r.kin.c : 0.0;
+            st.gabs = (step > 0) ? r.ga : 0.0;
         }
         st.arrested = arrest;
-        st.step = n;
+        st.step = step;
         st.status = in.status ? *in.status : 0;
         in.arrested = arrest;
         in.e_prev = en;
     }
+    // (the next instance's sums wait for this one's to be read)
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory");
 }
 
 // Control of the instances [i_begin, i_end), one block each (admission, precision change; the
 // steps themselves fold mode 0 into their last launches).
 template <typename S>
-__global__ void __launch_bounds__(32) k_engine_control(InstDesc<S>* __restrict__ insts, int i_begin, int i_end,
+__global__ void __launch_bounds__(32 * kControlWarps) k_engine_control(InstDesc<S>* __restrict__ insts, int i_begin, int i_end,
                                                        int mode) {
     const int ii = i_begin + blockIdx.x;
     if (ii >= i_end) return;
     InstDesc<S>& in = insts[ii];
     if (!in.active) return;
-    engine_control_warp(in, mode);
+    __shared__ ControlSums sh[kControlWarps - 1];
+    engine_control(in, mode, threadIdx.x >> 5, sh, 1);
 }
 
 
 
 // ---------------------------------------------------------------------------
 // Stage kernels.  The stage input is built while the x-planes are staged; the epilogue
-// writes l_s, or applies the RK4 update at stage 4.  Theories of at most five components run
-// the gradient walk (sky_grad.cuh, k_grad_stage), rho the marching tile (sky_march.cuh,
-// k_march_stage).
+// writes l_s, or applies the RK4 update.  Every theory runs the gradient walk (sky_grad.cuh,
+// k_grad_stage); rho's is over the pion components, between a walk over the rho components
+// (sky_rho.cuh, k_rho_stage) and the rho components' epilogue (k_rho_finish).
 // ---------------------------------------------------------------------------
-// What a tile's stage reads and writes (both kernels).  `half`: stage 1 works on the new field
+// What a tile's stage reads and writes.  `half`: stage 1 works on the new field
 // of the step in flight (1) or, at admission and after a precision change, on the current one (0).
 template <typename T>
 struct StageIo {
@@ -278,6 +336,7 @@ struct StageIo {
     const T *F, *Flo, *V, *l1, *l2;  // stage 3: the update's operands (V null: zero; Flo null: not compensated)
     // stages 1, 2: l_s.  Stage 3: F', its low parts and P.  Stage 4: F' (read) and P -> V'.
     T *out, *out_lo, *pv;
+    T* R;  // rho: where the stage's walk over the rho components leaves R (components 4 .. 12)
     T dtt;
     bool l2_is_l1;
 };
@@ -312,16 +371,20 @@ __device__ __forceinline__ StageIo<T> stage_io(const InstDesc<T>& in, const Para
     io.out = STAGE == 1 ? in.L[l1_slot(in, half)] : STAGE == 2 ? in.L[1] : in.F[cur ^ 1];
     io.out_lo = in.Flo[cur ^ 1];
     io.pv = in.V[cur ^ 1];
+    // R lies where the stage's output will (stage 4: in the slope that it does not read)
+    io.R = STAGE < 3 ? io.out : STAGE == 3 ? io.pv : io.l2_is_l1 ? in.L[1] : in.L[l1_slot(in, 0)];
     return io;
 }
 
-// The maps of a tile's sources (null: the source reads as zero).
+// The maps of a tile's sources (null: the source reads as zero); tm: the instance's maps of the
+// walk's components.
 template <typename T, int STAGE>
-__device__ __forceinline__ void stage_maps(const InstDesc<T>& in, const StageIo<T>& io, int half, TmaTile& tt) {
+__device__ __forceinline__ void stage_maps(const InstDesc<T>& in, const TmaMap* tm, const StageIo<T>& io, int half,
+                                           TmaTile& tt) {
     const int cur = STAGE == 1 ? in.cur ^ half : in.cur;
-    tt.map[0] = &in.tm[kMapF + cur];
-    tt.map[1] = io.V != nullptr ? &in.tm[kMapV + cur] : nullptr;
-    tt.map[2] = STAGE > 2 ? &in.tm[kMapL + (STAGE == 3 || io.l2_is_l1 ? l1_slot(in, 0) : 1)] : nullptr;
+    tt.map[0] = &tm[kMapF + cur];
+    tt.map[1] = io.V != nullptr ? &tm[kMapV + cur] : nullptr;
+    tt.map[2] = STAGE > 2 ? &tm[kMapL + (STAGE == 3 || io.l2_is_l1 ? l1_slot(in, 0) : 1)] : nullptr;
     tt.status = in.status;
 }
 
@@ -533,6 +596,28 @@ struct GradEpi {
     }
 };
 
+// Rho: the walk over the pion components takes R at the site and leaves H in its place
+// (k_rho_finish applies it).
+template <typename T, int STAGE, bool WIDE, bool TMA>
+struct RhoGradEpi : GradEpi<T, STAGE, 4, WIDE, TMA, false> {
+    using B = GradEpi<T, STAGE, 4, WIDE, TMA, false>;
+    using V = typename Lanes<T>::V;
+    static constexpr bool kCoupled = true;
+    __device__ __forceinline__ void coupling(int64_t s, int64_t N, bool own1, V (&R)[9]) {
+#pragma unroll
+        for (int m = 0; m < 9; ++m) R[m] = B::get(B::io.R + B::at(4 + m, N, s), own1);
+    }
+    __device__ __forceinline__ void coupled(int64_t s, int64_t N, bool own1, const V (&J)[9], const Params& p) {
+        V R[9];  // (read again, not held)
+        coupling(s, N, own1, R);
+#pragma unroll
+        for (int m = 0; m < 9; ++m) B::store(B::io.R + B::at(4 + m, N, s), rho_rest(R[m], J[m], p), own1);
+    }
+};
+template <template <typename> class Th, typename T, int STAGE, class M, bool TMA>
+using StageEpi = typename std::conditional<Th<T>::kId == SKY_THEORY_RHO, RhoGradEpi<T, STAGE, M::WIDE, TMA>,
+                                           GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>>::type;
+
 // A finished tile's partials: stage 1 the baryon number and (FP64) the energy, stage 4 the
 // gradient maxima and the kinetic sum.
 template <typename T, int STAGE>
@@ -562,7 +647,7 @@ __device__ __forceinline__ void tile_partials(const InstDesc<T>& in, int lt, con
 }
 
 // Tail of a step's stage-4 and stage-1 launches (total > 0: their blocks together): the last
-// block of the two to finish runs the control of every active instance of the group, one warp
+// block of the two to finish runs the control of every active instance of the group, four warps
 // per instance, so a step needs no separate launch for it.  Each block publishes its partials
 // (fence) before it is counted; the counter returns to 0 for the next step.  The tail sits after
 // the tile loop so that its registers do not add to the stencil loop's.
@@ -581,10 +666,14 @@ __device__ __forceinline__ void stage_tail(InstDesc<T>* ctl, const int* tile_ins
             __syncthreads();
             if (last_block) {
                 __threadfence();
-                const int nw = int(blockDim.x * blockDim.y) >> 5;
+                __shared__ ControlSums sh[4][kControlWarps - 1];
+                const int ng = int(blockDim.x * blockDim.y) / (32 * kControlWarps);  // 1 to 4
+                const int g = ltid / (32 * kControlWarps);
                 const int i1 = __ldg(tile_inst + t_end - 1) + 1;
-                for (int i = __ldg(tile_inst + t_begin) + (ltid >> 5); i < i1; i += nw)
-                    if (ctl[i].active) engine_control_warp(ctl[i], 0);
+                if (g < ng)
+                    for (int i = __ldg(tile_inst + t_begin) + g; i < i1; i += ng)
+                        if (ctl[i].active)
+                            engine_control(ctl[i], 0, (ltid >> 5) % kControlWarps, sh[g], 1 + g);
                 if (ltid == 0) *done = 0;
             }
         }
@@ -631,10 +720,11 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
         const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
         int xa, xe, y0, z0;
         march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
-        using Epi = GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>;
-        Epi epi{stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
-                STAGE == 1 && half && refresh_due(in), {nullptr, nullptr, nullptr, nullptr},
-                {nullptr, nullptr, nullptr, nullptr}};
+        using Epi = StageEpi<Th, T, STAGE, M, TMA>;
+        Epi epi{GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>{
+            stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
+            STAGE == 1 && half && refresh_due(in), {nullptr, nullptr, nullptr, nullptr},
+            {nullptr, nullptr, nullptr, nullptr}}};
         epi.z0 = z0;
         epi.y0 = y0;
         // what the staged sources have not brought into L2 already
@@ -651,45 +741,270 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
             ahead(1, epi.io.pv, kMapV + (in.cur ^ 1));
         }
         ahead(3, in.Dlt, kMapDlt);
-        if constexpr (TMA) stage_maps<T, STAGE>(in, epi.io, half, tt);
+        if constexpr (TMA) stage_maps<T, STAGE>(in, in.tm, epi.io, half, tt);
         __syncthreads();  // the previous tile's readers of coef are done
         if (first) coef = in.coef;
         __syncthreads();
         KSum es{0.0, 0.0}, bs{0.0, 0.0};
-        const bool ok = grad_tile<Th, M, T, NSRC, STAGE == 1, Epi, T, TMA>(sm, p, coef, epi.io.src, epi.io.a, epi.io.b,
-                                                                           xa, xe, y0, z0, epi, es, bs, &tt);
+        constexpr bool own_energy = energy_walk<T>(Th<T>::kId);  // else stage 1 sums the energy
+        const bool ok = grad_tile<Th, M, T, NSRC, STAGE == 1 ? (own_energy ? 2 : 1) : 0, Epi, T, TMA>(
+            sm, p, coef, epi.io.src, epi.io.a, epi.io.b, xa, xe, y0, z0, epi, es, bs, &tt);
         if (!ok) break;  // a copy did not arrive; the error bit is set and the tile's partials stay stale
-        tile_partials<T, STAGE>(in, lt, es, bs, epi.st, sizeof(T) == 8, shk, shm);
+        tile_partials<T, STAGE>(in, lt, es, bs, epi.st, !own_energy, shk, shm);
     }
     grid_dep_launch();  // the next launch may be scheduled while the last blocks finish
     stage_tail<T, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
 }
 
 // ---------------------------------------------------------------------------
-// Energy of FP32 instances: the FP64 density of the field (high plus low parts of a
-// compensated one), evaluated in its own walk.  Each value is converted once as it enters an
-// FP64 ring.  (Inside stage 1 the 60 tap differences of a five-component site each needed an
-// exact FP32 difference and two conversions: half of that stage's instructions.)
+// Rho's first walk of a stage: R of the stage input (sky_rho.cuh), over tiles of its own, each of
+// which gives three items, one per isospin component.
 // ---------------------------------------------------------------------------
-constexpr int kEnergyRows = kDensRows;
+template <class M, typename T, int STAGE, bool TMA>
+constexpr size_t rho_stage_bytes() {
+    return RhoPipe<M, T, T, stage_nsrc<STAGE>(), TMA>::bytes + (TMA ? 128 : 0);
+}
 
-template <template <typename> class Th>
-struct EnergyOp {
-    const Params& p;
-    KSum sum;
-    __device__ __forceinline__ void operator()(int64_t, int, const double (&phi)[Th<double>::C],
-                                               const double (&D)[3][Th<double>::C]) {
-        ksum_add(sum, Th<double>::energy(phi, D, p));
+template <class M, typename T, int STAGE, int MINB, bool TMA>
+__global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
+    k_rho_stage(const InstDesc<T>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end,
+                int half) {
+    constexpr int NSRC = stage_nsrc<STAGE>();
+    extern __shared__ __align__(128) unsigned char smraw[];
+    T* sm = reinterpret_cast<T*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    __shared__ uint64_t tma_bar;
+    __shared__ MarchCoef<T> coef;
+    TmaTile tt{&tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    if constexpr (TMA) {
+        if (first) mbar_init(&tma_bar, 1);
+        __syncthreads();
+    }
+    grid_dep_wait();
+    for (int q = 3 * t_begin + blockIdx.x; q < 3 * t_end; q += gridDim.x) {
+        const int t = q / 3, a = q - 3 * t;
+        const InstDesc<T>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;  // uniform across the block
+        if (STAGE == 2 && l2_is_l1(in)) continue;
+        const Params p = in.p;
+        int xa, xe, y0, z0;
+        march_origin(in.r_grid, t - in.r_tile_begin, M::BY, xa, xe, y0, z0, p.X);
+        const StageIo<T> io = stage_io<T, STAGE>(in, p, half);
+        const int64_t N = n_sites(p), c0 = (4 + a) * N;
+        const T* const src[3] = {io.src[0] + c0, io.src[1] ? io.src[1] + c0 : nullptr, io.src[2] + c0};
+        if constexpr (TMA) {
+            stage_maps<T, STAGE>(in, in.tmr, io, half, tt);
+            tt.x0 = a * p.X;
+        }
+        __syncthreads();  // the previous tile's readers of coef are done
+        if (first) coef = in.coef;
+        __syncthreads();
+        if (!rho_tile<M, T, NSRC, T, TMA>(sm, p, coef, src, io.a, io.b, xa, xe, y0, z0, io.R + c0, 3 * N, 3 * N,
+                                              &tt))
+            break;
+    }
+    grid_dep_launch();
+}
+
+// Rho's last kernel of a stage: the rho components' gradient 8 m_rho^2 X - H and what the
+// epilogue of the gradient walk does with the pions' (the rho components are neither normalised
+// nor projected).  Element by element over the nine components, 16 bytes per thread and array, an
+// equal share of them per item.  In the epilogue of the pion walk the same work was a chain of
+// dependent L2 round trips per plane and spilled: that walk 67 us at stage 3 of 64^3 FP32 sites
+// and 82 of 57 x 50 x 45 FP64 ones.
+template <typename T>
+struct Vec16 {
+    static constexpr int W = 16 / int(sizeof(T));
+    T v[W];
+    __device__ __forceinline__ void load(const T* p, int n) {
+        if (n == W) {
+            using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+            const V4 q = __ldcg(reinterpret_cast<const V4*>(p));
+            memcpy(v, &q, 16);
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) v[i] = i < n ? __ldcg(p + i) : T(0);
+        }
+    }
+    __device__ __forceinline__ void store(T* p, int n) const {
+        if (n == W) {
+            using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+            V4 q;
+            memcpy(&q, v, 16);
+            __stcg(reinterpret_cast<V4*>(p), q);
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                if (i < n) __stcg(p + i, v[i]);
+        }
+    }
+};
+constexpr int kRhoFinishThreads = 256;
+constexpr int kRhoFinishSplit = 2;  // items per tile of the walk over the rho components
+
+template <typename T, int STAGE>
+__global__ void __launch_bounds__(kRhoFinishThreads)
+    k_rho_finish(const InstDesc<T>* __restrict__ insts, InstDesc<T>* ctl, const int* __restrict__ tile_inst,
+                 int t_begin, int t_end, int half, int* done, int total) {
+    using V = Vec16<T>;
+    constexpr int W = V::W;
+    __shared__ KSum shk[kRhoFinishThreads / 32];
+    __shared__ double shm[kRhoFinishThreads / 32];
+    grid_dep_wait();
+    constexpr int K = kRhoFinishSplit;
+    for (int u = K * t_begin + blockIdx.x; u < K * t_end; u += gridDim.x) {
+        const int t = u / K;
+        const InstDesc<T>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;  // uniform across the block
+        if (STAGE == 2 && l2_is_l1(in)) continue;
+        const Params p = in.p;
+        const int lt = u - K * in.r_tile_begin, items = K * in.r_grid.count();
+        const StageIo<T> io = stage_io<T, STAGE>(in, p, half);
+        const bool refresh = STAGE == 1 && half && refresh_due(in);
+        T* const dlt = in.Dlt;
+        StageStats<T> st(p.vol);
+        const int64_t N = n_sites(p), c0 = 4 * N, nv = (9 * N + W - 1) / W;  // (component 4 starts on 16 bytes)
+        const int64_t v0 = nv * lt / items, v1 = nv * (lt + 1) / items;
+        for (int64_t q = v0 + threadIdx.x; q < v1; q += kRhoFinishThreads) {
+            const int64_t j = c0 + q * W;
+            const int n = int(min(int64_t(W), 13 * N - j));
+            V x, v, l, l2, lo, d, h, pv;
+            x.load(io.src[0] + j, n);
+            h.load(io.R + j, n);
+            if (STAGE > 1 && io.src[1]) v.load(io.src[1] + j, n);
+            if (STAGE > 2) l.load(io.src[2] + j, n);
+            if (STAGE == 3 && !io.l2_is_l1) l2.load(io.l2 + j, n);
+            if (STAGE == 3 && io.Flo) lo.load(io.Flo + j, n);
+            if (STAGE == 4) pv.load(io.pv + j, n);
+            if (dlt) d.load(dlt + j, n);
+            V o1, o2, o3;
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                T X = x.v[i];
+                const T vi = STAGE > 1 && io.src[1] ? v.v[i] : T(0);
+                if (STAGE > 1) X += io.a * vi;
+                if (STAGE > 2) X += io.b * l.v[i];
+                T g = rho_gradient(X, h.v[i], p);
+                if (dlt) {
+                    if (refresh) {  // d = g64(F): the correction becomes g64 - g32(F)
+                        const T g64 = d.v[i];
+                        d.v[i] = g64 - g;
+                        g = g64;
+                    } else {
+                        g += d.v[i];
+                    }
+                }
+                if constexpr (STAGE < 3) {
+                    o1.v[i] = -io.dtt * g;
+                } else if constexpr (STAGE == 3) {
+                    const T F[1] = {x.v[i]}, Fl[1] = {io.Flo ? lo.v[i] : T(0)}, V0[1] = {vi};
+                    const T b1[1] = {l.v[i]}, b2[1] = {io.l2_is_l1 ? l.v[i] : l2.v[i]}, b3[1] = {-io.dtt * g};
+                    T of[1], ol[1], op[1];
+                    update_field<T, 1>(F, Fl, io.Flo != nullptr, V0, b1, b2, b3, io.dtt, 0, 0, of, ol, op);
+                    o1.v[i] = of[0], o2.v[i] = ol[0], o3.v[i] = op[0];
+                } else {
+                    const T q1[1] = {pv.v[i]}, gg[1] = {g};
+                    T o[1];
+                    const T v2 = update_velocity<T, 1>(q1, gg, q1, io.dtt, 0, 0, o);
+                    if (i < n) {
+                        st.gradient(g);
+                        st.velocity(v2);
+                    }
+                    o1.v[i] = o[0];
+                }
+            }
+            if (refresh && dlt) d.store(dlt + j, n);
+            o1.store((STAGE == 4 ? io.pv : io.out) + j, n);
+            if constexpr (STAGE == 3) {
+                if (io.Flo) o2.store(io.out_lo + j, n);
+                o3.store(io.pv + j, n);
+            }
+        }
+        if constexpr (STAGE == 4) tile_partials<T, STAGE>(in, in.ntiles + lt, KSum{}, KSum{}, st, false, shk, shm);
+    }
+    grid_dep_launch();
+    stage_tail<T, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
+}
+
+// ---------------------------------------------------------------------------
+// Small FP32 rho lattices: all thirteen components in one walk, one site per thread.  The three
+// kernels of a stage above are faster where they fill the GPU; up to kFusedRhoSites sites their
+// launches, their smaller tiles' halos and the separate energy cost more than they give.  Step in
+// us, fused / separate: FP32 48^3 148 / 171, 57 x 50 x 45 237 / 249, 64^3 252 / 243;
+// defect-corrected 48^3 168 / 204, 64^3 306 / 295, 72^3 505 / 421, 96^3 786 / 700.
+// ---------------------------------------------------------------------------
+template <class M, int STAGE, bool TMA>
+constexpr size_t rho_fused_bytes() {
+    return rho_march_bytes<M>(stage_nsrc<STAGE>(), TMA) + (TMA ? 128 : 0);
+}
+
+template <int STAGE>
+struct RhoFusedEpi {
+    static constexpr int C = 13;
+    StageIo<float> io;
+    StageStats<float> st;
+    int nsky, unit_length;
+    float* dlt;
+    bool refresh;  // stage 1 after the defect refresh: dlt holds g64 of the field; replace it by g64 - g32
+    __device__ __forceinline__ void operator()(int64_t s, int64_t N, float (&g)[C]) {
+        if (dlt) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float d = __ldcg(dlt + c * N + s);
+                if (STAGE == 1 && refresh) {
+                    __stcg(dlt + c * N + s, d - g[c]);
+                    g[c] = d;
+                } else {
+                    g[c] += d;
+                }
+            }
+        }
+        if constexpr (STAGE < 3) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) __stcg(io.out + c * N + s, -io.dtt * g[c]);
+        } else if constexpr (STAGE == 3) {
+            float f0[C], fl[C], v0[C], a1[C], a2[C], fo[C], lo[C], pv[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int64_t j = c * N + s;
+                f0[c] = __ldcg(io.F + j);
+                fl[c] = io.Flo ? __ldcg(io.Flo + j) : 0.0f;
+                v0[c] = io.V ? __ldcg(io.V + j) : 0.0f;
+                a1[c] = __ldcg(io.l1 + j);
+                a2[c] = io.l2_is_l1 ? a1[c] : __ldcg(io.l2 + j);
+                g[c] = -io.dtt * g[c];  // l3
+            }
+            update_field<float, C>(f0, fl, io.Flo != nullptr, v0, a1, a2, g, io.dtt, nsky, unit_length, fo, lo, pv);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int64_t j = c * N + s;
+                __stcg(io.out + j, fo[c]);
+                if (io.Flo) __stcg(io.out_lo + j, lo[c]);
+                __stcg(io.pv + j, pv[c]);
+            }
+        } else {
+            float fo[C], pv[C], vv[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                st.gradient(g[c]);
+                fo[c] = __ldcg(io.out + c * N + s);
+                pv[c] = __ldcg(io.pv + c * N + s);
+            }
+            st.velocity(update_velocity<float, C>(pv, g, fo, io.dtt, nsky, unit_length, vv));
+#pragma unroll
+            for (int c = 0; c < C; ++c) __stcg(io.pv + c * N + s, vv[c]);
+        }
     }
 };
 
-template <template <typename> class Th, class M, bool TMA>
-__global__ void __launch_bounds__(M::NTHREADS, 2)
-    k_energy(const InstDesc<float>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end,
-             int half) {
+template <class M, int STAGE, bool TMA>
+__global__ void __launch_bounds__(M::NTHREADS)
+    k_rho_fused(const InstDesc<float>* __restrict__ insts, InstDesc<float>* ctl, const int* __restrict__ tile_inst,
+                int t_begin, int t_end, int half, int* done, int total) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    double* sm = reinterpret_cast<double*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    float* sm = reinterpret_cast<float*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
     __shared__ KSum shk[M::NTHREADS / 32];
+    __shared__ double shm[M::NTHREADS / 32];
     __shared__ uint64_t tma_bar;
     TmaTile tt{&tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
     if constexpr (TMA) {
@@ -699,122 +1014,6 @@ __global__ void __launch_bounds__(M::NTHREADS, 2)
     grid_dep_wait();
     for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
         const InstDesc<float>& in = insts[__ldg(tile_inst + t)];
-        if (!in.active) continue;
-        const Params p = in.p;
-        const int lt = t - in.e_tile_begin, cur = in.cur ^ half;
-        const MarchGrid mg{in.e_nz, in.e_ny, in.e_nx, in.e_xc};
-        int xa, xe, y0, z0;
-        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
-        const float* const src[3] = {in.F[cur], in.Flo[cur], nullptr};
-        const double r1[3] = {in.r1d[0], in.r1d[1], in.r1d[2]};
-        if constexpr (TMA) {
-            tt.map[0] = &in.tme[kMapF + cur];
-            tt.map[1] = in.Flo[cur] != nullptr ? &in.tme[kMapFlo + cur] : nullptr;
-            tt.status = in.status;
-        }
-        EnergyOp<Th> op{p, KSum{0.0, 0.0}};
-        if (!dens_tile<M, float, 2, TMA>(sm, p, r1, src, xa, xe, y0, z0, op, &tt)) break;
-        const KSum e = block_ksum(op.sum, shk);
-        if (threadIdx.x == 0 && threadIdx.y == 0) in.epart[lt] = e;
-    }
-    grid_dep_launch();
-}
-
-// ---------------------------------------------------------------------------
-// Rho's stages (13 components): the marching tile, one site per thread.
-// ---------------------------------------------------------------------------
-template <typename T, int STAGE, int CC>
-struct EngineEpi {
-    StageIo<T> io;
-    StageStats<T> st;
-    int nsky, unit_length;
-    T* dlt;
-    int refresh;
-    template <int C>
-    __device__ __forceinline__ void operator()(int64_t s, int64_t N, const T (&)[C], const T (&g32)[C]) {
-        static_assert(C == CC, "component count");
-        T g[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) g[c] = g32[c];
-        if (dlt) {
-            if (STAGE == 1 && refresh) {  // dlt = g64(F): the correction becomes g64 - g32(F)
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    g[c] = __ldcg(dlt + c * N + s);
-                    __stcg(dlt + c * N + s, g[c] - g32[c]);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < C; ++c) g[c] = g32[c] + __ldcg(dlt + c * N + s);
-            }
-        }
-        if constexpr (STAGE < 3) {
-#pragma unroll
-            for (int c = 0; c < C; ++c) __stcg(io.out + c * N + s, -io.dtt * g[c]);
-        } else if constexpr (STAGE == 3) {
-            T f0[C], fl[C], v0[C], a1[C], a2[C], fo[C], lo[C], pv[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int64_t j = c * N + s;
-                f0[c] = __ldcg(io.F + j);
-                fl[c] = io.Flo ? __ldcg(io.Flo + j) : T(0);
-                v0[c] = io.V ? __ldcg(io.V + j) : T(0);
-                a1[c] = __ldcg(io.l1 + j);
-                a2[c] = io.l2_is_l1 ? a1[c] : __ldcg(io.l2 + j);
-                g[c] = -io.dtt * g[c];  // l3
-            }
-            update_field<T, C>(f0, fl, io.Flo != nullptr, v0, a1, a2, g, io.dtt, nsky, unit_length, fo, lo, pv);
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int64_t j = c * N + s;
-                __stcg(io.out + j, fo[c]);
-                if (io.Flo) __stcg(io.out_lo + j, lo[c]);
-                __stcg(io.pv + j, pv[c]);
-            }
-        } else {
-            T fo[C], pv[C], vv[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                st.gradient(g[c]);
-                fo[c] = __ldcg(io.out + c * N + s);
-                pv[c] = __ldcg(io.pv + c * N + s);
-            }
-            st.velocity(update_velocity<T, C>(pv, g, fo, io.dtt, nsky, unit_length, vv));
-#pragma unroll
-            for (int c = 0; c < C; ++c) __stcg(io.pv + c * N + s, vv[c]);
-        }
-    }
-};
-
-template <class M, typename T, int STAGE, bool TMA>
-constexpr size_t march_stage_bytes() {
-    constexpr int nsrc = stage_nsrc<STAGE>();
-    return TMA ? M::template smem_bytes_tma<T>(nsrc) + 128 : M::template smem_bytes<T>(nsrc);
-}
-
-template <template <typename> class Th, class M, typename T, int STAGE, bool TMA>
-__global__ void __launch_bounds__(M::NTHREADS)
-    k_march_stage(const InstDesc<T>* __restrict__ insts, InstDesc<T>* ctl, const int* __restrict__ tile_inst,
-                  int t_begin, int t_end, int half, int* done, int total) {
-    constexpr int NSRC = stage_nsrc<STAGE>();
-    extern __shared__ __align__(128) unsigned char smraw[];
-    // TMA box copies land on 128-byte boundaries: the launch adds 128 bytes of slack
-    // and the ring starts at the first 128-byte boundary of the dynamic segment
-    T* sm = reinterpret_cast<T*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
-    __shared__ KSum shk[M::NTHREADS / 32];
-    __shared__ double shm[M::NTHREADS / 32];
-    __shared__ uint64_t tma_bar[2];
-    TmaTile tt{tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
-    if constexpr (TMA) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            mbar_init(&tma_bar[0], 1);
-            mbar_init(&tma_bar[1], 1);
-        }
-        __syncthreads();
-    }
-    grid_dep_wait();
-    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
-        const InstDesc<T>& in = insts[__ldg(tile_inst + t)];
         if (!in.active) continue;  // uniform across the block
         if (STAGE == 2 && l2_is_l1(in)) continue;
         const Params p = in.p;
@@ -822,18 +1021,114 @@ __global__ void __launch_bounds__(M::NTHREADS)
         const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
         int xa, xe, y0, z0;
         march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
-        using Epi = EngineEpi<T, STAGE, M::C>;
-        Epi epi{stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
-                STAGE == 1 && half && refresh_due(in)};
-        if constexpr (TMA) stage_maps<T, STAGE>(in, epi.io, half, tt);
+        RhoFusedEpi<STAGE> epi{stage_io<float, STAGE>(in, p, half), StageStats<float>(p.vol), p.nsky, p.unit_length,
+                               in.Dlt, STAGE == 1 && half && refresh_due(in)};
+        if constexpr (TMA) stage_maps<float, STAGE>(in, in.tm, epi.io, half, tt);
         KSum es{0.0, 0.0}, bs{0.0, 0.0};
-        const bool ok = march_tile<Th, M, T, NSRC, STAGE == 1, Epi, false, T, true, TMA>(
+        const bool ok = rho_march_tile<M, stage_nsrc<STAGE>(), STAGE == 1, TMA>(
             sm, p, epi.io.src, epi.io.a, epi.io.b, xa, xe, y0, z0, epi, es, bs, TMA ? &tt : nullptr);
         if (!ok) break;  // a copy did not arrive; the error bit is set and the tile's partials stay stale
-        tile_partials<T, STAGE>(in, lt, es, bs, epi.st, true, shk, shm);
+        tile_partials<float, STAGE>(in, lt, es, bs, epi.st, true, shk, shm);
     }
-    grid_dep_launch();  // the next launch may be scheduled while the last blocks finish
-    stage_tail<T, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
+    grid_dep_launch();
+    stage_tail<float, STAGE>(ctl, tile_inst, t_begin, t_end, done, total);
+}
+
+// ---------------------------------------------------------------------------
+// Energy of FP32 instances, and of rho in both precisions: the FP64 density of the field (high
+// plus low parts of a compensated one), evaluated in its own walk.  An FP32 value is converted
+// once as it enters the FP64 ring.  (Inside stage 1 the 60 tap differences of a five-component site each needed an
+// exact FP32 difference and two conversions: half of that stage's instructions.)
+// ---------------------------------------------------------------------------
+
+//
+// FP32 rho: the thirteen components and their staged FP32 planes in one walk fill an SM with a
+// block of 192 threads (60 us at 64^3 sites, and nothing beside it).  So a walk over the rho
+// components, three at a time, sums their own part and leaves the curls, and one over the pions
+// reads them.  (FP64, where 256 threads fit, keeps one walk: 35 us at 57 x 50 x 45 sites, and 41
+// in two.)
+template <template <typename> class Th>
+struct EnergyOp {
+    const Params& p;
+    const double* curl;
+    int64_t N;
+    KSum sum;
+    static constexpr int C = Th<double>::C;
+    __device__ __forceinline__ void operator()(int64_t s, int, const double (&phi)[C], const double (&D)[3][C]) {
+        if constexpr (std::is_same<Th<double>, RhoPion<double>>::value) {
+            double R[9];
+#pragma unroll
+            for (int m = 0; m < 9; ++m) R[m] = __ldcg(curl + m * N + s);
+            ksum_add(sum, Th<double>::energy(phi, D, R, p));
+        } else {
+            ksum_add(sum, Th<double>::energy(phi, D, p));
+        }
+    }
+};
+struct CurlOp {
+    const Params& p;
+    double* curl;  // of the isospin component
+    int64_t N;
+    KSum sum;
+    __device__ __forceinline__ void operator()(int64_t s, int, const double (&r)[3], const double (&D)[3][3]) {
+        const double R[3] = {D[0][1] - D[1][0], D[0][2] - D[2][0], D[1][2] - D[2][1]};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) __stcg(curl + q * N + s, R[q]);
+        ksum_add(sum, RhoPion<double>::rho_energy(r, R, p));
+    }
+};
+
+// CURL: rho's walk over the rho components (M::C = 3, three items per tile).
+template <template <typename> class Th, class M, typename S, bool TMA, bool CURL>
+__global__ void __launch_bounds__(M::NTHREADS, M::C > 5 ? 1 : 2)
+    k_energy(const InstDesc<S>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end,
+             int half) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    double* sm = reinterpret_cast<double*>(smraw + (TMA ? ((128u - (smem_addr(smraw) & 127u)) & 127u) : 0u));
+    __shared__ KSum shk[M::NTHREADS / 32];
+    __shared__ uint64_t tma_bar;
+    constexpr int NSRC = std::is_same<S, double>::value ? 1 : 2;
+    constexpr bool SPLIT = std::is_same<Th<double>, RhoPion<double>>::value;
+    constexpr int PER = CURL ? 3 : 1;
+    TmaTile tt{&tma_bar, 0u, {nullptr, nullptr, nullptr}, nullptr};
+    if constexpr (TMA) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(&tma_bar, 1);
+        __syncthreads();
+    }
+    grid_dep_wait();
+    for (int u = PER * t_begin + blockIdx.x; u < PER * t_end; u += gridDim.x) {
+        const int t = u / PER, a = u - PER * t;
+        const InstDesc<S>& in = insts[__ldg(tile_inst + t)];
+        if (!in.active) continue;
+        const Params p = in.p;
+        const int lt = t - in.e_tile_begin, cur = in.cur ^ half;
+        const MarchGrid mg{in.e_nz, in.e_ny, in.e_nx, in.e_xc};
+        int xa, xe, y0, z0;
+        march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
+        const double r1[3] = {in.r1d[0], in.r1d[1], in.r1d[2]};
+        const int64_t N = n_sites(p), c0 = CURL ? (4 + a) * N : 0;
+        const S* const src[3] = {in.F[cur] + c0, in.Flo[cur] ? in.Flo[cur] + c0 : nullptr, nullptr};
+        if constexpr (TMA) {
+            const TmaMap* tm = CURL ? in.tmc : in.tme;
+            tt.map[0] = &tm[kMapF + cur];
+            tt.map[1] = in.Flo[cur] != nullptr ? &tm[kMapFlo + cur] : nullptr;
+            tt.x0 = a * p.X;
+            tt.status = in.status;
+        }
+        KSum sum;
+        if constexpr (CURL) {
+            CurlOp op{p, in.curl + 3 * a * N, N, KSum{0.0, 0.0}};
+            if (!dens_tile<M, S, NSRC, TMA, true>(sm, p, r1, src, xa, xe, y0, z0, op, &tt, 3 * N)) break;
+            sum = op.sum;
+        } else {
+            EnergyOp<Th> op{p, in.curl, N, KSum{0.0, 0.0}};
+            if (!dens_tile<M, S, NSRC, TMA>(sm, p, r1, src, xa, xe, y0, z0, op, &tt)) break;
+            sum = op.sum;
+        }
+        const KSum e = block_ksum(sum, shk);
+        if (threadIdx.x == 0 && threadIdx.y == 0) in.epart[SPLIT ? 4 * lt + (CURL ? 1 + a : 0) : lt] = e;
+    }
+    grid_dep_launch();
 }
 
 // ---------------------------------------------------------------------------
@@ -845,47 +1140,72 @@ __global__ void __launch_bounds__(M::NTHREADS)
 struct DefectEpi {
     float* dlt;
     template <int C>
-    __device__ __forceinline__ void operator()(int64_t s, int64_t N, const double (&)[C], const double (&g)[C]) {
+    __device__ __forceinline__ void operator()(int64_t s, int64_t N, bool, const double (&)[C], const double (&g)[C]) {
 #pragma unroll
         for (int c = 0; c < C; ++c) dlt[c * N + s] = float(g[c]);
     }
-    template <int C>
-    __device__ __forceinline__ void operator()(int64_t s, int64_t N, bool, const double (&phi)[C],
-                                               const double (&g)[C]) {
-        (*this)(s, N, phi, g);
+};
+// Rho: R_j^a of the new field, in FP64, lies in slope buffer a (all three are free between
+// stage 4 and the next stage 1).
+struct RhoDefectEpi : DefectEpi {
+    static constexpr bool kCoupled = true;
+    const double* r[3];
+    const float *F, *Flo;
+    __device__ __forceinline__ void coupling(int64_t s, int64_t N, bool, double (&R)[9]) {
+#pragma unroll
+        for (int m = 0; m < 9; ++m) R[m] = __ldcg(r[m % 3] + (m / 3) * N + s);
+    }
+    __device__ __forceinline__ void coupled(int64_t s, int64_t N, bool, const double (&J)[9], const Params& p) {
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            const int64_t j = (4 + m) * N + s;
+            const double x = double(__ldcg(F + j)) + double(__ldcg(Flo + j));
+            const double R = __ldcg(r[m % 3] + (m / 3) * N + s);
+            dlt[j] = float(rho_gradient(x, rho_rest(R, J[m], p), p));
+        }
     }
 };
 
-// TBY: rows of the engine's FP32 tiles; the FP64 ring walks each as TBY / M::BY sub-tiles
-// (4-row sub-tiles for 13 components, whose FP64 ring of 8-row planes would not fit).
-template <template <typename> class Th, class M, int TBY>
+// TBY: rows of the engine's FP32 tiles; the FP64 ring walks each as TBY / M::BY sub-tiles.
+// RHO: the walk over the rho components (three items per tile, M::C = 3), else the gradient walk.
+template <template <typename> class Th, class M, int TBY, bool RHO>
 __global__ void __launch_bounds__(M::NTHREADS, 1)
-    k_march_defect(InstDesc<float>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end) {
+    k_defect(InstDesc<float>* __restrict__ insts, const int* __restrict__ tile_inst, int t_begin, int t_end) {
     static_assert(TBY % M::BY == 0, "sub-tiles of the engine tile's rows");
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(128) unsigned char smraw[];
     double* sm = reinterpret_cast<double*>(smraw);
+    constexpr int PER = RHO ? 3 : 1;
     grid_dep_wait();
-    for (int t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
-        const int ii = __ldg(tile_inst + t);
-        const InstDesc<float>& in = insts[ii];
+    for (int q = PER * t_begin + blockIdx.x; q < PER * t_end; q += gridDim.x) {
+        const int t = q / PER, a = q - PER * t;
+        const InstDesc<float>& in = insts[__ldg(tile_inst + t)];
         if (!in.active || !refresh_due(in)) continue;  // uniform across the block
         const Params p = in.p;
-        const int lt = t - in.tile_begin;
         const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
         int xa, xe, y0, z0;
-        march_origin(mg, lt, TBY, xa, xe, y0, z0, p.X);
-        const float* const src[3] = {in.F[in.cur ^ 1], in.Flo[in.cur ^ 1], nullptr};  // the new field
-        DefectEpi epi{in.Dlt};
-        KSum es{0.0, 0.0}, bs{0.0, 0.0};
-        [[maybe_unused]] MarchCoef<double> k;
-        if constexpr (M::C <= 5) k.init(p);
+        march_origin(mg, t - in.tile_begin, TBY, xa, xe, y0, z0, p.X);
+        const float *F = in.F[in.cur ^ 1], *Flo = in.Flo[in.cur ^ 1];  // the new field
+        const int64_t N = n_sites(p);
+        MarchCoef<double> k;
+        k.init(p);
         for (int sy = 0; sy < TBY && y0 + sy < p.Y; sy += M::BY) {
-            if constexpr (M::C <= 5)
-                grad_tile<Th, M, double, 2, 0, DefectEpi, float>(sm, p, k, src, 1.0, 0.0, xa, xe, y0 + sy, z0, epi, es,
-                                                                 bs);
-            else
-                march_tile<Th, M, double, 2, false, DefectEpi, false, float>(sm, p, src, 1.0, 0.0, xa, xe, y0 + sy,
-                                                                             z0, epi, es, bs);
+            if constexpr (RHO) {
+                const int64_t c0 = (4 + a) * N;
+                const float* const src[3] = {F + c0, Flo + c0, nullptr};
+                rho_tile<M, double, 2, float>(sm, p, k, src, 1.0, 0.0, xa, xe, y0 + sy, z0,
+                                              reinterpret_cast<double*>(in.L[a]), N, 3 * N);
+            } else {
+                const float* const src[3] = {F, Flo, nullptr};
+                KSum es{0.0, 0.0}, bs{0.0, 0.0};
+                using Epi = typename std::conditional<Th<double>::kId == SKY_THEORY_RHO, RhoDefectEpi, DefectEpi>::type;
+                Epi epi{DefectEpi{in.Dlt}};
+                if constexpr (HasCoupling<Epi>::value) {
+                    for (int i = 0; i < 3; ++i) epi.r[i] = reinterpret_cast<const double*>(in.L[i]);
+                    epi.F = F;
+                    epi.Flo = Flo;
+                }
+                grad_tile<Th, M, double, 2, 0, Epi, float>(sm, p, k, src, 1.0, 0.0, xa, xe, y0 + sy, z0, epi, es, bs);
+            }
         }
     }
 }
@@ -921,7 +1241,7 @@ template <template <typename> class Th, class M, typename S>
 __global__ void __launch_bounds__(M::NTHREADS, 1)
     k_engine_audit(const InstDesc<S>* __restrict__ d, MarchGrid mg, double* __restrict__ parts) {
     constexpr int NSRC = std::is_same<S, double>::value ? 1 : 2;
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(128) unsigned char smraw[];
     double* sm = reinterpret_cast<double*>(smraw);
     __shared__ KSum shk[M::NTHREADS / 32];
     const Params p = d->p;

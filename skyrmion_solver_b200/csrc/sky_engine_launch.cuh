@@ -13,22 +13,21 @@ namespace sky {
 // ---------------------------------------------------------------------------
 // shapes and launches per (theory, precision)
 // ---------------------------------------------------------------------------
-// Theories of at most five components run the gradient walk (sky_grad.cuh) in both precisions,
-// rho the marching tile (sky_march.cuh).
+// The theory of the stages' gradient walk: rho's is over the pion components and follows a walk
+// over the rho components (sky_rho.cuh).
 template <template <typename> class Th>
-constexpr bool is_walk() {
-    return Th<float>::C <= 5;
+constexpr bool is_rho() {
+    return Th<float>::kId == SKY_THEORY_RHO;
 }
 // Rows of a stage tile (32 columns).  FP64 walks: grad_rows64.  FP32 walks, which compute two
 // sites per thread: rows and blocks per SM such that the ring, one staging slot and G and H of
 // all blocks fit the SM's shared memory and the registers do not spill.  Gradient of 128^3 /
 // 64^3 sites, in us: nuclear 16 rows x 2 blocks 54 / 13, 8 x 3 62 / 13; omega 8 x 3 40 / 9,
 // 16 x 2 41 / 11; Coulomb 12 x 2 73 / 17, 8 x 2 80 / 15, 16 x 1 83 / 15 (one site per thread,
-// 8 rows x 2 blocks: 83 / 17, 60 / 14, 103 / 21).  Rho: 8 rows, or 4 in FP64, whose ring takes
-// 150 KB then (narrow rows only, two of stage 3/4's three sources staged).
+// 8 rows x 2 blocks: 83 / 17, 60 / 14, 103 / 21).  Omega's stages as a whole run 12 x 2, and
+// rho's, whose walk over the pions spills with 16.
 template <template <typename> class Th, typename T>
 constexpr int stage_rows() {
-    if (!is_walk<Th>()) return sizeof(T) == 8 ? 4 : 8;
     if (sizeof(T) == 8) return grad_rows64<Th>(true);
     constexpr int id = Th<float>::kId;
     return (id == SKY_THEORY_NUCLEAR || id == SKY_THEORY_LIGHTLY_BOUND) ? 16 : 12;
@@ -36,33 +35,45 @@ constexpr int stage_rows() {
 // Resident blocks per SM the stages are compiled for, and their x-chunks chosen with.
 template <template <typename> class Th, typename T>
 constexpr int stage_blocks() {
-    return (sizeof(T) == 4 && is_walk<Th>()) ? 2 : 1;
+    return sizeof(T) == 4 ? 2 : 1;
 }
-// Wide-row (16-byte copies) or narrow-row shape; FP64 rho has narrow rows only.
-template <template <typename> class Th, typename T>
-constexpr bool wide_allowed() {
-    return is_walk<Th>() || sizeof(T) == 4;
-}
+template <int C, template <typename> class Th, typename T, bool WIDE>
+using WalkShape = MarchShape<C, stage_rows<Th, T>(), WIDE, sizeof(T) == 8 ? 2 : 4>;
 template <template <typename> class Th, typename T, bool WIDE>
-using MShape = MarchShape<Th<T>::C, stage_rows<Th, T>(), WIDE && wide_allowed<Th, T>(),
-                          (sizeof(T) == 8 && is_walk<Th>()) ? 2 : 4>;
+using MShape = WalkShape<is_rho<Th>() ? 4 : Th<T>::C, Th, T, WIDE>;
 
 template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
 struct StageKernel {
     using M = MShape<Th, T, WIDE>;
     static auto kern() {
-        if constexpr (is_walk<Th>())
-            return k_grad_stage<Th, M, T, STAGE, stage_blocks<Th, T>(), TMA>;
+        if constexpr (is_rho<Th>())
+            return k_grad_stage<RhoPion, M, T, STAGE, stage_blocks<Th, T>(), TMA>;
         else
-            return k_march_stage<Th, M, T, STAGE, TMA>;
+            return k_grad_stage<Th, M, T, STAGE, stage_blocks<Th, T>(), TMA>;
     }
     static size_t smem() {
-        if constexpr (is_walk<Th>())
-            return grad_stage_bytes<Th, M, T, STAGE, TMA>();
+        if constexpr (is_rho<Th>())
+            return grad_stage_bytes<RhoPion, M, T, STAGE, TMA>();
         else
-            return march_stage_bytes<M, T, STAGE, TMA>();
+            return grad_stage_bytes<Th, M, T, STAGE, TMA>();
     }
-    static dim3 block() { return is_walk<Th>() ? dim3(GradBlock<M, T>::TZ, M::BY) : dim3(M::BZ, M::BY); }
+    static dim3 block() { return dim3(GradBlock<M, T>::TZ, M::BY); }
+};
+// Rho: the stage's walk over the rho components.
+template <typename T>
+constexpr int rho_rows() {
+    return sizeof(T) == 8 ? 8 : 12;
+}
+template <typename T>
+constexpr int rho_blocks() {
+    return sizeof(T) == 8 ? 2 : 3;
+}
+template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+struct RhoKernel {
+    using M = MarchShape<3, rho_rows<T>(), WIDE, sizeof(T) == 8 ? 2 : 4>;
+    static auto kern() { return k_rho_stage<M, T, STAGE, rho_blocks<T>(), TMA>; }
+    static size_t smem() { return rho_stage_bytes<M, T, STAGE, TMA>(); }
+    static dim3 block() { return dim3(GradBlock<M, T>::TZ, M::BY); }
 };
 
 // One-time kernel attribute setup (kept out of stream capture); returns the
@@ -80,10 +91,9 @@ static int kernel_setup(K kern, size_t smem, int threads, int* per_sm) {
     return SKY_OK;
 }
 
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+template <class SK>
 static int stage_setup(int* per_sm_out) {
     static int per_sm = 0;
-    using SK = StageKernel<Th, T, STAGE, WIDE, TMA>;
     if (per_sm == 0) {
         const dim3 b = SK::block();
         const int rc = kernel_setup(SK::kern(), SK::smem(), int(b.x * b.y), &per_sm);
@@ -93,10 +103,13 @@ static int stage_setup(int* per_sm_out) {
     return SKY_OK;
 }
 
-// Launch with programmatic dependent launch when option 4 asks for it.
+// Launch, programmatically dependent on its predecessor where `chained` (the kernel follows it in
+// the same stream, with no event in between) or when option 4 asks for it everywhere.  Every kernel
+// of a step waits for its predecessor before it reads anything, so the dependence is transitive; what
+// overlaps is the launch.
 template <class... Args, class... Given>
-static int launch_pdl(void (*kern)(Args...), int blocks, dim3 block, size_t smem, cudaStream_t st, Given... args) {
-    if (option(4) == 1) {
+static int launch_chain(bool chained, void (*kern)(Args...), int blocks, dim3 block, size_t smem, cudaStream_t st, Given... args) {
+    if (chained || option(4) == 1) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -115,68 +128,106 @@ static int launch_pdl(void (*kern)(Args...), int blocks, dim3 block, size_t smem
 
 template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
 static int launch_stage_w(const Group& g, const StageArgs& a, cudaStream_t st) {
+    using SK = StageKernel<Th, T, STAGE, WIDE, TMA>;
     int per_sm = 1;
-    int rc = stage_setup<Th, T, STAGE, WIDE, TMA>(&per_sm);
+    int rc = stage_setup<SK>(&per_sm);
     if (rc) return rc;
     const int n = a.t_end - a.t_begin;
     if (n <= 0) return SKY_OK;
+    InstDesc<T>* d = reinterpret_cast<InstDesc<T>*>(g.d_desc);
+    if constexpr (is_rho<Th>()) {
+        using RK = RhoKernel<Th, T, STAGE, WIDE, TMA>;
+        int rho_per_sm = 1;
+        if ((rc = stage_setup<RK>(&rho_per_sm))) return rc;
+        const int resident = num_sms() * rho_per_sm, items = 3 * (a.r_end - a.r_begin);
+        if ((rc = launch_chain(a.chained, RK::kern(), items < resident ? items : resident, RK::block(), RK::smem(), st, d,
+                             g.d_tile_inst + g.ntiles + g.entiles, a.r_begin, a.r_end, a.in_step)))
+            return rc;
+    }
     const int blocks = n < num_sms() * per_sm ? n : num_sms() * per_sm;
     int total = 0;
-    if (a.in_step && (STAGE == 1 || STAGE == 4)) {  // both launches that share the step's tail counter
+    const bool tail = a.in_step && (STAGE == 1 || STAGE == 4);  // both stages' last launches share the tail counter
+    if constexpr (is_rho<Th>()) {
+        if ((rc = launch_chain(true, SK::kern(), blocks, SK::block(), SK::smem(), st, d, d, g.d_tile_inst, a.t_begin,
+                               a.t_end, a.in_step, g.d_done, 0)))
+            return rc;
+        const int fi = kRhoFinishSplit * (a.r_end - a.r_begin), fb = fi < 4 * num_sms() ? fi : 4 * num_sms();
+        if (tail) total = 2 * fb;
+        return launch_chain(true, k_rho_finish<T, STAGE>, fb, dim3(kRhoFinishThreads), 0, st, d, d,
+                          g.d_tile_inst + g.ntiles + g.entiles, a.r_begin, a.r_end, a.in_step, g.d_done, total);
+    }
+    if (tail) {
         int other = 1;
-        if ((rc = stage_setup<Th, T, STAGE == 1 ? 4 : 1, WIDE, TMA>(&other))) return rc;
+        if ((rc = stage_setup<StageKernel<Th, T, STAGE == 1 ? 4 : 1, WIDE, TMA>>(&other))) return rc;
         total = blocks + (n < num_sms() * other ? n : num_sms() * other);
     }
-    InstDesc<T>* d = reinterpret_cast<InstDesc<T>*>(g.d_desc);
-    using SK = StageKernel<Th, T, STAGE, WIDE, TMA>;
-    return launch_pdl(SK::kern(), blocks, SK::block(), SK::smem(), st, d, d, g.d_tile_inst, a.t_begin, a.t_end,
+    return launch_chain(a.chained, SK::kern(), blocks, SK::block(), SK::smem(), st, d, d, g.d_tile_inst, a.t_begin, a.t_end,
                       a.in_step, g.d_done, total);
 }
 
 template <template <typename> class Th, typename T, int STAGE>
 static int launch_stage(const Group& g, const StageArgs& a, cudaStream_t st) {
-    if constexpr (wide_allowed<Th, T>()) {
+    // (FP64 rho has no TMA maps: tma_possible)
+    if constexpr (!(is_rho<Th>() && sizeof(T) == 8)) {
         if (g.all_tma) return launch_stage_w<Th, T, STAGE, true, true>(g, a, st);
-        if (g.all_wide) return launch_stage_w<Th, T, STAGE, true, false>(g, a, st);
     }
+    if (g.all_wide) return launch_stage_w<Th, T, STAGE, true, false>(g, a, st);
     return launch_stage_w<Th, T, STAGE, false, false>(g, a, st);
 }
 
-// Energy walk of a group's FP32 instances (theories of at most five components; the others'
-// energy is summed by stage 1), energy tiles [t_begin, t_end).
-template <template <typename> class Th, bool WIDE, bool TMA>
-static int energy_setup(int* per_sm_out) {
-    static int per_sm = 0;
-    using M = MarchShape<Th<double>::C, kEnergyRows, WIDE, 4>;
-    using Pipe = DensPipe<M, float, 2, TMA>;
-    if (per_sm == 0) {
-        const int rc = kernel_setup(k_energy<Th, M, TMA>, Pipe::bytes + (TMA ? 128 : 0), M::NTHREADS, &per_sm);
-        if (rc) return rc;
-    }
-    *per_sm_out = per_sm;
-    return SKY_OK;
+// Energy walk of a group's instances (energy_walk), energy tiles [t_begin, t_end).  CURL: FP32 rho's
+// walk over the rho components, which comes first.
+template <template <typename> class Th, typename T>
+constexpr bool split_energy() {
+    return is_rho<Th>() && sizeof(T) == 4;
 }
-template <template <typename> class Th, bool WIDE, bool TMA>
-static int launch_energy_w(const Group& g, const StageArgs& a, cudaStream_t st) {
-    using M = MarchShape<Th<double>::C, kEnergyRows, WIDE, 4>;
-    using Pipe = DensPipe<M, float, 2, TMA>;
+template <template <typename> class Th, typename T, bool WIDE, bool TMA, bool CURL>
+struct EnergyKernel {
+    using M = MarchShape<CURL ? 3 : split_energy<Th, T>() ? 4 : Th<double>::C, kDensRows, WIDE, sizeof(T) == 8 ? 2 : 4>;
+    using Pipe = DensPipe<M, T, sizeof(T) == 8 ? 1 : 2, TMA, CURL>;
+    static auto kern() {
+        if constexpr (split_energy<Th, T>())
+            return k_energy<RhoPion, M, T, TMA, CURL>;
+        else
+            return k_energy<Th, M, T, TMA, CURL>;
+    }
+    static size_t smem() { return Pipe::bytes + (TMA ? 128 : 0); }
+    static dim3 block() { return dim3(M::BZ, M::BY); }
+};
+template <class EK, typename T>
+static int launch_energy_k(const Group& g, const StageArgs& a, int per, cudaStream_t st) {
     int per_sm = 1;
-    int rc = energy_setup<Th, WIDE, TMA>(&per_sm);
+    int rc = stage_setup<EK>(&per_sm);
     if (rc) return rc;
-    const int n = a.t_end - a.t_begin;
+    const int n = per * (a.t_end - a.t_begin);
     if (n <= 0) return SKY_OK;
     const int blocks = n < num_sms() * per_sm ? n : num_sms() * per_sm;
-    return launch_pdl(k_energy<Th, M, TMA>, blocks, dim3(M::BZ, M::BY), Pipe::bytes + (TMA ? 128 : 0), st,
-                      reinterpret_cast<InstDesc<float>*>(g.d_desc), g.d_tile_inst + g.ntiles, a.t_begin, a.t_end,
-                      a.in_step);
+    return launch_chain(a.chained, EK::kern(), blocks, EK::block(), EK::smem(), st, reinterpret_cast<InstDesc<T>*>(g.d_desc),
+                      g.d_tile_inst + g.ntiles, a.t_begin, a.t_end, a.in_step);
+}
+template <template <typename> class Th, typename T, bool WIDE, bool TMA>
+static int launch_energy_w(const Group& g, const StageArgs& a, cudaStream_t st) {
+    if constexpr (split_energy<Th, T>()) {
+        const int rc = launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, true>, T>(g, a, 3, st);
+        if (rc) return rc;
+        StageArgs b = a;
+        b.chained = 1;
+        return launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, false>, T>(g, b, 1, st);
+    }
+    return launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, false>, T>(g, a, 1, st);
+}
+template <template <typename> class Th, typename T>
+static int launch_energy_p(const Group& g, const StageArgs& a, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+        if (g.all_tma) return launch_energy_w<Th, T, true, true>(g, a, st);
+    }
+    if (g.all_wide) return launch_energy_w<Th, T, true, false>(g, a, st);
+    return launch_energy_w<Th, T, false, false>(g, a, st);
 }
 template <template <typename> class Th>
 static int launch_energy_t(const Group& g, const StageArgs& a, cudaStream_t st) {
-    if constexpr (is_walk<Th>()) {
-        if (g.all_tma) return launch_energy_w<Th, true, true>(g, a, st);
-        if (g.all_wide) return launch_energy_w<Th, true, false>(g, a, st);
-        return launch_energy_w<Th, false, false>(g, a, st);
-    }
+    if (!g.prec) return launch_energy_p<Th, float>(g, a, st);
+    if constexpr (energy_walk<double>(Th<double>::kId)) return launch_energy_p<Th, double>(g, a, st);
     return SKY_OK;
 }
 template <template <typename> class Th, typename T>
@@ -194,28 +245,39 @@ static int stage_dispatch_prec(int prec, int stage, const Group& g, const StageA
     return prec ? launch_stage_any<Th, double>(stage, g, a, st) : launch_stage_any<Th, float>(stage, g, a, st);
 }
 
+template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+static int setup_stage() {
+    int n, rc = stage_setup<StageKernel<Th, T, STAGE, WIDE, TMA>>(&n);
+    if constexpr (is_rho<Th>()) {
+        if (!rc) rc = stage_setup<RhoKernel<Th, T, STAGE, WIDE, TMA>>(&n);
+    }
+    return rc;
+}
 template <template <typename> class Th, typename T, bool WIDE, bool TMA>
 static int setup_stages() {
     int n, rc;
-    if ((rc = stage_setup<Th, T, 1, WIDE, TMA>(&n)) || (rc = stage_setup<Th, T, 2, WIDE, TMA>(&n)) ||
-        (rc = stage_setup<Th, T, 3, WIDE, TMA>(&n)) || (rc = stage_setup<Th, T, 4, WIDE, TMA>(&n)))
+    if ((rc = setup_stage<Th, T, 1, WIDE, TMA>()) || (rc = setup_stage<Th, T, 2, WIDE, TMA>()) ||
+        (rc = setup_stage<Th, T, 3, WIDE, TMA>()) || (rc = setup_stage<Th, T, 4, WIDE, TMA>()))
         return rc;
-    if constexpr (sizeof(T) == 4 && is_walk<Th>()) return energy_setup<Th, WIDE, TMA>(&n);
-    return SKY_OK;
-}
-template <template <typename> class Th, typename T>
-static int setup_all() {
-    int rc;
-    if ((rc = setup_stages<Th, T, false, false>())) return rc;
-    if constexpr (wide_allowed<Th, T>()) {
-        if ((rc = setup_stages<Th, T, true, false>()) || (rc = setup_stages<Th, T, true, true>())) return rc;
+    if constexpr (energy_walk<T>(Th<T>::kId)) {
+        if constexpr (split_energy<Th, T>()) {
+            if ((rc = stage_setup<EnergyKernel<Th, T, WIDE, TMA, true>>(&n))) return rc;
+        }
+        return stage_setup<EnergyKernel<Th, T, WIDE, TMA, false>>(&n);
     }
     return SKY_OK;
 }
-
+template <template <typename> class Th, typename T>
+static int setup_prec(const Group& g) {
+    if constexpr (!(is_rho<Th>() && sizeof(T) == 8)) {
+        if (g.all_tma) return setup_stages<Th, T, true, true>();
+    }
+    return g.all_wide ? setup_stages<Th, T, true, false>() : setup_stages<Th, T, false, false>();
+}
+// Kernel attributes of the variants that a group's steps launch (kept out of stream capture).
 template <template <typename> class Th>
-static int setup_prec(int prec) {
-    return prec ? setup_all<Th, double>() : setup_all<Th, float>();
+static int setup_group_kernels(const Group& g) {
+    return g.prec ? setup_prec<Th, double>(g) : setup_prec<Th, float>(g);
 }
 
 // Tile geometry of a (theory, precision): rows of its stage tiles, the resident blocks per SM
@@ -223,45 +285,51 @@ static int setup_prec(int prec) {
 // not depend on the staging, so neither does the order of the per-tile partial sums.
 template <template <typename> class Th>
 static TileShapeInfo shape_of(int prec) {
-    return prec ? TileShapeInfo{stage_rows<Th, double>(), stage_blocks<Th, double>(), MShape<Th, double, true>::HZ}
-                : TileShapeInfo{stage_rows<Th, float>(), stage_blocks<Th, float>(), MShape<Th, float, true>::HZ};
+    return prec ? TileShapeInfo{stage_rows<Th, double>(), stage_blocks<Th, double>(), MShape<Th, double, true>::HZ,
+                                MShape<Th, double, true>::C, rho_rows<double>(),
+                                rho_blocks<double>()}
+                : TileShapeInfo{stage_rows<Th, float>(), stage_blocks<Th, float>(), MShape<Th, float, true>::HZ,
+                                MShape<Th, float, true>::C, rho_rows<float>(),
+                                rho_blocks<float>()};
 }
 
-// Defect refresh of the group's defect-corrected FP32 instances (those whose
-// refresh flag the stage-4 advance just set; the others' tiles are skipped).
-template <template <typename> class Th, bool WIDE>
-static int launch_defect_t(const Group& g, cudaStream_t st) {
-    // 4-row sub-tiles of an engine tile's rows, or 8 where they divide them and the ring fits
-    constexpr int rows = is_walk<Th>() && stage_rows<Th, float>() % 8 == 0 ? 8 : 4;
-    using M = MarchShape<Th<double>::C, rows, WIDE && is_walk<Th>()>;
-    auto kern = k_march_defect<Th, M, stage_rows<Th, float>()>;
-    size_t smem;
-    if constexpr (is_walk<Th>())
-        smem = GradPipe<Th, M, double, float, 2, false>::bytes;
-    else
-        smem = M::template smem_bytes<double, float>(2);
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(defect)", __LINE__);
-        if (rc) return rc;
-        int n = 0;
-        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, M::NTHREADS, smem), "occupancy",
-                        __LINE__);
-        if (rc) return rc;
-        per_sm = n < 1 ? 1 : n;
-    }
-    const int n = g.ntiles;
+// Defect refresh of the group's defect-corrected FP32 instances (those whose refresh is due; the
+// others' tiles are skipped).
+template <class M, int PER, class K>
+static int launch_defect_k(bool chained, K kern, size_t smem, int* per_sm, const Group& g, cudaStream_t st) {
+    int rc;
+    if (*per_sm == 0 && (rc = kernel_setup(kern, smem, M::NTHREADS, per_sm))) return rc;
+    const int n = PER * g.ntiles;
     if (n <= 0) return SKY_OK;
-    const int blocks = n < num_sms() * per_sm ? n : num_sms() * per_sm;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(reinterpret_cast<InstDesc<float>*>(g.d_desc), g.d_tile_inst, 0,
-                                                   n);
-    return check_cuda(cudaGetLastError(), "launch defect refresh", __LINE__);
+    const int blocks = n < num_sms() * *per_sm ? n : num_sms() * *per_sm;
+    return launch_chain(chained, kern, blocks, dim3(M::BZ, M::BY), smem, st,
+                        reinterpret_cast<InstDesc<float>*>(g.d_desc), g.d_tile_inst, 0, g.ntiles);
+}
+// TBY: rows of the stage tiles.
+template <template <typename> class Th, int TBY, bool WIDE>
+static int launch_defect_t(const Group& g, cudaStream_t st) {
+    // two sub-tiles of a 16-row engine tile, one of the others
+    constexpr int rows = TBY == 16 ? 8 : TBY;
+    static int per_sm = 0;
+    if constexpr (is_rho<Th>()) {
+        using R = MarchShape<3, rows, WIDE>;
+        using M = MarchShape<4, rows, WIDE>;
+        static int rho_per_sm = 0;
+        const int rc = launch_defect_k<R, 3>(false, k_defect<RhoPion, R, TBY, true>,
+                                             RhoPipe<R, double, float, 2, false>::bytes, &rho_per_sm, g, st);
+        if (rc) return rc;
+        return launch_defect_k<M, 1>(true, k_defect<RhoPion, M, TBY, false>,
+                                     GradPipe<RhoPion, M, double, float, 2, false>::bytes, &per_sm, g, st);
+    } else {
+        using M = MarchShape<Th<double>::C, rows, WIDE>;
+        return launch_defect_k<M, 1>(false, k_defect<Th, M, TBY, false>, GradPipe<Th, M, double, float, 2, false>::bytes,
+                                     &per_sm, g, st);
+    }
 }
 
-template <template <typename> class Th>
+template <template <typename> class Th, int TBY = stage_rows<Th, float>()>
 static int launch_defect_w(const Group& g, cudaStream_t st) {
-    return g.all_wide ? launch_defect_t<Th, true>(g, st) : launch_defect_t<Th, false>(g, st);
+    return g.all_wide ? launch_defect_t<Th, TBY, true>(g, st) : launch_defect_t<Th, TBY, false>(g, st);
 }
 
 // Energy audit of the RK4 dynamics (k_engine_audit).
@@ -322,7 +390,7 @@ static int audit_prec(const Group& g, const HostInst& h, cudaStream_t st, double
 
 template <template <typename> class Th>
 constexpr TheoryOps make_ops() {
-    return TheoryOps{shape_of<Th>, setup_prec<Th>, stage_dispatch_prec<Th>, launch_energy_t<Th>, launch_defect_w<Th>,
+    return TheoryOps{shape_of<Th>, setup_group_kernels<Th>, stage_dispatch_prec<Th>, launch_energy_t<Th>, launch_defect_w<Th>,
                      audit_prec<Th>};
 }
 

@@ -1,5 +1,5 @@
 // Gradient walk: one (y, z) tile of a lattice marched along x, for the theories with at
-// most five components.  It evaluates the energy gradient at every site of the stage
+// most five components (and rho's pions, sky_rho.cuh).  It evaluates the energy gradient at every site of the stage
 // input X = F + a V + b L and hands it to an epilogue; stage 1 also sums the FP64 energy
 // and baryon densities.
 //
@@ -73,6 +73,13 @@ struct HasGradBegin : std::false_type {};
 template <class E>
 struct HasGradBegin<E, std::void_t<decltype(std::declval<E&>().begin_site(int64_t(0), int64_t(0), true))>>
     : std::true_type {};
+
+// coupling(s, N, own1, R) and coupled(s, N, own1, J, p): what a walk over the pion components
+// (RhoPion) takes from and leaves for the other fields at the site.
+template <class E, class = void>
+struct HasCoupling : std::false_type {};
+template <class E>
+struct HasCoupling<E, std::void_t<decltype(E::kCoupled)>> : std::true_type {};
 
 __device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
@@ -150,7 +157,9 @@ __device__ __forceinline__ void axpy16(double2& v, double a, const double2& u) {
 // S != T (float arrays, FP64 ring): every source is staged and converted; X = F + a V.
 // Planes outside the lattice and points outside it in y and z read as zero.
 // ---------------------------------------------------------------------------
-template <class M, typename T, typename S, int NSRC, bool TMA, int NT, int R_ = 6>
+// STRIDED: the walk's components are not consecutive (every third of the rho field's nine): the
+// caller gives their stride, and TMA reads one map of 3 X planes per component (TmaTile::x0).
+template <class M, typename T, typename S, int NSRC, bool TMA, int NT, int R_ = 6, bool STRIDED = false>
 struct PlanePipe {
     static constexpr bool SAME = std::is_same<S, T>::value;
     static constexpr bool DIRECT = SAME && NSRC == 1;
@@ -182,10 +191,10 @@ struct PlanePipe {
     PO po;
 
     __device__ __forceinline__ PlanePipe(T* sm, const Params& p, const S* const (&src_)[3], T a, T b, int tid_, int y0_,
-                                         int z0_, TmaTile* tma_)
+                                         int z0_, TmaTile* tma_, int64_t cstride = 0)
         : ring(sm), stage(reinterpret_cast<S*>(reinterpret_cast<char*>(sm) + ring_bytes)), src(src_), w{T(1), a, b},
           tma(tma_), tid(tid_), y0(y0_), z0(z0_), X(p.X), YZ((int64_t)p.Y * p.Z), ns(0), e0(1) {
-        if constexpr (!TMA) po.init(p, n_sites(p), y0, z0, tid);
+        if constexpr (!TMA) po.init(p, STRIDED ? cstride : n_sites(p), y0, z0, tid);
 #pragma unroll
         for (int s = 1; s < NSRC; ++s)
             if (TMA ? tma->map[s] != nullptr : src[s] != nullptr) {
@@ -193,8 +202,13 @@ struct PlanePipe {
                 ++ns;
             }
     }
+    // the x coordinate of plane q in the maps (planes outside the lattice: outside the map)
+    __device__ __forceinline__ int plane(int q) const {
+        if constexpr (STRIDED) return unsigned(q) < unsigned(X) ? tma->x0 + q : 3 * X;
+        return q;
+    }
     __device__ __forceinline__ void box(void* dst, int s, int q) {
-        tma_load_plane(dst, tma->map[s], z0 - M::ZOFF, y0 - 2, q, 0, tma->bar);
+        tma_load_plane(dst, tma->map[s], z0 - M::ZOFF, y0 - 2, plane(q), 0, tma->bar);
     }
     static constexpr uint32_t kBox = uint32_t(SLOT * sizeof(S));
 
@@ -202,9 +216,9 @@ struct PlanePipe {
     __device__ __forceinline__ void ahead(int q) {
         if constexpr (TMA) {
             if (q >= X) return;
-            tma_prefetch_plane(tma->map[0], z0 - M::ZOFF, y0 - 2, q, 0);
-            if (NSRC > 1 && ns > 0) tma_prefetch_plane(tma->map[e0], z0 - M::ZOFF, y0 - 2, q, 0);
-            if (NSRC > 2 && ns > 1) tma_prefetch_plane(tma->map[2], z0 - M::ZOFF, y0 - 2, q, 0);
+            tma_prefetch_plane(tma->map[0], z0 - M::ZOFF, y0 - 2, plane(q), 0);
+            if (NSRC > 1 && ns > 0) tma_prefetch_plane(tma->map[e0], z0 - M::ZOFF, y0 - 2, plane(q), 0);
+            if (NSRC > 2 && ns > 1) tma_prefetch_plane(tma->map[2], z0 - M::ZOFF, y0 - 2, plane(q), 0);
         }
     }
     // Start the copies of plane q into `slot`.
@@ -392,10 +406,12 @@ struct PlanePipe {
 // sites: nuclear 110 us with 16 rows, 134 with 12; omega 89 and 89), else 12 at 168 registers
 // (Coulomb 147 with 12 and 230 with 16, where it spills; Berger 140).  8-row tiles with the
 // register queues of the earlier form: 154, 119, 200 and 173 us.  Every engine stage spills with
-// 16 (omega stage 1: 143 us against 114, stage 3: 222 against 173): 12.
+// 16 (omega stage 1: 143 us against 114, stage 3: 222 against 173): 12; so does rho's pion walk,
+// which also holds the nine sums of its couplings.
 template <template <typename> class Th>
 constexpr int grad_rows64(bool engine) {
-    return engine || Th<double>::kId == SKY_THEORY_COULOMB || Th<double>::kId == SKY_THEORY_BERGER ? 12 : 16;
+    constexpr int id = Th<double>::kId;
+    return engine || id == SKY_THEORY_COULOMB || id == SKY_THEORY_BERGER || id == SKY_THEORY_RHO ? 12 : 16;
 }
 
 // Shared memory of a gradient walk.
@@ -418,7 +434,7 @@ struct GradPipe {
 // TMA as march_tile's (sky_march.cuh); the epilogue gets the pair (or the site) at once:
 // epi(s, N, own1, phi, g) with s the first site and own1 whether the second is in the lattice.
 // DENS: the baryon density of the input is summed into bsum (per site in T), and for FP64 its
-// energy density into esum.  Returns false (every thread of the block) when a wait for a TMA
+// energy density into esum (DENS = 2: the baryon density only).  Returns false (every thread of the block) when a wait for a TMA
 // copy gave up.
 template <template <typename> class Th, class M, typename T, int NSRC, int DENS, class Epi, typename S = T,
           bool TMA = false>
@@ -548,7 +564,7 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
                 if constexpr (NL > 1) {
                     if (own1) ksum_add(bsum, double(L::get(bd, 1)));
                 }
-                if constexpr (sizeof(T) == 8) ksum_add(esum, Th<double>::energy(phi, D, p));
+                if constexpr (sizeof(T) == 8 && DENS == 1) ksum_add(esum, Th<double>::energy(phi, D, p));
             }
         }
         if constexpr (HasLoad<Epi>::value) {
@@ -559,6 +575,11 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
             V g[C];
             typename Th<V>::Stream st;
             st.begin(phi, D, p);
+            if constexpr (HasCoupling<Epi>::value) {
+                V R[9];
+                epi.coupling(s, N, own1, R);
+                st.couple(R, D, p);
+            }
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 V s6[6] = {Sp[0][c], Sp[1][c], Sp[2][c], V(0.0f), V(0.0f), V(0.0f)};
@@ -578,6 +599,12 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
                     }
                 }
                 st.add(c, s6, phi, D, g);
+            }
+            if constexpr (HasCoupling<Epi>::value) {
+                epi.coupled(s, N, own1, st.J, p);
+                // the values are read again, not held
+#pragma unroll
+                for (int c = 0; c < C; ++c) phi[c] = L::load(ring + o2 + lofs + c * PLANE);
             }
             st.end(phi, D, p, g);
             epi(s, N, own1, phi, g);
@@ -610,14 +637,14 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
 // column (x-2 .. x+1) in registers, which leaves nine reads per component and a ring of four
 // planes (x, whose y and z taps are read, x+1, x+2 and the one on its way), so that several
 // blocks share an SM.
-template <class M, typename S, int NSRC, bool TMA>
-using DensPipe = PlanePipe<M, double, S, NSRC, TMA, M::NTHREADS, 4>;
+template <class M, typename S, int NSRC, bool TMA, bool STRIDED = false>
+using DensPipe = PlanePipe<M, double, S, NSRC, TMA, M::NTHREADS, 4, STRIDED>;
 
-template <class M, typename S, int NSRC, bool TMA, class Op>
+template <class M, typename S, int NSRC, bool TMA, bool STRIDED = false, class Op>
 __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params& p, const double (&r1)[3],
                                           const S* const (&src)[3], int xa, int xe, int y0, int z0, Op& op,
-                                          TmaTile* tma = nullptr) {
-    using Pipe = DensPipe<M, S, NSRC, TMA>;
+                                          TmaTile* tma = nullptr, int64_t cstride = 0) {
+    using Pipe = DensPipe<M, S, NSRC, TMA, STRIDED>;
     constexpr int C = M::C, SLOT = M::SLOT, PLANE = M::PLANE, HZ = M::HZ;
     const int64_t YZ = (int64_t)p.Y * p.Z;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -627,7 +654,7 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
     const bool py = y >= hl && y < p.Y - hl, pz = z >= hl && z < p.Z - hl;
     const int q1 = xe + 1;
     const int lofs = (ty + 2) * HZ + (tx + M::ZOFF);
-    Pipe pipe(sm, p, src, 1.0, 1.0, tx + M::BZ * ty, y0, z0, tma);
+    Pipe pipe(sm, p, src, 1.0, 1.0, tx + M::BZ * ty, y0, z0, tma, cstride);
     if (!pipe.prologue(xa - 2, nullptr, 0)) return false;
     double qm2[C], qm1[C], qc[C], qp1[C];  // planes x-2 .. x+1 of the thread's column
 #pragma unroll
@@ -695,7 +722,7 @@ template <template <typename> class Th, class M>
 __global__ void __launch_bounds__(M::NTHREADS)
     k_grad_plain(Params p, const __grid_constant__ MarchCoef<double> k, MarchGrid mg, const double* __restrict__ field,
                  double* __restrict__ eg, double* __restrict__ l) {
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(128) unsigned char smraw[];
     double* sm = reinterpret_cast<double*>(smraw);
     PlainGradEpi epi{eg, l, -p.dt};
     const double* const src[3] = {field, nullptr, nullptr};
@@ -790,7 +817,7 @@ __global__ void __launch_bounds__(M::NTHREADS)
     k_plain_stage(Params p, const __grid_constant__ MarchCoef<double> k, MarchGrid mg, const double* __restrict__ in,
                   StageArrays a, double* __restrict__ counter_e, double* __restrict__ scratch_m,
                   double* __restrict__ err) {
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(128) unsigned char smraw[];
     double* sm = reinterpret_cast<double*>(smraw);
     __shared__ double shm[M::NTHREADS / 32];
     if (STAGE == 1 && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
@@ -842,7 +869,7 @@ template <template <typename> class Th, class M, int MODE>
 __global__ void __launch_bounds__(M::NTHREADS, M::C > 5 ? 1 : 2)
     k_dens_plain(Params p, const __grid_constant__ MarchCoef<double> k, MarchGrid mg, const double* __restrict__ field,
                  double* __restrict__ dens, double* __restrict__ scratch, double* __restrict__ out_dev) {
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(128) unsigned char smraw[];
     double* sm = reinterpret_cast<double*>(smraw);
     __shared__ KSum shk[32];
     DensOp<Th, MODE> op{p, dens, KSum{0.0, 0.0}};

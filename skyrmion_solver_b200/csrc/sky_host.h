@@ -17,7 +17,6 @@ int pack_core(const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf,
 int pack_params(int theory, const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf, Params* out);
 int num_sms();
 int ew_blocks(int64_t n);
-int choose_xc(int X, int tiles_yz, int resident);
 int option(int key);
 
 // The buffers of a drop-in step (C N values each).

@@ -6,7 +6,7 @@
 
 #include "sky_host.h"
 #include "sky_diag.cuh"
-#include "sky_grad.cuh"
+#include "sky_rho.cuh"
 #include "sky_kernels.cuh"
 
 namespace sky {
@@ -282,22 +282,6 @@ int ew_blocks(int64_t n) {
     return (int)b;
 }
 
-// x-chunk of a marching launch: minimise (waves of tiles over the resident
-// blocks) x (planes a block walks: chunk + 4 halo planes).
-int choose_xc(int X, int tiles_yz, int resident) {
-    int best = X, best_cost = -1;
-    for (int xc = 4; xc <= X; ++xc) {
-        const int nt = tiles_yz * ((X + xc - 1) / xc);
-        const int waves = (nt + resident - 1) / resident;
-        const int cost = waves * (xc + 4);
-        if (best_cost < 0 || cost < best_cost || (cost == best_cost && xc > best)) {
-            best_cost = cost;
-            best = xc;
-        }
-    }
-    return best;
-}
-
 // x-chunk of a walk whose first planes are loaded at once (sky_grad.cuh): minimise (waves of
 // tiles) x (planes computed + about three planes' time to fill the ring).
 int choose_chunk(int X, int tiles_yz, int resident) {
@@ -327,34 +311,6 @@ int option(int key) { return (key >= 0 && key < 5) ? g_options[key] : 0; }
 // ---------------------------------------------------------------------------
 // templated launchers
 // ---------------------------------------------------------------------------
-// BY = 8-row tiles, or 4 for FP64 rho (13 components), whose 8-row ring would
-// not fit in shared memory.
-template <template <typename> class Th, typename T, bool WIDE, int BY = 8>
-int launch_gradient_march(const Params& p, const T* field, T* eg, T* l, cudaStream_t st) {
-    using M = MarchShape<Th<T>::C, BY, WIDE>;
-    auto kern = k_march_plain<Th, M, T>;
-    const size_t smem = M::template smem_bytes<T>(1);
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute(march gradient)", __LINE__);
-        if (rc) return rc;
-        int n = 0;
-        rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, M::NTHREADS, smem), "occupancy",
-                        __LINE__);
-        if (rc) return rc;
-        per_sm = n < 1 ? 1 : n;
-    }
-    const int resident = num_sms() * per_sm;
-    const MarchGrid g0 = march_grid<M>(p, p.X);
-    const int xc_opt = option(1);
-    const int xc = xc_opt > 0 ? (xc_opt < p.X ? xc_opt : p.X) : choose_xc(p.X, g0.nz * g0.ny, resident);
-    const MarchGrid mg = march_grid<M>(p, xc);
-    const int blocks = mg.count() < resident ? mg.count() : resident;
-    kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, mg, field, eg, l);
-    return check_cuda(cudaGetLastError(), "launch march gradient", __LINE__);
-}
-
 // Geometry of a walk's launch: x-chunk (xc_opt, or 0: chosen), tiles and persistent blocks; one-time kernel attributes.
 template <class M, class K>
 int walk_geometry(K kern, size_t smem, const Params& p, int cap, int xc_opt, int* per_sm, MarchGrid* mg, int* blocks) {
@@ -397,6 +353,28 @@ int launch_gradient_walk(const Params& p, const double* field, double* eg, doubl
     k.init(p);
     kern<<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, field, eg, l);
     return check_cuda(cudaGetLastError(), "launch gradient walk", __LINE__);
+}
+
+// Rho: a walk over the rho components, then one over the pions'.
+template <bool WIDE>
+int launch_rho_gradient(const Params& p, const double* field, double* eg, double* l, cudaStream_t st) {
+    using R = MarchShape<3, grad_rows64<RhoPion>(false), WIDE, 2>;
+    using M = MarchShape<4, grad_rows64<RhoPion>(false), WIDE, 2>;
+    static int rho_per_sm = 0, per_sm = 0;
+    MarchGrid mg;
+    int blocks;
+    const size_t rho_smem = RhoPipe<R, double, double, 1, false>::bytes;
+    int rc = walk_geometry<R>(k_rho_plain<R>, rho_smem, p, 0, option(1), &rho_per_sm, &mg, &blocks);
+    if (rc) return rc;
+    MarchCoef<double> k;
+    k.init(p);
+    const int resident = num_sms() * rho_per_sm;
+    k_rho_plain<R><<<3 * mg.count() < resident ? 3 * mg.count() : resident, dim3(R::BZ, R::BY), rho_smem, st>>>(
+        p, k, mg, field, eg);
+    const size_t smem = GradPipe<RhoPion, M, double, double, 1, false>::bytes;
+    if ((rc = walk_geometry<M>(k_rho_pion_plain<M>, smem, p, 0, option(1), &per_sm, &mg, &blocks))) return rc;
+    k_rho_pion_plain<M><<<blocks, dim3(M::BZ, M::BY), smem, st>>>(p, k, mg, field, eg, l);
+    return check_cuda(cudaGetLastError(), "launch rho gradient walks", __LINE__);
 }
 
 template <template <typename> class Th, bool WIDE, int STAGE>
@@ -482,7 +460,8 @@ int grad64(const Params& p, const double* f, double* eg, double* l, cudaStream_t
             return wide64(p, f) ? launch_gradient_walk<Th, true>(p, f, eg, l, st)
                                 : launch_gradient_walk<Th, false>(p, f, eg, l, st);
         else
-            return launch_gradient_march<Th, double, false, 4>(p, f, eg, l, st);
+            return wide64(p, f) ? launch_rho_gradient<true>(p, f, eg, l, st)
+                                : launch_rho_gradient<false>(p, f, eg, l, st);
     }
     return launch_gradient<Th, double, double>(p, f, eg, l, st);
 }

@@ -493,6 +493,129 @@ struct Rho {
     }
 };
 
+// The rho gradient in two walks.  With S the second derivatives,
+//   R_j^a = sum_i d_i R^a_ij = sum_i (S_ii rho_j^a - S_ij rho_i^a)
+// is all that the gradient needs of the rho field's derivatives: sum_i dR(a, i, j, i) = R_j^a in
+// the back-reaction on the pions and sum_j dR(a, i, j, j) = -R_i^a in the rho field's own
+// gradient.  A walk over the rho components writes R (sky_rho.cuh); RhoPion is the walk over the
+// four pion components, which takes R at the site and leaves
+//   H_i^a = 8 R_i^a + 16 c_alpha sum_j dOmega(a, i, j, j),
+// so that the gradient of rho_i^a is 8 m_rho^2 rho_i^a - H_i^a.
+template <typename T>
+struct RhoPion {
+    static constexpr bool kMixed = true;
+    static constexpr int C = 4;
+    static constexpr int kId = SKY_THEORY_RHO;
+    struct Stream {
+        QuarticStream<T, C> q;
+        T gr[4];    // the back-reaction on the pions
+        T J[9];     // sum_j dOmega(a, i, j, j) at 3 i + a
+        __device__ __forceinline__ void begin(const T*, const T (&D)[3][C], const Params&) {
+            q.begin(D);
+#pragma unroll
+            for (int m = 0; m < 9; ++m) J[m] = T(0);
+        }
+        // R_j^a at 3 j + a
+        __device__ __forceinline__ void couple(const T (&R)[9], const T (&D)[3][C], const Params& p) {
+            const T ca16 = T(16.0 * p.c2);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) gr[a] = T(0);
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const T r = ca16 * R[3 * j + a];
+                    gr[0] += D[j][a + 1] * r;
+                    gr[a + 1] -= D[j][0] * r;
+                    const int b = (a + 1) % 3, c = (a + 2) % 3;
+                    // eps(a, b, c) D_j,c R^a on component b, and the same with b and c exchanged
+                    gr[b + 1] += D[j][c + 1] * r;
+                    gr[c + 1] -= D[j][b + 1] * r;
+                }
+        }
+        __device__ __forceinline__ void add(int m, const T (&S)[6], const T*, const T (&D)[3][C], T* g) {
+            g[m] = T(2) * (q.add(m, S, D) + (S[0] + S[1] + S[2]));
+            const T w[3] = {S[1] + S[2], S[0] + S[2], S[0] + S[1]};
+            // sum_j (S_ij,m D_j,nu - S_jj,m D_i,nu)
+            auto mm = [&](int i, int nu) -> T {
+                const int j = i == 0 ? 1 : 0, k = i == 2 ? 1 : 2;
+                T v = w[i] * D[i][nu];
+                v += S[sidx(i, j)] * D[j][nu];
+                v += S[sidx(i, k)] * D[k][nu];
+                return v;
+            };
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                if (m == 0) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) J[3 * i + a] += mm(i, a + 1);
+                } else {
+                    const int b = m - 1, c = (b + 1) % 3, a = (b + 2) % 3;  // eps(a, b, c) = 1
+                    J[3 * i + b] -= mm(i, 0);
+                    J[3 * i + a] += mm(i, c + 1);
+                    J[3 * i + c] -= mm(i, a + 1);
+                }
+            }
+        }
+        __device__ __forceinline__ void end(const T* phi, const T (&D)[3][C], const Params& p, T* g) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                g[a] -= T(2) * q.rest(a, D);
+                g[a] += gr[a];
+            }
+            g[0] -= T(2.0 * p.c0 * p.c0);
+            project<T, C>(g, phi, p.nsky);
+        }
+    };
+    // Rho::energy in two parts: the pions' with the coupling, from the curls
+    // R^a_xy, R^a_xz, R^a_yz (at 3 a) of the rho components ...
+    __device__ static T energy(const T* phi, const T (&D)[3][C], const T (&R)[9], const Params& p) {
+        T e = T(0), n[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            n[i] = D[i][0] * D[i][0] + D[i][1] * D[i][1] + D[i][2] * D[i][2] + D[i][3] * D[i][3];
+            e += n[i];
+        }
+        e += T(2) * T(p.c0 * p.c0) * (T(1) - phi[0]);
+        T om = T(0);
+        const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int i = pi[q], j = pj[q];
+            const T d = D[i][0] * D[j][0] + D[i][1] * D[j][1] + D[i][2] * D[j][2] + D[i][3] * D[j][3];
+            e += n[i] * n[j] - d * d;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int b = (a + 1) % 3, c = (a + 2) % 3;
+                om += R[3 * a + q] * ((D[i][0] * D[j][a + 1] - D[i][a + 1] * D[j][0]) +
+                                      (D[i][b + 1] * D[j][c + 1] - D[i][c + 1] * D[j][b + 1]));
+            }
+        }
+        e -= T(16.0 * p.c2) * om;
+        return e * T(p.vol);
+    }
+    // ... and one isospin component's own.
+    __device__ static T rho_energy(const T (&r)[3], const T (&R)[3], const Params& p) {
+        const T m = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        const T f = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+        return (T(4.0 * p.c1 * p.c1) * m + T(4) * f) * T(p.vol);
+    }
+    __device__ static T baryon(const T* phi, const T (&D)[3][C], const Params& p) {
+        return neg_det_b<T, C>(phi, D) * T(p.vol / (2.0 * M_PI * M_PI));
+    }
+};
+// H_i^a, and the gradient of rho_i^a (component 4 + 3 i + a) from its value and H_i^a.
+template <typename T>
+__device__ __forceinline__ T rho_rest(T R, T J, const Params& p) {
+    T h = T(16.0 * p.c2) * J;
+    h += T(8) * R;
+    return h;
+}
+template <typename T>
+__device__ __forceinline__ T rho_gradient(T rho, T H, const Params& p) {
+    return T(8.0 * p.c1 * p.c1) * rho - H;
+}
+
 // ===========================================================================
 // Berger-deformed Skyrme model, C = 4.  c0 = m_pi, c1 = kappa, c2 = alpha.
 // omega(a, b) = a0 b3 + a1 b2 - a2 b1 - a3 b0 (th/berger_skyrme/kernels.py:81-111)
