@@ -98,10 +98,19 @@ __global__ void k_convert_in(int64_t n, const double* __restrict__ src, S* __res
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dst[i] = src ? S(src[i]) : S(0);
 }
+// An instance's field (high plus low parts of a compensated one) and velocity in FP64; null: not
+// wanted.  Which halves are current, and whether the velocity counts as zero (the reference zeroes V
+// on arrest), is read from the device's own state: a read-back is then one launch and one
+// synchronisation where it fetched that state to the host first (38 us of the 144 that a step, its
+// record and the buffers of a frame take at 32^3 sites).
 template <typename S>
-__global__ void k_convert_out(int64_t n, const S* __restrict__ src, double* __restrict__ dst, int zero) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = zero ? 0.0 : double(src[i]);
+__global__ void k_read_state(const InstDesc<S>* __restrict__ d, int64_t n, double* __restrict__ field,
+                             double* __restrict__ velocity) {
+    const S *F = d->F[d->cur], *Flo = d->Flo[d->cur], *V = d->arrested ? nullptr : d->V[d->cur];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (field) field[i] = Flo ? double(F[i]) + double(Flo[i]) : double(F[i]);
+        if (velocity) velocity[i] = V ? double(V[i]) : 0.0;
+    }
 }
 __global__ void k_f32_to_f64(int64_t n, const float* __restrict__ s, double* __restrict__ d) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -1036,34 +1045,28 @@ int sky_engine_read(void* handle, int id, double* field, double* velocity, int o
     if (!h) return invalid("unknown instance id");
     cudaSetDevice(e->device);
     Group& g = e->groups[h->set][h->prec];
-    int cur = 0, arrested = 0;
-    int rc;
-    size_t sz = h->prec ? sizeof(InstDesc<double>) : sizeof(InstDesc<float>);
-    size_t ocur = h->prec ? offsetof(InstDesc<double>, cur) : offsetof(InstDesc<float>, cur);
-    size_t oarr = h->prec ? offsetof(InstDesc<double>, arrested) : offsetof(InstDesc<float>, arrested);
-    char* base = reinterpret_cast<char*>(g.d_desc) + sz * h->group_slot;
-    cudaMemcpyAsync(&cur, base + ocur, sizeof(int), cudaMemcpyDeviceToHost, e->stream);
-    cudaMemcpyAsync(&arrested, base + oarr, sizeof(int), cudaMemcpyDeviceToHost, e->stream);
-    if ((rc = check_cuda(cudaStreamSynchronize(e->stream), "sync", __LINE__))) return rc;
     const int64_t n = (int64_t)h->C * h->N;
+    int rc = SKY_OK;
+    auto convert = [&](double* f, double* v) {
+        if (h->prec)
+            k_read_state<double><<<ew_blocks(n), 256, 0, e->stream>>>(
+                reinterpret_cast<const InstDesc<double>*>(g.d_desc) + h->group_slot, n, f, v);
+        else
+            k_read_state<float><<<ew_blocks(n), 256, 0, e->stream>>>(
+                reinterpret_cast<const InstDesc<float>*>(g.d_desc) + h->group_slot, n, f, v);
+        return check_cuda(cudaGetLastError(), "convert out", __LINE__);
+    };
+    if (on_device) {
+        if ((field || velocity) && (rc = convert(field, velocity))) return rc;
+        return check_cuda(cudaStreamSynchronize(e->stream), "sync", __LINE__);
+    }
     double* tmp = nullptr;
-    if (!on_device && (rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * n), "cudaMalloc(read)", __LINE__)))
-        return rc;
+    if ((rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * n), "cudaMalloc(read)", __LINE__))) return rc;
     double* outs[2] = {field, velocity};
-    const void* srcs[2] = {h->F[cur], h->V[cur]};
     for (int k = 0; k < 2 && rc == SKY_OK; ++k) {
         if (!outs[k]) continue;
-        double* dst = on_device ? outs[k] : tmp;
-        const int zero = (k == 1 && arrested) ? 1 : 0;  // the reference zeroes V on arrest
-        if (h->prec)
-            k_convert_out<double><<<ew_blocks(n), 256, 0, e->stream>>>(n, (const double*)srcs[k], dst, zero);
-        else if (k == 0 && h->comp)
-            k_f32c_to_f64<<<ew_blocks(n), 256, 0, e->stream>>>(n, (const float*)srcs[k], (const float*)h->Flo[cur],
-                                                               dst, 0);
-        else
-            k_convert_out<float><<<ew_blocks(n), 256, 0, e->stream>>>(n, (const float*)srcs[k], dst, zero);
-        rc = check_cuda(cudaGetLastError(), "convert out", __LINE__);
-        if (!rc && !on_device)
+        rc = convert(k == 0 ? tmp : nullptr, k == 1 ? tmp : nullptr);
+        if (!rc)
             rc = check_cuda(cudaMemcpyAsync(outs[k], tmp, sizeof(double) * n, cudaMemcpyDeviceToHost, e->stream),
                             "download", __LINE__);
         if (!rc) rc = check_cuda(cudaStreamSynchronize(e->stream), "sync", __LINE__);

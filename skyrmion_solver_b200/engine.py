@@ -241,7 +241,7 @@ class Engine:
             field = torch.empty(m["C"] * N, dtype=torch.float64, device=dev)
             stream.synchronize()                           # the engine writes on its own stream
             self.read_device(iid, field)                   # synchronous on the engine's stream
-            en = torch.zeros(N, dtype=torch.float64, device=dev)
+            en = torch.empty(N, dtype=torch.float64, device=dev)   # every site is written
             fn = "sky_baryon_density" if density == "baryon" else "sky_energy_density"
             _lib.call(fn, m["theory"], i32p(m["p_i"]), len(m["p_i"]), f64p(m["p_f"]), len(m["p_f"]), _lib.dptr(en),
                       _lib.dptr(field), _lib.stream_ptr(stream))
