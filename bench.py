@@ -47,8 +47,7 @@ METRIC = "converged solves/s and p99 latency at 1e-6 rel. energy vs plain FP64; 
 UNIT = "solves/s"
 WORKLOAD = "omega_B4_rational_map_128^3_h0.15"
 CALIBRATION = os.path.join(ROOT, "profiles", "convergence_omega_B4_128.json")
-TRAFFIC = [os.path.join(ROOT, "profiles", f) for f in ("ncu_stage1_fp32d_omega128.md",
-                                                        "ncu_stage4_fp32d_omega128.md")]
+TRAFFIC = [os.path.join(ROOT, "profiles", f) for f in ("ncu_walks_fp32d_omega128.md",)]
 L = 128
 H = 0.15
 FAST = "fp32d"   # precision of the timed steps (the FP32 phase of the schedule)
@@ -59,18 +58,19 @@ INIT = {"mode": "rational_map", "baryon_number": 4, "scale": 2.0, "vacuum_shell"
 REL_ENERGY_TOL = 1e-6
 GRAD_TOL = 1e-6
 # passes over one C-component field per stage launch (reads + writes)
-STAGE_PASSES = {"stage1": 2, "stage2": 3, "stage3": 4, "stage4": 7}
+# (stage 3 reads F, V, l1, l2 and writes F' and P; stage 4 reads F, V, l2, F', P and writes V')
+STAGE_PASSES = {"stage1": 2, "stage2": 3, "stage3": 6, "stage4": 6}
 
 
 def stage_passes(stage, precision):
     """Field-sized passes (reads + writes of one C-component FP32 array) of one stage launch.
-    Compensated field (fp32c, fp32d): stage 1 also reads the low parts (FP64 densities of hi + lo),
-    stage 4 reads and writes them.  fp32d: every stage reads the correction; every 16th step the
+    Compensated field (fp32c, fp32d): stage 1 (with its energy walk) also reads the high and low
+    parts for the FP64 density of hi + lo, stage 3 reads and writes the low parts.  fp32d: every stage reads the correction; every 16th step the
     defect kernel reads hi and lo and writes it, and stage 1 rewrites it (4/16 per step, counted
     with stage 1, whose timing includes the defect kernel)."""
     n = STAGE_PASSES[stage]
     if precision in ("fp32c", "fp32d"):
-        n += {"stage1": 1, "stage4": 2}.get(stage, 0)
+        n += {"stage1": 2, "stage3": 2}.get(stage, 0)
     if precision == "fp32d":
         n += 1 + (4 / 16 if stage == "stage1" else 0)
     return n
@@ -480,7 +480,7 @@ def run_ours(args):
     # per-launch-kind timing (CUDA events on the engine stream, un-captured launches)
     stages = eng.time_stages(max(5, min(50, K)))
     dom = max(("stage1", "stage2", "stage3", "stage4"), key=lambda k: stages[k])
-    alg_bytes = STAGE_PASSES[dom] * C * 4 * N                 # minimal fused schedule: 16 C s per step
+    alg_bytes = STAGE_PASSES[dom] * C * 4 * N                 # minimal fused schedule: 17 C s per step
     fmt_bytes = stage_passes(dom, FAST) * C * 4 * N           # with the compensated format's extra arrays
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (stages[dom] * 1e-3) / 1e9
@@ -607,14 +607,14 @@ def run_ours(args):
         "final": final,
         "steps_rate": {"ms_per_step": ms_step, "site_steps_per_s": world * N * 1e3 / ms_step,
                        "hbm_gbs_step": step_bytes / (ms_step * 1e-3) / 1e9},
-        "roofline": {"bound": "hbm", "kernel": f"k_march_stage<Omega,float,{dom[-1]}>"
-                     + (" + k_march_defect" if dom == "stage1" and FAST == "fp32d" else ""),
+        "roofline": {"bound": "hbm", "kernel": f"k_grad_stage<Omega,float,{dom[-1]}>"
+                     + (" + k_energy + k_defect" if dom == "stage1" and FAST == "fp32d" else ""),
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind, "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes,
                      "format_bytes_per_launch": fmt_bytes, "format_achieved": fmt_bytes / (stages[dom] * 1e-3) / 1e9,
                      "issue_active": load_issue_active(dom),
                      "note": "algorithmic bytes: the minimal fused schedule's passes of one C-component FP32 "
-                             "field (stage 1: 2, stage 2: 3, stage 3: 4, stage 4: 7); format bytes add the "
+                             "field (stage 1: 2, stage 2: 3, stage 3: 6, stage 4: 6); format bytes add the "
                              "compensated field's low parts and the defect correction",
                      "launch_ms": stages[dom], "stage_ms": stages},
         "plain_fp64": plain,

@@ -51,16 +51,15 @@ const char* sky_version(void);
 const char* sky_last_error(void);
 
 /* Library-wide tuning options.  Key 0: kernel family of the reference-layout
- * gradient (sky_gradient_step / sky_arrested_newton_step) for theories with at
- * most five components: 1 = marching x-plane kernels (default), 0 = 3-D tile
- * kernels.  Key 1: x-chunk of those marching launches (0 = automatic).  Key 2:
+ * gradient and densities (sky_gradient_step / sky_arrested_newton_step): 1 =
+ * marching x-plane kernels (default), 0 = 3-D tile kernels.  Key 1: x-chunk of those marching launches (0 = automatic).  Key 2:
  * staging of the resident engine's stage kernels, 1 = tensor-memory-accelerator
  * box copies (default; lattices whose Z gives 16-byte row pitches), 0 = per-thread
  * cp.async copies; it applies to instances admitted afterwards
  * (sky_engine_set_staging changes one instance).
- * Key 3: 1 = the FP32 stages of theories whose gradient needs no mixed second
- * derivatives (omega) compute two adjacent z-sites per thread with packed FP32x2
- * arithmetic; 0 = one site per thread (default).  Applies at admission.
+ * Key 3: 0 or 1, recorded as the z-pair flag of FP32 omega instances at admission.
+ * It selects nothing: every FP32 gradient walk computes two adjacent z-sites per
+ * thread with packed FP32x2 arithmetic.
  * Key 4: 1 = the engine's stage launches use programmatic dependent launch, so a
  * launch is scheduled while the previous one's last blocks finish (each waits for
  * the previous launch before reading its results), 0 = plain stream order (default;
@@ -317,11 +316,11 @@ int sky_engine_retile(void* engine, int id, int xc);
 /* Staging of an instance's planes in the marching stage kernels: tma = 1 copies
  * each haloed plane with one tensor-memory-accelerator box copy per source (Z *
  * element size a multiple of 16 bytes; not FP64 rho), 0 with per-thread cp.async
- * copies; pair = 1 runs two z-sites per thread with packed FP32x2 arithmetic (TMA,
- * FP32 omega only).  Admission takes both from library options 2 and 3; a group of
- * instances of one theory and precision stages by TMA (z-pairs) only when every
- * member does.  The state and the pending arrest decision carry over; the
- * stagings are bitwise identical, z-pairs agree to FP32 rounding. */
+ * copies; pair (TMA, FP32 omega only) is recorded and selects nothing: every FP32
+ * gradient walk computes two z-sites per thread with packed FP32x2 arithmetic.
+ * Admission takes both from library options 2 and 3; a group of instances of one
+ * theory and precision stages by TMA only when every member does.  The state and
+ * the pending arrest decision carry over; the stagings are bitwise identical. */
 int sky_engine_set_staging(void* engine, int id, int tma, int pair);
 int sky_engine_get_staging(void* engine, int id, int* tma, int* pair);
 /* Steps between refreshes of a defect-corrected instance's FP64 correction

@@ -1,12 +1,11 @@
 """Autotuner for the engine's per-instance tiling and plane staging.
 
-The marching stage kernels split a lattice into (x-chunk, 8-row y, 32-column z)
+The stage kernels split a lattice into (x-chunk, 8- to 16-row y, 32-column z)
 tiles; the x-chunk sets how many tiles one launch has (and so how evenly they
 spread over the 148 SMs) against how many halo planes each block re-reads.  The
 planes of a tile are staged either by TMA box copies or by per-thread cp.async
-copies, and an FP32 omega tile can run as z-pairs (16 x 8 threads, two z-sites
-each, packed FP32x2 arithmetic) instead of one site per thread (32 x 8).
-``sky_engine_add`` picks the chunk with a cost model and the staging from the
+copies (the z-pair flag of an FP32 omega instance is timed too, but every FP32
+gradient walk computes z-pairs, so it changes nothing).  ``sky_engine_add`` picks the chunk with a cost model and the staging from the
 library options; this module measures instead: for one (theory, precision,
 lattice shape, device) it admits a probe instance, times a few steps per
 candidate (staging, chunk) with CUDA events on the engine's stream
@@ -15,8 +14,7 @@ file so that a serving process tunes each shape once.
 
 Tiling changes only the order of the per-tile energy partial sums, so a tuned
 instance follows the same trajectory as an untuned one (``tests/test_march.py``);
-the two stagings are bitwise identical and z-pairs agree to FP32 rounding
-(``tests/test_tma.py``).
+the stagings are bitwise identical (``tests/test_tma.py``).
 """
 from __future__ import annotations
 

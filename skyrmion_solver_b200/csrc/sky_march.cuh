@@ -19,8 +19,7 @@ namespace sky {
 // 16 / sizeof(T) so that every 16-byte chunk of a row starts on a 16-byte boundary
 // and lies wholly inside or (as the first chunk at z0 = 0) wholly outside the lattice
 // in z; a chunk crossing z = Z copies its in-lattice part and zero-fills the rest.
-constexpr size_t kMaxSmemPerBlock = 232448;  // 227 KB of dynamic shared memory per block
-
+//
 // ZP: columns staged on each side of a wide row's 32 (4, or 2 for 8-byte values, whose
 // 16-byte chunks start at z0 - 2).
 template <int C_, int BY_, bool WIDE_ = false, int ZP = 4>
@@ -34,10 +33,8 @@ struct MarchShape {
     static constexpr int NTHREADS = BZ * BY;
 };
 
-// Per-tile TMA state of a marching kernel: the kernel's two mbarriers
-// (initialised once per launch; planes alternate between them when two are in
-// flight), the parity bit of the phase each one completes next, the maps of the
-// tile's sources (null: the source reads as zero) and the launch-wide error word
+// Per-tile TMA state of a walk: the kernel's mbarrier (initialised once per launch), the
+// parity of the phase it completes next, the maps of the tile's sources (null: the source reads as zero) and the launch-wide error word
 // that a timed-out wait sets.
 struct TmaTile {
     uint64_t* bar;

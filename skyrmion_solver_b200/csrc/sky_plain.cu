@@ -302,9 +302,8 @@ int choose_chunk(int X, int tiles_yz, int resident) {
 // reference-layout gradient and densities (1 = marching kernels, 0 = 3-D tile
 // kernels); key 1 = x-chunk of those marching launches (0 = automatic); key 2 =
 // staging of the engine's stage kernels (1 = TMA box copies, 0 = cp.async); key 3 =
-// z-pair tiles for the FP32 stages of theories without mixed derivatives (1 = on; off
-// by default: on the omega 128^3 stages they issue a third fewer instructions per site
-// but run at half the resident warps, and measured no faster).
+// kept and reported, selects nothing: every FP32 gradient walk computes z-pairs; key 4 =
+// programmatic dependent launch of every stage kernel, in one stream.
 static int g_options[5] = {1, 0, 1, 0, 0};
 int option(int key) { return (key >= 0 && key < 5) ? g_options[key] : 0; }
 

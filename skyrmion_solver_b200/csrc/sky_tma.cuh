@@ -89,10 +89,6 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 // grid has signalled (or exited), the dependent kernel may be scheduled.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ void prefetch_tmap(const TmaMap* map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map->m) : "memory");
-}
-
 // One tile copy of the box at (z, y, x, c) of `map` into shared memory at dst,
 // completing on `bar`; the destination is the issuing CTA's own shared memory.
 __device__ __forceinline__ void tma_load_plane(void* dst, const TmaMap* map, int z, int y, int x, int c,

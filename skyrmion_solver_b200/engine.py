@@ -152,7 +152,8 @@ class Engine:
         self._call("sky_engine_retile", int(iid), int(xc))
 
     def set_staging(self, iid: int, tma: bool, pair: bool = False):
-        """Plane staging of this instance: TMA box copies or cp.async, and z-pair tiles."""
+        """Plane staging of this instance: TMA box copies or cp.async; the z-pair flag is kept and
+        reported (every FP32 walk computes z-pairs)."""
         self._call("sky_engine_set_staging", int(iid), int(bool(tma)), int(bool(pair)))
 
     def staging(self, iid: int) -> tuple:
@@ -301,4 +302,5 @@ class Engine:
 def instance_bytes(C: int, N: int, precision: str = "fp32") -> int:
     """Device bytes one instance occupies (7 state / slope arrays + small per-tile scratch)."""
     es = 4 if precision == "fp32" else 8
-    return 7 * es * C * N + 8192 * 48 + N // 4
+    curls = 72 * N if C > 5 and precision == "fp32" else 0   # rho's energy walks
+    return 7 * es * C * N + curls + 8192 * 48 + N // 4

@@ -68,7 +68,8 @@ class Result:
 def instance_bytes(C: int, N: int, precision: str = "fp32") -> int:
     """Device bytes of one engine instance: 7 state / slope arrays plus per-tile partials and the stats ring."""
     es = 4 if precision == "fp32" else 8
-    return 7 * es * C * N + 8192 * 48 + (N // 256 + 1) * 48
+    curls = 72 * N if C > 5 and precision == "fp32" else 0   # rho's energy walks
+    return 7 * es * C * N + curls + 8192 * 48 + (N // 256 + 1) * 48
 
 
 def fp32_gradient_floor(p_f) -> float:
