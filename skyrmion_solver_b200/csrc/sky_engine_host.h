@@ -21,6 +21,8 @@ struct HostInst {
     Params p{};
     int64_t N = 0;
     int C = 0;
+    void* arena = nullptr;  // one allocation that holds every array below
+    void* parts = nullptr;  // the partials' own allocation once sky_engine_retile has changed their sizes
     void* F[2] = {nullptr, nullptr};
     void* Flo[2] = {nullptr, nullptr};
     void* Dlt = nullptr;
