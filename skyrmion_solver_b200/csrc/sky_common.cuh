@@ -26,10 +26,12 @@ struct Params {
     double vol;         // p_f[6] (cell volume)
     double dt;          // p_f[7]
     double c0, c1, c2;  // theory couplings (see sky_pack_params)
+    int Zp;             // values from one (x, y) row to the next: Z, or more in the engine's own arrays
 };
 
+// Values of one component, the rows' padding included: the stride between components.
 __host__ __device__ inline int64_t n_sites(const Params& p) {
-    return (int64_t)p.X * p.Y * p.Z;
+    return (int64_t)p.X * p.Y * p.Zp;
 }
 
 // ---------------------------------------------------------------------------

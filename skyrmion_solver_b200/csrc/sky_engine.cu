@@ -63,9 +63,15 @@ static int launch_defect(const Group& g, cudaStream_t st) {
 }
 static int setup_group(const Group& g) { return kernel_ops(g.set).setup(g); }
 
-// Whether every instance of a group can use the wide-row kernels: Z a multiple of
-// 16 / sizeof(T) (the buffers are cudaMalloc'd, hence 256-byte aligned).
-static bool wide_ok(int prec, int Z) { return Z % (prec ? 2 : 4) == 0; }
+// Row pitch of an instance's arrays: Z rounded up to four values, so that the rows of every
+// lattice start on 16-byte boundaries and are staged by TMA or in 16-byte chunks.  With the
+// caller's pitch an odd Z could only be copied value by value, and with two or three sources that
+// took the stages longer than before they were gradient walks.  Step in us with the caller's pitch /
+// padded: Coulomb FP64 63^3 208 / 149, omega FP64 49^3 102 / 83, nuclear FP32 75 x 83 x 61 169 / 115,
+// rho defect-corrected 63^3 358 / 286.
+static int row_pitch(int Z) { return (Z + 3) / 4 * 4; }
+// Whether the caller's rows have such a pitch: the staging of those instances can be chosen.
+static bool rows_aligned(int prec, int Z) { return Z % (prec ? 2 : 4) == 0; }
 
 // Stage tiles of an instance for x-chunk request `xc` (0: chosen).
 static void tile_geometry(const HostInst& h, int request, int* xc, int* nz, int* ny, int* nx) {
@@ -93,10 +99,19 @@ static int launch_control(const Group& g, int ib, int ie, int mode, cudaStream_t
 // ---------------------------------------------------------------------------
 // conversion kernels (FP64 reference layout <-> engine storage)
 // ---------------------------------------------------------------------------
+// The caller's arrays have rows of Z values, the engine's of Zp.
+__device__ __forceinline__ int64_t caller_index(int64_t i, int Z, int Zp) {
+    if (Z == Zp) return i;
+    const uint32_t row = uint32_t(i) / uint32_t(Zp), z = uint32_t(i) - row * uint32_t(Zp);
+    return z < uint32_t(Z) ? int64_t(row) * Z + z : -1;
+}
+// n: values of the engine's array, padding included (it reads as zero; a null src too)
 template <typename S>
-__global__ void k_convert_in(int64_t n, const double* __restrict__ src, S* __restrict__ dst) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = src ? S(src[i]) : S(0);
+__global__ void k_convert_in(int64_t n, int Z, int Zp, const double* __restrict__ src, S* __restrict__ dst) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = caller_index(i, Z, Zp);
+        dst[i] = src && j >= 0 ? S(src[j]) : S(0);
+    }
 }
 // An instance's field (high plus low parts of a compensated one) and velocity in FP64; null: not
 // wanted.  Which halves are current, and whether the velocity counts as zero (the reference zeroes V
@@ -107,9 +122,12 @@ template <typename S>
 __global__ void k_read_state(const InstDesc<S>* __restrict__ d, int64_t n, double* __restrict__ field,
                              double* __restrict__ velocity) {
     const S *F = d->F[d->cur], *Flo = d->Flo[d->cur], *V = d->arrested ? nullptr : d->V[d->cur];
+    const int Z = d->p.Z, Zp = d->p.Zp;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (field) field[i] = Flo ? double(F[i]) + double(Flo[i]) : double(F[i]);
-        if (velocity) velocity[i] = V ? double(V[i]) : 0.0;
+        const int64_t j = caller_index(i, Z, Zp);
+        if (j < 0) continue;
+        if (field) field[j] = Flo ? double(F[i]) + double(Flo[i]) : double(F[i]);
+        if (velocity) velocity[j] = V ? double(V[i]) : 0.0;
     }
 }
 __global__ void k_f32_to_f64(int64_t n, const float* __restrict__ s, double* __restrict__ d) {
@@ -120,11 +138,13 @@ __global__ void k_f64_to_f32(int64_t n, const double* __restrict__ s, float* __r
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         d[i] = float(s[i]);
 }
-// FP64 -> compensated FP32 pair (hi = nearest float, lo = nearest float of the remainder)
-__global__ void k_f64_to_f32c(int64_t n, const double* __restrict__ s, float* __restrict__ hi,
+// FP64 -> compensated FP32 pair (hi = nearest float, lo = nearest float of the remainder).  Z: the
+// source's rows, Zp unless it is the caller's array.
+__global__ void k_f64_to_f32c(int64_t n, int Z, int Zp, const double* __restrict__ s, float* __restrict__ hi,
                               float* __restrict__ lo) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = s[i];
+        const int64_t j = caller_index(i, Z, Zp);
+        const double v = j >= 0 ? s[j] : 0.0;
         const float h = float(v);
         hi[i] = h;
         lo[i] = float(v - double(h));
@@ -148,17 +168,17 @@ static int encode_maps(const HostInst& h, InstDesc<S>& d) {
                                   h.L[0], h.L[1], h.L[2], h.Dlt};
     for (int k = 0; k < kNumMaps; ++k) {
         if (!arrs[k]) continue;
-        int rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, sh.components, sh.hz,
+        int rc = encode_plane_map(&d.tm[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.p.Zp, sh.components, sh.hz,
                                   sh.rows + 4);
         if (!rc && h.set == SKY_THEORY_RHO)
             // the rho components: those of one isospin component are 3 N apart, and its planes X long
             rc = encode_plane_map(&d.tmr[k], reinterpret_cast<const S*>(arrs[k]) + 4 * h.N, (int)sizeof(S), 3 * h.p.X,
-                                  h.p.Y, h.p.Z, 3, sh.hz, sh.rho_rows + 4);
+                                  h.p.Y, h.p.Z, h.p.Zp, 3, sh.hz, sh.rho_rows + 4);
         if (!rc && k < kNumEnergyMaps && split_energy(h.set, h.prec))
             rc = encode_plane_map(&d.tmc[k], reinterpret_cast<const S*>(arrs[k]) + 4 * h.N, (int)sizeof(S), 3 * h.p.X,
-                                  h.p.Y, h.p.Z, 3, 40, kDensRows + 4);
+                                  h.p.Y, h.p.Z, h.p.Zp, 3, 40, kDensRows + 4);
         if (!rc && k < kNumEnergyMaps && energy_walk(h.set, h.prec))
-            rc = encode_plane_map(&d.tme[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, sh.components, 40,
+            rc = encode_plane_map(&d.tme[k], arrs[k], (int)sizeof(S), h.p.X, h.p.Y, h.p.Z, h.p.Zp, sh.components, 40,
                                   kDensRows + 4);
         if (rc) return rc;
     }
@@ -225,7 +245,6 @@ static int rebuild_group_t(Engine& e, Group& g) {
     std::vector<InstDesc<S>> descs;
     std::vector<int> tile_inst, e_tile_inst, r_tile_inst;
     int tb = 0;
-    g.all_wide = true;
     g.any_defect = false;
     g.all_tma = !g.members.empty();
     for (size_t k = 0; k < g.members.size(); ++k) {
@@ -249,7 +268,6 @@ static int rebuild_group_t(Engine& e, Group& g) {
         }
         h.group_slot = (int)k;
         if (h.defect) g.any_defect = true;
-        if (!wide_ok(h.prec, h.p.Z)) g.all_wide = false;
         descs.push_back(d);
         for (int t = 0; t < h.ntiles; ++t) tile_inst.push_back((int)k);
         if (energy_walk(h.set, h.prec)) e_tile_inst.insert(e_tile_inst.end(), h.entiles, (int)k);
@@ -336,23 +354,22 @@ static void take_partials(Carver& c, HostInst& h) {
     c.take(h.gpart, sizeof(double) * 4 * grad_partials(h.set, h.ntiles, h.rgrid.count()));
 }
 
-// Whether an instance's planes can be staged by TMA box copies: the option is on,
-// the row pitch Z * sizeof(T) is a multiple of 16 bytes, and its (theory,
-// precision) has TMA kernels (every one but FP64 rho).
-static bool tma_possible(const HostInst& h) {
-    return wide_ok(h.prec, h.p.Z) && !(h.prec && theory_components(h.theory) > 5);
-}
-static bool tma_ok_for(const HostInst& h) { return option(2) == 1 && tma_possible(h); }
+// Whether an instance's (theory, precision) has TMA kernels: every one but FP64 rho.
+static bool tma_kernels(const HostInst& h) { return !(h.prec && theory_components(h.theory) > 5); }
+// Whether its staging is the caller's to choose and see.  The arrays of the others, whose rows are
+// padded, follow the library's option.
+static bool tma_possible(const HostInst& h) { return rows_aligned(h.prec, h.p.Z) && tma_kernels(h); }
 // Whether the z-pair flag applies to an instance (TMA staging, FP32, omega).
 static bool pair_possible(const HostInst& h) { return h.prec == 0 && h.theory == SKY_THEORY_OMEGA; }
 
 static int alloc_inst(Engine& e, HostInst& h) {
     const size_t es = h.prec ? sizeof(double) : sizeof(float);
-    h.set = kernel_set(h.theory, h.prec, h.N);
-    h.tma = tma_ok_for(h);
-    h.pair = h.tma && option(3) == 1 && pair_possible(h);
+    h.set = kernel_set(h.theory, h.prec, h.sites);
+    h.tma = option(2) == 1 && tma_kernels(h);
+    h.pair = h.tma && tma_possible(h) && option(3) == 1 && pair_possible(h);
     const size_t fb = es * (size_t)h.C * (size_t)h.N;
-    if ((int64_t)h.C * h.N >= ((int64_t)1 << 31)) return invalid("lattice too large for the marching kernels");
+    if ((int64_t)h.C * h.sites >= ((int64_t)1 << 31) || (int64_t)h.C * h.N >= (int64_t)0xffffffff)
+        return invalid("lattice too large for the marching kernels");
     tile_geometry(h, h.xc_request, &h.xc, &h.tnz, &h.tny, &h.tnx);
     h.ntiles = h.tnz * h.tny * h.tnx;
     h.entiles = h.ntiles;
@@ -401,7 +418,8 @@ static int alloc_inst(Engine& e, HostInst& h) {
 }
 
 static int upload(Engine& e, HostInst& h, const double* field, const double* velocity, bool on_device) {
-    const int64_t n = (int64_t)h.C * h.N;
+    const int64_t n = (int64_t)h.C * h.N, nc = (int64_t)h.C * h.sites;  // values here, and of the caller's
+    const int Z = h.p.Z, Zp = h.p.Zp;
     double* tmp = nullptr;
     int rc = SKY_OK;
     const double* srcs[2] = {field, velocity};
@@ -409,20 +427,20 @@ static int upload(Engine& e, HostInst& h, const double* field, const double* vel
     for (int k = 0; k < 2; ++k) {
         const double* src = srcs[k];
         if (src && !on_device) {
-            if (!tmp && (rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * n), "cudaMalloc(upload)", __LINE__)))
+            if (!tmp && (rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * nc), "cudaMalloc(upload)", __LINE__)))
                 return rc;
-            if ((rc = check_cuda(cudaMemcpyAsync(tmp, src, sizeof(double) * n, cudaMemcpyHostToDevice, e.stream),
+            if ((rc = check_cuda(cudaMemcpyAsync(tmp, src, sizeof(double) * nc, cudaMemcpyHostToDevice, e.stream),
                                  "upload", __LINE__)))
                 break;
             src = tmp;
         }
         if (h.prec)
-            k_convert_in<double><<<ew_blocks(n), 256, 0, e.stream>>>(n, src, reinterpret_cast<double*>(dsts[k]));
+            k_convert_in<double><<<ew_blocks(n), 256, 0, e.stream>>>(n, Z, Zp, src, reinterpret_cast<double*>(dsts[k]));
         else if (k == 0 && h.comp)
-            k_f64_to_f32c<<<ew_blocks(n), 256, 0, e.stream>>>(n, src, reinterpret_cast<float*>(h.F[0]),
+            k_f64_to_f32c<<<ew_blocks(n), 256, 0, e.stream>>>(n, Z, Zp, src, reinterpret_cast<float*>(h.F[0]),
                                                               reinterpret_cast<float*>(h.Flo[0]));
         else
-            k_convert_in<float><<<ew_blocks(n), 256, 0, e.stream>>>(n, src, reinterpret_cast<float*>(dsts[k]));
+            k_convert_in<float><<<ew_blocks(n), 256, 0, e.stream>>>(n, Z, Zp, src, reinterpret_cast<float*>(dsts[k]));
         if ((rc = check_cuda(cudaGetLastError(), "convert", __LINE__))) break;
         if (tmp) cudaStreamSynchronize(e.stream);
     }
@@ -656,6 +674,8 @@ int sky_engine_add(void* handle, int theory, const int32_t* p_i, int32_t n_pi, c
     h.prec = precision == 1 ? 1 : 0;
     h.comp = precision >= 2 ? 1 : 0;
     h.defect = precision == 3 ? 1 : 0;
+    h.sites = n_sites(h.p);
+    h.p.Zp = row_pitch(h.p.Z);
     h.N = n_sites(h.p);
     h.C = h.p.C;
     if ((rc = alloc_inst(*e, h))) return rc;
@@ -746,7 +766,7 @@ int sky_engine_set_precision(void* handle, int id, int precision) {
                 k_f32_to_f64<<<ew_blocks(n), 256, 0, e->stream>>>(n, (const float*)srcs[k], (double*)dsts[k]);
         } else {                  // FP64 -> FP32 (+ low part)
             if (fieldk && nh.comp)
-                k_f64_to_f32c<<<ew_blocks(n), 256, 0, e->stream>>>(n, (const double*)srcs[k], (float*)dsts[k],
+                k_f64_to_f32c<<<ew_blocks(n), 256, 0, e->stream>>>(n, h.p.Zp, h.p.Zp, (const double*)srcs[k], (float*)dsts[k],
                                                                    (float*)nh.Flo[0]);
             else
                 k_f64_to_f32<<<ew_blocks(n), 256, 0, e->stream>>>(n, (const double*)srcs[k], (float*)dsts[k]);
@@ -848,7 +868,7 @@ int sky_engine_set_staging(void* handle, int id, int tma, int pair) {
     if (tma && !tma_possible(h))
         return invalid("TMA staging needs Z * element size a multiple of 16 bytes (and no FP64 rho)");
     if (pair && !(tma && pair_possible(h))) return invalid("z-pair tiles need TMA staging and an FP32 omega instance");
-    if (h.tma == tma && h.pair == pair) return SKY_OK;
+    if (!tma_possible(h) || (h.tma == tma && h.pair == pair)) return SKY_OK;
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
     h.tma = tma;
@@ -861,7 +881,7 @@ int sky_engine_get_staging(void* handle, int id, int* tma, int* pair) {
     if (!e || !tma || !pair) return invalid("null argument");
     HostInst* hp = find(e, id);
     if (!hp) return invalid("unknown instance id");
-    *tma = hp->tma;
+    *tma = hp->tma && tma_possible(*hp);
     *pair = hp->pair;
     return SKY_OK;
 }
@@ -1052,7 +1072,7 @@ int sky_engine_read(void* handle, int id, double* field, double* velocity, int o
     if (!h) return invalid("unknown instance id");
     cudaSetDevice(e->device);
     Group& g = e->groups[h->set][h->prec];
-    const int64_t n = (int64_t)h->C * h->N;
+    const int64_t n = (int64_t)h->C * h->N, nc = (int64_t)h->C * h->sites;
     int rc = SKY_OK;
     auto convert = [&](double* f, double* v) {
         if (h->prec)
@@ -1068,13 +1088,13 @@ int sky_engine_read(void* handle, int id, double* field, double* velocity, int o
         return check_cuda(cudaStreamSynchronize(e->stream), "sync", __LINE__);
     }
     double* tmp = nullptr;
-    if ((rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * n), "cudaMalloc(read)", __LINE__))) return rc;
+    if ((rc = check_cuda(cudaMalloc(&tmp, sizeof(double) * nc), "cudaMalloc(read)", __LINE__))) return rc;
     double* outs[2] = {field, velocity};
     for (int k = 0; k < 2 && rc == SKY_OK; ++k) {
         if (!outs[k]) continue;
         rc = convert(k == 0 ? tmp : nullptr, k == 1 ? tmp : nullptr);
         if (!rc)
-            rc = check_cuda(cudaMemcpyAsync(outs[k], tmp, sizeof(double) * n, cudaMemcpyDeviceToHost, e->stream),
+            rc = check_cuda(cudaMemcpyAsync(outs[k], tmp, sizeof(double) * nc, cudaMemcpyDeviceToHost, e->stream),
                             "download", __LINE__);
         if (!rc) rc = check_cuda(cudaStreamSynchronize(e->stream), "sync", __LINE__);
     }

@@ -430,15 +430,6 @@ __device__ __forceinline__ double ld_early(const double* p) {
     return v;
 }
 template <bool ONCE>
-__device__ __forceinline__ float ld_early(const float* p) {
-    float v;
-    if constexpr (ONCE)
-        asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    else
-        asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-template <bool ONCE>
 __device__ __forceinline__ float2 ld_early2(const float* p) {
     float2 v;
     if constexpr (ONCE)
@@ -449,10 +440,11 @@ __device__ __forceinline__ float2 ld_early2(const float* p) {
 }
 
 // Epilogue of the gradient walk's stages: a thread's pair of FP32 sites, or its FP64 site, at
-// once.  WIDE: Z is a multiple of four (FP32), so the pair is one aligned 8-byte access.
+// once.  The row pitch is a multiple of four, so a pair is one aligned 8-byte access; where Z is
+// odd, the second lane of a row's last pair is padding, which nothing reads as a site.
 // EARLY: stage 3's operands are loaded before the point arithmetic (where 168 registers hold
 // both: without mixed derivatives); stage 4's two always are.
-template <typename T, int STAGE, int C, bool WIDE, bool TMA, bool EARLY>
+template <typename T, int STAGE, int C, bool TMA, bool EARLY>
 struct GradEpi {
     using L = Lanes<T>;
     using V = typename L::V;
@@ -468,23 +460,17 @@ struct GradEpi {
     V op[STAGE == 3 ? 5 : STAGE == 4 ? 2 : 1][STAGE > 2 ? C : 1];  // the update's operands at the site
 
     template <bool ONCE = true>
-    static __device__ __forceinline__ V get(const T* p, bool own1) {
+    static __device__ __forceinline__ V get(const T* p) {
         if constexpr (NL == 1)
             return ld_early<ONCE>(p);
-        else if constexpr (WIDE)
-            return P2(ld_early2<ONCE>(p));
         else
-            return P2(ld_early<ONCE>(p), own1 ? ld_early<ONCE>(p + 1) : 0.0f);
+            return P2(ld_early2<ONCE>(p));
     }
-    static __device__ __forceinline__ void store(T* p, V v, bool own1) {
-        if constexpr (NL == 1) {
+    static __device__ __forceinline__ void store(T* p, V v) {
+        if constexpr (NL == 1)
             __stcs(p, v);
-        } else if constexpr (WIDE) {
+        else
             __stcs(reinterpret_cast<float2*>(p), v.v);
-        } else {
-            __stcs(p, v.v.x);
-            if (own1) __stcs(p + 1, v.v.y);
-        }
     }
     // The next plane of the operands into L2, so that the loads at the site do not wait for DRAM:
     // box prefetches by one thread, or 128-byte lines by each row.
@@ -509,11 +495,11 @@ struct GradEpi {
         }
     }
     static constexpr int M_TZ = 32 / NL;
-    __device__ __forceinline__ void begin_site(int64_t s, int64_t N, bool own1) {
+    __device__ __forceinline__ void begin_site(int64_t s, int64_t N, bool) {
         if constexpr (NL > 1) {
             if (dlt) {
 #pragma unroll
-                for (int c = 0; c < C; ++c) d[c] = get(dlt + at(c, N, s), own1);
+                for (int c = 0; c < C; ++c) d[c] = get(dlt + at(c, N, s));
             }
         }
     }
@@ -521,26 +507,26 @@ struct GradEpi {
     static __device__ __forceinline__ uint32_t at(int c, int64_t N, int64_t s) {
         return uint32_t(c) * uint32_t(N) + uint32_t(s);
     }
-    __device__ __forceinline__ void load(int64_t s, int64_t N, bool own1) {
-        if constexpr (EARLY || STAGE == 4) operands(s, N, own1);
+    __device__ __forceinline__ void load(int64_t s, int64_t N, bool) {
+        if constexpr (EARLY || STAGE == 4) operands(s, N);
     }
-    __device__ __forceinline__ void operands(int64_t s, int64_t N, bool own1) {
+    __device__ __forceinline__ void operands(int64_t s, int64_t N) {
         if constexpr (STAGE == 3) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const uint32_t j = at(c, N, s);
-                op[0][c] = get(io.F + j, own1);
-                op[1][c] = io.Flo ? get(io.Flo + j, own1) : V(0.0f);
-                op[2][c] = io.V ? get(io.V + j, own1) : V(0.0f);
-                op[3][c] = get(io.l1 + j, own1);
-                op[4][c] = io.l2_is_l1 ? op[3][c] : get(io.l2 + j, own1);
+                op[0][c] = get(io.F + j);
+                op[1][c] = io.Flo ? get(io.Flo + j) : V(0.0f);
+                op[2][c] = io.V ? get(io.V + j) : V(0.0f);
+                op[3][c] = get(io.l1 + j);
+                op[4][c] = io.l2_is_l1 ? op[3][c] : get(io.l2 + j);
             }
         }
         if constexpr (STAGE == 4) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
-                op[0][c] = get(io.out + at(c, N, s), own1);
-                op[1][c] = get(io.pv + at(c, N, s), own1);
+                op[0][c] = get(io.out + at(c, N, s));
+                op[1][c] = get(io.pv + at(c, N, s));
             }
         }
     }
@@ -553,7 +539,7 @@ struct GradEpi {
                 if (STAGE == 1 && refresh) {  // d = g64(F): the correction becomes g64 - g32(F)
 #pragma unroll
                     for (int c = 0; c < C; ++c) {
-                        store(dlt + at(c, N, s), d[c] - g32[c], own1);
+                        store(dlt + at(c, N, s), d[c] - g32[c]);
                         g[c] = d[c];
                     }
                 } else {
@@ -564,9 +550,9 @@ struct GradEpi {
         }
         if constexpr (STAGE < 3) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) store(io.out + at(c, N, s), V(-io.dtt) * g[c], own1);
+            for (int c = 0; c < C; ++c) store(io.out + at(c, N, s), V(-io.dtt) * g[c]);
         } else if constexpr (STAGE == 3) {
-            if constexpr (!EARLY) operands(s, N, own1);
+            if constexpr (!EARLY) operands(s, N);
             V fo[C], lo[C], pv[C];
 #pragma unroll
             for (int c = 0; c < C; ++c) g[c] = V(-io.dtt) * g[c];  // l3
@@ -589,9 +575,9 @@ struct GradEpi {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const uint32_t j = at(c, N, s);
-                store(io.out + j, fo[c], own1);
-                if (io.Flo) store(io.out_lo + j, lo[c], own1);
-                store(io.pv + j, pv[c], own1);
+                store(io.out + j, fo[c]);
+                if (io.Flo) store(io.out_lo + j, lo[c]);
+                store(io.pv + j, pv[c]);
             }
         } else {
             V (&fo)[C] = op[0], (&pv)[C] = op[1];
@@ -609,32 +595,32 @@ struct GradEpi {
                 for (int c = 0; c < C; ++c) L::set(pv[c], l, ov[c]);
             }
 #pragma unroll
-            for (int c = 0; c < C; ++c) store(io.pv + at(c, N, s), pv[c], own1);
+            for (int c = 0; c < C; ++c) store(io.pv + at(c, N, s), pv[c]);
         }
     }
 };
 
 // Rho: the walk over the pion components takes R at the site and leaves H in its place
 // (k_rho_finish applies it).
-template <typename T, int STAGE, bool WIDE, bool TMA>
-struct RhoGradEpi : GradEpi<T, STAGE, 4, WIDE, TMA, false> {
-    using B = GradEpi<T, STAGE, 4, WIDE, TMA, false>;
+template <typename T, int STAGE, bool TMA>
+struct RhoGradEpi : GradEpi<T, STAGE, 4, TMA, false> {
+    using B = GradEpi<T, STAGE, 4, TMA, false>;
     using V = typename Lanes<T>::V;
     static constexpr bool kCoupled = true;
-    __device__ __forceinline__ void coupling(int64_t s, int64_t N, bool own1, V (&R)[9]) {
+    __device__ __forceinline__ void coupling(int64_t s, int64_t N, bool, V (&R)[9]) {
 #pragma unroll
-        for (int m = 0; m < 9; ++m) R[m] = B::template get<false>(B::io.R + B::at(4 + m, N, s), own1);
+        for (int m = 0; m < 9; ++m) R[m] = B::template get<false>(B::io.R + B::at(4 + m, N, s));
     }
     __device__ __forceinline__ void coupled(int64_t s, int64_t N, bool own1, const V (&J)[9], const Params& p) {
         V R[9];  // (read again, not held)
         coupling(s, N, own1, R);
 #pragma unroll
-        for (int m = 0; m < 9; ++m) B::store(B::io.R + B::at(4 + m, N, s), rho_rest(R[m], J[m], p), own1);
+        for (int m = 0; m < 9; ++m) B::store(B::io.R + B::at(4 + m, N, s), rho_rest(R[m], J[m], p));
     }
 };
 template <template <typename> class Th, typename T, int STAGE, class M, bool TMA>
-using StageEpi = typename std::conditional<Th<T>::kId == SKY_THEORY_RHO, RhoGradEpi<T, STAGE, M::WIDE, TMA>,
-                                           GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>>::type;
+using StageEpi = typename std::conditional<Th<T>::kId == SKY_THEORY_RHO, RhoGradEpi<T, STAGE, TMA>,
+                                           GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed>>::type;
 
 // A finished tile's partials: stage 1 the baryon number and (FP64) the energy, stage 4 the
 // gradient maxima and the kinetic sum.
@@ -739,7 +725,7 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
         int xa, xe, y0, z0;
         march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
         using Epi = StageEpi<Th, T, STAGE, M, TMA>;
-        Epi epi{GradEpi<T, STAGE, M::C, M::WIDE, TMA, !Th<T>::kMixed>{
+        Epi epi{GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed>{
             stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
             STAGE == 1 && half && refresh_due(in), {nullptr, nullptr, nullptr, nullptr},
             {nullptr, nullptr, nullptr, nullptr}}};
@@ -833,28 +819,16 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
 template <typename T>
 struct Vec16 {
     static constexpr int W = 16 / int(sizeof(T));
+    using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
     T v[W];
-    __device__ __forceinline__ void load(const T* p, int n) {
-        if (n == W) {
-            using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-            const V4 q = __ldcs(reinterpret_cast<const V4*>(p));
-            memcpy(v, &q, 16);
-        } else {
-#pragma unroll
-            for (int i = 0; i < W; ++i) v[i] = i < n ? __ldcs(p + i) : T(0);
-        }
+    __device__ __forceinline__ void load(const T* p) {
+        const V4 q = __ldcs(reinterpret_cast<const V4*>(p));
+        memcpy(v, &q, 16);
     }
-    __device__ __forceinline__ void store(T* p, int n) const {
-        if (n == W) {
-            using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-            V4 q;
-            memcpy(&q, v, 16);
-            __stcs(reinterpret_cast<V4*>(p), q);
-        } else {
-#pragma unroll
-            for (int i = 0; i < W; ++i)
-                if (i < n) __stcs(p + i, v[i]);
-        }
+    __device__ __forceinline__ void store(T* p) const {
+        V4 q;
+        memcpy(&q, v, 16);
+        __stcs(reinterpret_cast<V4*>(p), q);
     }
 };
 constexpr int kRhoFinishThreads = 256;
@@ -881,20 +855,21 @@ __global__ void __launch_bounds__(kRhoFinishThreads)
         const bool refresh = STAGE == 1 && half && refresh_due(in);
         T* const dlt = in.Dlt;
         StageStats<T> st(p.vol);
-        const int64_t N = n_sites(p), c0 = 4 * N, nv = (9 * N + W - 1) / W;  // (component 4 starts on 16 bytes)
+        const int64_t N = n_sites(p), c0 = 4 * N, nv = 9 * N / W;  // (rows are whole vectors)
         const int64_t v0 = nv * lt / items, v1 = nv * (lt + 1) / items;
         for (int64_t q = v0 + threadIdx.x; q < v1; q += kRhoFinishThreads) {
             const int64_t j = c0 + q * W;
-            const int n = int(min(int64_t(W), 13 * N - j));
+            // values that are sites (the others pad the row; they take no part in the statistics)
+            const int n = STAGE < 4 || p.Zp == p.Z ? W : p.Z - int(uint32_t(j) % uint32_t(p.Zp));
             V x, v, l, l2, lo, d, h, pv;
-            x.load(io.src[0] + j, n);
-            h.load(io.R + j, n);
-            if (STAGE > 1 && io.src[1]) v.load(io.src[1] + j, n);
-            if (STAGE > 2) l.load(io.src[2] + j, n);
-            if (STAGE == 3 && !io.l2_is_l1) l2.load(io.l2 + j, n);
-            if (STAGE == 3 && io.Flo) lo.load(io.Flo + j, n);
-            if (STAGE == 4) pv.load(io.pv + j, n);
-            if (dlt) d.load(dlt + j, n);
+            x.load(io.src[0] + j);
+            h.load(io.R + j);
+            if (STAGE > 1 && io.src[1]) v.load(io.src[1] + j);
+            if (STAGE > 2) l.load(io.src[2] + j);
+            if (STAGE == 3 && !io.l2_is_l1) l2.load(io.l2 + j);
+            if (STAGE == 3 && io.Flo) lo.load(io.Flo + j);
+            if (STAGE == 4) pv.load(io.pv + j);
+            if (dlt) d.load(dlt + j);
             V o1, o2, o3;
 #pragma unroll
             for (int i = 0; i < W; ++i) {
@@ -931,11 +906,11 @@ __global__ void __launch_bounds__(kRhoFinishThreads)
                     o1.v[i] = o[0];
                 }
             }
-            if (refresh && dlt) d.store(dlt + j, n);
-            o1.store((STAGE == 4 ? io.pv : io.out) + j, n);
+            if (refresh && dlt) d.store(dlt + j);
+            o1.store((STAGE == 4 ? io.pv : io.out) + j);
             if constexpr (STAGE == 3) {
-                if (io.Flo) o2.store(io.out_lo + j, n);
-                o3.store(io.pv + j, n);
+                if (io.Flo) o2.store(io.out_lo + j);
+                o3.store(io.pv + j);
             }
         }
         if constexpr (STAGE == 4) tile_partials<T, STAGE>(in, in.ntiles + lt, KSum{}, KSum{}, st, false, shk, shm);

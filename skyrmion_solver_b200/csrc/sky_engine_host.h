@@ -19,7 +19,8 @@ struct HostInst {
     int defect = 0;  // ... and a defect-corrected gradient (precision 3)
     int defect_period = kDefectRefresh;  // steps between refreshes of the correction
     Params p{};
-    int64_t N = 0;
+    int64_t sites = 0;  // lattice sites: values of a component in the caller's arrays
+    int64_t N = 0;      // values of a component here, rows padded to p.Zp (n_sites)
     int C = 0;
     void* arena = nullptr;  // one allocation that holds every array below
     void* parts = nullptr;  // the partials' own allocation once sky_engine_retile has changed their sizes
@@ -54,7 +55,6 @@ struct Group {
     int* d_done = nullptr;     // blocks of the current step's stage-1 and stage-4 launches finished (0 between steps)
     int desc_cap = 0, tile_cap = 0;
     int ntiles = 0, entiles = 0, rtiles = 0;
-    bool all_wide = true;   // every member can use the wide-row (16-byte staged) kernels
     bool any_defect = false;  // holds a defect-corrected instance (launch the defect refresh)
     bool all_tma = false;     // every member has TMA plane maps (launch the TMA stage kernels)
 };

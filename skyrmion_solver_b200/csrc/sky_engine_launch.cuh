@@ -1,5 +1,5 @@
-// Launch side of the engine kernels for one theory: tile shapes, kernel variants (wide or
-// narrow rows, TMA or cp.async copies) and the table of entry points that sky_engine.cu calls.
+// Launch side of the engine kernels for one theory: tile shapes, kernel variants (TMA or
+// cp.async copies) and the table of entry points that sky_engine.cu calls.
 #pragma once
 
 #include <cmath>
@@ -37,14 +37,12 @@ template <template <typename> class Th, typename T>
 constexpr int stage_blocks() {
     return sizeof(T) == 4 ? 2 : 1;
 }
-template <int C, template <typename> class Th, typename T, bool WIDE>
-using WalkShape = MarchShape<C, stage_rows<Th, T>(), WIDE, sizeof(T) == 8 ? 2 : 4>;
-template <template <typename> class Th, typename T, bool WIDE>
-using MShape = WalkShape<is_rho<Th>() ? 4 : Th<T>::C, Th, T, WIDE>;
+template <template <typename> class Th, typename T>
+using MShape = MarchShape<is_rho<Th>() ? 4 : Th<T>::C, stage_rows<Th, T>(), true, sizeof(T) == 8 ? 2 : 4>;
 
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, int STAGE, bool TMA>
 struct StageKernel {
-    using M = MShape<Th, T, WIDE>;
+    using M = MShape<Th, T>;
     static auto kern() {
         if constexpr (is_rho<Th>())
             return k_grad_stage<RhoPion, M, T, STAGE, stage_blocks<Th, T>(), TMA>;
@@ -68,9 +66,9 @@ template <typename T>
 constexpr int rho_blocks() {
     return sizeof(T) == 8 ? 2 : 3;
 }
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, int STAGE, bool TMA>
 struct RhoKernel {
-    using M = MarchShape<3, rho_rows<T>(), WIDE, sizeof(T) == 8 ? 2 : 4>;
+    using M = MarchShape<3, rho_rows<T>(), true, sizeof(T) == 8 ? 2 : 4>;
     static auto kern() { return k_rho_stage<M, T, STAGE, rho_blocks<T>(), TMA>; }
     static size_t smem() { return rho_stage_bytes<M, T, STAGE, TMA>(); }
     static dim3 block() { return dim3(GradBlock<M, T>::TZ, M::BY); }
@@ -126,9 +124,9 @@ static int launch_chain(bool chained, void (*kern)(Args...), int blocks, dim3 bl
     return check_cuda(cudaGetLastError(), "launch engine kernel", __LINE__);
 }
 
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, int STAGE, bool TMA>
 static int launch_stage_w(const Group& g, const StageArgs& a, cudaStream_t st) {
-    using SK = StageKernel<Th, T, STAGE, WIDE, TMA>;
+    using SK = StageKernel<Th, T, STAGE, TMA>;
     int per_sm = 1;
     int rc = stage_setup<SK>(&per_sm);
     if (rc) return rc;
@@ -136,7 +134,7 @@ static int launch_stage_w(const Group& g, const StageArgs& a, cudaStream_t st) {
     if (n <= 0) return SKY_OK;
     InstDesc<T>* d = reinterpret_cast<InstDesc<T>*>(g.d_desc);
     if constexpr (is_rho<Th>()) {
-        using RK = RhoKernel<Th, T, STAGE, WIDE, TMA>;
+        using RK = RhoKernel<Th, T, STAGE, TMA>;
         int rho_per_sm = 1;
         if ((rc = stage_setup<RK>(&rho_per_sm))) return rc;
         const int resident = num_sms() * rho_per_sm, items = 3 * (a.r_end - a.r_begin);
@@ -158,7 +156,7 @@ static int launch_stage_w(const Group& g, const StageArgs& a, cudaStream_t st) {
     }
     if (tail) {
         int other = 1;
-        if ((rc = stage_setup<StageKernel<Th, T, STAGE == 1 ? 4 : 1, WIDE, TMA>>(&other))) return rc;
+        if ((rc = stage_setup<StageKernel<Th, T, STAGE == 1 ? 4 : 1, TMA>>(&other))) return rc;
         total = blocks + (n < num_sms() * other ? n : num_sms() * other);
     }
     return launch_chain(a.chained, SK::kern(), blocks, SK::block(), SK::smem(), st, d, d, g.d_tile_inst, a.t_begin, a.t_end,
@@ -169,10 +167,9 @@ template <template <typename> class Th, typename T, int STAGE>
 static int launch_stage(const Group& g, const StageArgs& a, cudaStream_t st) {
     // (FP64 rho has no TMA maps: tma_possible)
     if constexpr (!(is_rho<Th>() && sizeof(T) == 8)) {
-        if (g.all_tma) return launch_stage_w<Th, T, STAGE, true, true>(g, a, st);
+        if (g.all_tma) return launch_stage_w<Th, T, STAGE, true>(g, a, st);
     }
-    if (g.all_wide) return launch_stage_w<Th, T, STAGE, true, false>(g, a, st);
-    return launch_stage_w<Th, T, STAGE, false, false>(g, a, st);
+    return launch_stage_w<Th, T, STAGE, false>(g, a, st);
 }
 
 // Energy walk of a group's instances (energy_walk), energy tiles [t_begin, t_end).  CURL: FP32 rho's
@@ -181,9 +178,9 @@ template <template <typename> class Th, typename T>
 constexpr bool split_energy() {
     return is_rho<Th>() && sizeof(T) == 4;
 }
-template <template <typename> class Th, typename T, bool WIDE, bool TMA, bool CURL>
+template <template <typename> class Th, typename T, bool TMA, bool CURL>
 struct EnergyKernel {
-    using M = MarchShape<CURL ? 3 : split_energy<Th, T>() ? 4 : Th<double>::C, kDensRows, WIDE, sizeof(T) == 8 ? 2 : 4>;
+    using M = MarchShape<CURL ? 3 : split_energy<Th, T>() ? 4 : Th<double>::C, kDensRows, true, sizeof(T) == 8 ? 2 : 4>;
     using Pipe = DensPipe<M, T, sizeof(T) == 8 ? 1 : 2, TMA, CURL>;
     static auto kern() {
         if constexpr (split_energy<Th, T>())
@@ -205,24 +202,23 @@ static int launch_energy_k(const Group& g, const StageArgs& a, int per, cudaStre
     return launch_chain(a.chained, EK::kern(), blocks, EK::block(), EK::smem(), st, reinterpret_cast<InstDesc<T>*>(g.d_desc),
                       g.d_tile_inst + g.ntiles, a.t_begin, a.t_end, a.in_step);
 }
-template <template <typename> class Th, typename T, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, bool TMA>
 static int launch_energy_w(const Group& g, const StageArgs& a, cudaStream_t st) {
     if constexpr (split_energy<Th, T>()) {
-        const int rc = launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, true>, T>(g, a, 3, st);
+        const int rc = launch_energy_k<EnergyKernel<Th, T, TMA, true>, T>(g, a, 3, st);
         if (rc) return rc;
         StageArgs b = a;
         b.chained = 1;
-        return launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, false>, T>(g, b, 1, st);
+        return launch_energy_k<EnergyKernel<Th, T, TMA, false>, T>(g, b, 1, st);
     }
-    return launch_energy_k<EnergyKernel<Th, T, WIDE, TMA, false>, T>(g, a, 1, st);
+    return launch_energy_k<EnergyKernel<Th, T, TMA, false>, T>(g, a, 1, st);
 }
 template <template <typename> class Th, typename T>
 static int launch_energy_p(const Group& g, const StageArgs& a, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
-        if (g.all_tma) return launch_energy_w<Th, T, true, true>(g, a, st);
+        if (g.all_tma) return launch_energy_w<Th, T, true>(g, a, st);
     }
-    if (g.all_wide) return launch_energy_w<Th, T, true, false>(g, a, st);
-    return launch_energy_w<Th, T, false, false>(g, a, st);
+    return launch_energy_w<Th, T, false>(g, a, st);
 }
 template <template <typename> class Th>
 static int launch_energy_t(const Group& g, const StageArgs& a, cudaStream_t st) {
@@ -245,34 +241,34 @@ static int stage_dispatch_prec(int prec, int stage, const Group& g, const StageA
     return prec ? launch_stage_any<Th, double>(stage, g, a, st) : launch_stage_any<Th, float>(stage, g, a, st);
 }
 
-template <template <typename> class Th, typename T, int STAGE, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, int STAGE, bool TMA>
 static int setup_stage() {
-    int n, rc = stage_setup<StageKernel<Th, T, STAGE, WIDE, TMA>>(&n);
+    int n, rc = stage_setup<StageKernel<Th, T, STAGE, TMA>>(&n);
     if constexpr (is_rho<Th>()) {
-        if (!rc) rc = stage_setup<RhoKernel<Th, T, STAGE, WIDE, TMA>>(&n);
+        if (!rc) rc = stage_setup<RhoKernel<Th, T, STAGE, TMA>>(&n);
     }
     return rc;
 }
-template <template <typename> class Th, typename T, bool WIDE, bool TMA>
+template <template <typename> class Th, typename T, bool TMA>
 static int setup_stages() {
     int n, rc;
-    if ((rc = setup_stage<Th, T, 1, WIDE, TMA>()) || (rc = setup_stage<Th, T, 2, WIDE, TMA>()) ||
-        (rc = setup_stage<Th, T, 3, WIDE, TMA>()) || (rc = setup_stage<Th, T, 4, WIDE, TMA>()))
+    if ((rc = setup_stage<Th, T, 1, TMA>()) || (rc = setup_stage<Th, T, 2, TMA>()) ||
+        (rc = setup_stage<Th, T, 3, TMA>()) || (rc = setup_stage<Th, T, 4, TMA>()))
         return rc;
     if constexpr (energy_walk<T>(Th<T>::kId)) {
         if constexpr (split_energy<Th, T>()) {
-            if ((rc = stage_setup<EnergyKernel<Th, T, WIDE, TMA, true>>(&n))) return rc;
+            if ((rc = stage_setup<EnergyKernel<Th, T, TMA, true>>(&n))) return rc;
         }
-        return stage_setup<EnergyKernel<Th, T, WIDE, TMA, false>>(&n);
+        return stage_setup<EnergyKernel<Th, T, TMA, false>>(&n);
     }
     return SKY_OK;
 }
 template <template <typename> class Th, typename T>
 static int setup_prec(const Group& g) {
     if constexpr (!(is_rho<Th>() && sizeof(T) == 8)) {
-        if (g.all_tma) return setup_stages<Th, T, true, true>();
+        if (g.all_tma) return setup_stages<Th, T, true>();
     }
-    return g.all_wide ? setup_stages<Th, T, true, false>() : setup_stages<Th, T, false, false>();
+    return setup_stages<Th, T, false>();
 }
 // Kernel attributes of the variants that a group's steps launch (kept out of stream capture).
 template <template <typename> class Th>
@@ -285,11 +281,11 @@ static int setup_group_kernels(const Group& g) {
 // not depend on the staging, so neither does the order of the per-tile partial sums.
 template <template <typename> class Th>
 static TileShapeInfo shape_of(int prec) {
-    return prec ? TileShapeInfo{stage_rows<Th, double>(), stage_blocks<Th, double>(), MShape<Th, double, true>::HZ,
-                                MShape<Th, double, true>::C, rho_rows<double>(),
+    return prec ? TileShapeInfo{stage_rows<Th, double>(), stage_blocks<Th, double>(), MShape<Th, double>::HZ,
+                                MShape<Th, double>::C, rho_rows<double>(),
                                 rho_blocks<double>()}
-                : TileShapeInfo{stage_rows<Th, float>(), stage_blocks<Th, float>(), MShape<Th, float, true>::HZ,
-                                MShape<Th, float, true>::C, rho_rows<float>(),
+                : TileShapeInfo{stage_rows<Th, float>(), stage_blocks<Th, float>(), MShape<Th, float>::HZ,
+                                MShape<Th, float>::C, rho_rows<float>(),
                                 rho_blocks<float>()};
 }
 
@@ -306,14 +302,14 @@ static int launch_defect_k(bool chained, K kern, size_t smem, int* per_sm, const
                         reinterpret_cast<InstDesc<float>*>(g.d_desc), g.d_tile_inst, 0, g.ntiles);
 }
 // TBY: rows of the stage tiles.
-template <template <typename> class Th, int TBY, bool WIDE>
+template <template <typename> class Th, int TBY = stage_rows<Th, float>()>
 static int launch_defect_t(const Group& g, cudaStream_t st) {
     // two sub-tiles of a 16-row engine tile, one of the others
     constexpr int rows = TBY == 16 ? 8 : TBY;
     static int per_sm = 0;
     if constexpr (is_rho<Th>()) {
-        using R = MarchShape<3, rows, WIDE>;
-        using M = MarchShape<4, rows, WIDE>;
+        using R = MarchShape<3, rows, true>;
+        using M = MarchShape<4, rows, true>;
         static int rho_per_sm = 0;
         const int rc = launch_defect_k<R, 3>(false, k_defect<RhoPion, R, TBY, true>,
                                              RhoPipe<R, double, float, 2, false>::bytes, &rho_per_sm, g, st);
@@ -321,15 +317,10 @@ static int launch_defect_t(const Group& g, cudaStream_t st) {
         return launch_defect_k<M, 1>(true, k_defect<RhoPion, M, TBY, false>,
                                      GradPipe<RhoPion, M, double, float, 2, false>::bytes, &per_sm, g, st);
     } else {
-        using M = MarchShape<Th<double>::C, rows, WIDE>;
+        using M = MarchShape<Th<double>::C, rows, true>;
         return launch_defect_k<M, 1>(false, k_defect<Th, M, TBY, false>, GradPipe<Th, M, double, float, 2, false>::bytes,
                                      &per_sm, g, st);
     }
-}
-
-template <template <typename> class Th, int TBY = stage_rows<Th, float>()>
-static int launch_defect_w(const Group& g, cudaStream_t st) {
-    return g.all_wide ? launch_defect_t<Th, TBY, true>(g, st) : launch_defect_t<Th, TBY, false>(g, st);
 }
 
 // Energy audit of the RK4 dynamics (k_engine_audit).
@@ -340,7 +331,7 @@ constexpr int audit_rows() {
 
 template <template <typename> class Th, typename S>
 static int audit_t(const Group& g, const HostInst& h, cudaStream_t st, double* out2) {
-    using M = MarchShape<Th<double>::C, audit_rows<Th>(), false>;
+    using M = MarchShape<Th<double>::C, audit_rows<Th>(), true, std::is_same<S, double>::value ? 2 : 4>;
     constexpr int NSRC = std::is_same<S, double>::value ? 1 : 2;
     auto kern = k_engine_audit<Th, M, S>;
     const size_t smem = DensPipe<M, S, NSRC, false>::bytes;
@@ -390,7 +381,7 @@ static int audit_prec(const Group& g, const HostInst& h, cudaStream_t st, double
 
 template <template <typename> class Th>
 constexpr TheoryOps make_ops() {
-    return TheoryOps{shape_of<Th>, setup_group_kernels<Th>, stage_dispatch_prec<Th>, launch_energy_t<Th>, launch_defect_w<Th>,
+    return TheoryOps{shape_of<Th>, setup_group_kernels<Th>, stage_dispatch_prec<Th>, launch_energy_t<Th>, launch_defect_t<Th>,
                      audit_prec<Th>};
 }
 

@@ -5,16 +5,16 @@ namespace sky {
 
 // FP32 rho of at most kFusedRhoSites sites: 8 rows of all thirteen components, one site per thread.
 constexpr int kFusedRows = 8;
-template <int STAGE, bool WIDE, bool TMA>
+template <int STAGE, bool TMA>
 struct FusedKernel {
-    using M = MarchShape<13, kFusedRows, WIDE>;
+    using M = MarchShape<13, kFusedRows, true>;
     static auto kern() { return k_rho_fused<M, STAGE, TMA>; }
     static size_t smem() { return rho_fused_bytes<M, STAGE, TMA>(); }
     static dim3 block() { return dim3(M::BZ, M::BY); }
 };
-template <int STAGE, bool WIDE, bool TMA>
+template <int STAGE, bool TMA>
 static int launch_fused_w(const Group& g, const StageArgs& a, cudaStream_t st) {
-    using FK = FusedKernel<STAGE, WIDE, TMA>;
+    using FK = FusedKernel<STAGE, TMA>;
     int per_sm = 1;
     int rc = stage_setup<FK>(&per_sm);
     if (rc) return rc;
@@ -26,8 +26,7 @@ static int launch_fused_w(const Group& g, const StageArgs& a, cudaStream_t st) {
 }
 template <int STAGE>
 static int launch_fused(const Group& g, const StageArgs& a, cudaStream_t st) {
-    if (g.all_tma) return launch_fused_w<STAGE, true, true>(g, a, st);
-    return g.all_wide ? launch_fused_w<STAGE, true, false>(g, a, st) : launch_fused_w<STAGE, false, false>(g, a, st);
+    return g.all_tma ? launch_fused_w<STAGE, true>(g, a, st) : launch_fused_w<STAGE, false>(g, a, st);
 }
 static int fused_stage(int, int stage, const Group& g, const StageArgs& a, cudaStream_t st) {
     switch (stage) {
@@ -37,17 +36,16 @@ static int fused_stage(int, int stage, const Group& g, const StageArgs& a, cudaS
         default: return launch_fused<4>(g, a, st);
     }
 }
-template <bool WIDE, bool TMA>
+template <bool TMA>
 static int setup_fused_w() {
     int n, rc;
-    if ((rc = stage_setup<FusedKernel<1, WIDE, TMA>>(&n)) || (rc = stage_setup<FusedKernel<2, WIDE, TMA>>(&n)) ||
-        (rc = stage_setup<FusedKernel<3, WIDE, TMA>>(&n)))
+    if ((rc = stage_setup<FusedKernel<1, TMA>>(&n)) || (rc = stage_setup<FusedKernel<2, TMA>>(&n)) ||
+        (rc = stage_setup<FusedKernel<3, TMA>>(&n)))
         return rc;
-    return stage_setup<FusedKernel<4, WIDE, TMA>>(&n);
+    return stage_setup<FusedKernel<4, TMA>>(&n);
 }
 static int setup_fused(const Group& g) {
-    if (g.all_tma) return setup_fused_w<true, true>();
-    return g.all_wide ? setup_fused_w<true, false>() : setup_fused_w<false, false>();
+    return g.all_tma ? setup_fused_w<true>() : setup_fused_w<false>();
 }
 static TileShapeInfo fused_shape(int) {
     return TileShapeInfo{kFusedRows, 1, MarchShape<13, kFusedRows, true>::HZ, 13, 0, 0};
@@ -55,5 +53,5 @@ static TileShapeInfo fused_shape(int) {
 
 extern const TheoryOps kRhoOps = make_ops<Rho>();
 extern const TheoryOps kFusedRhoOps = {fused_shape, setup_fused, fused_stage, launch_energy_t<Rho>,
-                                       launch_defect_w<Rho, kFusedRows>, audit_prec<Rho>};
+                                       launch_defect_t<Rho, kFusedRows>, audit_prec<Rho>};
 }  // namespace sky

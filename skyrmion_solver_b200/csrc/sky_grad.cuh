@@ -193,7 +193,7 @@ struct PlanePipe {
     __device__ __forceinline__ PlanePipe(T* sm, const Params& p, const S* const (&src_)[3], T a, T b, int tid_, int y0_,
                                          int z0_, TmaTile* tma_, int64_t cstride = 0)
         : ring(sm), stage(reinterpret_cast<S*>(reinterpret_cast<char*>(sm) + ring_bytes)), src(src_), w{T(1), a, b},
-          tma(tma_), tid(tid_), y0(y0_), z0(z0_), X(p.X), YZ((int64_t)p.Y * p.Z), ns(0), e0(1) {
+          tma(tma_), tid(tid_), y0(y0_), z0(z0_), X(p.X), YZ((int64_t)p.Y * p.Zp), ns(0), e0(1) {
         if constexpr (!TMA) po.init(p, STRIDED ? cstride : n_sites(p), y0, z0, tid);
 #pragma unroll
         for (int s = 1; s < NSRC; ++s)
@@ -456,7 +456,7 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
     T* Hs = Gs + P::CM * PLANE;
 
     const int64_t N = n_sites(p);
-    const int64_t YZ = (int64_t)p.Y * p.Z;
+    const int64_t YZ = (int64_t)p.Y * p.Zp;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = y0 + ty, z = z0 + NL * tx;
     const bool own = (y < p.Y) && (z < p.Z);
@@ -476,7 +476,7 @@ __device__ __forceinline__ bool grad_tile(T* __restrict__ sm, const Params& p, c
     // ring offsets of planes x-2 .. x+2 (and, with six slots, x+3)
     int o0 = 0, o1 = SLOT, o2 = 2 * SLOT, o3 = 3 * SLOT, o4 = 4 * SLOT, o5 = 5 * SLOT;
     int nslot = 0;  // slot of plane x - 2
-    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
+    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Zp + z;
     // the second derivatives are taken with the opposite sign, as the streamed point arithmetic
     // wants them (no negations to issue)
     const V r1x = V(k.r1[0]), r1y = V(k.r1[1]), r1z = V(k.r1[2]);
@@ -646,7 +646,7 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
                                           TmaTile* tma = nullptr, int64_t cstride = 0) {
     using Pipe = DensPipe<M, S, NSRC, TMA, STRIDED>;
     constexpr int C = M::C, SLOT = M::SLOT, PLANE = M::PLANE, HZ = M::HZ;
-    const int64_t YZ = (int64_t)p.Y * p.Z;
+    const int64_t YZ = (int64_t)p.Y * p.Zp;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = y0 + ty, z = z0 + tx;
     const bool own = (y < p.Y) && (z < p.Z);
@@ -670,7 +670,7 @@ __device__ __forceinline__ bool dens_tile(double* __restrict__ sm, const Params&
     }
     if (xa + 3 <= q1) pipe.issue(xa + 3, 1);
     int k = 2;  // slot of plane x
-    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
+    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Zp + z;
     for (int x = xa; x < xe; ++x, s += YZ) {
         const double* P0 = sm + k * SLOT + lofs;
         const double* P2 = sm + ((k + 2) & 3) * SLOT + lofs;

@@ -15,8 +15,8 @@ namespace sky {
 
 // A row of a staged plane holds z = z0 - ZOFF .. z0 - ZOFF + HZ - 1.  Narrow rows
 // (36 values: z0-2 .. z0+33) are filled element by element; wide rows (40 values:
-// z0-4 .. z0+35) are filled with 16-byte copies, which needs Z to be a multiple of
-// 16 / sizeof(T) so that every 16-byte chunk of a row starts on a 16-byte boundary
+// z0-4 .. z0+35) are filled with 16-byte copies, which needs the row pitch Zp to be a multiple
+// of 16 / sizeof(T) so that every 16-byte chunk of a row starts on a 16-byte boundary
 // and lies wholly inside or (as the first chunk at z0 = 0) wholly outside the lattice
 // in z; a chunk crossing z = Z copies its in-lattice part and zero-fills the rest.
 //
@@ -65,13 +65,14 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Per-thread element offsets of the haloed plane: element k of thread tid is
 // idx = tid + k*NTHREADS of the slot, i.e. (c, yy, zz) = decompose(idx); its
-// global offset within the x-plane is c*N + gy*Z + gz (int32), or -1 when the
+// global offset within the x-plane is c*N + gy*Zp + gz (32 bits), or all ones when the
 // point lies outside the lattice in y or z (or idx is past the slot).  The
-// host guarantees C*N < 2^31 for marching launches.
+// host guarantees C*N < 2^32 - 1 for marching launches.
 template <class M, int NT = M::NTHREADS>
 struct PlaneOffsets {
     static constexpr int NPER = (M::SLOT + NT - 1) / NT;
-    int off[NPER];
+    static constexpr uint32_t kNone = 0xffffffffu;
+    uint32_t off[NPER];
     __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0, int tid) {
 #pragma unroll
         for (int k = 0; k < NPER; ++k) {
@@ -82,7 +83,7 @@ struct PlaneOffsets {
             const int yy = row - c * M::HY;
             const int gy = y0 - 2 + yy, gz = z0 - M::ZOFF + zz;
             const bool ok = idx < M::SLOT && gy >= 0 && gy < p.Y && gz >= 0 && gz < p.Z;
-            off[k] = ok ? static_cast<int>(c * N + (int64_t)gy * p.Z + gz) : -1;
+            off[k] = ok ? static_cast<uint32_t>(c * N + (int64_t)gy * p.Zp + gz) : kNone;
         }
     }
 };
@@ -96,7 +97,7 @@ struct PlaneChunks {
     static constexpr int CPR = M::HZ / VW;
     static constexpr int NCHS = M::C * M::HY * CPR;
     static constexpr int NCH = (NCHS + NT - 1) / NT;
-    int off[NCH];
+    uint32_t off[NCH];
     int nb[NCH];
     __device__ __forceinline__ void init(const Params& p, int64_t N, int y0, int z0, int tid) {
         static_assert(M::WIDE && M::HZ % VW == 0, "16-byte chunks need the wide row layout");
@@ -109,7 +110,7 @@ struct PlaneChunks {
             const int yy = row - c * M::HY;
             const int gy = y0 - 2 + yy, gz0 = z0 - M::ZOFF + cz * VW;
             const bool ok = ci < NCHS && gy >= 0 && gy < p.Y && gz0 >= 0 && gz0 < p.Z;
-            off[k] = ok ? static_cast<int>(c * N + (int64_t)gy * p.Z + gz0) : 0;
+            off[k] = ok ? static_cast<uint32_t>(c * N + (int64_t)gy * p.Zp + gz0) : 0;
             nb[k] = ok ? int(sizeof(T)) * min(VW, p.Z - gz0) : 0;
         }
     }
@@ -149,7 +150,7 @@ __device__ __forceinline__ void plane_issue(T* __restrict__ stage, const PlaneOf
     for (int k = 0; k < PlaneOffsets<M, NT>::NPER; ++k) {
         const int idx = tid + k * NT;
         if (M::SLOT % NT == 0 || idx < M::SLOT) {
-            const bool ok = xok && po.off[k] >= 0;
+            const bool ok = xok && po.off[k] != PlaneOffsets<M, NT>::kNone;
 #pragma unroll
             for (int s = 0; s < NSRC; ++s) {
                 const T* g = src[s];

@@ -191,7 +191,7 @@ int pack_core(const int32_t* p_i, int32_t n_pi, const double* p_f, int32_t n_pf,
     memset(&q, 0, sizeof(q));
     q.X = p_i[0];
     q.Y = p_i[1];
-    q.Z = p_i[2];
+    q.Z = q.Zp = p_i[2];
     q.halo = p_i[3];
     q.C = p_i[5];
     q.nsky = p_i[5];

@@ -53,7 +53,7 @@ __device__ __forceinline__ bool rho_tile(T* __restrict__ sm, const Params& p, co
     T* Az = Wy + P::YP;                                                       // u_x(rho_z), z-halo
     T* Wz = Az + P::ZP;                                                       // d_x rho_x + d_y rho_y, z-halo
 
-    const int64_t YZ = (int64_t)p.Y * p.Z;
+    const int64_t YZ = (int64_t)p.Y * p.Zp;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = y0 + ty, z = z0 + NL * tx;
     const bool own = (y < p.Y) && (z < p.Z);
@@ -72,7 +72,7 @@ __device__ __forceinline__ bool rho_tile(T* __restrict__ sm, const Params& p, co
 
     int o0 = 0, o1 = SLOT, o2 = 2 * SLOT, o3 = 3 * SLOT, o4 = 4 * SLOT, o5 = 5 * SLOT;
     int nslot = 0;
-    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Z + z;
+    int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Zp + z;
     const V r1x = V(k.r1[0]), r1y = V(k.r1[1]), r1z = V(k.r1[2]);
     const V r2x = V(k.r2[0]), r2y = V(k.r2[1]), r2z = V(k.r2[2]);
     for (int x = xa; x < xe; ++x, s += YZ) {

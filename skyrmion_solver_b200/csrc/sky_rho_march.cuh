@@ -16,6 +16,8 @@ constexpr size_t rho_march_bytes(int nsrc, bool tma) {
     return size_t(rho_march_slots(nsrc, tma)) * M::SLOT * sizeof(float);
 }
 
+// Combine the thread's own staged chunks (source type S) into a ring slot of
+// type T: X = F + a V + b L.
 template <class M, int NSRC, typename T, typename S = T, int NT = M::NTHREADS>
 __device__ __forceinline__ void plane_combine_wide(T* __restrict__ slot, const S* __restrict__ stage, T a, T b,
                                                    int tid) {
@@ -41,22 +43,6 @@ __device__ __forceinline__ void plane_combine_wide(T* __restrict__ slot, const S
     }
 }
 
-// Combine the thread's own staged elements (source type S) into a ring slot of
-// type T: X = F + a V + b L.
-template <class M, int NSRC, typename T, typename S = T, int NT = M::NTHREADS>
-__device__ __forceinline__ void plane_combine(T* __restrict__ slot, const S* __restrict__ stage, T a, T b, int tid) {
-#pragma unroll
-    for (int k = 0; k < PlaneOffsets<M, NT>::NPER; ++k) {
-        const int idx = tid + k * NT;
-        if (M::SLOT % NT == 0 || idx < M::SLOT) {
-            T v = T(stage[idx]);
-            if (NSRC > 1) v += a * T(stage[M::SLOT + idx]);
-            if (NSRC > 2) v += b * T(stage[2 * M::SLOT + idx]);
-            slot[idx] = v;
-        }
-    }
-}
-
 // Raw first-difference sum c_m f[m*st], c = (1, -8, 0, 8, -1) for m = -2..2.
 template <typename T>
 __device__ __forceinline__ T diff5(const T* f, int st) {
@@ -74,7 +60,7 @@ __device__ __forceinline__ bool rho_march_tile(float* __restrict__ sm, const Par
                                                KSum& bsum, TmaTile* tma) {
     using T = float;
     constexpr int C = M::C;
-    static_assert(!TMA || M::WIDE, "TMA staging: wide rows");
+    static_assert(M::WIDE, "the engine's rows are padded to whole 16-byte chunks");
     constexpr bool DIRECT = NSRC == 1;
     constexpr int R = rho_march_slots(NSRC, TMA) - (DIRECT ? 0 : (TMA ? NSRC - 1 : NSRC));  // ring slots
     constexpr int DST = DIRECT ? R * M::SLOT : M::SLOT;  // distance between the sources' copies
@@ -82,24 +68,19 @@ __device__ __forceinline__ bool rho_march_tile(float* __restrict__ sm, const Par
     T* stage = sm + R * M::SLOT;
 
     const int64_t N = n_sites(p);
-    const int64_t YZ = (int64_t)p.Y * p.Z;
+    const int64_t YZ = (int64_t)p.Y * p.Zp;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = y0 + ty, z = z0 + tx;
     const bool own = (y < p.Y) && (z < p.Z);
     StencilCoef<T> k;
     k.init(p);
-    // element offsets (narrow rows) or 16-byte chunks (wide rows) of the haloed plane
-    using PO = typename std::conditional<M::WIDE, PlaneChunks<M, T>, PlaneOffsets<M>>::type;
-    PO po;
+    PlaneChunks<M, T> po;  // 16-byte chunks of the haloed plane
     po.init(p, N, y0, z0, tx + M::BZ * ty);
     const int q0 = xa - 2, q1 = xe + 1;
     const int lofs = (ty + 2) * M::HZ + (tx + M::ZOFF);  // thread's site within a component plane
     auto issue = [&](int64_t base, bool xok, int dslot) {
         T* dst = DIRECT ? ring + dslot * M::SLOT : stage;
-        if constexpr (M::WIDE)
-            plane_issue_wide<M, NSRC, T, DST>(dst, po, src, base, xok, tx + M::BZ * ty, src[0]);
-        else
-            plane_issue<M, NSRC, T, DST>(dst, po, src, base, xok, tx + M::BZ * ty, src[0]);
+        plane_issue_wide<M, NSRC, T, DST>(dst, po, src, base, xok, tx + M::BZ * ty, src[0]);
     };
     // TMA: thread 0 copies plane qq of every present source (a plane outside the lattice arrives as
     // zeros); source 0 into ring slot dslot, further sources into the staging slots
@@ -186,10 +167,7 @@ __device__ __forceinline__ bool rho_march_tile(float* __restrict__ sm, const Par
         } else {
             cp_async_wait_all();
             __syncthreads();  // (A), as above
-            if constexpr (M::WIDE)
-                plane_combine_wide<M, NSRC, T>(ring + slot * M::SLOT, stage, a, b, tx + M::BZ * ty);
-            else
-                plane_combine<M, NSRC, T>(ring + slot * M::SLOT, stage, a, b, tx + M::BZ * ty);
+            plane_combine_wide<M, NSRC, T>(ring + slot * M::SLOT, stage, a, b, tx + M::BZ * ty);
             if (q < q1) issue((int64_t)(q + 1) * YZ, q + 1 >= 0 && q + 1 < p.X, 0);
             __syncthreads();  // (B) slot complete
         }
@@ -202,7 +180,7 @@ __device__ __forceinline__ bool rho_march_tile(float* __restrict__ sm, const Par
             const T* Pp1 = ring + ((slot + R - 1) % R) * M::SLOT + lofs;
             const T* Pp2 = ring + slot * M::SLOT + lofs;
             const Mask mk = site_mask(p, x, y, z);
-            const int64_t s = (int64_t)x * YZ + (int64_t)y * p.Z + z;
+            const int64_t s = (int64_t)x * YZ + (int64_t)y * p.Zp + z;
             // baryon density of an FP32 stage input, from the FP32 derivatives the gradient uses
             // (its FP64 sum needs no more than FP32 per-site accuracy; only the energy, which
             // decides the arrest, is evaluated in FP64)

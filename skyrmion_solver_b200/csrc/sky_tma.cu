@@ -29,18 +29,18 @@ static PfnEncodeTiled encode_fn() {
     return fn;
 }
 
-int encode_plane_map(TmaMap* out, const void* base, int esize, int X, int Y, int Z, int C, int hz, int hy) {
+int encode_plane_map(TmaMap* out, const void* base, int esize, int X, int Y, int Z, int Zp, int C, int hz, int hy) {
     if (!out || !base) return invalid("null tensor-map argument");
     if (esize != 4 && esize != 8) return invalid("TMA plane maps hold FP32 or FP64 values");
     const uint64_t es = (uint64_t)esize;
-    const uint64_t N = (uint64_t)X * Y * Z;
+    const uint64_t N = (uint64_t)X * Y * Zp;
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return invalid("TMA plane map: base not 16-byte aligned");
-    if ((Z * es) % 16 != 0 || (N * es) % 16 != 0) return invalid("TMA plane map: row pitch not a multiple of 16 B");
+    if (Zp < Z || (Zp * es) % 16 != 0 || (N * es) % 16 != 0) return invalid("TMA plane map: row pitch not a multiple of 16 B");
     if ((hz * es) % 16 != 0 || hz > 256 || hy > 256 || C > 256) return invalid("TMA plane map: box out of range");
     PfnEncodeTiled fn = encode_fn();
     if (!fn) return invalid("cuTensorMapEncodeTiled is not available from the driver");
     const cuuint64_t dims[4] = {(cuuint64_t)Z, (cuuint64_t)Y, (cuuint64_t)X, (cuuint64_t)C};
-    const cuuint64_t strides[3] = {(cuuint64_t)(Z * es), (cuuint64_t)((uint64_t)Y * Z * es), (cuuint64_t)(N * es)};
+    const cuuint64_t strides[3] = {(cuuint64_t)(Zp * es), (cuuint64_t)((uint64_t)Y * Zp * es), (cuuint64_t)(N * es)};
     const cuuint32_t box[4] = {(cuuint32_t)hz, (cuuint32_t)hy, 1u, (cuuint32_t)C};
     const cuuint32_t estride[4] = {1u, 1u, 1u, 1u};
     const CUresult r = fn(&out->m, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,

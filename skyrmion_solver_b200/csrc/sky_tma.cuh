@@ -110,6 +110,6 @@ __device__ __forceinline__ void tma_prefetch_plane(const TmaMap* map, int z, int
 // Host: encode the plane-box map of a C-component lattice array of element size
 // `esize` (4 or 8) with dimensions (X, Y, Z): box (hz, hy, 1, C).  Returns 0 on
 // success, else a sky_status (invalid argument when an alignment rule fails).
-int encode_plane_map(TmaMap* out, const void* base, int esize, int X, int Y, int Z, int C, int hz, int hy);
+int encode_plane_map(TmaMap* out, const void* base, int esize, int X, int Y, int Z, int Zp, int C, int hz, int hy);
 
 }  // namespace sky

@@ -65,8 +65,13 @@ class Result:
         return self.finished - self.arrival
 
 
+def stored_sites(p_i) -> int:
+    """Values of one component in the engine's arrays: rows of Z padded to a multiple of four."""
+    return int(p_i[0]) * int(p_i[1]) * (-(-int(p_i[2]) // 4) * 4)
+
+
 def instance_bytes(C: int, N: int, precision: str = "fp32") -> int:
-    """Device bytes of one engine instance: 7 state / slope arrays plus per-tile partials and the stats ring."""
+    """Device bytes of one engine instance of N stored sites: 7 state / slope arrays plus per-tile partials and the stats ring."""
     es = 4 if precision == "fp32" else 8
     curls = 72 * N if C > 5 and precision == "fp32" else 0   # rho's energy walks
     return 7 * es * C * N + curls + 8192 * 48 + (N // 256 + 1) * 48
@@ -167,7 +172,7 @@ class Server:
         t = self.now()
         while self.pending and self.pending[0].arrival <= t:
             req = self.pending[0]
-            C, N = int(req.p_i[5]), int(req.p_i[6])
+            C, N = int(req.p_i[5]), stored_sites(req.p_i)
             need = instance_bytes(C, N, "fp64" if self.polish else "fp32")
             if self.live and (self.engine.bytes + need > self.mem_cap or self.free_bytes() - need < self.reserve):
                 break                                   # wait for a retirement to free memory
