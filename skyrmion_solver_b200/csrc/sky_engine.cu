@@ -22,6 +22,16 @@ constexpr int kGraphSteps = 8;  // steps captured per graph replay
 // and a server that admits or retires a request every chunk of 64 steps would do it every chunk.
 constexpr int kDirectSteps = 64;
 
+// A captured run of steps.  Bit k of `refresh`: its step k refreshes defect corrections (it may do so
+// where none is due: the kernels look at each instance).
+struct StepGraph {
+    int nsteps;
+    unsigned refresh;
+    cudaGraphExec_t exec;
+};
+// An engine keeps this many patterns of refreshes; beyond them every captured step has one.
+constexpr size_t kMaxGraphs = 8;
+
 struct Engine {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -30,9 +40,7 @@ struct Engine {
     std::map<int, HostInst> insts;
     int next_id = 0;
     Group groups[kNumKernelSets][2];
-    cudaGraphExec_t graph = nullptr;   // kGraphSteps steps
-    cudaGraphExec_t graph1 = nullptr;  // one step (the remainder of a step call)
-    bool graph_valid = false, graph1_valid = false;
+    std::vector<StepGraph> graphs;     // of the current instance set
     int graph_pdl = -1;                // option 4 when the graphs were captured
     int direct_steps = 0;              // steps launched kernel by kernel since the instance set changed
     int64_t bytes = 0;
@@ -228,10 +236,19 @@ static InstDesc<S> make_desc(const HostInst& h, int tile_begin, int e_tile_begin
     return d;
 }
 
+static void drop_graphs(Engine& e) {
+    for (StepGraph& g : e.graphs) cudaGraphExecDestroy(g.exec);
+    e.graphs.clear();
+}
+
 // Rebuild a group's device descriptor array and tile list.  Device-updated
 // control fields (e_prev, step, arrested, cur) of existing members are kept.
 template <typename S>
 static int rebuild_group_t(Engine& e, Group& g) {
+    int rc0 = check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__);
+    drop_graphs(e);
+    e.direct_steps = 0;
+    if (rc0) return rc0;
     // gather current device state of the members (they may move slots)
     std::vector<InstDesc<S>> dev_old;
     if (g.d_desc && g.desc_cap > 0) {
@@ -307,8 +324,6 @@ static int rebuild_group_t(Engine& e, Group& g) {
                         "write tile list", __LINE__);
         if (rc) return rc;
     }
-    e.graph_valid = e.graph1_valid = false;
-    e.direct_steps = 0;
     return check_cuda(cudaStreamSynchronize(e.stream), "sync", __LINE__);
 }
 
@@ -475,12 +490,13 @@ static int init_instance(Engine& e, HostInst& h, int mode) {
 // each kind is issued for every non-empty group before the next kind.
 enum { kKindS2 = 0, kKindS3, kKindS4, kKindDefect, kKindEnergy, kKindS1, kNumKinds };
 
-static int launch_kind(Engine& e, int kind, cudaStream_t st) {
+// serial: every kind in one stream.
+static int launch_kind(Engine& e, int kind, bool serial, cudaStream_t st) {
     for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr) {
             Group& g = e.groups[t][pr];
             if (g.members.empty()) continue;
-            const int chained = kind == kKindS3 || kind == kKindEnergy || kind == kKindS1;
+            const int chained = serial || kind == kKindS3 || kind == kKindEnergy || kind == kKindS1;
             const StageArgs a{0, g.ntiles, 1, 0, g.rtiles, chained};
             int rc = SKY_OK;
             switch (kind) {
@@ -496,54 +512,79 @@ static int launch_kind(Engine& e, int kind, cudaStream_t st) {
     return SKY_OK;
 }
 
-// Record one step.  Stage 4 runs on a second stream beside the work on the new field, except
-// under programmatic dependent launch, which orders the kernels of one stream.
-static int record_step(Engine& e) {
+// Whether stage 4 runs on a second stream, beside the work on the new field.  It gains where blocks
+// of both fit an SM or the new field's work is more than one kernel: FP32, and rho in FP64 (graph
+// step in us, one stream / two: omega FP32 128^3 323 / 313, nuclear FP32 64^3 84 / 80, rho FP64 64^3
+// 404 / 373).  FP64 stages and the small FP32 rho lattices' fill an SM with one block, and there the
+// programmatic launches of one stream are worth more (omega FP64 64^3 104 / 109, nuclear FP64 96^3
+// 259 / 268, rho FP32 56^3 196 / 204).
+static bool two_streams(const Engine& e) {
+    if (option(4) == 1) return false;
+    for (int t = 0; t < kNumKernelSets; ++t)
+        for (int pr = 0; pr < 2; ++pr)
+            if (!e.groups[t][pr].members.empty() && energy_walk(t, pr)) return true;
+    return false;
+}
+
+// Record one step; refresh: it refreshes the defect corrections that are due.  The refresh replaces the
+// correction that stage 4 reads: it and its stage 1 come after stage 4, and they alone.
+static int record_step(Engine& e, bool refresh) {
     int rc;
-    if ((rc = launch_kind(e, kKindS2, e.stream)) || (rc = launch_kind(e, kKindS3, e.stream))) return rc;
-    const bool fork = option(4) == 0;
+    const bool fork = two_streams(e), serial = !fork;
     cudaStream_t side = fork ? e.side : e.stream;
+    if ((rc = launch_kind(e, kKindS2, serial, e.stream)) || (rc = launch_kind(e, kKindS3, serial, e.stream))) return rc;
     if (fork) {
         if ((rc = check_cuda(cudaEventRecord(e.forked, e.stream), "fork", __LINE__)) ||
             (rc = check_cuda(cudaStreamWaitEvent(side, e.forked, 0), "fork", __LINE__)))
             return rc;
     }
-    bool any_defect = false;
-    for (int t = 0; t < kNumKernelSets; ++t) any_defect = any_defect || e.groups[t][0].any_defect;
     auto join = [&]() -> int {
         if (!fork) return SKY_OK;
         const int r = check_cuda(cudaEventRecord(e.joined, side), "join", __LINE__);
         return r ? r : check_cuda(cudaStreamWaitEvent(e.stream, e.joined, 0), "join", __LINE__);
     };
-    // the refresh replaces the correction that stage 4 reads: it and its stage 1 come after stage 4
-    if ((rc = launch_kind(e, kKindS4, side)) || (rc = launch_kind(e, kKindEnergy, e.stream))) return rc;
-    if (any_defect && ((rc = join()) || (rc = launch_kind(e, kKindDefect, e.stream)))) return rc;
-    if ((rc = launch_kind(e, kKindS1, e.stream))) return rc;
-    return any_defect ? SKY_OK : join();
+    if ((rc = launch_kind(e, kKindS4, serial, side)) || (rc = launch_kind(e, kKindEnergy, serial, e.stream))) return rc;
+    if (refresh && ((rc = join()) || (rc = launch_kind(e, kKindDefect, false, e.stream)))) return rc;
+    if ((rc = launch_kind(e, kKindS1, serial, e.stream))) return rc;
+    return refresh ? SKY_OK : join();
 }
 
+// Bit k: the k-th step from now refreshes an instance's defect correction (refresh_due, whose step
+// count HostInst::steps mirrors).
+static unsigned refresh_pattern(const Engine& e, int nsteps) {
+    unsigned m = 0;
+    for (const auto& kv : e.insts) {
+        const HostInst& h = kv.second;
+        if (!h.active || !h.defect) continue;
+        const int period = h.defect_period > 0 ? h.defect_period : kDefectRefresh;
+        for (int k = 0; k < nsteps; ++k)
+            if ((h.steps + k + 1) % period == 0) m |= 1u << k;
+    }
+    return m;
+}
+static void count_steps(Engine& e, int n) {
+    for (auto& kv : e.insts)
+        if (kv.second.active) kv.second.steps += n;
+}
+
+// Kernels of a step without a defect refresh.
 static int count_launches(Engine& e) {
     int n = 0;
     for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty())
-                // stages 2, 3, 4, 1 (rho: three kernels each), [defect,] [energy] (FP32 rho: two each)
-                n += 4 * (t == SKY_THEORY_RHO ? 3 : 1) + (energy_walk(t, pr) ? (split_energy(t, pr) ? 2 : 1) : 0) +
-                     ((pr == 0 && e.groups[t][pr].any_defect) ? (t == SKY_THEORY_RHO || t == kFusedRho ? 2 : 1) : 0);
+                // stages 2, 3, 4, 1 (rho: three kernels each), [energy] (FP32 rho: two)
+                n += 4 * (t == SKY_THEORY_RHO ? 3 : 1) + (energy_walk(t, pr) ? (split_energy(t, pr) ? 2 : 1) : 0);
     return n;
 }
 
 // Capture `nsteps` steps of the current instance set into *exec.
-static int capture_steps(Engine& e, int nsteps, cudaGraphExec_t* exec) {
-    if (*exec) {
-        cudaGraphExecDestroy(*exec);
-        *exec = nullptr;
-    }
+static int capture_steps(Engine& e, int nsteps, unsigned refresh, cudaGraphExec_t* exec) {
     cudaGraph_t graph;
     int rc = check_cuda(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal), "begin capture",
                         __LINE__);
     if (rc) return rc;
-    for (int s = 0; s < nsteps && rc == SKY_OK; ++s) rc = record_step(e);
+    for (int s = 0; s < nsteps && rc == SKY_OK; ++s) rc = record_step(e, (refresh >> s & 1) != 0);
     cudaError_t ce = cudaStreamEndCapture(e.stream, &graph);
     if (rc) {
         if (ce == cudaSuccess) cudaGraphDestroy(graph);
@@ -556,16 +597,28 @@ static int capture_steps(Engine& e, int nsteps, cudaGraphExec_t* exec) {
 }
 
 // The step graphs: kGraphSteps steps, and one step for the remainder of a call, each captured
-// when a call first wants it.  Each step depends only on device-side state, so replaying them is
-// the same as launching the kernels one by one.
-static int step_graph(Engine& e, int nsteps, cudaGraphExec_t* exec, bool* valid) {
-    if (*valid) return SKY_OK;
+// when a call first wants it, for every pattern of refreshes that comes up (with one period and
+// instances admitted between calls of whole periods: two).  Each step depends only on device-side
+// state, so replaying them is the same as launching the kernels one by one.
+static int step_graph(Engine& e, int nsteps, unsigned refresh, cudaGraphExec_t* exec) {
+    for (;;) {
+        for (const StepGraph& g : e.graphs)
+            if (g.nsteps == nsteps && g.refresh == refresh) {
+                *exec = g.exec;
+                return SKY_OK;
+            }
+        const unsigned every = (1u << nsteps) - 1;
+        if (e.graphs.size() < kMaxGraphs || refresh == every) break;
+        refresh = every;
+    }
     int rc = SKY_OK;
     for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr)
             if (!e.groups[t][pr].members.empty() && (rc = setup_group(e.groups[t][pr]))) return rc;
-    if ((rc = capture_steps(e, nsteps, exec))) return rc;
-    *valid = true;
+    StepGraph g{nsteps, refresh, nullptr};
+    if ((rc = capture_steps(e, nsteps, refresh, &g.exec))) return rc;
+    e.graphs.push_back(g);
+    *exec = g.exec;
     return SKY_OK;
 }
 
@@ -640,8 +693,7 @@ int sky_engine_destroy(void* handle) {
     if (!e) return SKY_OK;
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
-    if (e->graph) cudaGraphExecDestroy(e->graph);
-    if (e->graph1) cudaGraphExecDestroy(e->graph1);
+    drop_graphs(*e);
     for (auto& kv : e->insts) free_inst(kv.second);
     for (int t = 0; t < kNumKernelSets; ++t)
         for (int p = 0; p < 2; ++p) {
@@ -947,25 +999,25 @@ int sky_engine_step(void* handle, int nsteps) {
     int rc;
     int done = 0;
     if (e->graph_pdl != option(4)) {
-        e->graph_valid = e->graph1_valid = false;
+        cudaStreamSynchronize(e->stream);
+        drop_graphs(*e);
         e->graph_pdl = option(4);
     }
-    if (!e->graph_valid && !e->graph1_valid && e->direct_steps + nsteps <= kDirectSteps) {
-        for (; done < nsteps; ++done)
-            if ((rc = record_step(*e))) return rc;
+    if (e->graphs.empty() && e->direct_steps + nsteps <= kDirectSteps) {
+        for (; done < nsteps; ++done) {
+            if ((rc = record_step(*e, refresh_pattern(*e, 1) != 0))) return rc;
+            count_steps(*e, 1);
+        }
         e->direct_steps += nsteps;
     }
-    while (nsteps - done >= kGraphSteps) {
-        if ((rc = step_graph(*e, kGraphSteps, &e->graph, &e->graph_valid))) return rc;
-        if ((rc = check_cuda(cudaGraphLaunch(e->graph, e->stream), "graph launch", __LINE__))) return rc;
-        done += kGraphSteps;
+    while (done < nsteps) {
+        const int n = nsteps - done >= kGraphSteps ? kGraphSteps : 1;
+        cudaGraphExec_t exec;
+        if ((rc = step_graph(*e, n, refresh_pattern(*e, n), &exec))) return rc;
+        if ((rc = check_cuda(cudaGraphLaunch(exec, e->stream), "graph launch", __LINE__))) return rc;
+        count_steps(*e, n);
+        done += n;
     }
-    for (; done < nsteps; ++done) {
-        if ((rc = step_graph(*e, 1, &e->graph1, &e->graph1_valid))) return rc;
-        if ((rc = check_cuda(cudaGraphLaunch(e->graph1, e->stream), "graph launch", __LINE__))) return rc;
-    }
-    for (auto& kv : e->insts)
-        if (kv.second.active) kv.second.steps += nsteps;
     return SKY_OK;
 }
 
@@ -1118,7 +1170,7 @@ int sky_engine_time_stages(void* handle, int nsteps, double* ms_out) {
     for (int s = 0; s < nsteps && rc == SKY_OK; ++s) {
         for (int k = 0; k < kNumKinds && rc == SKY_OK; ++k) {
             cudaEventRecord(ev[k], e->stream);
-            rc = launch_kind(*e, k, e->stream);
+            rc = launch_kind(*e, k, false, e->stream);
         }
         if (rc) break;
         cudaEventRecord(ev[kNumKinds], e->stream);
@@ -1131,8 +1183,7 @@ int sky_engine_time_stages(void* handle, int nsteps, double* ms_out) {
     }
     for (int k = 0; k <= kNumKinds; ++k) cudaEventDestroy(ev[k]);
     if (rc) return rc;
-    for (auto& kv : e->insts)
-        if (kv.second.active) kv.second.steps += nsteps;
+    count_steps(*e, nsteps);
     // report in the order stage 1, 2, 3, 4, control, advance
     // stage 1 with the defect refresh and the FP32 energy walk
     ms_out[0] = (acc[kKindS1] + acc[kKindDefect] + acc[kKindEnergy]) / nsteps;
