@@ -90,7 +90,7 @@ static void tile_geometry(const HostInst& h, int request, int* xc, int* nz, int*
     if (request > 0)
         *xc = request < h.p.X ? request : h.p.X;
     else
-        *xc = choose_chunk(h.p.X, *nz * *ny, resident);
+        *xc = choose_chunk(h.p.X, *nz * *ny, resident, sh.blocks);
     *nx = (h.p.X + *xc - 1) / *xc;
 }
 

@@ -27,7 +27,7 @@ struct StepBuffers {
 };
 int arrested_step(int theory, const Params& p, const StepBuffers& b, double* s_e, double* s_m, double prev_energy,
                   double* new_energy, double* err, cudaStream_t st);
-int choose_chunk(int X, int tiles_yz, int resident);
+int choose_chunk(int X, int tiles_yz, int resident, int per_sm = 1);
 int gradient_fp64(int theory, const Params& p, const double* f, double* eg, double* l, cudaStream_t st);
 int density_fp64(int theory, const Params& p, int mode, const double* f, double* dens, double* scratch,
                  double* out_dev, cudaStream_t st);
