@@ -490,12 +490,13 @@ static int init_instance(Engine& e, HostInst& h, int mode) {
 // each kind is issued for every non-empty group before the next kind.
 enum { kKindS2 = 0, kKindS3, kKindS4, kKindDefect, kKindEnergy, kKindS1, kNumKinds };
 
-// serial: every kind in one stream.
-static int launch_kind(Engine& e, int kind, bool serial, cudaStream_t st) {
+// serial: every kind in one stream.  late: 1 the groups with a late update only, 0 the others only,
+// -1 all.
+static int launch_kind(Engine& e, int kind, bool serial, cudaStream_t st, int late = -1) {
     for (int t = 0; t < kNumKernelSets; ++t)
         for (int pr = 0; pr < 2; ++pr) {
             Group& g = e.groups[t][pr];
-            if (g.members.empty()) continue;
+            if (g.members.empty() || (late >= 0 && late != int(late_update(t, pr)))) continue;
             const int chained = serial || kind == kKindS3 || kind == kKindEnergy || kind == kKindS1;
             const StageArgs a{0, g.ntiles, 1, 0, g.rtiles, chained};
             int rc = SKY_OK;
@@ -543,7 +544,10 @@ static int record_step(Engine& e, bool refresh) {
         const int r = check_cuda(cudaEventRecord(e.joined, side), "join", __LINE__);
         return r ? r : check_cuda(cudaStreamWaitEvent(e.stream, e.joined, 0), "join", __LINE__);
     };
-    if ((rc = launch_kind(e, kKindS4, serial, side)) || (rc = launch_kind(e, kKindEnergy, serial, e.stream))) return rc;
+    // a late update's stage 4 comes before its stage 1
+    if ((rc = launch_kind(e, kKindS4, serial, side, 0)) || (rc = launch_kind(e, kKindS4, serial, e.stream, 1)) ||
+        (rc = launch_kind(e, kKindEnergy, serial, e.stream)))
+        return rc;
     if (refresh && ((rc = join()) || (rc = launch_kind(e, kKindDefect, false, e.stream)))) return rc;
     if ((rc = launch_kind(e, kKindS1, serial, e.stream))) return rc;
     return refresh ? SKY_OK : join();

@@ -12,16 +12,22 @@
 // fly from F, V and the previous slope.
 //
 // F' needs no l4.  So stage 3 already writes the new field, into the other half of a
-// ping-pong pair, and P = V + (l1 + 2 l2 + 2 l3)/6 instead of l3; stage 4 adds l4 / 6,
-// projects and leaves V'.  The work on the new field -- its energy and the next step's l1
-// (stage 1) -- then depends on stage 3 only and runs beside stage 4:
+// ping-pong pair, and the sum l1 + 2 l2 + 2 l3 instead of l3; stage 4 adds l4, projects and leaves
+// V'.  The work on the new field -- its energy and the next step's l1 (stage 1) -- then depends on
+// stage 3 only and runs beside stage 4:
 //   stage 2 -> stage 3 -> { stage 4 | [defect refresh,] [FP32 energy,] stage 1 } -> control.
-// The last block of the two branches to finish runs every instance's control: it reduces the
+// l1 alternates between two buffers, since stage 4 of an arrested step reads the old one (l2 = l1)
+// while stage 1 writes the new one.
+//
+// Where one block fills an SM (FP64 stages of at most five components, the fused FP32 rho kernels)
+// nothing runs beside stage 4, and the split update's array more would only cost: there stage 3
+// writes l3 and stage 4 updates field and velocity (late_update); stage 1 follows it.
+//
+// The last block of stages 4 and 1 to finish runs every instance's control: it reduces the
 // energy, baryon number and stage-4 gradient (compensated, fixed order), records the step's
 // (energy, err) exactly as do_arrested_newton_flow returns them, takes the arrest decision for
 // the next step (the velocity is treated as zero when killkinen is set and the energy rose,
-// core/integrator.py:403-407) and flips the halves.  l1 alternates between two buffers, since
-// stage 4 of an arrested step reads the old one (l2 = l1) while stage 1 writes the new one.
+// core/integrator.py:403-407) and flips the halves.
 #pragma once
 
 #include <string.h>
@@ -68,6 +74,12 @@ constexpr bool energy_walk(int set) {
     return set != kFusedRho && (sizeof(T) == 4 || set == SKY_THEORY_RHO);
 }
 
+// Whether stage 4 updates the field (else stage 3 does).
+template <typename T>
+constexpr bool late_update(int set) {
+    return set == kFusedRho || (sizeof(T) == 8 && set != SKY_THEORY_RHO);
+}
+
 // Device-resident state of one instance.
 template <typename S>
 struct InstDesc {
@@ -83,9 +95,10 @@ struct InstDesc {
     S* F[2];           // ping-pong field
     S* Flo[2];         // ping-pong low parts of a compensated FP32 field (null otherwise)
     S* Dlt;            // defect correction g64 - g32 of a defect-corrected FP32 instance (null otherwise)
-    S* V[2];           // ping-pong velocity (the next half holds P between stages 3 and 4)
+    S* V[2];           // ping-pong velocity (the next half holds l1 + 2 l2 + 2 l3 between stages 3 and 4)
     double* curl;      // FP32 rho: R^a_xy, R^a_xz, R^a_yz (at 3 a) of the field whose energy is being summed
-    S* L[3];           // slopes: l1 of this step and of the next in L[0] and L[2] (see cur_l1), l2 in L[1]
+    S* L[3];           // slopes: l2 in L[1]; l1 of this step and of the next in L[0] and L[2] (l1_slot), or with
+                       // a late update l1 in L[0] and l3 in L[2]
     KSum* epart;       // energy partials, per energy tile (k_energy; FP32 rho: four each) or per stage tile (stage 1)
     KSum* bpart;       // per-tile baryon partials (stage 1)
     double* gpart;     // per-tile [signed max, abs max of stage-4 g, kinetic KSum (s, c)] (4 doubles / tile)
@@ -111,20 +124,19 @@ struct InstDesc {
 };
 
 // The field's update at one site: F' = F + dt (V + (l1 + l2 + l3)/6), then the theory's
-// normalisation of the first nsky components; and P = V + (l1 + 2 l2 + 2 l3)/6.
+// normalisation of the first nsky components; and sum = l1 + 2 l2 + 2 l3.
 // With a compensated field (comp) F is the unevaluated sum hi + lo of two FP32
 // values: the update and the normalisation run in FP64 and the result is
 // split back into hi + lo, so increments far below one FP32 ulp of F still accumulate.
 template <typename T, int C>
 __device__ __forceinline__ void update_field(const T (&f0)[C], const T (&flo)[C], bool comp, const T (&v0)[C],
                                              const T (&l1)[C], const T (&l2)[C], const T (&l3)[C], T dtt, int nsky,
-                                             int unit_length, T (&fo)[C], T (&lo)[C], T (&pv)[C]) {
+                                             int unit_length, T (&fo)[C], T (&lo)[C], T (&sum)[C]) {
     T inc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        const T b = l2[c] + l3[c], a = l1[c] + b;
-        pv[c] = v0[c] + (a + b) * T(1.0 / 6.0);
-        inc[c] = dtt * (v0[c] + a * T(1.0 / 6.0));
+        sum[c] = l1[c] + T(2) * l2[c] + T(2) * l3[c];
+        inc[c] = dtt * (v0[c] + (l1[c] + l2[c] + l3[c]) * T(1.0 / 6.0));
         lo[c] = T(0);
     }
     if (!comp) {
@@ -172,14 +184,15 @@ __device__ __forceinline__ void update_field(const T (&f0)[C], const T (&flo)[C]
     }
 }
 
-// The velocity's update: V' = P + l4 / 6, projected orthogonal to the first nsky components of
-// the new field (a compensated field's high parts); returns |V'|^2.
+// The velocity's update: V' = V + (l1 + 2 l2 + 2 l3 + l4)/6 -- the small terms are summed before
+// the velocity, which is rounded once (kept as V + (l1 + 2 l2 + 2 l3)/6 between the stages it was
+// rounded twice: up to one ulp from the exact sum instead of half of one) -- projected orthogonal to
+// the first nsky components of the new field (a compensated field's high parts); returns |V'|^2.
 template <typename T, int C>
-__device__ __forceinline__ T update_velocity(const T (&pv)[C], const T (&g)[C], const T (&fo)[C], T dtt, int nsky,
-                                             int unit_length, T (&vv)[C]) {
-    const T w = -dtt * T(1.0 / 6.0);
+__device__ __forceinline__ T update_velocity(const T (&v0)[C], const T (&sum)[C], const T (&g)[C], const T (&fo)[C],
+                                             T dtt, int nsky, int unit_length, T (&vv)[C]) {
 #pragma unroll
-    for (int c = 0; c < C; ++c) vv[c] = pv[c] + w * g[c];
+    for (int c = 0; c < C; ++c) vv[c] = v0[c] + (sum[c] + -dtt * g[c]) * T(1.0 / 6.0);
     if (unit_length) {
         T lm = T(0);
 #pragma unroll
@@ -202,9 +215,9 @@ __device__ __forceinline__ bool refresh_due(const InstDesc<S>& in) {
     return in.Dlt != nullptr && (in.step + 1) % period == 0;
 }
 // The buffer of the current step's l1 (half 0) or of the next one's (half 1).
-template <typename S>
+template <bool LATE, typename S>
 __device__ __forceinline__ int l1_slot(const InstDesc<S>& in, int half) {
-    return (in.cur ^ half) ? 2 : 0;
+    return !LATE && (in.cur ^ half) ? 2 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -333,8 +346,10 @@ template <typename T>
 struct StageIo {
     const T* src[3];   // sources of the stage input
     T a, b;            // their weights
-    const T *F, *Flo, *V, *l1, *l2;  // stage 3: the update's operands (V null: zero; Flo null: not compensated)
-    // stages 1, 2: l_s.  Stage 3: F', its low parts and P.  Stage 4: F' (read) and P -> V'.
+    const T *F, *Flo, *V, *l1, *l2;  // the update's operands (V null: zero; Flo null: not compensated)
+    T* l3;                           // late update
+    // stages 1, 2: l_s.  Stage 3: F', its low parts and the slopes' sum.  Stage 4: F' (read) and the
+    // sum, which V' replaces.  Late update: stage 3 l3, stage 4 F', its low parts and V'.
     T *out, *out_lo, *pv;
     T* R;  // rho: where the stage's walk over the rho components leaves R (components 4 .. 12)
     T dtt;
@@ -351,7 +366,7 @@ __device__ __forceinline__ bool l2_is_l1(const InstDesc<T>& in) {
     return in.arrested && !in.refresh;
 }
 
-template <typename T, int STAGE>
+template <bool LATE, typename T, int STAGE>
 __device__ __forceinline__ StageIo<T> stage_io(const InstDesc<T>& in, const Params& p, int half) {
     const int cur = STAGE == 1 ? in.cur ^ half : in.cur;
     StageIo<T> io;
@@ -359,7 +374,8 @@ __device__ __forceinline__ StageIo<T> stage_io(const InstDesc<T>& in, const Para
     io.F = in.F[cur];
     io.Flo = in.Flo[cur];
     io.V = in.arrested ? nullptr : in.V[cur];
-    io.l1 = in.L[l1_slot(in, 0)];
+    io.l1 = in.L[l1_slot<LATE>(in, 0)];
+    io.l3 = in.L[2];
     io.l2 = io.l2_is_l1 ? io.l1 : in.L[1];  // the step's l2
     io.dtt = T(p.dt);
     const T hdt = T(0.5 * p.dt);
@@ -368,23 +384,23 @@ __device__ __forceinline__ StageIo<T> stage_io(const InstDesc<T>& in, const Para
     io.src[2] = STAGE == 3 ? io.l1 : io.l2;
     io.a = STAGE == 4 ? io.dtt : hdt;
     io.b = STAGE == 3 ? T(0.25) * io.dtt : T(0.5) * io.dtt;
-    io.out = STAGE == 1 ? in.L[l1_slot(in, half)] : STAGE == 2 ? in.L[1] : in.F[cur ^ 1];
+    io.out = STAGE == 1 ? in.L[l1_slot<LATE>(in, half)] : STAGE == 2 ? in.L[1] : LATE && STAGE == 3 ? io.l3 : in.F[cur ^ 1];
     io.out_lo = in.Flo[cur ^ 1];
     io.pv = in.V[cur ^ 1];
     // R lies where the stage's output will (stage 4: in the slope that it does not read)
-    io.R = STAGE < 3 ? io.out : STAGE == 3 ? io.pv : io.l2_is_l1 ? in.L[1] : in.L[l1_slot(in, 0)];
+    io.R = STAGE < 3 ? io.out : STAGE == 3 ? io.pv : io.l2_is_l1 ? in.L[1] : in.L[l1_slot<LATE>(in, 0)];
     return io;
 }
 
 // The maps of a tile's sources (null: the source reads as zero); tm: the instance's maps of the
 // walk's components.
-template <typename T, int STAGE>
+template <bool LATE, typename T, int STAGE>
 __device__ __forceinline__ void stage_maps(const InstDesc<T>& in, const TmaMap* tm, const StageIo<T>& io, int half,
                                            TmaTile& tt) {
     const int cur = STAGE == 1 ? in.cur ^ half : in.cur;
     tt.map[0] = &tm[kMapF + cur];
     tt.map[1] = io.V != nullptr ? &tm[kMapV + cur] : nullptr;
-    tt.map[2] = STAGE > 2 ? &tm[kMapL + (STAGE == 3 || io.l2_is_l1 ? l1_slot(in, 0) : 1)] : nullptr;
+    tt.map[2] = STAGE > 2 ? &tm[kMapL + (STAGE == 3 || io.l2_is_l1 ? l1_slot<LATE>(in, 0) : 1)] : nullptr;
     tt.status = in.status;
 }
 
@@ -442,10 +458,13 @@ __device__ __forceinline__ float2 ld_early2(const float* p) {
 // Epilogue of the gradient walk's stages: a thread's pair of FP32 sites, or its FP64 site, at
 // once.  The row pitch is a multiple of four, so a pair is one aligned 8-byte access; where Z is
 // odd, the second lane of a row's last pair is padding, which nothing reads as a site.
-// EARLY: stage 3's operands are loaded before the point arithmetic (where 168 registers hold
-// both: without mixed derivatives); stage 4's two always are.
-template <typename T, int STAGE, int C, bool TMA, bool EARLY>
+// EARLY: the field update's operands are loaded before the point arithmetic (where 168 registers
+// hold both: without mixed derivatives); of a stage 4 that updates the velocity only, F' and the
+// slopes' sum always are, and the velocity, which the staged planes have brought into L2, is not.
+template <typename T, int STAGE, int C, bool TMA, bool EARLY, bool LATE>
 struct GradEpi {
+    static constexpr bool UPDATE = STAGE == (LATE ? 4 : 3);  // the stage that updates the field
+    static constexpr int NOP = UPDATE ? 5 : STAGE == 4 ? 3 : 1;
     using L = Lanes<T>;
     using V = typename L::V;
     static constexpr int NL = L::NL;
@@ -457,7 +476,7 @@ struct GradEpi {
     const T* ahead[4];  // operands that the stage reads at the site only (null: none), and their maps
     const TmaMap* ahead_map[4];
     V d[NL > 1 ? C : 1];  // the correction of the site's pair
-    V op[STAGE == 3 ? 5 : STAGE == 4 ? 2 : 1][STAGE > 2 ? C : 1];  // the update's operands at the site
+    V op[NOP][NOP > 1 ? C : 1];  // the update's operands at the site
 
     template <bool ONCE = true>
     static __device__ __forceinline__ V get(const T* p) {
@@ -508,21 +527,20 @@ struct GradEpi {
         return uint32_t(c) * uint32_t(N) + uint32_t(s);
     }
     __device__ __forceinline__ void load(int64_t s, int64_t N, bool) {
-        if constexpr (EARLY || STAGE == 4) operands(s, N);
+        if constexpr (EARLY || (STAGE == 4 && !UPDATE)) operands(s, N);
     }
     __device__ __forceinline__ void operands(int64_t s, int64_t N) {
-        if constexpr (STAGE == 3) {
+        if constexpr (UPDATE) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const uint32_t j = at(c, N, s);
                 op[0][c] = get(io.F + j);
-                op[1][c] = io.Flo ? get(io.Flo + j) : V(0.0f);
+                op[1][c] = LATE ? get(io.l3 + j) : io.Flo ? get(io.Flo + j) : V(0.0f);
                 op[2][c] = io.V ? get(io.V + j) : V(0.0f);
                 op[3][c] = get(io.l1 + j);
                 op[4][c] = io.l2_is_l1 ? op[3][c] : get(io.l2 + j);
             }
-        }
-        if constexpr (STAGE == 4) {
+        } else if constexpr (STAGE == 4) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 op[0][c] = get(io.out + at(c, N, s));
@@ -548,28 +566,28 @@ struct GradEpi {
                 }
             }
         }
-        if constexpr (STAGE < 3) {
+        if constexpr (STAGE < 3 || (LATE && STAGE == 3)) {
 #pragma unroll
             for (int c = 0; c < C; ++c) store(io.out + at(c, N, s), V(-io.dtt) * g[c]);
         } else if constexpr (STAGE == 3) {
             if constexpr (!EARLY) operands(s, N);
-            V fo[C], lo[C], pv[C];
+            V fo[C], lo[C], sum[C];
 #pragma unroll
             for (int c = 0; c < C; ++c) g[c] = V(-io.dtt) * g[c];  // l3
 #pragma unroll
             for (int l = 0; l < NL; ++l) {
-                T F[C], Fl[C], v[C], b1[C], b2[C], b3[C], of[C], ol[C], pn[C];
+                T F[C], Fl[C], v[C], b1[C], b2[C], b3[C], of[C], ol[C], sn[C];
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
                     F[c] = L::get(op[0][c], l), Fl[c] = L::get(op[1][c], l), v[c] = L::get(op[2][c], l);
                     b1[c] = L::get(op[3][c], l), b2[c] = L::get(op[4][c], l), b3[c] = L::get(g[c], l);
                 }
-                update_field<T, C>(F, Fl, io.Flo != nullptr, v, b1, b2, b3, io.dtt, nsky, unit_length, of, ol, pn);
+                update_field<T, C>(F, Fl, io.Flo != nullptr, v, b1, b2, b3, io.dtt, nsky, unit_length, of, ol, sn);
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
                     L::set(fo[c], l, of[c]);
                     L::set(lo[c], l, ol[c]);
-                    L::set(pv[c], l, pn[c]);
+                    L::set(sum[c], l, sn[c]);
                 }
             }
 #pragma unroll
@@ -577,25 +595,43 @@ struct GradEpi {
                 const uint32_t j = at(c, N, s);
                 store(io.out + j, fo[c]);
                 if (io.Flo) store(io.out_lo + j, lo[c]);
-                store(io.pv + j, pv[c]);
+                store(io.pv + j, sum[c]);
+            }
+        } else if constexpr (LATE) {
+            static_assert(NL == 1, "FP64 sites");
+            if constexpr (!EARLY) operands(s, N);
+            T zero[C], of[C], ol[C], sum[C], ov[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                zero[c] = T(0);
+                st.gradient(g[c]);
+            }
+            update_field<T, C>(op[0], zero, false, op[2], op[3], op[4], op[1], io.dtt, nsky, unit_length, of, ol, sum);
+            st.velocity(update_velocity<T, C>(op[2], sum, g, of, io.dtt, nsky, unit_length, ov));
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                store(io.out + at(c, N, s), of[c]);
+                store(io.pv + at(c, N, s), ov[c]);
             }
         } else {
-            V (&fo)[C] = op[0], (&pv)[C] = op[1];
+            V (&fo)[C] = op[0], (&sum)[C] = op[1], (&v0)[C] = op[2];
+#pragma unroll
+            for (int c = 0; c < C; ++c) v0[c] = io.V ? get(io.V + at(c, N, s)) : V(0.0f);
 #pragma unroll
             for (int l = 0; l < NL; ++l) {
                 if (l == 1 && !own1) break;
-                T F[C], v[C], gg[C], ov[C];
+                T F[C], v[C], sm[C], gg[C], ov[C];
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
-                    F[c] = L::get(fo[c], l), v[c] = L::get(pv[c], l), gg[c] = L::get(g[c], l);
+                    F[c] = L::get(fo[c], l), v[c] = L::get(v0[c], l), sm[c] = L::get(sum[c], l), gg[c] = L::get(g[c], l);
                     st.gradient(gg[c]);
                 }
-                st.velocity(update_velocity<T, C>(v, gg, F, io.dtt, nsky, unit_length, ov));
+                st.velocity(update_velocity<T, C>(v, sm, gg, F, io.dtt, nsky, unit_length, ov));
 #pragma unroll
-                for (int c = 0; c < C; ++c) L::set(pv[c], l, ov[c]);
+                for (int c = 0; c < C; ++c) L::set(sum[c], l, ov[c]);
             }
 #pragma unroll
-            for (int c = 0; c < C; ++c) store(io.pv + at(c, N, s), pv[c]);
+            for (int c = 0; c < C; ++c) store(io.pv + at(c, N, s), sum[c]);
         }
     }
 };
@@ -603,8 +639,8 @@ struct GradEpi {
 // Rho: the walk over the pion components takes R at the site and leaves H in its place
 // (k_rho_finish applies it).
 template <typename T, int STAGE, bool TMA>
-struct RhoGradEpi : GradEpi<T, STAGE, 4, TMA, false> {
-    using B = GradEpi<T, STAGE, 4, TMA, false>;
+struct RhoGradEpi : GradEpi<T, STAGE, 4, TMA, false, false> {
+    using B = GradEpi<T, STAGE, 4, TMA, false, false>;
     using V = typename Lanes<T>::V;
     static constexpr bool kCoupled = true;
     __device__ __forceinline__ void coupling(int64_t s, int64_t N, bool, V (&R)[9]) {
@@ -620,7 +656,7 @@ struct RhoGradEpi : GradEpi<T, STAGE, 4, TMA, false> {
 };
 template <template <typename> class Th, typename T, int STAGE, class M, bool TMA>
 using StageEpi = typename std::conditional<Th<T>::kId == SKY_THEORY_RHO, RhoGradEpi<T, STAGE, TMA>,
-                                           GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed>>::type;
+                                           GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed, late_update<T>(Th<T>::kId)>>::type;
 
 // A finished tile's partials: stage 1 the baryon number and (FP64) the energy, stage 4 the
 // gradient maxima and the kinetic sum.
@@ -725,8 +761,9 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
         int xa, xe, y0, z0;
         march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
         using Epi = StageEpi<Th, T, STAGE, M, TMA>;
-        Epi epi{GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed>{
-            stage_io<T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
+        constexpr bool LATE = late_update<T>(Th<T>::kId);
+        Epi epi{GradEpi<T, STAGE, M::C, TMA, !Th<T>::kMixed, LATE>{
+            stage_io<LATE, T, STAGE>(in, p, half), StageStats<T>(p.vol), p.nsky, p.unit_length, in.Dlt,
             STAGE == 1 && half && refresh_due(in), {nullptr, nullptr, nullptr, nullptr},
             {nullptr, nullptr, nullptr, nullptr}}};
         epi.z0 = z0;
@@ -736,16 +773,19 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
             epi.ahead[k] = a;
             epi.ahead_map[k] = a != nullptr ? &in.tm[map] : nullptr;
         };
-        if constexpr (STAGE == 3) {
+        if constexpr (LATE && STAGE == 4) {
+            ahead(0, epi.io.l3, kMapL + 2);
+            ahead(1, epi.io.l2_is_l1 ? nullptr : epi.io.l1, kMapL);
+        } else if constexpr (STAGE == 3 && !LATE) {
             ahead(0, epi.io.Flo, kMapFlo + in.cur);
             ahead(1, epi.io.l2_is_l1 ? nullptr : epi.io.l2, kMapL + 1);
         }
-        if constexpr (STAGE == 4) {
+        if constexpr (STAGE == 4 && !LATE) {
             ahead(0, epi.io.out, kMapF + (in.cur ^ 1));
             ahead(1, epi.io.pv, kMapV + (in.cur ^ 1));
         }
         ahead(3, in.Dlt, kMapDlt);
-        if constexpr (TMA) stage_maps<T, STAGE>(in, in.tm, epi.io, half, tt);
+        if constexpr (TMA) stage_maps<LATE, T, STAGE>(in, in.tm, epi.io, half, tt);
         __syncthreads();  // the previous tile's readers of coef are done
         if (first) coef = in.coef;
         __syncthreads();
@@ -793,11 +833,11 @@ __global__ void __launch_bounds__(GradBlock<M, T>::NT, MINB)
         const Params p = in.p;
         int xa, xe, y0, z0;
         march_origin(in.r_grid, t - in.r_tile_begin, M::BY, xa, xe, y0, z0, p.X);
-        const StageIo<T> io = stage_io<T, STAGE>(in, p, half);
+        const StageIo<T> io = stage_io<false, T, STAGE>(in, p, half);
         const int64_t N = n_sites(p), c0 = (4 + a) * N;
         const T* const src[3] = {io.src[0] + c0, io.src[1] ? io.src[1] + c0 : nullptr, io.src[2] + c0};
         if constexpr (TMA) {
-            stage_maps<T, STAGE>(in, in.tmr, io, half, tt);
+            stage_maps<false, T, STAGE>(in, in.tmr, io, half, tt);
             tt.x0 = a * p.X;
         }
         __syncthreads();  // the previous tile's readers of coef are done
@@ -851,7 +891,7 @@ __global__ void __launch_bounds__(kRhoFinishThreads)
         if (STAGE == 2 && l2_is_l1(in)) continue;
         const Params p = in.p;
         const int lt = u - K * in.r_tile_begin, items = K * in.r_grid.count();
-        const StageIo<T> io = stage_io<T, STAGE>(in, p, half);
+        const StageIo<T> io = stage_io<false, T, STAGE>(in, p, half);
         const bool refresh = STAGE == 1 && half && refresh_due(in);
         T* const dlt = in.Dlt;
         StageStats<T> st(p.vol);
@@ -896,9 +936,9 @@ __global__ void __launch_bounds__(kRhoFinishThreads)
                     update_field<T, 1>(F, Fl, io.Flo != nullptr, V0, b1, b2, b3, io.dtt, 0, 0, of, ol, op);
                     o1.v[i] = of[0], o2.v[i] = ol[0], o3.v[i] = op[0];
                 } else {
-                    const T q1[1] = {pv.v[i]}, gg[1] = {g};
+                    const T V0[1] = {vi}, sum[1] = {pv.v[i]}, gg[1] = {g};
                     T o[1];
-                    const T v2 = update_velocity<T, 1>(q1, gg, q1, io.dtt, 0, 0, o);
+                    const T v2 = update_velocity<T, 1>(V0, sum, gg, V0, io.dtt, 0, 0, o);
                     if (i < n) {
                         st.gradient(g);
                         st.velocity(v2);
@@ -952,40 +992,31 @@ struct RhoFusedEpi {
                 }
             }
         }
-        if constexpr (STAGE < 3) {
+        if constexpr (STAGE < 4) {
 #pragma unroll
             for (int c = 0; c < C; ++c) __stcg(io.out + c * N + s, -io.dtt * g[c]);
-        } else if constexpr (STAGE == 3) {
-            float f0[C], fl[C], v0[C], a1[C], a2[C], fo[C], lo[C], pv[C];
+        } else {
+            float f0[C], fl[C], v0[C], a1[C], a2[C], a3[C], fo[C], lo[C], sum[C], vv[C];
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const int64_t j = c * N + s;
+                st.gradient(g[c]);
                 f0[c] = __ldcg(io.F + j);
                 fl[c] = io.Flo ? __ldcg(io.Flo + j) : 0.0f;
                 v0[c] = io.V ? __ldcg(io.V + j) : 0.0f;
                 a1[c] = __ldcg(io.l1 + j);
                 a2[c] = io.l2_is_l1 ? a1[c] : __ldcg(io.l2 + j);
-                g[c] = -io.dtt * g[c];  // l3
+                a3[c] = __ldcg(io.l3 + j);
             }
-            update_field<float, C>(f0, fl, io.Flo != nullptr, v0, a1, a2, g, io.dtt, nsky, unit_length, fo, lo, pv);
+            update_field<float, C>(f0, fl, io.Flo != nullptr, v0, a1, a2, a3, io.dtt, nsky, unit_length, fo, lo, sum);
+            st.velocity(update_velocity<float, C>(v0, sum, g, fo, io.dtt, nsky, unit_length, vv));
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const int64_t j = c * N + s;
                 __stcg(io.out + j, fo[c]);
                 if (io.Flo) __stcg(io.out_lo + j, lo[c]);
-                __stcg(io.pv + j, pv[c]);
+                __stcg(io.pv + j, vv[c]);
             }
-        } else {
-            float fo[C], pv[C], vv[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                st.gradient(g[c]);
-                fo[c] = __ldcg(io.out + c * N + s);
-                pv[c] = __ldcg(io.pv + c * N + s);
-            }
-            st.velocity(update_velocity<float, C>(pv, g, fo, io.dtt, nsky, unit_length, vv));
-#pragma unroll
-            for (int c = 0; c < C; ++c) __stcg(io.pv + c * N + s, vv[c]);
         }
     }
 };
@@ -1014,9 +1045,9 @@ __global__ void __launch_bounds__(M::NTHREADS)
         const MarchGrid mg{in.tiles_nz, in.tiles_ny, in.tiles_nx, in.xc};
         int xa, xe, y0, z0;
         march_origin(mg, lt, M::BY, xa, xe, y0, z0, p.X);
-        RhoFusedEpi<STAGE> epi{stage_io<float, STAGE>(in, p, half), StageStats<float>(p.vol), p.nsky, p.unit_length,
+        RhoFusedEpi<STAGE> epi{stage_io<true, float, STAGE>(in, p, half), StageStats<float>(p.vol), p.nsky, p.unit_length,
                                in.Dlt, STAGE == 1 && half && refresh_due(in)};
-        if constexpr (TMA) stage_maps<float, STAGE>(in, in.tm, epi.io, half, tt);
+        if constexpr (TMA) stage_maps<true, float, STAGE>(in, in.tm, epi.io, half, tt);
         KSum es{0.0, 0.0}, bs{0.0, 0.0};
         const bool ok = rho_march_tile<M, stage_nsrc<STAGE>(), STAGE == 1, TMA>(
             sm, p, epi.io.src, epi.io.a, epi.io.b, xa, xe, y0, z0, epi, es, bs, TMA ? &tt : nullptr);

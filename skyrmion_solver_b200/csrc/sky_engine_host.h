@@ -94,6 +94,7 @@ inline int energy_partials(int set, int prec, int entiles) { return split_energy
 inline int grad_partials(int set, int ntiles, int rtiles) {
     return ntiles + (set == SKY_THEORY_RHO ? kRhoFinishSplit * rtiles : 0);
 }
+inline bool late_update(int set, int prec) { return prec ? late_update<double>(set) : late_update<float>(set); }
 inline bool energy_walk(int set, int prec) { return prec ? energy_walk<double>(set) : energy_walk<float>(set); }
 
 }  // namespace sky

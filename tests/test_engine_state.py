@@ -77,3 +77,29 @@ def test_rows_are_padded_to_sixteen_byte_chunks(precision, z):
         f, v = eng.read(i)
         assert np.max(np.abs(f - F)) <= (0.0 if precision == "fp64" else 2.0 ** -24 * np.max(np.abs(F)))
         assert not np.any(v)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp32c"])
+@pytest.mark.parametrize("name,dims", [("nuclear", (9, 17, 36)), ("omega", (9, 13, 33)), ("coulomb", (9, 13, 34)),
+                                       ("rho", (9, 13, 36)), ("rho", (57, 57, 57))])
+def test_velocity_is_rounded_once(name, precision, dims):
+    """V' = V + (l1 + 2 l2 + 2 l3 + l4)/6 with an FP32 velocity near one and increments far below it:
+    the increment is summed first, so V' is the exact sum rounded once, at most half a unit in the
+    last place of values in [0.5, 1] (2^-25) away.  To that comes the increment's own FP32 error, at
+    most the 2e-5 of its maximum that the engine's FP32 gradients are held to, and the units in which
+    an increment is summed (four roundings of 2^-24 of it).  No projection (unit_length = 0)."""
+    from skyrmion_solver_b200.engine import Engine
+    _, p_i, p_f = params_for(name, dims)
+    p_i, p_f = p_i.copy(), p_f.copy()
+    p_i[8] = p_i[10] = 0
+    p_f[7] = 1e-8
+    F, V = inputs(int(p_i[5]), dims, seed=6)
+    V = np.random.default_rng(8).uniform(0.5, 1.0 - 1e-3, size=F.shape).astype(np.float32).astype(np.float64)
+    _, Vo, _, _, _ = O.arrested_newton_step(O.THEORIES[name], F, V, p_i, p_f, 0.0)
+    inc = float(np.max(np.abs(Vo - V)))
+    assert 2.0 ** -24 < inc < 1e-3
+    with Engine(0) as eng:
+        i = eng.add(name, (p_i, p_f), F, V, precision=precision)
+        eng.step(1)
+        _, v = eng.read(i)
+    assert float(np.max(np.abs(v - Vo))) <= 2.0 ** -25 + (2e-5 + 2.0 ** -22) * inc
