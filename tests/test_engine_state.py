@@ -79,6 +79,24 @@ def test_rows_are_padded_to_sixteen_byte_chunks(precision, z):
         assert not np.any(v)
 
 
+@pytest.mark.parametrize("dims", [(56, 56, 56), (57, 57, 57), (49, 61, 60), (13, 25, 37)])
+@pytest.mark.parametrize("precision", ["fp32", "fp32d"])
+def test_rho_state_with_a_refresh_in_every_step(precision, dims):
+    """The largest lattice of the fused FP32 rho kernels and the smallest of the separate walks (odd
+    rows and whole chunks) over three steps; defect-corrected, the correction is refreshed in each of
+    them, so that the refresh kernels, the stage 1 that follows them and stages with a correction
+    that is not zero all run."""
+    run_against_oracle("rho", dims, precision, steps=3, period=1 if precision == "fp32d" else None)
+
+
+@pytest.mark.parametrize("dims", [(6, 16, 32), (5, 17, 33), (9, 11, 31), (7, 13, 62), (8, 33, 34)])
+@pytest.mark.parametrize("name", ["nuclear", "omega", "coulomb", "berger", "lightly_bound"])
+def test_state_with_refreshes_at_tile_edges(name, dims):
+    """Defect-corrected FP32 with a refresh in every second step, at the edges of the 12- and 16-row,
+    32-column tiles."""
+    run_against_oracle(name, dims, "fp32d", steps=3, period=2)
+
+
 @pytest.mark.parametrize("precision", ["fp32", "fp32c"])
 @pytest.mark.parametrize("name,dims", [("nuclear", (9, 17, 36)), ("omega", (9, 13, 33)), ("coulomb", (9, 13, 34)),
                                        ("rho", (9, 13, 36)), ("rho", (57, 57, 57))])
