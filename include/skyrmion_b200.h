@@ -52,11 +52,14 @@ const char* sky_last_error(void);
 
 /* Library-wide tuning options.  Key 0: kernel family of the reference-layout
  * gradient and densities (sky_gradient_step / sky_arrested_newton_step): 1 =
- * marching x-plane kernels (default), 0 = 3-D tile kernels.  Key 1: x-chunk of those marching launches (0 = automatic).  Key 2:
+ * marching x-plane kernels (default), 0 = 3-D tile kernels.  Key 1: x-chunk of the
+ * marching gradients, alone and in the step's stages (0 = automatic); the densities
+ * choose theirs.  Key 2:
  * staging of the resident engine's stage kernels, 1 = tensor-memory-accelerator
- * box copies (default; lattices whose Z gives 16-byte row pitches), 0 = per-thread
- * cp.async copies; it applies to instances admitted afterwards
- * (sky_engine_set_staging changes one instance).
+ * box copies (default), 0 = per-thread cp.async copies; it applies to instances
+ * admitted afterwards (sky_engine_set_staging changes one instance whose Z gives
+ * 16-byte row pitches; the rows of the others are padded in the engine's arrays,
+ * and their staging is the library's).
  * Key 3: 0 or 1, recorded as the z-pair flag of FP32 omega instances at admission.
  * It selects nothing: every FP32 gradient walk computes two adjacent z-sites per
  * thread with packed FP32x2 arithmetic.
@@ -316,7 +319,8 @@ int sky_engine_retile(void* engine, int id, int xc);
 /* Staging of an instance's planes in the marching stage kernels: tma = 1 copies
  * each haloed plane with one tensor-memory-accelerator box copy per source (Z *
  * element size a multiple of 16 bytes; not FP64 rho), 0 with per-thread cp.async
- * copies; pair (TMA, FP32 omega only) is recorded and selects nothing: every FP32
+ * copies; an instance with other rows, which the engine pads, has the library's staging,
+ * reports 0 and takes 0 only; pair (TMA, FP32 omega only) is recorded and selects nothing: every FP32
  * gradient walk computes two z-sites per thread with packed FP32x2 arithmetic.
  * Admission takes both from library options 2 and 3; a group of instances of one
  * theory and precision stages by TMA only when every member does.  The state and

@@ -306,7 +306,7 @@ int choose_chunk(int X, int tiles_yz, int resident, int per_sm) {
 
 // Library options (sky_set_option): key 0 = kernel family of the
 // reference-layout gradient and densities (1 = marching kernels, 0 = 3-D tile
-// kernels); key 1 = x-chunk of those marching launches (0 = automatic); key 2 =
+// kernels); key 1 = x-chunk of the marching gradients, the drop-in step's among them (0 = automatic); key 2 =
 // staging of the engine's stage kernels (1 = TMA box copies, 0 = cp.async); key 3 =
 // kept and reported, selects nothing: every FP32 gradient walk computes z-pairs; key 4 =
 // programmatic dependent launch of every stage kernel, in one stream.
@@ -391,7 +391,7 @@ int launch_stage_walk(const Params& p, const double* in, const StageArrays& a, d
     static int per_sm = 0;
     MarchGrid mg;
     int blocks;
-    int rc = walk_geometry<M>(kern, smem, p, kMaxRedBlocks, 0, &per_sm, &mg, &blocks);
+    int rc = walk_geometry<M>(kern, smem, p, kMaxRedBlocks, option(1), &per_sm, &mg, &blocks);
     if (rc) return rc;
     MarchCoef<double> k;
     k.init(p);
