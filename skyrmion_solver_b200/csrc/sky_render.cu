@@ -142,6 +142,10 @@ __device__ __forceinline__ float texel(const float4* v, float) { return __ldg(&v
 __device__ __forceinline__ float4 texel(const float4* v, float4) { return __ldg(v); }
 __device__ __forceinline__ float density(float v) { return v; }
 __device__ __forceinline__ float density(const float4& v) { return v.x; }
+// What makes a vector's colour a number (pion_rgb: its third component gives the lightness; a
+// direction in the other two that is none gives black).
+__device__ __forceinline__ float lightness(float) { return 0.0f; }
+__device__ __forceinline__ float lightness(const float4& v) { return fabsf(v.w); }
 __device__ __forceinline__ float mix1(float a, float b, float t) { return a + (b - a) * t; }
 __device__ __forceinline__ float4 mix1(const float4& a, const float4& b, float t) {
     return make_float4(a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.w + (b.w - a.w) * t);
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(256) k_render(const float4* __restrict__ vol, 
     const float floor_norm = PION ? rp.levelset - 2.0e-6f * (1.0f + fabsf(rp.levelset)) : 0.5f / 9.0f - 2.0e-6f;
     float gx = INFINITY, gy = 0.0f, gz = 0.0f;  // the cell whose corners are held
     Tex c[8];
-    bool empty = false;
+    bool empty = false;  // every sample of the cell adds nothing
     for (int i = 0; i < rp.max_steps;) {
         const float ux = __fadd_rn(__fmul_rn(p0, kx), cx), uy = __fadd_rn(__fmul_rn(p1, ky), cy), uz = __fadd_rn(__fmul_rn(p2, kz), cz);
         const float fx = floorf(ux), fy = floorf(uy), fz = floorf(uz);
@@ -266,15 +270,16 @@ __global__ void __launch_bounds__(256) k_render(const float4* __restrict__ vol, 
             c[2] = texel(r10 + x0, Tex{}), c[3] = texel(r10 + x1, Tex{});
             c[4] = texel(r01 + x0, Tex{}), c[5] = texel(r01 + x1, Tex{});
             c[6] = texel(r11 + x0, Tex{}), c[7] = texel(r11 + x1, Tex{});
-            float hi = density(c[0]), ab = fabsf(hi);
-            bool number = hi == hi;
+            float hi = density(c[0]), ab = fabsf(hi), light = lightness(c[0]);
 #pragma unroll
             for (int k = 1; k < 8; ++k) {
                 const float d = density(c[k]);
-                number = number && d == d;
                 hi = fmaxf(hi, d);
-                ab = fmaxf(ab, fabsf(d));
+                ab += fabsf(d);
+                light += lightness(c[k]);
             }
+            // (a sum that a NaN or an infinity enters is not below the bound)
+            const bool number = ab < 1.0e30f && light < 1.0e30f;
             const float top = (hi + 4.0e-6f * ab - rp.dmin) * inv_denom;
             const int faces = (fx <= nlx || fx >= nhx) + (fy <= nly || fy >= nhy) + (fz <= nlz || fz >= nhz);
             empty = may_skip && number && faces < 2 && top + 2.0e-6f * fabsf(top) < floor_norm;
