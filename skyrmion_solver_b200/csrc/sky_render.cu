@@ -147,8 +147,10 @@ __device__ __forceinline__ float density(const float4& v) { return v.x; }
 __device__ __forceinline__ float lightness(float) { return 0.0f; }
 __device__ __forceinline__ float lightness(const float4& v) { return fabsf(v.w); }
 __device__ __forceinline__ float mix1(float a, float b, float t) { return a + (b - a) * t; }
-__device__ __forceinline__ float4 mix1(const float4& a, const float4& b, float t) {
-    return make_float4(a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.w + (b.w - a.w) * t);
+template <class F, class C>
+__device__ __forceinline__ float trilinear(const C (&c)[8], F get, float wx, float wy, float wz) {
+    return mix1(mix1(mix1(get(c[0]), get(c[1]), wx), mix1(get(c[2]), get(c[3]), wx), wy),
+                mix1(mix1(get(c[4]), get(c[5]), wx), mix1(get(c[6]), get(c[7]), wx), wy), wz);
 }
 
 // The transfer table is read from a shared-memory copy: lanes index different entries,
@@ -190,6 +192,10 @@ __device__ __forceinline__ float3 pion_rgb(float nx, float ny, float nz) {
 // that is sure to stay in the cell.  Cells within reach of two box faces, whose edges are drawn
 // black, are always sampled.  1200 x 900 pixels of a 128^3 volume with pion colours: 10.9 ms when
 // every sample fetched its corners, 2.1 ms now.
+// With pion colours a sample interpolates the density first, and the vector and its colour only above
+// the level set: in a noisy volume few cells are empty, and there holding corners alone was slower
+// than fetching them (density noise of 30 %, 128^3, 400 x 300 pixels: 1.76 ms fetched, 2.21 held, 1.70
+// with the density first; 1200 x 900 11.0, 12.9, 9.8).
 //
 // The march's roundings are written out -- the position's step fused, the texel coordinate not,
 // the pion colouring's excess over the level set fused -- so that a position and a colour do not
@@ -247,11 +253,13 @@ __global__ void __launch_bounds__(256) k_render(const float4* __restrict__ vol, 
     const float qx = 1.0f / (st0 * kx), qy = 1.0f / (st1 * ky), qz = 1.0f / (st2 * kz);
     // density below which a sample adds nothing: the transfer table is transparent below its
     // second entry, the pion colouring below the level set
-    const bool may_skip = PION ? rp.tscale >= 0.0f && isfinite(rp.tscale) && isfinite(rp.oscale) : isfinite(rp.oscale);
+    const bool finite_scale = isfinite(rp.oscale);
+    const bool may_skip = !PION || (rp.tscale >= 0.0f && isfinite(rp.tscale));
     const float floor_norm = PION ? rp.levelset - 2.0e-6f * (1.0f + fabsf(rp.levelset)) : 0.5f / 9.0f - 2.0e-6f;
     float gx = INFINITY, gy = 0.0f, gz = 0.0f;  // the cell whose corners are held
     Tex c[8];
     bool empty = false;  // every sample of the cell adds nothing
+    bool black = false;  // a sample of the cell that does not exceed the level set adds nothing
     for (int i = 0; i < rp.max_steps;) {
         const float ux = __fadd_rn(__fmul_rn(p0, kx), cx), uy = __fadd_rn(__fmul_rn(p1, ky), cy), uz = __fadd_rn(__fmul_rn(p2, kz), cz);
         const float fx = floorf(ux), fy = floorf(uy), fz = floorf(uz);
@@ -279,10 +287,11 @@ __global__ void __launch_bounds__(256) k_render(const float4* __restrict__ vol, 
                 light += lightness(c[k]);
             }
             // (a sum that a NaN or an infinity enters is not below the bound)
-            const bool number = ab < 1.0e30f && light < 1.0e30f;
+            black = finite_scale && light < 1.0e30f;
+            const bool number = ab < 1.0e30f;
             const float top = (hi + 4.0e-6f * ab - rp.dmin) * inv_denom;
             const int faces = (fx <= nlx || fx >= nhx) + (fy <= nly || fy >= nhy) + (fz <= nlz || fz >= nhz);
-            empty = may_skip && number && faces < 2 && top + 2.0e-6f * fabsf(top) < floor_norm;
+            empty = may_skip && black && number && faces < 2 && top + 2.0e-6f * fabsf(top) < floor_norm;
         }
         if (empty) {
             // the samples up to the last one sure to be in this cell, and the step out of it
@@ -311,17 +320,23 @@ __global__ void __launch_bounds__(256) k_render(const float4* __restrict__ vol, 
             return;
         }
         const float wx = ux - fx, wy = uy - fy, wz = uz - fz;
-        const Tex sv = mix1(mix1(mix1(c[0], c[1], wx), mix1(c[2], c[3], wx), wy),
-                            mix1(mix1(c[4], c[5], wx), mix1(c[6], c[7], wx), wy), wz);
+        const float d = trilinear(c, [](const Tex& q) { return density(q); }, wx, wy, wz);
         float cr, cg, cb, ca;
         if constexpr (!PION) {
-            const float4 e = transfer(tf, fminf(fmaxf(__fmul_rn(density(sv) - rp.dmin, inv_denom), 0.0f), 1.0f));
+            const float4 e = transfer(tf, fminf(fmaxf(__fmul_rn(d - rp.dmin, inv_denom), 0.0f), 1.0f));
             cr = e.x, cg = e.y, cb = e.z, ca = e.w * rp.oscale;
         } else {
-            float inp = __fmul_rn(__fmaf_rn(density(sv) - rp.dmin, inv_denom, -rp.levelset), rp.tscale);
+            float inp = __fmul_rn(__fmaf_rn(d - rp.dmin, inv_denom, -rp.levelset), rp.tscale);
             if (inp < 0.0f) inp = 0.0f;
-            const float3 rgb = pion_rgb(sv.y, sv.z, sv.w);
-            cr = inp * rgb.x, cg = inp * rgb.y, cb = inp * rgb.z, ca = inp * rp.oscale;
+            if (inp == 0.0f && black) {
+                // below the level set: the colour would be multiplied by zero
+                cr = cg = cb = ca = 0.0f;
+            } else {
+                const float3 rgb = pion_rgb(trilinear(c, [](const Tex& q) { return q.y; }, wx, wy, wz),
+                                            trilinear(c, [](const Tex& q) { return q.z; }, wx, wy, wz),
+                                            trilinear(c, [](const Tex& q) { return q.w; }, wx, wy, wz));
+                cr = inp * rgb.x, cg = inp * rgb.y, cb = inp * rgb.z, ca = inp * rp.oscale;
+            }
         }
         cr *= ca;
         cg *= ca;
