@@ -14,11 +14,16 @@
 namespace sky {
 
 constexpr int kDiagCluster = 8;
+// Clusters whose partials (two doubles for each of n sums) fit the scratch below the result and the
+// completion counter at 2 kMaxRedBlocks.
+constexpr int diag_clusters(int n) { return 2 * kMaxRedBlocks / (2 * n); }
+constexpr bool diag_fits(int n) { return diag_clusters(n) >= 1 && 2 * n * diag_clusters(n) <= 2 * kMaxRedBlocks; }
 
 // Reduce the block's NS sums over the grid in a fixed order.  Partial c of cluster c sits at
 // scratch[2 NS c]; the results replace the partials' first NS values.
 template <int NS, int NT>
 __device__ __forceinline__ void finish_sums(const KSum (&v)[NS], double* __restrict__ scratch) {
+    static_assert(diag_fits(NS) && 2 * kMaxRedBlocks + 1 < kScratchDoubles, "partials below the counter");
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ KSum part[NS][NT / 32];

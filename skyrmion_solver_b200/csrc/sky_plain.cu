@@ -557,7 +557,7 @@ int diag_walk(K kern, const Params& p, const double* f, double* scratch, int n, 
     const size_t smem = DensPipe<M, double, 1, false>::bytes;
     MarchGrid mg;
     int blocks;
-    const int cap = kScratchDoubles / (2 * n) * kDiagCluster;
+    const int cap = diag_clusters(n) * kDiagCluster;
     int rc = walk_geometry<M>(kern, smem, p, cap, 0, per_sm, &mg, &blocks);
     if (rc) return rc;
     blocks = (blocks + kDiagCluster - 1) / kDiagCluster * kDiagCluster;
