@@ -24,18 +24,20 @@ constexpr bool is_rho() {
 // all blocks fit the SM's shared memory and the registers do not spill.  Gradient of 128^3 /
 // 64^3 sites, in us: nuclear 16 rows x 2 blocks 54 / 13, 8 x 3 62 / 13; omega 8 x 3 40 / 9,
 // 16 x 2 41 / 11; Coulomb 12 x 2 73 / 17, 8 x 2 80 / 15, 16 x 1 83 / 15 (one site per thread,
-// 8 rows x 2 blocks: 83 / 17, 60 / 14, 103 / 21).  Omega's stages as a whole run 12 x 2, and
-// rho's, whose walk over the pions spills with 16.
+// 8 rows x 2 blocks: 83 / 17, 60 / 14, 103 / 21).  Omega's stages run 8 x 3: with 12 x 2 whole steps
+// took longer and left more of a last tile empty (step in us, 12 x 2 / 16 x 2 / 8 x 3 / one site per
+// thread with 8 x 2 blocks: 48^3 63 / 67 / 62 / 60, 64^3 78 / 83 / 72 / 74, 112^3 269 / 288 / 263 / 246,
+// 128^3 315 / 331 / 311 / 322).  Rho's walk over the pions spills with 16.
 template <template <typename> class Th, typename T>
 constexpr int stage_rows() {
     if (sizeof(T) == 8) return grad_rows64<Th>(true);
     constexpr int id = Th<float>::kId;
-    return (id == SKY_THEORY_NUCLEAR || id == SKY_THEORY_LIGHTLY_BOUND) ? 16 : 12;
+    return id == SKY_THEORY_NUCLEAR || id == SKY_THEORY_LIGHTLY_BOUND ? 16 : id == SKY_THEORY_OMEGA ? 8 : 12;
 }
 // Resident blocks per SM the stages are compiled for, and their x-chunks chosen with.
 template <template <typename> class Th, typename T>
 constexpr int stage_blocks() {
-    return sizeof(T) == 4 ? 2 : 1;
+    return sizeof(T) == 8 ? 1 : stage_rows<Th, T>() == 8 ? 3 : 2;
 }
 template <template <typename> class Th, typename T>
 using MShape = MarchShape<is_rho<Th>() ? 4 : Th<T>::C, stage_rows<Th, T>(), true, sizeof(T) == 8 ? 2 : 4>;

@@ -420,10 +420,10 @@ struct GradPipe {
     static constexpr bool GH = Th<T>::kMixed;
     static constexpr int CM = 4;  // components with mixed derivatives: the pion field
     static constexpr size_t gh_bytes = GH ? size_t(CM) * (M::PLANE + M::HY * M::BZ) * sizeof(T) : 0;
-    // the late ring where the full one would leave one FP32 block on an SM (228 KB, less 1 KB and
-    // the static variables of each block)
+    // the late ring where the full one would leave one FP32 block fewer on an SM than its stages run
+    // with: two, or three of eight-row tiles (228 KB, less 1 KB and the static variables of each)
     static constexpr bool LATE = TMA && NSRC == 3 && sizeof(T) == 4 && sizeof(S) == 4 &&
-                                 size_t(8) * M::SLOT * sizeof(T) + gh_bytes > 114000;
+                                 size_t(8) * M::SLOT * sizeof(T) + gh_bytes > (M::BY == 8 ? 76000 : 114000);
     using Pipe = PlanePipe<M, T, S, NSRC, TMA, GradBlock<M, T>::NT, LATE ? 5 : 6>;
     static constexpr size_t bytes = Pipe::bytes + gh_bytes;
     // staging slots that G and H can stand in for during the prologue

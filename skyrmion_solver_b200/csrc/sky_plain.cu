@@ -284,18 +284,19 @@ int ew_blocks(int64_t n) {
 
 // x-chunk of a walk whose first planes are loaded at once (sky_grad.cuh): minimise (waves of
 // tiles) x (planes computed + about three planes' time to fill the ring).  resident: tiles that run
-// at once, per_sm of them on an SM; two that share one take 1.4 times as long as one alone.  Without
-// that factor small FP32 lattices got more and shorter tiles than pay: step in us with the chunk
-// chosen without / with it, nuclear FP32 40^3 65.3 / 59.5 (chunks of 1 / 2 planes), 48^3 71.0 / 62.7
-// (1 / 2), omega FP32 56^3 74.4 / 71.3 (2 / 4), Coulomb FP32 48^3 76.2 / 73.1 (2 / 3).
+// at once, per_sm of them on an SM.  Tiles that share an SM slow each other down: two take 1.4 times
+// as long as one alone (1.25 where there is room for three, which take 1.7; steps over chunks of 1 to
+// 48 planes of 25 lattices).  Without those factors small FP32 lattices got more and shorter tiles
+// than pay: step in us with the chunk chosen without / with it, nuclear FP32 40^3 65.3 / 59.5 (chunks
+// of 1 / 2 planes), 48^3 71.0 / 62.7 (1 / 2), Coulomb FP32 48^3 76.2 / 73.1 (2 / 3).
 int choose_chunk(int X, int tiles_yz, int resident, int per_sm) {
-    const int shared = per_sm > 1 ? 14 : 10;
+    const int f2 = per_sm > 2 ? 25 : 28, full = per_sm > 2 ? 34 : per_sm > 1 ? f2 : 20;
     int best = X;
     int64_t best_cost = -1;
     for (int xc = 1; xc <= X; ++xc) {
         const int64_t nt = (int64_t)tiles_yz * ((X + xc - 1) / xc), rest = nt % resident;
-        const int64_t waves = nt / resident * shared + (rest == 0 ? 0 : rest * per_sm <= resident ? 10 : shared);
-        const int64_t cost = waves * (xc + 3);
+        const int last = rest == 0 ? 0 : rest * per_sm <= resident ? 20 : rest * per_sm <= 2 * resident ? f2 : full;
+        const int64_t cost = (nt / resident * full + last) * (xc + 3);
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && xc > best)) {
             best_cost = cost;
             best = xc;
