@@ -3,19 +3,10 @@ the accounting of the bytes they take."""
 import numpy as np
 import pytest
 
+from tests._profile import trace, traced
 from tests.test_march import inputs, params_for
 
 pytestmark = pytest.mark.gpu
-
-
-def _runtime_calls(fn):
-    """Names of the CUDA runtime calls that fn makes."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        fn()
-        torch.cuda.synchronize()
-    return [e.name for e in prof.events()]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32d"])
@@ -27,17 +18,20 @@ def test_a_request_takes_and_frees_one_block_of_memory(precision):
     from skyrmion_solver_b200.engine import Engine
     th, p_i, p_f = params_for("nuclear", (24, 20, 28))
     F = torch.from_numpy(inputs(4, (24, 20, 28))[0]).cuda()
-    with Engine(0) as eng:
-        eng.add("nuclear", (p_i, p_f), F, None, precision=precision)
-        before = eng.bytes
-        got = []
-        calls = _runtime_calls(lambda: got.append(eng.add("nuclear", (p_i, p_f), F, None, precision=precision)))
-        assert "cudaLaunchKernel" in calls or "cudaLaunchKernelExC" in calls   # the calls are recorded
-        assert calls.count("cudaMalloc") == 1
-        taken = eng.bytes - before
-        calls = _runtime_calls(lambda: eng.remove(got[0]))
-        assert calls.count("cudaFree") == 1
-        assert eng.bytes == before and taken > 0
+
+    def run():
+        with Engine(0) as eng:
+            eng.add("nuclear", (p_i, p_f), F, None, precision=precision)
+            before = eng.bytes
+            got = []
+            calls = [e["name"] for e in trace(
+                lambda: got.append(eng.add("nuclear", (p_i, p_f), F, None, precision=precision)))]
+            assert calls.count("cudaMalloc") == 1
+            taken = eng.bytes - before
+            calls = [e["name"] for e in trace(lambda: eng.remove(got[0]))]
+            assert calls.count("cudaFree") == 1
+            assert eng.bytes == before and taken > 0
+    traced(run)
 
 
 def test_bytes_follow_a_retiled_instance():

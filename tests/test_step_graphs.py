@@ -4,6 +4,7 @@ refreshes fall on different steps."""
 import numpy as np
 import pytest
 
+from tests._profile import trace, traced
 from tests.test_march import inputs, params_for
 
 pytestmark = pytest.mark.gpu
@@ -75,22 +76,16 @@ def test_captured_steps_with_refreshes_out_of_phase():
     _same(*out)
 
 
-def _kernels(fn):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        fn()
-        torch.cuda.synchronize()
-    return [e.name for e in prof.events()]
-
-
 def test_only_steps_with_a_refresh_run_its_kernel():
     """A step without a defect refresh launches no refresh kernel (and does not order stage 1 after
     stage 4 for its sake)."""
     from skyrmion_solver_b200.engine import Engine
-    with Engine(0) as eng:
-        _engine(eng, [("omega", "fp32d", SMALL)], [None])
-        for due in (0, 1, 0, 1):     # steps 1-8, 9-16, ..
-            names = _kernels(lambda: eng.step(8))
-            assert sum("k_grad_stage" in k for k in names) >= 8
-            assert sum("k_defect" in k for k in names) == due
+
+    def run():
+        with Engine(0) as eng:
+            _engine(eng, [("omega", "fp32d", SMALL)], [None])
+            for due in (0, 1, 0, 1):     # steps 1-8, 9-16, ..
+                names = [e["name"] for e in trace(lambda: eng.step(8)) if "grid" in e.get("args", {})]
+                assert sum("k_grad_stage" in k for k in names) >= 8
+                assert sum("k_defect" in k for k in names) == due
+    traced(run)

@@ -1,33 +1,19 @@
 """Library options of the reference-layout walks: the x-chunk (key 1) reaches the drop-in step."""
-import json
-
 import numpy as np
 import pytest
 
 from oracle import skyrme_oracle as O
 from tests import _golden as G
 from tests._gpu import host
+from tests._profile import trace, traced
 from tests.test_march import _set_option, options  # noqa: F401  (fixture)
 from tests.test_walks import _simulation
 
 pytestmark = pytest.mark.gpu
 
 
-def _grids(fn, kernel, path):
-    """Blocks of the launches of `kernel` that fn makes."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        fn()
-        torch.cuda.synchronize()
-    prof.export_chrome_trace(str(path))
-    with open(path) as fh:
-        ev = json.load(fh)["traceEvents"]
-    return [int(np.prod(e["args"]["grid"])) for e in ev if kernel in e.get("name", "") and "grid" in e.get("args", {})]
-
-
 @pytest.mark.parametrize("name", ["nuclear", "omega", "coulomb"])
-def test_the_chunk_option_reaches_the_step(options, name, tmp_path):  # noqa: F811
+def test_the_chunk_option_reaches_the_step(options, name):  # noqa: F811
     """One (16-row at most, 32-column) tile column of 24 planes: a chunk of 24 gives one block per
     stage, of 4 six.  The results do not depend on it (bitwise), and match the oracle."""
     dims = (24, 12, 32)
@@ -36,11 +22,12 @@ def test_the_chunk_option_reaches_the_step(options, name, tmp_path):  # noqa: F8
         _set_option(1, xc)
         th, sim, F, V = _simulation(name, dims)
         prev = O.total_energy(O.THEORIES[name], F, sim.p_i_h, sim.p_f_h)
-        out = []
-        grids = _grids(lambda: out.append(sim.step(prev)), "k_plain_stage", tmp_path / ("t%d.json" % xc))
+        out = sim.step(prev)
+        runs[xc] = (out, host(sim.Field), host(sim.Velocity), host(sim.EnergyGradient))
         if xc:
+            grids = [int(np.prod(e["args"]["grid"])) for e in traced(lambda: trace(lambda: sim.step(prev)))
+                     if "k_plain_stage" in e["name"] and "grid" in e.get("args", {})]
             assert grids == [24 // xc] * 4
-        runs[xc] = (out[0], host(sim.Field), host(sim.Velocity), host(sim.EnergyGradient))
     for xc in (24, 4):
         assert runs[xc][0] == runs[0][0]
         assert all(np.array_equal(a, b) for a, b in zip(runs[xc][1:], runs[0][1:]))
