@@ -187,7 +187,9 @@ struct PlanePipe {
     int64_t YZ;
     int ns;       // extra sources present (TMA: V may be absent, then L takes the first staging slot)
     int e0;       // the first of them
-    using PO = typename std::conditional<M::WIDE, PlaneChunks<M, S, NT>, PlaneOffsets<M, NT>>::type;
+    static constexpr bool ROWS = !M::WIDE && M::C > 5 && DIRECT;
+    using PO = typename std::conditional<M::WIDE, PlaneChunks<M, S, NT>,
+                                         typename std::conditional<ROWS, PlaneRows<M, NT>, PlaneOffsets<M, NT>>::type>::type;
     PO po;
 
     __device__ __forceinline__ PlanePipe(T* sm, const Params& p, const S* const (&src_)[3], T a, T b, int tid_, int y0_,
@@ -240,7 +242,9 @@ struct PlanePipe {
             const S* const g[3] = {src[1], src[2], nullptr};
             S* d0 = SAME ? reinterpret_cast<S*>(ring + slot * SLOT) : stage;
             S* d1 = SAME ? stage : stage + SLOT;
-            if constexpr (M::WIDE) {
+            if constexpr (ROWS) {
+                plane_issue_rows<M, S, NT>(d0, po, src[0], base, xok);
+            } else if constexpr (M::WIDE) {
                 plane_issue_wide<M, 1, S, SLOT, NT>(d0, po, f, base, xok, tid, src[0]);
                 if constexpr (NSRC > 1) plane_issue_wide<M, NSRC - 1, S, SLOT, NT>(d1, po, g, base, xok, tid, src[0]);
             } else {
