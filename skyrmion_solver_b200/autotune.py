@@ -4,8 +4,9 @@ The stage kernels split a lattice into (x-chunk, 8- to 16-row y, 32-column z)
 tiles; the x-chunk sets how many tiles one launch has (and so how evenly they
 spread over the 148 SMs) against how many halo planes each block re-reads.  The
 planes of a tile are staged either by TMA box copies or by per-thread cp.async
-copies (the z-pair flag of an FP32 omega instance is timed too, but every FP32
-gradient walk computes z-pairs, so it changes nothing).  ``sky_engine_add`` picks the chunk with a cost model and the staging from the
+copies (the z-pair flag of an FP32 omega instance is listed too; every FP32
+gradient walk computes z-pairs, so it selects nothing and takes the times of the
+same staging without it).  ``sky_engine_add`` picks the chunk with a cost model and the staging from the
 library options; this module measures instead: for one (theory, precision,
 lattice shape, device) it admits a probe instance, times a few steps per
 candidate (staging, chunk) with CUDA events on the engine's stream
@@ -124,7 +125,10 @@ def tune(theory, p_i, p_f, precision: str = "fp32c", field=None, device: int = 0
         t = {}
         # every candidate starts from the same field: a flow that has begun to arrest runs
         # cheaper steps (stage 2 skips an arrested step), which would favour later candidates
-        for st in stagings:
+        for st in sorted(stagings, key=lambda st: st[1]):
+            if st[1]:                       # the same kernels as without the flag
+                t.update({(k[0], 1, k[2]): ms for k, ms in t.items() if k[:2] == (int(st[0]), 0)})
+                continue
             for xc in candidate_chunks(X):
                 iid = eng.add(theory, packed, field, None, precision=precision)
                 eng.set_staging(iid, *st)
