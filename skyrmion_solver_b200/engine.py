@@ -303,5 +303,5 @@ def instance_bytes(C: int, N: int, precision: str = "fp32") -> int:
     """Device bytes one instance of N stored sites (rows padded to four values) occupies (7 state / slope arrays + small
     per-tile scratch)."""
     es = 4 if precision == "fp32" else 8
-    curls = 72 * N if C > 5 and precision == "fp32" else 0   # rho's energy walks
+    curls = 72 * N if C > 5 and precision == "fp32" and N > 56 ** 3 else 0   # rho's energy walks
     return 7 * es * C * N + curls + 8192 * 48 + N // 4

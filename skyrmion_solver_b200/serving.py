@@ -73,7 +73,7 @@ def stored_sites(p_i) -> int:
 def instance_bytes(C: int, N: int, precision: str = "fp32") -> int:
     """Device bytes of one engine instance of N stored sites: 7 state / slope arrays plus per-tile partials and the stats ring."""
     es = 4 if precision == "fp32" else 8
-    curls = 72 * N if C > 5 and precision == "fp32" else 0   # rho's energy walks
+    curls = 72 * N if C > 5 and precision == "fp32" and N > 56 ** 3 else 0   # rho's energy walks
     return 7 * es * C * N + curls + 8192 * 48 + (N // 256 + 1) * 48
 
 
