@@ -17,9 +17,12 @@ namespace sky {
 
 constexpr int kStatsCap = 8192;
 constexpr int kGraphSteps = 8;  // steps captured per graph replay
-// Steps launched kernel by kernel after a change of the instance set before they are captured:
-// capturing and instantiating eight steps takes about as long as launching 64 (a millisecond),
-// and a server that admits or retires a request every chunk of 64 steps would do it every chunk.
+// Steps launched kernel by kernel after a change of the instance set before they are captured: a
+// server that admits or retires a request every chunk would capture every chunk.  A served request,
+// launched / captured, in ms: nuclear FP64 32^3, 8 steps 1.55 / 1.85, 64 steps 5.57 / 5.80; 64^3, 64
+// steps 13.7 / 13.6; defect-corrected 32^3, 64 steps 4.2 / 6.1, 64^3 9.9 / 11.4 (two patterns of
+// refreshes to capture, and to destroy with the next change).  Beyond 64 steps the replays' smaller
+// gaps between kernels pay for the capture.
 constexpr int kDirectSteps = 64;
 
 // A captured run of steps.  Bit k of `refresh`: its step k refreshes defect corrections (it may do so
@@ -490,7 +493,8 @@ static int init_instance(Engine& e, HostInst& h, int mode) {
 // each kind is issued for every non-empty group before the next kind.
 enum { kKindS2 = 0, kKindS3, kKindS4, kKindDefect, kKindEnergy, kKindS1, kNumKinds };
 
-// serial: every kind in one stream.  late: 1 the groups with a late update only, 0 the others only,
+// serial: every kind in one stream; else the first kind after the fork may follow an event's record,
+// which changes nothing for a chained launch (launch_chain).  late: 1 the groups with a late update only, 0 the others only,
 // -1 all.
 static int launch_kind(Engine& e, int kind, bool serial, cudaStream_t st, int late = -1) {
     for (int t = 0; t < kNumKernelSets; ++t)

@@ -1,6 +1,6 @@
 // Resident engine kernels: the arrested-Newton / RK4 step of
-// core/integrator.py:284-410 as fused stage launches plus a small control
-// launch, for a batch of lattice instances at once.
+// core/integrator.py:284-410 as fused stage launches, whose last block runs the control,
+// for a batch of lattice instances at once.
 //
 // With k1 = dt V, k2 = dt (V + l1/2), k3 = dt (V + l2/2), k4 = dt (V + l3) the
 // stage inputs of the reference schedule are
@@ -84,7 +84,7 @@ constexpr bool late_update(int set) {
 template <typename S>
 struct InstDesc {
     TmaMap tm[kNumMaps];  // plane maps of F[0..1], Flo[0..1], V[0..1], L[0..2], Dlt (when tma is set)
-    TmaMap tme[kNumEnergyMaps];  // energy-tile maps of F and Flo (FP32 instances of at most five components)
+    TmaMap tme[kNumEnergyMaps];  // energy-tile maps of F and Flo (FP32 instances with an energy walk; rho: the pions')
     TmaMap tmc[kNumEnergyMaps];  // FP32 rho: energy-tile maps of the rho components (as tmr)
     TmaMap tmr[kNumMaps];  // rho: maps of the rho components, 3 planes-long x axes of one isospin component each
     int tma;              // the stage kernels stage this instance's planes with TMA
@@ -221,9 +221,9 @@ __device__ __forceinline__ int l1_slot(const InstDesc<S>& in, int half) {
 }
 
 // ---------------------------------------------------------------------------
-// Control of one instance: reduces the stage-1 partials (energy and baryon number
-// of the field entering this step) and the previous step's stage-4 gradient
-// partials, records StepStats and sets the arrest flag.
+// Control of one instance: reduces the partials of the step that ends -- energy and baryon
+// number of its new field (stage 1 and the energy walk), its stage-4 gradient and kinetic sum --
+// records StepStats and sets the arrest flag.
 // ---------------------------------------------------------------------------
 // mode 0: end of a step (advances the instance, arrest decision); 1: admission (step 0, no
 // arrest); 2: resume after a precision change (keeps the pending arrest decision).

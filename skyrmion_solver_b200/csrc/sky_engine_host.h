@@ -72,7 +72,7 @@ struct TileShapeInfo {
 // [r_begin, r_end): tiles of rho's walk over the rho components.
 struct StageArgs {
     int t_begin, t_end, in_step, r_begin, r_end;
-    int chained;  // the launch follows its predecessor in the stream with no event in between
+    int chained;  // a kernel of the step precedes the launch in its stream (launch_chain)
 };
 struct TheoryOps {
     TileShapeInfo (*shape)(int prec);

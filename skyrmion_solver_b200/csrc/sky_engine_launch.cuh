@@ -103,10 +103,11 @@ static int stage_setup(int* per_sm_out) {
     return SKY_OK;
 }
 
-// Launch, programmatically dependent on its predecessor where `chained` (the kernel follows it in
-// the same stream, with no event in between) or when option 4 asks for it everywhere.  Every kernel
-// of a step waits for its predecessor before it reads anything, so the dependence is transitive; what
-// overlaps is the launch.
+// Launch, programmatically dependent on its predecessor where `chained` (a kernel of the step precedes
+// it in the same stream) or when option 4 asks for it everywhere.  Every kernel of a step waits for its
+// predecessor before it reads anything, so the dependence is transitive; what overlaps is the launch.
+// An event recorded between the two (a fork, a timing pass) only turns the programmatic dependence of
+// a launch outside a graph into a full one; in a captured step it leaves no node and no trace.
 template <class... Args, class... Given>
 static int launch_chain(bool chained, void (*kern)(Args...), int blocks, dim3 block, size_t smem, cudaStream_t st, Given... args) {
     if (chained || option(4) == 1) {

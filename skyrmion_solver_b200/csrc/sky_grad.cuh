@@ -743,8 +743,8 @@ __global__ void __launch_bounds__(M::NTHREADS)
 // field, and the next stage's field F + f_{s+1} k_s, all at the site whose gradient the walk has
 // just formed; stage 4 also writes EG and applies do_rk4_kernel (:143-177) in place.  The stage
 // fields alternate between two buffers, so every stage reads one haloed array.
-// A step then moves 30 arrays of C N values where the separate kernels moved 48, in five
-// launches (with the energy) instead of thirteen: 1.12 -> 0.72 ms for omega at 128^3.
+// A step then moves 31 arrays of C N values, the energy's read included, where the separate kernels
+// moved 49, in five launches instead of thirteen: 1.12 -> 0.70 ms for omega at 128^3.
 struct StageArrays {
     double *V, *F;
     const double *l1, *l2, *l3;  // slopes of the earlier stages
