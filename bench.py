@@ -58,7 +58,8 @@ INIT = {"mode": "rational_map", "baryon_number": 4, "scale": 2.0, "vacuum_shell"
 REL_ENERGY_TOL = 1e-6
 GRAD_TOL = 1e-6
 # passes over one C-component field per stage launch (reads + writes)
-# (stage 3 reads F, V, l1, l2 and writes F' and P; stage 4 reads F, V, l2, F', P and writes V')
+# (stage 3 reads F, V, l1, l2 and writes F' and the slopes' sum; stage 4 reads F, V, l2, F' and that sum
+# and writes V')
 STAGE_PASSES = {"stage1": 2, "stage2": 3, "stage3": 6, "stage4": 6}
 
 
@@ -120,7 +121,8 @@ def load_issue_active(stage):
 
 
 def load_traffic(stage):
-    """Per-launch DRAM bytes (read + write) of one stage kernel from the committed ncu summary, or None."""
+    """Per-launch DRAM bytes (read + write) of one stage from the committed ncu summary (stage 1 with its
+    energy walk, as it is timed; the defect kernel of every 16th step apart), or None."""
     import re
     for path in TRAFFIC:
         if os.path.exists(path):
