@@ -74,7 +74,7 @@ __device__ __forceinline__ bool rho_tile(T* __restrict__ sm, const Params& p, co
     int nslot = 0;
     int64_t s = (int64_t)xa * YZ + (int64_t)y * p.Zp + z;
     const V r1x = V(k.r1[0]), r1y = V(k.r1[1]), r1z = V(k.r1[2]);
-    const V r2x = V(k.r2[0]), r2y = V(k.r2[1]), r2z = V(k.r2[2]);
+    const V r2x = V(-k.r2[0]), r2y = V(-k.r2[1]), r2z = V(-k.r2[2]);  // (of negated tap sums)
     for (int x = xa; x < xe; ++x, s += YZ) {
         const int pslot = nslot == 0 ? R - 1 : nslot - 1;
         if (x > xa && pipe.meet(true)) {  // plane x - 1 is finished: its sums may be overwritten
@@ -108,26 +108,26 @@ __device__ __forceinline__ bool rho_tile(T* __restrict__ sm, const Params& p, co
             {
                 V m2, m1, p1, p2;
                 L::ztaps(fx, m2, m1, p1, p2);
-                rx = L::mask(r2z * tap_second(m2, m1, x0, p1, p2), pz0, pz1);
-                rx += L::mask(r2y * tap_second(L::load(fx - 2 * HZ), L::load(fx - HZ), x0, L::load(fx + HZ),
+                rx = L::mask(r2z * tap_second_neg(m2, m1, x0, p1, p2), pz0, pz1);
+                rx += L::mask(r2y * tap_second_neg(L::load(fx - 2 * HZ), L::load(fx - HZ), x0, L::load(fx + HZ),
                                                L::load(fx + 2 * HZ)), py, py);
             }
             {
                 const V m2 = L::load(ring + o0 + oy), m1 = L::load(ring + o1 + oy);
                 const V p1 = L::load(ring + o3 + oy), p2 = L::load(ring + o4 + oy);
                 L::store(Ay + yofs, tap_first(m2, m1, p1, p2));
-                ry = L::mask(r2x * tap_second(m2, m1, y0v, p1, p2), px, px);
+                ry = L::mask(r2x * tap_second_neg(m2, m1, y0v, p1, p2), px, px);
                 V a2, a1, b1, b2;
                 L::ztaps(fy, a2, a1, b1, b2);
-                ry += L::mask(r2z * tap_second(a2, a1, y0v, b1, b2), pz0, pz1);
+                ry += L::mask(r2z * tap_second_neg(a2, a1, y0v, b1, b2), pz0, pz1);
                 L::store(Wz + zofs, wz(dxx, uy(oy)));
             }
             {
                 const V m2 = L::load(ring + o0 + oz), m1 = L::load(ring + o1 + oz);
                 const V p1 = L::load(ring + o3 + oz), p2 = L::load(ring + o4 + oz);
                 L::store(Az + zofs, tap_first(m2, m1, p1, p2));
-                rz = L::mask(r2x * tap_second(m2, m1, z0v, p1, p2), px, px);
-                rz += L::mask(r2y * tap_second(L::load(fz - 2 * HZ), L::load(fz - HZ), z0v, L::load(fz + HZ),
+                rz = L::mask(r2x * tap_second_neg(m2, m1, z0v, p1, p2), px, px);
+                rz += L::mask(r2y * tap_second_neg(L::load(fz - 2 * HZ), L::load(fz - HZ), z0v, L::load(fz + HZ),
                                                L::load(fz + 2 * HZ)), py, py);
                 L::store(Wy + yofs, wy(dxx, uz(oz)));
             }
