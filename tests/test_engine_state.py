@@ -121,3 +121,32 @@ def test_velocity_is_rounded_once(name, precision, dims):
         eng.step(1)
         _, v = eng.read(i)
     assert float(np.max(np.abs(v - Vo))) <= 2.0 ** -25 + (2e-5 + 2.0 ** -22) * inc
+
+
+@pytest.mark.parametrize("name,precision", [("nuclear", "fp32d"), ("omega", "fp32"), ("coulomb", "fp64"), ("rho", "fp32d"),
+                                            ("rho", "fp64")])
+@pytest.mark.parametrize("z", [33, 38])
+def test_padded_rows_in_both_stagings(name, precision, z):
+    """Rows that are no whole chunks in the caller's arrays: TMA boxes and cp.async chunks of the padded
+    ones give bitwise the same records and state (a box ends at the last site, a chunk is cut there)."""
+    from skyrmion_solver_b200 import _lib
+    from skyrmion_solver_b200.engine import Engine
+    dims = (11, 19, z)
+    _, p_i, p_f = params_for(name, dims)
+    F, V = inputs(int(p_i[5]), dims, seed=12)
+    old = int(_lib.load().sky_get_option(2))
+    out = []
+    try:
+        for tma in (1, 0):
+            _lib.call("sky_set_option", 2, tma)
+            with Engine(0) as eng:
+                i = eng.add(name, (p_i, p_f), F, V, precision=precision)
+                if precision == "fp32d":
+                    eng.set_defect_period(i, 3)
+                eng.step(7)
+                s = eng.stats(i)
+                out.append(((s.energy, s.baryon, s.err, s.gabs, s.kinetic),) + eng.read(i))
+    finally:
+        _lib.call("sky_set_option", 2, old)
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
